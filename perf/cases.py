@@ -288,7 +288,7 @@ def _predictor():
     """The band predictor a program trains once and keeps."""
     if "predictor" not in _kept:
         predictor = learned.Predictor()
-        predictor.train(pairs=100_000, epochs=4, batch=1024, seed=2024)
+        predictor.train(pairs=400_000, epochs=4, batch=1024, seed=2024)
         _kept["predictor"] = predictor.parameters() + (predictor.margins(),)
     return _kept["predictor"]
 
