@@ -23,6 +23,7 @@
 #include "affine.cuh"
 #include "affine_kernel.cuh"
 #include "banded.cuh"
+#include "long_kernel.cuh"
 #include "pack.cuh"
 
 namespace dinara {
@@ -531,7 +532,7 @@ struct PhaseTimer {
 // then whole). Otherwise the band's score, a real alignment's, says how wide a band would prove a score
 // that good: g gap letters outside it must cost more than the score, g > (4 (open - extend) + best (rows +
 // columns) - 2 score) / (best - 2 extend). The pair goes round again at that width (at least twice the
-// last, rounded up to 1,024 diagonals) unless this is the `last` round or that band's strips of
+// last, rounded up to 256 diagonals) unless this is the `last` round or that band's strips of
 // `strip_columns` would sweep three fifths of its rows or more: then to the whole-matrix list. With `swept`
 // null, every pair is routed to `first_width`. With `proven`, a pair whose band proves its score leaves the
 // width there (by pair - proven_first).
@@ -565,7 +566,7 @@ __global__ void wide_route_kernel(const PairShape *__restrict__ shapes, const ui
         const int64_t g = (4 * (int64_t(open) - extend) + int64_t(best) * (rows + columns) - 2 * score) / per_letter + 2;
         const int64_t delta = columns > rows ? columns - rows : rows - columns;
         width = max(2 * done, g + delta + 2);
-        width = (width + 1023) / 1024 * 1024;
+        width = (width + 255) / 256 * 256;
     }
     const bool banded = !last && width < (int64_t(1) << 30) && band_low_for_width(rows, columns, width) != INT32_MIN &&
                         10 * (strip_columns + width) < 6 * rows;
@@ -576,6 +577,62 @@ __global__ void wide_route_kernel(const PairShape *__restrict__ shapes, const ui
     } else {
         whole[atomicAdd(whole_count, 1u)] = pair;
     }
+}
+
+// Whether the 16-bit strips of affine_long_kernel hold a table's cells: entries that fit a byte, and a step
+// (the largest shifted entry plus a gap's opening, in size) of at most kLongStep.
+bool long_serves(const AffineBatch &batch, const AffineTable &table) {
+    if (batch.local || batch.bits != 2 || !table.packed16) return false;
+    int32_t entry = 0;
+    for (int r = 0; r < table.size; ++r)
+        for (int c = 0; c < table.size; ++c) {
+            const int32_t v = table.entries[r * 32 + c] - 2 * table.extend;
+            if (v < -128 || v > 127) return false;
+            entry = std::max(entry, std::abs(v));
+        }
+    return int64_t(entry) + std::abs(int64_t(table.open) - table.extend) <= kLongStep;
+}
+
+// One launch of the block-a-pair sweep over `count` pairs of `order`, each over its whole matrix or its
+// band of `widths` (by item): the 16-bit strips where they hold the table's cells, else 32 bits.
+void sweep_long(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, KernelArgs args,
+                const uint32_t *order, int64_t count, const int32_t *widths) {
+    const TableArgs targs = table_args(table, false);
+    args.carry_stride = int64_t(batch.max_rows) + 1;
+    ClockSpan clock(gpu, kClassWhole, gpu->stream);
+    if (long_serves(batch, table)) {
+        // Four warps a block when the batch fills the GPU with them, eight for a batch too small to.
+        const int warps = count >= 4 * int64_t(gpu->multiprocessors) ? kLongWarps / 2 : kLongWarps;
+        int per_sm = 0;
+        DINARA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, affine_long_kernel, 32 * warps, 0));
+        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(int64_t(per_sm) * gpu->multiprocessors, count));
+        LongArgs a;
+        std::memset(&a, 0, sizeof a);
+        a.tape = args.tape;
+        a.shapes = args.shapes;
+        a.order = order;
+        a.band_widths = widths;
+        a.count = uint32_t(count);
+        a.open = args.open;
+        a.extend = args.extend;
+        for (int r = 0; r < 4; ++r) a.rows8[r] = targs.rows8[r];
+        a.scores = args.scores;
+        a.carry_stride = args.carry_stride;
+        a.carry = gpu->carry.ensure<int2>(size_t(blocks * args.carry_stride));
+        affine_long_kernel<<<unsigned(blocks), 32 * warps, 0, gpu->stream>>>(a);
+    } else {
+        KernelFn fn = widths ? &affine_wide_kernel<false, true> : &affine_wide_kernel<false, false>;
+        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(persistent_blocks(gpu, fn), count));
+        args.carry = gpu->carry.ensure<int2>(size_t(blocks * args.carry_stride));
+        args.order = order;
+        args.band_widths = widths;
+        args.begin = 0;
+        args.end = uint32_t(count);
+        fn<<<unsigned(blocks), kBlock, 0, gpu->stream>>>(args, targs, nullptr);
+    }
+    DINARA_CUDA(cudaGetLastError());
+    clock.stop();
+    gpu->launches += 1;
 }
 
 // Scores of long global pairs (the block-a-pair class) by a widening band: a first round sweeps each pair
@@ -589,16 +646,16 @@ __global__ void wide_route_kernel(const PairShape *__restrict__ shapes, const ui
 void widening_band(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, const uint32_t *order,
                    int64_t count, KernelArgs args, int32_t *proven = nullptr, int64_t proven_first = 0) {
     if (count <= 0) return;
-    const TableArgs targs = table_args(table, false);
     int32_t best = -128;
     for (int r = 0; r < table.size; ++r)
         for (int c = 0; c < table.size; ++c) best = std::max(best, table.entries[r * 32 + c]);
+    const int32_t strip_columns = proven ? kRecordStrip : long_serves(batch, table) ? kLongStrip : 16 * kBlock;
+    const int32_t first_width = long_serves(batch, table) ? 256 : 2048;
     uint32_t *lists = gpu->wide_pending.ensure<uint32_t>(5 * size_t(count));
     uint32_t *whole = lists + 2 * count;
     int32_t *widths = reinterpret_cast<int32_t *>(lists + 3 * count);
     unsigned int *counts = gpu->class_counts.ensure<unsigned int>(20) + 9;  // [0] next, [1] whole
     DINARA_CUDA(cudaMemsetAsync(counts + 1, 0, sizeof(unsigned int), gpu->stream));
-    constexpr int32_t kFirstWidth = 2048;
     constexpr int kBandRounds = 2;
     const uint32_t *pending = order;
     const int32_t *swept = nullptr;
@@ -608,48 +665,22 @@ void widening_band(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
         int32_t *next_widths = widths + (round & 1) * count;
         DINARA_CUDA(cudaMemsetAsync(counts, 0, sizeof(unsigned int), gpu->stream));
         wide_route_kernel<<<unsigned((left + 255) / 256), 256, 0, gpu->stream>>>(
-            batch.shapes, pending, swept, left, kFirstWidth, round == kBandRounds, args.scores, best, table.open,
+            batch.shapes, pending, swept, left, first_width, round == kBandRounds, args.scores, best, table.open,
             table.extend, next, next_widths, counts, whole, counts + 1, proven, proven_first,
-            proven ? kRecordStrip : 16 * kBlock);
+            strip_columns);
         DINARA_CUDA(cudaGetLastError());
         gpu->launches += 1;
         unsigned int routed = 0;
         read_back(gpu, &routed, counts, sizeof routed);
         left = routed;
         if (left == 0) break;
-        int64_t blocks = persistent_blocks(gpu, &affine_wide_kernel<false, true>);
-        blocks = std::max<int64_t>(1, std::min(blocks, left));
-        args.carry_stride = int64_t(batch.max_rows) + 1;
-        args.carry = gpu->carry.ensure<int2>(size_t(blocks * args.carry_stride));
-        args.order = next;
-        args.band_widths = next_widths;
-        args.begin = 0;
-        args.end = uint32_t(left);
-        ClockSpan clock(gpu, kClassWhole, gpu->stream);
-        affine_wide_kernel<false, true><<<unsigned(blocks), kBlock, 0, gpu->stream>>>(args, targs, nullptr);
-        DINARA_CUDA(cudaGetLastError());
-        clock.stop();
-        gpu->launches += 1;
+        sweep_long(gpu, batch, table, args, next, left, next_widths);
         pending = next;
         swept = next_widths;
     }
     unsigned int swept_whole = 0;
     if (!proven) read_back(gpu, &swept_whole, counts + 1, sizeof swept_whole);
-    if (swept_whole > 0) {
-        int64_t blocks = persistent_blocks(gpu, &affine_wide_kernel<false, false>);
-        blocks = std::max<int64_t>(1, std::min<int64_t>(blocks, swept_whole));
-        args.carry_stride = int64_t(batch.max_rows) + 1;
-        args.carry = gpu->carry.ensure<int2>(size_t(blocks * args.carry_stride));
-        args.order = whole;
-        args.band_widths = nullptr;
-        args.begin = 0;
-        args.end = swept_whole;
-        ClockSpan clock(gpu, kClassWhole, gpu->stream);
-        affine_wide_kernel<false, false><<<unsigned(blocks), kBlock, 0, gpu->stream>>>(args, targs, nullptr);
-        DINARA_CUDA(cudaGetLastError());
-        clock.stop();
-        gpu->launches += 1;
-    }
+    if (swept_whole > 0) sweep_long(gpu, batch, table, args, whole, swept_whole, nullptr);
 }
 
 void affine_launch_all(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, const Schedule &schedule,
@@ -727,6 +758,7 @@ PairLimits whole_limits_of(const AffineBatch &batch, const AffineTable &table) {
     PairLimits limits;
     if (batch.bits != 2 || !table.packed16) return limits;
     limits.wide = 1;
+    limits.long_strips = long_serves(batch, table) ? 1 : 0;
     const int32_t gaps = std::abs(table.open) + std::abs(table.extend);
     if (gaps > 8000) return limits;
     if (batch.local) {

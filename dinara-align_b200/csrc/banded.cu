@@ -73,14 +73,15 @@ __global__ void __launch_bounds__(kBlock) banded_kernel(BandedBatch b) {
 
     for (int64_t base = int64_t(warp) * GPW; base < b.count; base += int64_t(warps) * GPW) {
         const int64_t item = base + group;
-        const bool live = item < b.count;
+        bool live = item < b.count;
         uint32_t pair = 0;
         PairShape sh{0, 0, 0, 0};
         if (live) {
             pair = b.order[item];
             sh = b.shapes[pair];
         }
-        const int rows = int(sh.rows), cols = int(sh.columns);
+        int rows = int(sh.rows);
+        const int cols = int(sh.columns);
         const int low = live ? band_low_for(rows, cols) : 0;
         const int first_place = member * C;  // this lane's first place in the band
         int warp_rows = live ? rows : 0;
@@ -105,6 +106,29 @@ __global__ void __launch_bounds__(kBlock) banded_kernel(BandedBatch b) {
         for (int r0 = 1; r0 <= warp_rows; r0 += 16) {
             // Selectors of the 32 letters from column r0 + low + first_place on (letter index one less);
             // columns outside the pair read letter 0, which no real cell's value depends on.
+            // Every 64 rows a pair whose band can no longer prove its score is left to the whole-matrix sweep: from
+            // here its score gains at most the best shifted entry a row. At 5% errors a pair of 50,000 letters
+            // leaves after some 500 rows, where its band took 9 ms to its end; a pair that the band proves goes on
+            // as before.
+            if (r0 > 1 && (r0 & 63) == 1) {
+                int32_t most = H[0];
+#pragma unroll
+                for (int k = 1; k < C; ++k) most = max(most, H[k]);
+#pragma unroll
+                for (int span = 1; span < G; span <<= 1) most = max(most, __shfl_xor_sync(kFull, most, span, G));
+                const int64_t reach = int64_t(most) + int64_t(max(b.best - 2 * extend, 0)) * (rows - r0 + 1) +
+                                      int64_t(rows + cols) * extend;
+                if (live && r0 <= rows && !band_proves(reach, rows, cols, low, b.best, open, extend)) {
+                    if (member == 0) {
+                        if (b.proven) b.proven[pair] = 0;
+                        b.leftovers[atomicAdd(b.leftover_count, 1u)] = pair;
+                    }
+                    live = false;
+                    rows = 0;
+                }
+                warp_rows = warp_max(live ? rows : 0);
+                if (warp_rows < r0) break;
+            }
             uint32_t codes[2];
             run_of_letters(b.tape, sh.second_word, live ? cols : 0, r0 + low + first_place - 1, codes);
             uint32_t window[32];

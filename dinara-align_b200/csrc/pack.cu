@@ -107,7 +107,12 @@ __device__ void classify_pair(const PairShape *__restrict__ shapes, const uint32
         const bool pairs16 = cls != kWideClass && !record && !empty && limits.whole > 0 &&
                              (limits.local ? swept * limits.best + int64_t(shape.rows) * limits.row_step <= limits.whole
                                            : 2 * swept <= limits.whole && 2 * int64_t(shape.rows) <= limits.whole);
-        if (pairs16) cls += kWholePairsClass;
+        if (pairs16) {
+            cls += kWholePairsClass;
+        } else if (!record && limits.long_strips && shape.rows >= kLongSide && shape.columns >= kLongSide) {
+            cls = kWideClass;
+            strips = (shape.columns + 4095) / 4096;
+        }
         if (strips > 255) strips = 255;
     }
     uint32_t rows = shape.rows >> 2;

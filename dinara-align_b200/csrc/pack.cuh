@@ -29,6 +29,9 @@ constexpr int kWideClass = 12;
 constexpr int kBandRecordClass = 13;
 // A pair a whole block sweeps (kWideClass), scoring without a CIGAR: at least this tall and this wide.
 constexpr uint32_t kWideRows = 4096, kWideColumns = 2048;
+// With the 16-bit strips: a pair of two strips or more, each way. (600 pairs of 3,000 letters: 8.6 ms in 32 bits,
+// a warp a pair, 5.2 in strips; 4,000 of them 25.3 and 16.7.)
+constexpr uint32_t kLongSide = 1024 + 1;
 struct Schedule {
     const uint32_t *order;
     int64_t counts[kClasses];
@@ -43,6 +46,9 @@ struct PairLimits {
     int32_t whole = 0;
     int32_t local = 0;
     int32_t wide = 0;
+    // Scoring without a CIGAR, globally: the 16-bit strips of a long pair serve the batch's table. Then pairs of
+    // at least kLongSide x kLongSide that no 16-bit pair sweep takes go to kWideClass too.
+    int32_t long_strips = 0;
     // Local: a pair fits when best x swept columns + rows x row_step is at most `whole`.
     int32_t best = 1;
     int32_t row_step = 0;

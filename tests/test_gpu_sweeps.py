@@ -1,0 +1,66 @@
+"""The sweeps' own edges against the oracle: strips and lane groups at their widths and a column either side, the
+16-bit forms at their limits and a step past them, hits cut to their rows, kept fronts at their sizes, the
+first round's list, and the gradients' slices. Every result is an exact integer or text, except the gradients."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+BIG = 1 << 40
+PROTEIN = "ACDEFGHIKLMNPQRSTVWY"
+THIRTY_TWO = "ABCDEFGHIJKLMNOPQRSTUVWXYZ012345"
+
+
+def _mutated(rng, source, rate, alphabet):
+    out = []
+    for letter in source:
+        roll = rng.random()
+        if roll < rate / 2:
+            out.append(rng.choice(list(alphabet)))
+        elif roll < 3 * rate / 4:
+            continue
+        elif roll < rate:
+            out.append(letter + rng.choice(list(alphabet)))
+        else:
+            out.append(letter)
+    return "".join(out)
+
+
+def _text(rng, length, alphabet="ACGT"):
+    return "".join(np.asarray(list(alphabet))[rng.integers(0, len(alphabet), size=length)])
+
+
+def _table(scoring):
+    return np.asarray(scoring.table, dtype=np.int8)
+
+
+def _tabulated(da, rng, alphabet, opening=-10, extension=-1):
+    size = len(alphabet)
+    table = rng.integers(-4, 3, size=(size, size))
+    table = np.triu(table, 1) + np.triu(table, 1).T + np.diag(rng.integers(3, 9, size))
+    return da.Scoring.tabulated(alphabet, [int(v) for v in table.reshape(-1)], opening, extension)
+
+
+# ---- long pairs in strips of 1,024 columns ------------------------------------------------------------
+
+# The last three: steps (largest shifted entry plus opening) of 100, the strips' limit, and 101 and 180, past it.
+@pytest.mark.parametrize("entries", [(0, -4, -6, -2), (2, -4, -4, -2), (1, -1, 0, -1), (40, -20, -40, -10),
+                                     (41, -20, -40, -10), (60, -60, -100, -10)])
+def test_long_pairs_in_strips(da, oracle, entries):
+    """Pairs past 16-bit pair sweeps: one strip and a letter, whole strips and a letter either side, more than
+    eight strips (a warp's second), bands proven, bands widened and bands given up for the whole matrix."""
+    rng = np.random.default_rng(abs(sum(entries)) + 5)
+    scoring = da.Scoring.uniform(*entries)
+    refs, queries = [], []
+    for rows, columns, rate in ((1025, 1025, 0.05), (2600, 2048, 0.4), (2049, 2600, 0.3), (3071, 3072, 0.02),
+                                (4100, 4097, 0.1), (5000, 5000, 0.003), (5000, 1025, 0.0), (1025, 5000, 0.0),
+                                (9300, 9300, 0.01), (9300, 9217, 0.25)):
+        source = _text(rng, max(rows, columns))
+        refs.append(source[:rows])
+        queries.append(_mutated(rng, source, rate, "ACGT")[:columns] if rate else _text(rng, columns))
+    tape = da.Tape.of(refs, queries)
+    coded = np.concatenate([oracle.codes(text) for pair in zip(refs, queries) for text in pair])
+    op, ex = oracle.kernel_gaps(scoring.opening, scoring.extension)
+    expected = oracle.batch_scores(coded, tape.offsets, _table(scoring), 4, op, ex, oracle.GLOBAL, threads=8)
+    np.testing.assert_array_equal(da.scores_tape(tape, scoring), expected)
