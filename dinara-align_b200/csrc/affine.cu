@@ -39,6 +39,7 @@ using namespace sweep;
 struct WalkArgs {
     const uint32_t *tape;
     const PairShape *shapes;
+    const PairShape *whole_shapes;  // the pairs as given, when `shapes` are their hits' rows (else the same)
     const uint64_t *decisions;
     const uint64_t *decisions_extra;  // the band's leftovers, swept whole afterwards
     // Per pair: 0 whole matrix, 1 band, 2 whole matrix in decisions_extra, 3 and 4 the 16-bit pair band's
@@ -82,6 +83,7 @@ __global__ void walk_kernel(WalkArgs a) {
     const int64_t pair = a.first_pair + k;
     const PairShape sh = a.shapes[pair];
     const int rows = int(sh.rows), cols = int(sh.columns);
+    constexpr int per_tape_word = 32 / BITS;
     uint32_t *runs = reinterpret_cast<uint32_t *>(a.slots + a.slot_offsets[k]);
     int64_t run_count = 0, text = 0;
     int row, column;
@@ -240,10 +242,74 @@ __global__ void walk_kernel(WalkArgs a) {
     a.lengths[k] = text;
     a.run_counts[k] = run_count;
     int64_t *span = a.spans + 4 * k;
-    span[0] = row;
-    span[1] = end_row;
+    // A hit's rows start at a packed word of their reference.
+    const int64_t rows_before = int64_t(sh.first_word - a.whole_shapes[pair].first_word) * per_tape_word;
+    span[0] = end_row > 0 ? rows_before + row : 0;
+    span[1] = end_row > 0 ? rows_before + end_row : 0;
     span[2] = column;
     span[3] = end_col;
+}
+
+// Four letters from `at` on, which need not be aligned (device letter buffers keep 16 bytes of room past the last
+// letter): the word under its first letter and the one after.
+__device__ __forceinline__ uint32_t four_letters(const uint8_t *at) {
+    const uintptr_t address = reinterpret_cast<uintptr_t>(at);
+    const uint32_t *aligned = reinterpret_cast<const uint32_t *>(address & ~uintptr_t(3));
+    return __funnelshift_r(__ldg(aligned), __ldg(aligned + 1), uint32_t(address & 3u) * 8u);
+}
+
+// as_alignment's placement (scoring.mojo:724-744): a local alignment's letters placed at the last place they
+// occur in their sequence (at 0 when there are none). A warp a side: 32 places at a time from the last one
+// down, each lane holding its place's first eight letters against the alignment's, and the warp the rest of
+// the letters of a place that agrees. (One host thread took 19 ms for 5,000 reads in targets of 3,000.)
+__global__ void last_places_kernel(const uint8_t *__restrict__ letters, const int64_t *__restrict__ offsets,
+                                   int64_t first_pair, int64_t count, int64_t *__restrict__ spans) {
+    const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (warp >= 2 * count) return;
+    const int64_t k = 2 * first_pair + warp;
+    int64_t *span = spans + 2 * warp;
+    const int64_t start = span[0], letters_in = span[1] - span[0];
+    const uint8_t *text = letters + offsets[k];
+    const int64_t length = offsets[k + 1] - offsets[k];
+    int64_t place = letters_in > 0 ? start : 0;
+    if (letters_in > 0) {
+        // The first eight letters, or all of fewer, of each place by a mask.
+        auto mask = [&](int64_t n) { return n >= 4 ? ~0u : n <= 0 ? 0u : (1u << (8 * n)) - 1u; };
+        const uint32_t mask0 = mask(letters_in), mask1 = mask(letters_in - 4);
+        const uint32_t key0 = four_letters(text + start) & mask0;
+        const uint32_t key1 = letters_in > 4 ? four_letters(text + start + 4) & mask1 : 0u;
+        bool found = false;
+        for (int64_t top = length - letters_in; top > start && !found; top -= 32) {
+            const int64_t at = top - lane;
+            bool alike = false;
+            if (at > start) {
+                alike = (four_letters(text + at) & mask0) == key0;
+                if (alike && letters_in > 4) alike = (four_letters(text + at + 4) & mask1) == key1;
+            }
+            unsigned candidates = __ballot_sync(kFull, alike);
+            while (candidates && !found) {
+                const int64_t candidate = top - (__ffs(candidates) - 1);
+                candidates &= candidates - 1;
+                bool differs = false;
+                for (int64_t i = 8 + 4 * lane; i < letters_in; i += 128) {
+                    const uint32_t keep = mask(letters_in - i);
+                    if ((four_letters(text + candidate + i) ^ four_letters(text + start + i)) & keep) {
+                        differs = true;
+                        break;
+                    }
+                }
+                if (!__any_sync(kFull, differs)) {
+                    place = candidate;
+                    found = true;
+                }
+            }
+        }
+    }
+    if (lane == 0) {
+        span[0] = place;
+        span[1] = place + letters_in;
+    }
 }
 
 // Each pair's CIGAR text from its runs, which the walk left back to front: a warp a pair, 32 runs at a time
@@ -430,6 +496,17 @@ KernelFn pick_pairs_kernel(int cls, bool local) {
         case 2: return local ? &affine_pairs_kernel<16, 16, true> : &affine_pairs_kernel<16, 16, false>;
         case 3: return local ? &affine_pairs_kernel<16, 20, true> : &affine_pairs_kernel<16, 20, false>;
         default: return local ? &affine_pairs_kernel<32, 16, true> : &affine_pairs_kernel<32, 16, false>;
+    }
+}
+
+// The same keeping each hit's rows (local).
+KernelFn pick_hits_kernel(int cls) {
+    switch (cls) {
+        case 0: return &affine_pairs_kernel<4, 16, true, true>;
+        case 1: return &affine_pairs_kernel<8, 16, true, true>;
+        case 2: return &affine_pairs_kernel<16, 16, true, true>;
+        case 3: return &affine_pairs_kernel<16, 20, true, true>;
+        default: return &affine_pairs_kernel<32, 16, true, true>;
     }
 }
 
@@ -1140,6 +1217,62 @@ void free_end_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTabl
     timer.stop();
 }
 
+// Each local pair's shape cut to the rows its best alignment can span (by pair), from a score sweep of the pairs
+// the 16-bit pair sweeps take; the rest keep their whole shape. Recording a cell costs about seven times
+// scoring it in 16-bit pairs (its flags, their packing and the decisions' store, in 32 bits), so the cut
+// pays for its sweep once it leaves out a seventh of a pair's rows: a read of 575 letters in a target of
+// 3,000 leaves out three quarters. Null when no pair takes a 16-bit sweep.
+const PairShape *hit_shapes(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, int32_t *scores,
+                            int64_t first, int64_t count) {
+    const PairLimits limits = whole_limits_of(batch, table);
+    if (limits.whole <= 0) return nullptr;
+    const Schedule order = dinara::schedule(gpu, batch.shapes, nullptr, first, count, false, false, limits);
+    int64_t taken = 0;
+    for (int cls = 0; cls < kAffineShapes; ++cls) taken += order.counts[kWholePairsClass + cls];
+    if (taken == 0) return nullptr;
+    PairShape *hits = gpu->hits.ensure<PairShape>(size_t(batch.pairs));
+    if (taken < count)
+        DINARA_CUDA(cudaMemcpyAsync(hits + first, batch.shapes + first, size_t(count) * sizeof(PairShape),
+                                    cudaMemcpyDeviceToDevice, gpu->stream));
+    const TableArgs targs = table_args(table, true);
+    KernelArgs args;
+    std::memset(&args, 0, sizeof args);
+    args.tape = batch.tape;
+    args.shapes = batch.shapes;
+    args.order = order.order;
+    args.open = table.open;
+    args.extend = table.extend;
+    args.scores = scores;
+    args.hits = hits;
+    args.best_entry = limits.best;
+    const Buckets b = buckets_of(order);
+    PhaseTimer timer(gpu, &gpu->record_ms);
+    for (int cls = kAffineShapes - 1; cls >= 0; --cls) {
+        const int bucket = kWholePairsClass + cls;
+        const int64_t pairs = b.end[bucket] - b.begin[bucket];
+        if (pairs <= 0) continue;
+        KernelFn fn = pick_hits_kernel(cls);
+        const int groups_per_block = kBlock / affine_lanes(cls);
+        const int64_t needed = (pairs + 2 * groups_per_block - 1) / (2 * groups_per_block);
+        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(persistent_blocks(gpu, fn), needed));
+        args.carry = nullptr;
+        args.carry_stride = 0;
+        if (batch.max_columns > uint32_t(affine_lanes(cls) * affine_columns(cls))) {
+            args.carry_stride = int64_t(batch.max_rows) + 1;
+            args.carry = gpu->carry.ensure<int2>(size_t(blocks * groups_per_block * args.carry_stride));
+        }
+        args.begin = uint32_t(b.begin[bucket]);
+        args.end = uint32_t(b.end[bucket]);
+        ClockSpan clock(gpu, kClassWhole, gpu->stream);
+        fn<<<unsigned(blocks), kBlock, 0, gpu->stream>>>(args, targs, nullptr);
+        DINARA_CUDA(cudaGetLastError());
+        clock.stop();
+        gpu->launches += 1;
+    }
+    timer.stop();
+    return hits;
+}
+
 // Long global pairs of an alignment batch: their scores by the widening band, and each pair's proven width
 // (by pair - first_pair; 0 for a pair its band left to the whole matrix), so that its recording sweeps its
 // band's rows alone. Null when the range holds no long pair.
@@ -1222,8 +1355,14 @@ void affine_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
     tally_swept(gpu, batch.shapes, first, count, band, leftovers, left);
 }
 
-int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, bool eqx,
+int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &whole_batch, const AffineTable &table, bool eqx,
                           int32_t *scores, int64_t *spans, int64_t first_pair, int64_t count) {
+    // A local batch records each pair's hit's rows alone: its pairs, from here on, are those rows.
+    AffineBatch batch = whole_batch;
+    if (batch.local) {
+        const PairShape *hits = hit_shapes(gpu, batch, table, scores, first_pair, count);
+        if (hits) batch.shapes = hits;
+    }
     const bool band = band_serves(batch, table);
     const bool uniform = !table.packed16 || batch.bits == 8;
     // Per pair: its decisions' words, its layout and its CIGAR slot, then the offsets by exclusive scans.
@@ -1331,6 +1470,7 @@ int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &batch, const Affin
     std::memset(&w, 0, sizeof w);
     w.tape = batch.tape;
     w.shapes = batch.shapes;
+    w.whole_shapes = whole_batch.shapes;
     w.decisions = decisions;
     w.decisions_extra = extra ? extra : decisions;
     w.layouts = layouts;
@@ -1380,6 +1520,15 @@ int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &batch, const Affin
     DINARA_CUDA(cudaGetLastError());
     gpu->launches += 1;
     return total;
+}
+
+void last_places(dinara_gpu *gpu, const uint8_t *letters, const int64_t *offsets, int64_t first_pair, int64_t count,
+                 int64_t *spans) {
+    if (count <= 0) return;
+    last_places_kernel<<<unsigned((2 * count * 32 + 255) / 256), 256, 0, gpu->stream>>>(letters, offsets, first_pair,
+                                                                                      count, spans);
+    DINARA_CUDA(cudaGetLastError());
+    gpu->launches += 1;
 }
 
 }  // namespace dinara

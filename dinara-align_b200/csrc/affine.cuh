@@ -82,4 +82,10 @@ void affine_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
 int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, bool eqx,
                           int32_t *scores, int64_t *spans, int64_t first_pair, int64_t count);
 
+// Moves the spans (4 a pair of the range, as affine_alignments leaves them) of a local batch's alignments to where
+// the reference places them: the last place their letters occur in each sequence. `letters` and `offsets` are
+// the batch's ASCII tape on the device.
+void last_places(dinara_gpu *gpu, const uint8_t *letters, const int64_t *offsets, int64_t first_pair, int64_t count,
+                 int64_t *spans);
+
 }  // namespace dinara

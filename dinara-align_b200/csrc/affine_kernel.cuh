@@ -71,7 +71,24 @@ struct KernelArgs {
     // diagonals[diagonal_offsets[pair - first_pair] + row + column].
     unsigned long long *diagonals;
     const int64_t *diagonal_offsets;
+    // Local hits' rows (affine_pairs_kernel<..., TRACK>): each pair's shape cut to the rows its best alignment
+    // can span (hit_rows), by pair, for a recording sweep of those rows alone; `best_entry` the table's.
+    PairShape *hits;
+    int32_t best_entry;
 };
+
+// The rows, ending with `end_row`, that a local alignment of `score` ending there can span, its first one at
+// a packed word's first letter (0-based). Its pairs are at most the columns, each worth at most `best_entry`,
+// so its score leaves room for at most (best_entry * columns + open - score) / -extend + 1 deletions; with no
+// cost a letter (extend 0) it may span every row.
+__host__ __device__ inline int hit_first_row(int end_row, int columns, int32_t score, int32_t best_entry, int32_t open,
+                                             int32_t extend) {
+    if (extend >= 0) return 0;
+    const int64_t room = int64_t(best_entry) * columns + open - score;
+    const int64_t deletions = room < 0 ? 0 : room / -int64_t(extend) + 1;
+    const int64_t first = int64_t(end_row) - columns - deletions;
+    return first > 0 ? int(first) & ~15 : 0;
+}
 
 // The lowest diagonal (column less row) of a band of `width` diagonals holding a pair's main and end
 // diagonals, the slack shared either side; INT32_MIN when the band cannot hold both.
@@ -569,8 +586,14 @@ __device__ __forceinline__ uint32_t pair_selector(uint32_t a, uint32_t b) { retu
 __device__ __forceinline__ uint32_t half_selector_a(uint32_t y) { return 17u * y + 128u; }
 __device__ __forceinline__ uint32_t half_selector_b(uint32_t y) { return 17u * y + 196u; }
 
-template <int G, int C, bool LOCAL>
+// With TRACK (local), each half's best keeps the first row that reaches it (a strict rise moves it, a rare branch:
+// a hit raises its lane's best about once a row), and the pair's shape cut to its hit's rows goes to p.hits. A
+// local alignment then records those rows alone: every optimal path to the hit's end starts within them, so
+// along the walked path each cell is the whole matrix's and every other cell at most its own, and each
+// decision comes out the same.
+template <int G, int C, bool LOCAL, bool TRACK = false>
 __global__ void __launch_bounds__(kBlock) affine_pairs_kernel(KernelArgs p, TableArgs t, const int32_t *__restrict__) {
+    static_assert(LOCAL || !TRACK, "hits are local");
     constexpr int W = G * C;
     constexpr int GPW = 32 / G;
     __shared__ uint32_t rows8[4];
@@ -614,6 +637,8 @@ __global__ void __launch_bounds__(kBlock) affine_pairs_kernel(KernelArgs p, Tabl
         const int warp_strips = warp_max(max(strips[0], strips[1]));
         uint32_t best2 = 0;
         int32_t reported[2] = {0, 0};
+        // TRACK: each half's best over the strips so far and its first row.
+        int32_t hit[2] = {0, 0}, hit_row[2] = {0, 0}, strip_row[2] = {0, 0};
 
         for (int s = 0; s < warp_strips; ++s) {
             bool strip_live[2];
@@ -708,7 +733,12 @@ __global__ void __launch_bounds__(kBlock) affine_pairs_kernel(KernelArgs p, Tabl
 #pragma unroll
                         for (int k = 1; k + 1 < C; k += 2) row_best = __vimax3_s16x2(row_best, H[k], H[k + 1]);
                         if (C % 2 == 0) row_best = __vimax3_s16x2(row_best, H[C - 1], H[C - 1]);
-                        best2 = __viaddmax_s16x2(row_best, halves(-lift, -lift), best2);
+                        const uint32_t raised = __viaddmax_s16x2(row_best, halves(-lift, -lift), best2);
+                        if (TRACK && raised != best2) {
+                            if ((raised ^ best2) & 0xFFFFu) strip_row[0] = row;
+                            if ((raised ^ best2) >> 16) strip_row[1] = row;
+                        }
+                        best2 = raised;
                     }
                     if (member == G - 1 && s + 1 < warp_strips)
                         p.carry[slot * p.carry_stride + row] = make_int2(int32_t(H[C - 1]), int32_t(I));
@@ -730,11 +760,45 @@ __global__ void __launch_bounds__(kBlock) affine_pairs_kernel(KernelArgs p, Tabl
                     }
                 }
             }
+            if (TRACK) {
+                // The strip's best joins the others': higher, or as high from an earlier row.
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int32_t value = h == 0 ? low_of(best2) : high_of(best2);
+                    if (value > hit[h] || (value == hit[h] && strip_row[h] < hit_row[h])) {
+                        hit[h] = value;
+                        hit_row[h] = strip_row[h];
+                    }
+                    strip_row[h] = 0;
+                }
+                best2 = 0;
+            }
             __syncwarp();
         }
 
         // Results: a local score is the group's best, a global one the corner (one lane holds it) shifted back.
-        if (LOCAL) {
+        if (TRACK) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                for (int span = 1; span < G; span <<= 1) {
+                    const int32_t theirs = __shfl_xor_sync(kFull, hit[h], span, G);
+                    const int32_t their_row = __shfl_xor_sync(kFull, hit_row[h], span, G);
+                    if (theirs > hit[h] || (theirs == hit[h] && their_row < hit_row[h])) {
+                        hit[h] = theirs;
+                        hit_row[h] = their_row;
+                    }
+                }
+                if (live[h] && member == 0) {
+                    // No hit (a best of 0) leaves no row to record.
+                    const int first = hit_first_row(hit_row[h], cols[h], hit[h], p.best_entry, open, extend);
+                    PairShape cut = sh[h];
+                    cut.first_word += uint32_t(first / 16);
+                    cut.rows = hit[h] > 0 ? uint32_t(hit_row[h] - first) : 0u;
+                    p.hits[pair[h]] = cut;
+                }
+            }
+        } else if (LOCAL) {
 #pragma unroll
             for (int span = 1; span < G; span <<= 1) best2 = __vimax_s16x2_relu(best2, __shfl_xor_sync(kFull, best2, span, G));
             if (member == 0) {

@@ -396,16 +396,6 @@ void gather_tape(int64_t pairs, const char *const *references, const int64_t *re
     }
 }
 
-// as_alignment's placement (scoring.mojo:724-744): a local alignment's letters placed at the last place
-// they occur in their sequence; `start`/`end` are where the walk found them.
-int64_t last_place(const char *text, int64_t length, int64_t start, int64_t end) {
-    const int64_t k = end - start;
-    if (k <= 0) return 0;
-    for (int64_t at = length - k; at > start; --at)
-        if (text[at] == text[start] && std::memcmp(text + at, text + start, size_t(k)) == 0) return at;
-    return start;
-}
-
 // A large batch runs as units of pairs, each packed, swept and walked while later units' letters are
 // still crossing the bus and earlier units' results are being moved into the caller's buffers.
 
@@ -1379,15 +1369,7 @@ int64_t dinara_gpu_alignments_tape(dinara_gpu *gpu, int64_t pairs, const char *l
                         span[2] = 0;
                         span[3] = columns;
                     } else {
-                        const int64_t *w = walked + 4 * k;
-                        const char *reference = letters + offsets[2 * p];
-                        const char *query = letters + offsets[2 * p + 1];
-                        const int64_t r0 = last_place(reference, rows, w[0], w[1]);
-                        const int64_t c0 = last_place(query, columns, w[2], w[3]);
-                        span[0] = r0;
-                        span[1] = r0 + (w[1] - w[0]);
-                        span[2] = c0;
-                        span[3] = c0 + (w[3] - w[2]);
+                        std::memcpy(span, walked + 4 * k, 4 * sizeof(int64_t));
                     }
                 }
             });
@@ -1402,6 +1384,8 @@ int64_t dinara_gpu_alignments_tape(dinara_gpu *gpu, int64_t pairs, const char *l
             unit.count = count;
             unit.total = affine_alignments(ctx, batch, checked.table, eqx != 0, scores_device, spans_device, first,
                                            count);
+            if (local)
+                last_places(ctx, streamed.letters_device, streamed.offsets_device, first, count, spans_device);
             unit.layout = StageLayout(count, unit.total, local);
             uint8_t *stage = finisher.stage_for(int64_t(k), unit.layout.bytes);
             unit.stage = stage;

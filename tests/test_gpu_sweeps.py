@@ -64,3 +64,45 @@ def test_long_pairs_in_strips(da, oracle, entries):
     op, ex = oracle.kernel_gaps(scoring.opening, scoring.extension)
     expected = oracle.batch_scores(coded, tape.offsets, _table(scoring), 4, op, ex, oracle.GLOBAL, threads=8)
     np.testing.assert_array_equal(da.scores_tape(tape, scoring), expected)
+
+
+# ---- local alignments recorded over their hits' rows ----------------------------------------------------
+
+@pytest.mark.parametrize("alphabet", ["ACGT", "ACGTN", PROTEIN])
+def test_hits_in_long_targets(da, oracle, alphabet):
+    """Queries planted once, twice alike (the first hit wins, its letters placed at their last occurrence) and not
+    at all, at shape widths and a column either side, in targets whose hits start at every letter of a packed
+    word; repeats of one letter; gaps that cost nothing a letter, whose hits may span any rows."""
+    rng = np.random.default_rng(len(alphabet))
+    refs, queries = [], []
+    for trial, width in enumerate((1, 7, 16, 17, 63, 64, 65, 128, 129, 256, 257, 320, 321, 511, 512, 513, 800)):
+        query = _text(rng, width, alphabet)
+        lead = 100 + trial
+        for copies in (1, 2, 0):
+            target = _text(rng, lead, alphabet)
+            for _ in range(copies):
+                target += query + _text(rng, 200, alphabet)
+            target += _text(rng, 400, alphabet)
+            refs.append(target)
+            queries.append(_mutated(rng, query, 0.06, alphabet))
+    refs += [alphabet[0] * 300, alphabet[0] * 300, alphabet[0] * 40, "", alphabet[1] * 30]
+    queries += [alphabet[0] * 20, alphabet[1] * 9, alphabet[0] * 120, alphabet[0], ""]
+    tape = da.Tape.of(refs, queries)
+    coded = np.concatenate([oracle.codes(text, alphabet) for pair in zip(refs, queries) for text in pair if text])
+    scorings = [_tabulated(da, rng, alphabet), da.Scoring.uniform(2, -4, -4, -2, alphabet),
+                da.Scoring.uniform(2, -3, -5, 0, alphabet)]
+    for scoring in scorings:
+        op, ex = oracle.kernel_gaps(scoring.opening, scoring.extension)
+        expected, cigars = oracle.batch_alignments(coded, tape.offsets, _table(scoring), len(alphabet), op, ex,
+                                                   oracle.LOCAL, threads=8)
+        np.testing.assert_array_equal(da.scores_tape(tape, scoring, da.Mode.local()), expected)
+        found = da.alignments(refs, queries, scoring, da.Mode.local())
+        assert [a.score for a in found] == list(expected)
+        assert [a.cigar for a in found] == cigars
+        for a, ref, query in zip(found, refs, queries):
+            rows = ref[a.reference_start:a.reference_end]
+            columns = query[a.query_start:a.query_end]
+            top, bottom = a.gapped(ref, query)
+            assert (top.replace("-", ""), bottom.replace("-", "")) == (rows, columns)
+            assert a.reference_start == (ref.rfind(rows) if rows else 0)
+            assert a.query_start == (query.rfind(columns) if columns else 0)
