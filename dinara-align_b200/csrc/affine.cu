@@ -23,6 +23,7 @@
 #include "affine.cuh"
 #include "affine_kernel.cuh"
 #include "banded.cuh"
+#include "free_kernel.cuh"
 #include "long_kernel.cuh"
 #include "pack.cuh"
 
@@ -1012,11 +1013,13 @@ __global__ void diagonal_counts_kernel(const PairShape *__restrict__ shapes, int
     counts[k] = sh.rows > 0 && sh.columns > 0 ? int64_t(sh.rows) + sh.columns + 1 : 0;
 }
 
-// An extension's result from its sweep, one thread a pair. With a Z-drop (`diagonals`), the stop is read
+// An extension's result from its sweep, a warp a pair. With a Z-drop (`diagonals`), the stop is read
 // from the anti-diagonals' bests in order as scored.mojo:272-300 reads them: a best above zero at or
 // above the best so far is the new stop (later anti-diagonals win ties); one below it ends the sweep when
 // it lies more than `zdrop` plus `slack` a diagonal between them (each's reference less query letters)
-// below it. Otherwise the sweep's best cell is the stop. The span runs from the origin to the stop, or
+// below it. The warp reads 32 at once: each lane's best so far is a prefix maximum (of equal ones the latest),
+// and the first lane whose own drops ends the sweep with the stop before it. Otherwise the sweep's best cell is
+// the stop. The span runs from the origin to the stop, or
 // (swept from the ends) from the stop counted back to the ends. With an end bonus and no early end, the
 // alignment reaching the query's far end wins when its score plus the bonus passes the stop's
 // (scoring.mojo:704-710), compared without the sum: the bonus may be near 2^63.
@@ -1027,7 +1030,8 @@ __global__ void extension_finish_kernel(const PairShape *__restrict__ shapes, in
                                         int64_t end_bonus, const int32_t *__restrict__ reach_scores,
                                         const int64_t *__restrict__ reach_spans, int32_t *__restrict__ scores,
                                         int64_t *__restrict__ spans) {
-    const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t k = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     if (k >= count) return;
     const int64_t pair = first + k;
     const PairShape sh = shapes[pair];
@@ -1036,28 +1040,61 @@ __global__ void extension_finish_kernel(const PairShape *__restrict__ shapes, in
     bool dropped = false;
     if (diagonals && rows > 0 && columns > 0) {
         const unsigned long long *kept = diagonals + diagonal_offsets[k];
+        int32_t best_so_far = 0;
         int64_t best_row = 0, best_diagonal = 0;
-        best = 0;
-        for (int64_t d = 2; d <= rows + columns; ++d) {
-            const unsigned long long key = kept[d];
-            const int64_t most = int64_t(int32_t(uint32_t(key >> 32) ^ 0x80000000u));
-            const int64_t furthest = int64_t(key & 0xffffffffu);
-            if (most > 0 && most >= best) {
-                best = most;
-                best_row = furthest;
-                best_diagonal = d;
-            } else if (most < best) {
-                const int64_t lean = 2 * furthest - d, best_lean = 2 * best_row - best_diagonal;
-                const int64_t apart = lean > best_lean ? lean - best_lean : best_lean - lean;
-                if (best - most > zdrop + slack * apart) {
-                    dropped = true;
-                    break;
+        for (int64_t d0 = 2; d0 <= rows + columns && !dropped; d0 += 32) {
+            const int64_t d = d0 + lane;
+            const bool inside = d <= rows + columns;
+            const unsigned long long word = inside ? kept[d] : 0ull;
+            const int32_t most = inside ? int32_t(uint32_t(word >> 32) ^ 0x80000000u) : 0;
+            const int64_t furthest = int64_t(word & 0xffffffffu);
+            // The best up to and with this lane's: a value above zero, and the latest lane that has it (-1: the
+            // best before these).
+            int32_t through = inside && most > 0 && most >= best_so_far ? most : best_so_far;
+            int from = inside && most > 0 && most >= best_so_far ? lane : -1;
+#pragma unroll
+            for (int span = 1; span < 32; span <<= 1) {
+                const int32_t before = __shfl_up_sync(kFull, through, span);
+                const int before_from = __shfl_up_sync(kFull, from, span);
+                if (lane >= span && (before > through || (before == through && before_from > from))) {
+                    through = before;
+                    from = before_from;
                 }
             }
+            // The best before this lane's own: the lane before's.
+            int32_t standing = __shfl_up_sync(kFull, through, 1);
+            int standing_from = __shfl_up_sync(kFull, from, 1);
+            if (lane == 0) {
+                standing = best_so_far;
+                standing_from = -1;
+            }
+            const int source = max(standing_from, 0);
+            const int64_t from_row = __shfl_sync(kFull, furthest, source);
+            const int64_t standing_row = standing_from >= 0 ? from_row : best_row;
+            const int64_t standing_diagonal = standing_from >= 0 ? d0 + standing_from : best_diagonal;
+            bool drops = false;
+            if (inside && most < standing) {
+                const int64_t lean = 2 * furthest - d, best_lean = 2 * standing_row - standing_diagonal;
+                const int64_t apart = lean > best_lean ? lean - best_lean : best_lean - lean;
+                drops = int64_t(standing) - most > zdrop + slack * apart;
+            }
+            const unsigned dropping = __ballot_sync(kFull, drops);
+            dropped = dropping != 0;
+            // The stop as it stands: before the first lane that drops, or after all 32.
+            const int last = dropped ? __ffs(dropping) - 1 : 31;
+            const int32_t value = dropped ? __shfl_sync(kFull, standing, last) : __shfl_sync(kFull, through, last);
+            const int value_from = dropped ? __shfl_sync(kFull, standing_from, last) : __shfl_sync(kFull, from, last);
+            if (value_from >= 0) {
+                best_row = __shfl_sync(kFull, furthest, value_from);
+                best_diagonal = d0 + value_from;
+            }
+            best_so_far = value;
         }
+        best = best_so_far;
         row = best_row;
         column = best_diagonal - best_row;
     }
+    if (lane != 0) return;
     int64_t span[4] = {from_end ? rows - row : 0, from_end ? rows : row, from_end ? columns - column : 0,
                        from_end ? columns : column};
     if (end_bonus > 0 && !dropped && end_bonus > best - int64_t(reach_scores[pair])) {
@@ -1069,7 +1106,84 @@ __global__ void extension_finish_kernel(const PairShape *__restrict__ shapes, in
         for (int j = 0; j < 4; ++j) spans[4 * k + j] = span[j];
 }
 
-// Global scores with free ends: every pair over its whole matrix in 32 bits, one shape (32 lanes of 16
+// Which pairs the 16-bit free-end sweep takes (a table of up to four letters on the 2-bit tape, its shifted
+// entries a byte): a shifted cell reaches at most the best entry times the columns swept plus the rows and
+// columns swept times -extend, held to half of 30,000 less the gaps for the sum of a group's two pairs, and
+// falls at most a few gap openings below zero.
+PairLimits free_limits_of(const AffineBatch &batch, const AffineTable &table) {
+    PairLimits limits;
+    const int32_t gaps = std::abs(table.open) + std::abs(table.extend);
+    if (batch.bits != 2 || !table.packed16 || gaps > 2000) return limits;
+    int32_t best = 1;
+    for (int r = 0; r < table.size; ++r)
+        for (int c = 0; c < table.size; ++c) {
+            best = std::max(best, table.entries[r * 32 + c]);
+            const int32_t shifted = table.entries[r * 32 + c] - 2 * table.extend;
+            if (shifted < -128 || shifted > 127) return limits;
+        }
+    limits.local = 1;  // the local form of the limit
+    limits.whole = (30000 - 4 * gaps) / 2;
+    limits.best = best - table.extend;
+    limits.row_step = std::max(-table.extend, 1);  // an extension's rows fit 16 bits too
+    return limits;
+}
+
+// An extension's sweep takes eight places a lane, twice a class's lanes at most.
+KernelFn pick_extension_kernel(int cls) {
+    switch (cls) {
+        case 0: return &extension_pairs_kernel<8, 8>;
+        case 1: return &extension_pairs_kernel<16, 8>;
+        default: return &extension_pairs_kernel<32, 8>;
+    }
+}
+
+KernelFn pick_free_kernel(int cls) {
+    switch (cls) {
+        case 0: return &free_pairs_kernel<4, 16>;
+        case 1: return &free_pairs_kernel<8, 16>;
+        case 2: return &free_pairs_kernel<16, 16>;
+        case 3: return &free_pairs_kernel<16, 20>;
+        default: return &free_pairs_kernel<32, 16>;
+    }
+}
+
+// One free-end sweep of a scheduled batch: the 16-bit classes' pairs, then the rest in 32 bits.
+void launch_free(dinara_gpu *gpu, const AffineBatch &batch, const Schedule &order, KernelFn general, KernelArgs args,
+                 const TableArgs &targs, const int32_t *table32) {
+    const Buckets b = buckets_of(order);
+    auto launch = [&](KernelFn fn, int lanes, int width, int pairs_a_group, int64_t begin, int64_t end) {
+        if (end <= begin) return;
+        const int64_t per_block = int64_t(pairs_a_group) * kBlock / lanes;
+        const int64_t blocks =
+            std::max<int64_t>(1, std::min<int64_t>(persistent_blocks(gpu, fn), (end - begin + per_block - 1) / per_block));
+        args.carry = nullptr;
+        args.carry_stride = 0;
+        if (batch.max_columns > uint32_t(width)) {
+            args.carry_stride = int64_t(batch.max_rows) + 1;
+            args.carry = gpu->carry.ensure<int2>(size_t(blocks * (kBlock / lanes) * args.carry_stride));
+        }
+        args.begin = uint32_t(begin);
+        args.end = uint32_t(end);
+        ClockSpan clock(gpu, kClassWhole, gpu->stream);
+        fn<<<dim3(unsigned(blocks)), kBlock, 0, gpu->stream>>>(args, targs, table32);
+        DINARA_CUDA(cudaGetLastError());
+        clock.stop();
+        gpu->launches += 1;
+    };
+    for (int cls = kAffineShapes - 1; cls >= 0; --cls) {
+        const int64_t begin = b.begin[kWholePairsClass + cls], end = b.end[kWholePairsClass + cls];
+        if (batch.extension) {
+            const int lanes = std::min(2 * affine_lanes(cls), 32);
+            launch(pick_extension_kernel(cls), lanes, 8 * lanes, 2, begin, end);
+        } else {
+            launch(pick_free_kernel(cls), affine_lanes(cls), affine_lanes(cls) * affine_columns(cls), 2, begin, end);
+        }
+    }
+    launch(general, 32, 512, 1, b.begin[kAffineShapes - 1], b.end[0]);
+}
+
+// Global scores with free ends: pairs whose values fit it in the 16-bit pair sweep (free_limits_of), the rest
+// over their whole matrix in 32 bits, one shape (32 lanes of 16
 // columns, strips of 512) with the table in shared memory, the free-end form of the sweep. With `spans`
 // (4 a pair of the range, by pair - first), each pair's span as the reference places it
 // (scoring.mojo:690-722 mode_span, scored.mojo:616-633 started_span): its end, of equal best ends the one
@@ -1120,7 +1234,8 @@ void free_end_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTabl
         reach_spans = gpu->reach_spans.ensure<int64_t>(4 * size_t(count));
         free_end_scores(gpu, reaching, table, reach_scores, first, count, reach_spans);
     }
-    const Schedule order = dinara::schedule(gpu, batch.shapes, nullptr, first, count, false, false, PairLimits());
+    const PairLimits limits = free_limits_of(batch, table);
+    const Schedule order = dinara::schedule(gpu, batch.shapes, nullptr, first, count, false, false, limits);
     int32_t *table32 = nullptr;
     upload_table32(gpu, table, false, &table32);
     const TableArgs targs = table_args(table, false);
@@ -1172,24 +1287,19 @@ void free_end_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTabl
             args.diagonal_offsets = diagonal_offsets;
         }
     }
-    int64_t total = 0;
-    for (int cls = 0; cls < kClasses; ++cls) total += order.counts[cls];
-    int64_t blocks = persistent_blocks(gpu, fn);
-    blocks = std::max<int64_t>(1, std::min<int64_t>(blocks, (total + kBlock / 32 - 1) / (kBlock / 32)));
-    if (batch.max_columns > 512u) {
-        args.carry_stride = int64_t(batch.max_rows) + 1;
-        args.carry = gpu->carry.ensure<int2>(size_t(blocks * (kBlock / 32) * args.carry_stride));
-    }
-    args.begin = 0;
-    args.end = uint32_t(total);
     PhaseTimer timer(gpu, &gpu->kernel_ms);
-    ClockSpan clock(gpu, kClassWhole, gpu->stream);
-    fn<<<dim3(unsigned(blocks)), kBlock, 0, gpu->stream>>>(args, targs, table32);
-    DINARA_CUDA(cudaGetLastError());
-    clock.stop();
-    gpu->launches += 1;
+    const unsigned pair_blocks = unsigned((count + 255) / 256);
+    // With no letter free at the ends, every pair's end is its corner: the sweep back alone gives its score.
+    const bool corner_ends = spans && !batch.extension && batch.free_reference_end == 0 && batch.free_query_end == 0;
+    if (corner_ends) {
+        extents_kernel<<<pair_blocks, 256, 0, gpu->stream>>>(batch.shapes, first, count, ends);
+        DINARA_CUDA(cudaGetLastError());
+        gpu->launches += 1;
+    } else {
+        launch_free(gpu, batch, order, fn, args, targs, table32);
+    }
     if (batch.extension) {
-        extension_finish_kernel<<<unsigned((count + 255) / 256), 256, 0, gpu->stream>>>(
+        extension_finish_kernel<<<unsigned((count * 32 + 255) / 256), 256, 0, gpu->stream>>>(
             batch.shapes, first, count, batch.from_end, ends, args.diagonals, args.diagonal_offsets, batch.zdrop,
             -int64_t(table.extend), batch.end_bonus, reach_scores, reach_spans, scores, spans);
         DINARA_CUDA(cudaGetLastError());
@@ -1197,22 +1307,27 @@ void free_end_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTabl
     } else if (spans) {
         // The sweep back: each pair's prefixes to its end, backwards, the start's free letters free at the
         // (backward) end and none at its start; its scores, the same, go to scratch.
-        KernelArgs back = args;
-        back.scores = gpu->free_scores.ensure<int32_t>(size_t(batch.pairs));
-        back.extents = ends;
-        back.free_ends_out = ends + count;
-        back.free_highest = 0;
-        back.free_reference_start = 0;
-        back.free_reference_end = batch.free_reference_start;
-        back.free_query_start = 0;
-        back.free_query_end = batch.free_query_start;
-        ClockSpan back_clock(gpu, kClassWhole, gpu->stream);
-        fn<<<dim3(unsigned(blocks)), kBlock, 0, gpu->stream>>>(back, targs, table32);
+        // With no letter free at the starts, every pair starts at its origin and needs none.
+        const bool origin_starts = !corner_ends && batch.free_reference_start == 0 && batch.free_query_start == 0;
+        if (!origin_starts) {
+            KernelArgs back = args;
+            if (!corner_ends) {
+                back.scores = gpu->free_scores.ensure<int32_t>(size_t(batch.pairs));
+                back.known = scores;
+                back.best_entry = limits.whole > 0 ? limits.best + table.extend : 0;
+            }
+            back.extents = ends;
+            back.free_ends_out = ends + count;
+            back.free_highest = 0;
+            back.free_reference_start = 0;
+            back.free_reference_end = batch.free_reference_start;
+            back.free_query_start = 0;
+            back.free_query_end = batch.free_query_start;
+            launch_free(gpu, batch, order, fn, back, targs, table32);
+        }
+        free_spans_kernel<<<pair_blocks, 256, 0, gpu->stream>>>(ends, origin_starts ? ends : ends + count, count, spans);
         DINARA_CUDA(cudaGetLastError());
-        back_clock.stop();
-        free_spans_kernel<<<unsigned((count + 255) / 256), 256, 0, gpu->stream>>>(ends, ends + count, count, spans);
-        DINARA_CUDA(cudaGetLastError());
-        gpu->launches += 2;
+        gpu->launches += 1;
     }
     timer.stop();
 }

@@ -75,6 +75,7 @@ struct KernelArgs {
     // can span (hit_rows), by pair, for a recording sweep of those rows alone; `best_entry` the table's.
     PairShape *hits;
     int32_t best_entry;
+    const int32_t *known;  // free_pairs_kernel, sweeping back: each pair's score, by pair
 };
 
 // The rows, ending with `end_row`, that a local alignment of `score` ending there can span, its first one at
@@ -147,6 +148,34 @@ struct TableArgs {
 // whose first `free` letters go unaligned for nothing, a gap from where they end past them.
 __device__ __forceinline__ int32_t free_edge(int letters, int free, int32_t open, int32_t extend) {
     return letters <= free ? 0 : open + (letters - free - 1) * extend;
+}
+
+// The best end with free letters of a pair with an empty side, and its place (row << 32 | column). scored.mojo:155-176:
+// the run along the other side's edge, ending within its free letters at the end. Of equal ends, the furthest
+// when the run goes along the reference and the highest end is favoured (or along the query and the lowest),
+// else the nearest; free_edge never rises with the letters, so the equal ones run from the nearest allowed to
+// the last that still scores as it does.
+__device__ __forceinline__ void empty_side_end(int rows, int cols, int free_rs, int free_re, int free_qs, int free_qe,
+                                               bool highest, int32_t open, int32_t extend, int32_t &value, int64_t &at) {
+    value = 0;
+    at = 0;
+    if (rows == 0 && cols == 0) return;
+    const bool along_reference = rows > 0;
+    const int length = along_reference ? rows : cols;
+    const int start_free = along_reference ? free_rs : free_qs;
+    const int lo = max(length - (along_reference ? free_re : free_qe), 0);
+    value = free_edge(lo, start_free, open, extend);
+    int reach = lo, beyond = length;
+    if (along_reference == highest) {
+        while (reach < beyond) {
+            const int mid = beyond - (beyond - reach) / 2;
+            if (free_edge(mid, start_free, open, extend) == value)
+                reach = mid;
+            else
+                beyond = mid - 1;
+        }
+    }
+    at = along_reference ? int64_t(reach) << 32 : int64_t(reach);
 }
 
 // One pair per group of G lanes; see the file's notes. Persistent: each warp takes its next GPW pairs of
@@ -513,33 +542,8 @@ __global__ void __launch_bounds__(kBlock) affine_kernel(KernelArgs p, TableArgs 
                 if (ORIGIN) {
                     // An extension's stop: the group's best above zero, or the origin.
                 } else if (!work) {
-                    if (rows == 0 && cols == 0) {
-                        free_best = 0;
-                        free_at = 0;
-                    } else {
-                        // scored.mojo:155-176: the run along the other side's edge, ending within its free
-                        // letters at the end. Of equal ends, the furthest when the run goes along the
-                        // reference and the highest end is favoured (or along the query and the lowest),
-                        // else the nearest; free_edge never rises with the letters, so the equal ones run
-                        // from the nearest allowed to the last that still scores as it does.
-                        const bool along_reference = rows > 0;
-                        const int length = along_reference ? rows : cols;
-                        const int start_free = along_reference ? free_rs : free_qs;
-                        const int lo = max(length - (along_reference ? free_re : free_qe), 0);
-                        const int32_t top = free_edge(lo, start_free, open, extend);
-                        int reach = lo, beyond = length;
-                        if (along_reference == highest) {
-                            while (reach < beyond) {
-                                const int mid = beyond - (beyond - reach) / 2;
-                                if (free_edge(mid, start_free, open, extend) == top)
-                                    reach = mid;
-                                else
-                                    beyond = mid - 1;
-                            }
-                        }
-                        free_best = top;
-                        free_at = along_reference ? int64_t(reach) << 32 : int64_t(reach);
-                    }
+                    empty_side_end(rows, cols, free_rs, free_re, free_qs, free_qe, highest, open, extend, free_best,
+                                   free_at);
                 } else {
                     if (cols <= free_qe) offer(free_edge(rows, free_rs, open, extend), rows, 0);
                     if (rows <= free_re) offer(free_edge(cols, free_qs, open, extend), 0, cols);

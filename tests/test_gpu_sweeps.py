@@ -106,3 +106,50 @@ def test_hits_in_long_targets(da, oracle, alphabet):
             assert (top.replace("-", ""), bottom.replace("-", "")) == (rows, columns)
             assert a.reference_start == (ref.rfind(rows) if rows else 0)
             assert a.query_start == (query.rfind(columns) if columns else 0)
+
+
+# ---- free ends and extensions in 16-bit halves ----------------------------------------------------------
+
+WIDTHS = (1, 8, 9, 15, 16, 17, 63, 64, 65, 127, 128, 129, 255, 256, 257, 320, 321, 512, 513, 700)
+
+
+def _placed_pairs(rng, alphabet):
+    refs, queries = [], []
+    for width in WIDTHS:
+        source = _text(rng, width, alphabet)
+        for flank in (0, 1, 15, 16, 90):
+            refs.append(_text(rng, flank, alphabet) + source + _text(rng, 2 * flank, alphabet))
+            queries.append(_mutated(rng, source, 0.08, alphabet))
+    return refs, queries
+
+
+def _span(a):
+    return a.reference_start, a.reference_end, a.query_start, a.query_end
+
+
+# The last two: gaps past the 16-bit forms' limit, and values past it on the longer pairs.
+@pytest.mark.parametrize("alphabet,entries", [("ACGT", (2, -4, -4, -2)), ("ACGT", (1, -3, -5, 0)),
+                                              ("ACGTN", (2, -4, -6, -1)), (THIRTY_TWO, (5, -2, -10, -1)),
+                                              ("ACGT", (5, -4, -2000, -1)), ("ACGT", (40, -30, -40, -30))])
+def test_free_ends_and_extensions_at_the_widths(da, oracle, alphabet, entries):
+    rng = np.random.default_rng(len(alphabet) + abs(sum(entries)))
+    scoring = da.Scoring.uniform(*entries, alphabet)
+    refs, queries = _placed_pairs(rng, alphabet)
+    # Queries that part from their references half way, for the Z-drop.
+    for k in range(0, len(queries), 3):
+        queries[k] = queries[k][:len(queries[k]) // 2] + _text(rng, len(queries[k]) // 2, alphabet)
+    op, ex = oracle.kernel_gaps(scoring.opening, scoring.extension)
+    coded = [(oracle.codes(r, alphabet), oracle.codes(q, alphabet)) for r, q in zip(refs, queries)]
+    size, table = len(alphabet), _table(scoring)
+    for counts in ((BIG, BIG, 0, 0), (0, BIG, 0, 0), (BIG, 0, 0, 0), (0, 0, BIG, BIG), (9, 20, 0, 4)):
+        mode = da.Mode.ends_free(*counts)
+        found = da.alignments(refs, queries, scoring, mode)
+        expected = [oracle.free_ends_alignment(a, b, table, size, op, ex, *counts) for a, b in coded]
+        assert [(a.score, a.cigar, _span(a)) for a in found] == expected
+        assert da.scores(refs, queries, scoring, mode) == [score for score, _c, _s in expected]
+    for anchor in (da.Anchor.START, da.Anchor.END):
+        for zdrop, bonus in ((-1, -1), (25, 8), (0, -1)):
+            found = da.alignments(refs, queries, scoring, da.Mode.extension(0, anchor, zdrop=zdrop, end_bonus=bonus))
+            expected = [oracle.extension_alignment(a, b, table, size, op, ex, anchor == da.Anchor.END, bonus, zdrop=zdrop)
+                        for a, b in coded]
+            assert [(a.score, a.cigar, _span(a)) for a in found] == expected
