@@ -10,7 +10,8 @@
 // CPU only. Here one warp takes one pair: its lanes compute a cost's front, diagonals 32 apart, each
 // sliding over its matches; every front is kept in the warp's arena of device memory; lane 0 traces back
 // through them and writes the CIGAR. Warps take pairs from a queue, longest first. A pair whose fronts
-// outgrow its warp's arena goes onto a list that runs again on fewer warps with larger arenas.
+// outgrow its warp's arena goes on in blocks of a shared pool, and one past those goes onto a list that runs again on
+// fewer warps with larger arenas.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -26,7 +27,17 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWaveBlock = 128;
-constexpr int32_t kUnreached = -(1 << 30);
+// Fronts are kept as 16-bit columns when every pair's letters fit (a front's place then takes 7 bytes under
+// gap-affine costs instead of 13, and a pair's fronts about half the arena), else 32-bit; an empty place is the
+// type's lowest value.
+template <class V>
+constexpr int32_t kUnreached = sizeof(V) == 2 ? -32768 : -(1 << 30);
+constexpr int64_t kShortLetters = 32000;
+// Past its arena a warp's fronts go on in blocks of a pool that the launch's warps share, each taken by setting
+// its bit and given back when the pair is done; a pair that finds none free runs again with a larger arena.
+constexpr int64_t kBlockBytes = int64_t(1) << 20;
+constexpr int64_t kMostBlocks = 1024;
+constexpr int kBlocksAPair = 4;
 // A pair's slot in the cost table and in `results` while it waits for a larger arena.
 constexpr int64_t kRetry = INT64_MIN;
 
@@ -50,6 +61,9 @@ struct WaveArgs {
     bool trace;
     uint8_t *arena;
     int64_t arena_bytes;     // a warp's
+    int64_t blocks_at;       // the pool's first byte in `arena`
+    uint32_t *blocks_taken;  // a bit a block, `block_words` words; null: no pool
+    int32_t block_words;
     int32_t table_entries;   // cost entries at the start of each arena
     int64_t *results;        // per pair: its cost, or its code
     const int64_t *slot_offsets;
@@ -59,27 +73,49 @@ struct WaveArgs {
     unsigned int *retry_count;
 };
 
-__device__ __forceinline__ uint8_t letter_of(const uint8_t *s, int32_t length, int32_t i, bool reversed) {
-    return __ldg(s + (reversed ? length - 1 - i : i));
+// Eight bytes from `at` on, which need not be aligned (device letter buffers start on a 16-byte boundary and keep 16
+// bytes of room past the last letter): the two aligned words they lie in.
+__device__ __forceinline__ uint64_t eight_bytes(const uint8_t *at) {
+    const uintptr_t address = reinterpret_cast<uintptr_t>(at);
+    const uint64_t *aligned = reinterpret_cast<const uint64_t *>(address & ~uintptr_t(7));
+    const uint32_t shift = uint32_t(address & 7u) * 8u;
+    const uint64_t low = __ldg(aligned), high = __ldg(aligned + 1);
+    return shift ? (low >> shift) | (high << (64u - shift)) : low;
 }
 
-// The furthest column a diagonal's matches take a front from `column` (row column - diagonal).
-__device__ __forceinline__ int32_t slide(const uint8_t *first, int32_t columns, const uint8_t *second, int32_t rows,
-                                         int32_t column, int32_t diagonal, bool reversed) {
-    int32_t row = column - diagonal;
-    while (column < columns && row < rows &&
-           letter_of(first, columns, column, reversed) == letter_of(second, rows, row, reversed)) {
-        ++column;
-        ++row;
+// Eight letters of a sequence from letter `i` on as it is read: forwards, the first in the low byte; reversed, the
+// first in the high byte (letter i is then s[length - 1 - i]). No byte before `letters`, the buffer's first, is
+// read; what lies past the sequence is for the caller to leave out.
+__device__ __forceinline__ uint64_t eight_letters(const uint8_t *letters, const uint8_t *s, int32_t length, int32_t i,
+                                                  bool reversed) {
+    if (!reversed) return eight_bytes(s + i);
+    const int64_t at = (s - letters) + length - 8 - i;
+    return at >= 0 ? eight_bytes(letters + at) : eight_bytes(letters) << (-8 * at);
+}
+
+// The furthest column a diagonal's matches take a front from `column` (row column - diagonal), eight letters a
+// step: a letter at a time, each pair of loads waited for the one before.
+__device__ __forceinline__ int32_t slide(const uint8_t *letters, const uint8_t *first, int32_t columns,
+                                         const uint8_t *second, int32_t rows, int32_t column, int32_t diagonal,
+                                         bool reversed) {
+    int32_t left = min(columns - column, rows - (column - diagonal));
+    while (left > 0) {
+        const uint64_t apart = eight_letters(letters, first, columns, column, reversed) ^
+                               eight_letters(letters, second, rows, column - diagonal, reversed);
+        const int32_t alike = apart ? (reversed ? __clzll(apart) : __ffsll(apart) - 1) >> 3 : 8;
+        column += min(alike, left);
+        if (alike < 8) break;
+        left -= 8;
     }
     return column;
 }
 
 // A front's value on a diagonal: unreached outside its diagonals, before cost zero, or where empty.
+template <class V>
 __device__ __forceinline__ int32_t front_at(const uint8_t *arena, const CostEntry &e, int32_t layer, int32_t k) {
-    if (e.lo > e.hi || k < e.lo || k > e.hi) return kUnreached;
+    if (e.lo > e.hi || k < e.lo || k > e.hi) return kUnreached<V>;
     const int32_t width = e.hi - e.lo + 1;
-    return reinterpret_cast<const int32_t *>(arena + e.offset)[int64_t(layer) * width + (k - e.lo)];
+    return reinterpret_cast<const V *>(arena + e.offset)[int64_t(layer) * width + (k - e.lo)];
 }
 
 __device__ __forceinline__ CostEntry entry_of(const CostEntry *table, int32_t s) {
@@ -163,6 +199,7 @@ struct CigarOut {
 
 // The trace of diagonal transition (diagonal_cigar, traceback.mojo:803-900): from the corner, each cost
 // undoes the matches its front slid over and the edit `furthest_source` names.
+template <class V>
 __device__ bool trace_edit(const WaveArgs &a, const uint8_t *arena, const CostEntry *table, int32_t distance,
                            int32_t columns, int32_t rows, CigarOut &out) {
     const char matched = a.eqx ? '=' : 'M', substituted = a.eqx ? 'X' : 'M';
@@ -170,8 +207,8 @@ __device__ bool trace_edit(const WaveArgs &a, const uint8_t *arena, const CostEn
     for (int32_t score = distance; score > 0; --score) {
         const CostEntry back = table[score - 1];
         int move;
-        const int32_t best = furthest_source(front_at(arena, back, 0, diagonal), front_at(arena, back, 0, diagonal - 1),
-                                             front_at(arena, back, 0, diagonal + 1), diagonal, columns, rows, move);
+        const int32_t best = furthest_source(front_at<V>(arena, back, 0, diagonal), front_at<V>(arena, back, 0, diagonal - 1),
+                                             front_at<V>(arena, back, 0, diagonal + 1), diagonal, columns, rows, move);
         if (best < 0 || best > column) return false;
         out.add(matched, column - best);
         if (move == 0) {
@@ -192,19 +229,21 @@ __device__ bool trace_edit(const WaveArgs &a, const uint8_t *arena, const CostEn
 }
 
 // Layers of a gap-affine front: the alignment front, the first sequence's gap layer, the second's, and
-// the flags (a byte each, after the three int32 layers).
+// the flags (a byte each, after the three layers).
 constexpr int kAligned = 0, kFirst = 1, kSecond = 2;
 constexpr uint8_t kOpenedFirst = 8, kOpenedSecond = 16;
 
+template <class V>
 __device__ __forceinline__ uint8_t flag_at(const uint8_t *arena, const CostEntry &e, int32_t k) {
     const int32_t width = e.hi - e.lo + 1;
-    return (arena + e.offset + 12 * int64_t(width))[k - e.lo];
+    return (arena + e.offset + 3 * int64_t(sizeof(V)) * width)[k - e.lo];
 }
 
 // The gap-affine trace (gap_affine.mojo:2028-2124): in the alignment layer the source that won the front
 // (a substitution from the front `x` back, or a gap layer at the same cost, entered after the matches
 // back to its column); in a gap layer a letter of its sequence, then the opening or the extension its
 // flag names, an extension on a tie. On the first row or column the rest is a gap along it.
+template <class V>
 __device__ bool trace_affine(const WaveArgs &a, const uint8_t *arena, const CostEntry *table, int32_t cost,
                              int32_t columns, int32_t rows, CigarOut &out) {
     const char matched = a.eqx ? '=' : 'M', substituted = a.eqx ? 'X' : 'M';
@@ -235,9 +274,9 @@ __device__ bool trace_affine(const WaveArgs &a, const uint8_t *arena, const Cost
                 continue;
             }
             const CostEntry e = table[spent];
-            const int source = flag_at(arena, e, k) & 7;
-            const int32_t entry = source == kAligned ? front_at(arena, entry_of(table, spent - a.x), kAligned, k) + 1
-                                                     : front_at(arena, e, source, k);
+            const int source = flag_at<V>(arena, e, k) & 7;
+            const int32_t entry = source == kAligned ? front_at<V>(arena, entry_of(table, spent - a.x), kAligned, k) + 1
+                                                     : front_at<V>(arena, e, source, k);
             if (entry <= c) {
                 out.add(matched, c - entry);
                 c = entry;
@@ -251,7 +290,7 @@ __device__ bool trace_affine(const WaveArgs &a, const uint8_t *arena, const Cost
             }
         } else {
             const CostEntry e = table[spent];
-            const bool opened = (flag_at(arena, e, k) & (current == kFirst ? kOpenedFirst : kOpenedSecond)) != 0;
+            const bool opened = (flag_at<V>(arena, e, k) & (current == kFirst ? kOpenedFirst : kOpenedSecond)) != 0;
             if (current == kFirst) {
                 out.add('D', 1);
                 c -= 1;
@@ -285,13 +324,16 @@ __device__ bool trace_affine(const WaveArgs &a, const uint8_t *arena, const Cost
     return false;
 }
 
-template <bool EDIT>
+template <bool EDIT, class V>
 __global__ void __launch_bounds__(kWaveBlock) wavefront_kernel(WaveArgs a) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = (int64_t(blockIdx.x) * kWaveBlock + threadIdx.x) >> 5;
-    uint8_t *arena = a.arena + warp * a.arena_bytes;
-    CostEntry *table = reinterpret_cast<CostEntry *>(arena);
-    const int64_t data_begin = int64_t(a.table_entries) * int64_t(sizeof(CostEntry));
+    // The warp's own arena (its cost entries, then fronts), and where its fronts go on once that is full: every
+    // offset counts from the launch's first byte.
+    uint8_t *const arena = a.arena;
+    const int64_t own_begin = warp * a.arena_bytes;
+    CostEntry *table = reinterpret_cast<CostEntry *>(arena + own_begin);
+    const int64_t data_begin = own_begin + int64_t(a.table_entries) * int64_t(sizeof(CostEntry));
     for (;;) {
         uint32_t item = 0;
         if (lane == 0) item = atomicAdd(a.next, 1u);
@@ -304,7 +346,9 @@ __global__ void __launch_bounds__(kWaveBlock) wavefront_kernel(WaveArgs a) {
         const uint8_t *second = a.letters + p1;
         const int32_t columns = int32_t(p1 - p0), rows = int32_t(p2 - p1);
         const int32_t target = columns - rows;
-        int64_t used = data_begin;
+        int64_t used = data_begin, room_end = own_begin + a.arena_bytes;
+        int held_blocks = 0;
+        int32_t held[kBlocksAPair];
         bool overflow = false, found = false;
         int32_t s = 0;
         for (;; ++s) {
@@ -342,10 +386,39 @@ __global__ void __launch_bounds__(kWaveBlock) wavefront_kernel(WaveArgs a) {
             lo = max(lo, -rows);
             hi = min(hi, columns);
             const int32_t width = hi >= lo ? hi - lo + 1 : 0;
-            const int64_t bytes = ((EDIT ? 4 * int64_t(width) : 13 * int64_t(width)) + 15) & ~int64_t(15);
-            if (used + bytes > a.arena_bytes) {
-                overflow = true;
-                break;
+            constexpr int64_t kPlaceBytes = EDIT ? int64_t(sizeof(V)) : 3 * int64_t(sizeof(V)) + 1;
+            const int64_t bytes = (kPlaceBytes * width + 15) & ~int64_t(15);
+            if (used + bytes > room_end) {
+                // A free block of the pool, searched from a word of the warp's own on.
+                int32_t block = -1;
+                if (a.blocks_taken && held_blocks < kBlocksAPair && bytes <= kBlockBytes) {
+                    if (lane == 0) {
+                        for (int w = 0; w < a.block_words && block < 0; ++w) {
+                            const int word = int((warp + w) % a.block_words);
+                            uint32_t taken = *const_cast<volatile uint32_t *>(a.blocks_taken + word);
+                            while (taken != ~0u) {  // each turn takes a bit or sees one more taken
+                                const uint32_t bit = (~taken) & (taken + 1u);
+                                const uint32_t before = atomicOr(a.blocks_taken + word, bit);
+                                if (!(before & bit)) {
+                                    block = 32 * word + __ffs(bit) - 1;
+                                    break;
+                                }
+                                taken |= bit;
+                            }
+                        }
+                    }
+                    block = __shfl_sync(kFull, block, 0);
+                }
+                if (block < 0) {
+                    overflow = true;
+                    break;
+                }
+#pragma unroll
+                for (int b = 0; b < kBlocksAPair; ++b)
+                    if (b == held_blocks) held[b] = block;
+                ++held_blocks;
+                used = a.blocks_at + int64_t(block) * kBlockBytes;
+                room_end = used + kBlockBytes;
             }
             if (lane == 0) {
                 CostEntry e;
@@ -354,34 +427,34 @@ __global__ void __launch_bounds__(kWaveBlock) wavefront_kernel(WaveArgs a) {
                 e.offset = used;
                 table[s] = e;
             }
-            int32_t *aligned = reinterpret_cast<int32_t *>(arena + used);
+            V *aligned = reinterpret_cast<V *>(arena + used);
             bool hit = false;
             for (int32_t k = lo + lane; k <= hi; k += 32) {
                 int32_t value;
                 if (s == 0) {
-                    value = slide(first, columns, second, rows, 0, 0, a.reversed);
+                    value = slide(a.letters, first, columns, second, rows, 0, 0, a.reversed);
                     if (!EDIT) {
-                        aligned[width + (k - lo)] = kUnreached;
-                        aligned[2 * width + (k - lo)] = kUnreached;
+                        aligned[width + (k - lo)] = V(kUnreached<V>);
+                        aligned[2 * width + (k - lo)] = V(kUnreached<V>);
                         (reinterpret_cast<uint8_t *>(aligned + 3 * width))[k - lo] = 0;
                     }
                 } else if (EDIT) {
                     int move;
-                    const int32_t best = furthest_source(front_at(arena, same_e, 0, k), front_at(arena, same_e, 0, k - 1),
-                                                         front_at(arena, same_e, 0, k + 1), k, columns, rows, move);
-                    value = best < 0 ? kUnreached : slide(first, columns, second, rows, best, k, a.reversed);
+                    const int32_t best = furthest_source(front_at<V>(arena, same_e, 0, k), front_at<V>(arena, same_e, 0, k - 1),
+                                                         front_at<V>(arena, same_e, 0, k + 1), k, columns, rows, move);
+                    value = best < 0 ? kUnreached<V> : slide(a.letters, first, columns, second, rows, best, k, a.reversed);
                 } else {
-                    const int32_t same = front_at(arena, same_e, kAligned, k);
-                    const int32_t opened_below = front_at(arena, open_first_e, kAligned, k - 1);
-                    const int32_t extended_below = front_at(arena, ext_first_e, kFirst, k - 1);
-                    const int32_t opened_above = front_at(arena, open_second_e, kAligned, k + 1);
-                    const int32_t extended_above = front_at(arena, ext_second_e, kSecond, k + 1);
+                    const int32_t same = front_at<V>(arena, same_e, kAligned, k);
+                    const int32_t opened_below = front_at<V>(arena, open_first_e, kAligned, k - 1);
+                    const int32_t extended_below = front_at<V>(arena, ext_first_e, kFirst, k - 1);
+                    const int32_t opened_above = front_at<V>(arena, open_second_e, kAligned, k + 1);
+                    const int32_t extended_above = front_at<V>(arena, ext_second_e, kSecond, k + 1);
                     const int32_t below = max(opened_below, extended_below);
                     const int32_t above = max(opened_above, extended_above);
-                    const int32_t first_gap = below >= 0 && below < columns ? below + 1 : kUnreached;
-                    const int32_t second_gap = above >= 0 && above - k <= rows ? above : kUnreached;
+                    const int32_t first_gap = below >= 0 && below < columns ? below + 1 : kUnreached<V>;
+                    const int32_t second_gap = above >= 0 && above - k <= rows ? above : kUnreached<V>;
                     const int32_t substituted =
-                        same >= 0 && same < columns && same - k < rows ? same + 1 : kUnreached;
+                        same >= 0 && same < columns && same - k < rows ? same + 1 : kUnreached<V>;
                     const int32_t gapped = max(first_gap, second_gap);
                     // Ties as WFA2-lib's backtrace breaks them (gap_affine.mojo:984-1006): a substitution,
                     // then a letter of the first sequence alone before one of the second, and an extension
@@ -391,12 +464,12 @@ __global__ void __launch_bounds__(kWaveBlock) wavefront_kernel(WaveArgs a) {
                     if (opened_above > extended_above) flag |= kOpenedSecond;
                     if (!(substituted >= gapped)) flag |= first_gap >= second_gap ? kFirst : kSecond;
                     const int32_t start = max(substituted, gapped);
-                    value = start >= 0 ? slide(first, columns, second, rows, start, k, a.reversed) : kUnreached;
-                    aligned[width + (k - lo)] = first_gap;
-                    aligned[2 * width + (k - lo)] = second_gap;
+                    value = start >= 0 ? slide(a.letters, first, columns, second, rows, start, k, a.reversed) : kUnreached<V>;
+                    aligned[width + (k - lo)] = V(first_gap);
+                    aligned[2 * width + (k - lo)] = V(second_gap);
                     (reinterpret_cast<uint8_t *>(aligned + 3 * width))[k - lo] = flag;
                 }
-                aligned[k - lo] = value;
+                aligned[k - lo] = V(value);
                 if (k == target && value >= columns) hit = true;
             }
             used += bytes;
@@ -423,8 +496,8 @@ __global__ void __launch_bounds__(kWaveBlock) wavefront_kernel(WaveArgs a) {
                     out.slot = a.slots + a.slot_offsets[pair];
                     out.capacity = 2 * (int64_t(columns) + rows) + 8;
                     out.forward = a.reversed;
-                    const bool traced = EDIT ? trace_edit(a, arena, table, s, columns, rows, out)
-                                             : trace_affine(a, arena, table, s, columns, rows, out);
+                    const bool traced = EDIT ? trace_edit<V>(a, arena, table, s, columns, rows, out)
+                                             : trace_affine<V>(a, arena, table, s, columns, rows, out);
                     out.flush();
                     length = out.written;
                     if (!traced || out.overflow) {
@@ -436,6 +509,11 @@ __global__ void __launch_bounds__(kWaveBlock) wavefront_kernel(WaveArgs a) {
                 }
             }
             if (a.lengths) a.lengths[pair] = length;
+            // The pair's blocks back to the pool, once nothing reads them.
+            __threadfence();
+#pragma unroll
+            for (int b = 0; b < kBlocksAPair; ++b)
+                if (b < held_blocks) atomicAnd(a.blocks_taken + held[b] / 32, ~(1u << (held[b] & 31)));
         }
         __syncwarp();
     }
@@ -476,6 +554,8 @@ __global__ void wave_gather_kernel(const char *__restrict__ slots, const int64_t
     char *to = out + offsets[warp];
     for (int64_t i = lane; i < n; i += 32) to[i] = backwards ? from[n - 1 - i] : from[i];
 }
+
+using WaveFn = void (*)(WaveArgs);
 
 int64_t gcd(int64_t a, int64_t b) {
     while (b) {
@@ -551,6 +631,11 @@ int64_t cost_alignments(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, 
                                                           int(pairs), 0, 32, stream));
     int64_t slot_total = 0;
     read_back(gpu, &slot_total, slot_offsets + pairs, sizeof(int64_t));
+    uint32_t longest = 0;  // the longest pair's letters, and one
+    read_back(gpu, &longest, keys_sorted, sizeof longest);
+    const bool short_columns = int64_t(longest) <= kShortLetters;
+    WaveFn fn = plan.edit ? (short_columns ? &wavefront_kernel<true, int16_t> : &wavefront_kernel<true, int32_t>)
+                          : (short_columns ? &wavefront_kernel<false, int16_t> : &wavefront_kernel<false, int32_t>);
     char *slots = trace ? gpu->walk_out.ensure<char>(size_t(slot_total) + 8) : nullptr;
     int64_t *lengths = gpu->cigar_lengths.ensure<int64_t>(size_t(pairs) + 1);
     DINARA_CUDA(cudaMemsetAsync(lengths, 0, (size_t(pairs) + 1) * sizeof(int64_t), stream));
@@ -572,15 +657,20 @@ int64_t cost_alignments(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, 
     // with sixteen times the room on as many warps as the budget holds.
     int64_t arena_bytes = int64_t(256) << 10;
     const int64_t budget = int64_t(2) << 30;
-    const int64_t resident_warps = int64_t(gpu->multiprocessors) * (2048 / 32);
+    int per_sm = 0;
+    DINARA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kWaveBlock, 0));
+    const int64_t resident_warps = int64_t(gpu->multiprocessors) * std::max(per_sm, 1) * (kWaveBlock / 32);
     int rounds = 0;
     while (live > 0) {
         int64_t warps = std::min<int64_t>(resident_warps, budget / arena_bytes);
         warps = std::max<int64_t>(1, std::min<int64_t>(warps, live));
         const int64_t warps_per_block = kWaveBlock / 32;
         const int64_t blocks = (warps + warps_per_block - 1) / warps_per_block;
-        uint8_t *arena = gpu->wavefront.ensure<uint8_t>(size_t(blocks * warps_per_block * arena_bytes));
-        DINARA_CUDA(cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned int), stream));
+        // The first launch's pool: room for every pair's blocks, up to 1 GB in all.
+        const int64_t own_bytes = blocks * warps_per_block * arena_bytes;
+        const int64_t pool = rounds == 0 ? std::min<int64_t>(kMostBlocks, (kBlocksAPair * live + 31) / 32 * 32) : 0;
+        uint8_t *arena = gpu->wavefront.ensure<uint8_t>(size_t(own_bytes + pool * kBlockBytes));
+        DINARA_CUDA(cudaMemsetAsync(counters, 0, 64 * sizeof(unsigned int), stream));
         WaveArgs args;
         std::memset(&args, 0, sizeof args);
         args.letters = letters;
@@ -600,6 +690,9 @@ int64_t cost_alignments(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, 
         args.trace = trace;
         args.arena = arena;
         args.arena_bytes = arena_bytes;
+        args.blocks_at = own_bytes;
+        args.blocks_taken = pool > 0 ? counters + 16 : nullptr;
+        args.block_words = int32_t(pool / 32);
         args.table_entries = int32_t(std::min<int64_t>(arena_bytes / 16 / int64_t(sizeof(CostEntry)), INT32_MAX - 1));
         args.results = results;
         args.slot_offsets = slot_offsets;
@@ -608,10 +701,7 @@ int64_t cost_alignments(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, 
         args.retry = retry;
         args.retry_count = counters + 1;
         ClockSpan clock(gpu, kClassTrace, stream);
-        if (plan.edit)
-            wavefront_kernel<true><<<unsigned(blocks), kWaveBlock, 0, stream>>>(args);
-        else
-            wavefront_kernel<false><<<unsigned(blocks), kWaveBlock, 0, stream>>>(args);
+        fn<<<unsigned(blocks), kWaveBlock, 0, stream>>>(args);
         DINARA_CUDA(cudaGetLastError());
         clock.stop();
         gpu->launches += 1;

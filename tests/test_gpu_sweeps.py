@@ -153,3 +153,38 @@ def test_free_ends_and_extensions_at_the_widths(da, oracle, alphabet, entries):
             expected = [oracle.extension_alignment(a, b, table, size, op, ex, anchor == da.Anchor.END, bonus, zdrop=zdrop)
                         for a, b in coded]
             assert [(a.score, a.cigar, _span(a)) for a in found] == expected
+
+
+# ---- alignments under Costs: kept fronts in 16 bits, in 32 and in the shared blocks ---------------------------
+
+@pytest.mark.parametrize("letters", [31_998, 32_002])
+def test_fronts_either_side_of_16_bits(da, oracle, letters):
+    """A pair whose two sides hold 32,000 letters at most keeps 16-bit fronts, a longer one 32-bit: few edits, runs of
+    one letter at both ends (slides that meet the sequences' ends), both tie rules."""
+    rng = np.random.default_rng(letters)
+    half = letters // 2
+    source = "A" * 40 + _text(rng, half - 80) + "C" * 40
+    query = list(source)
+    for place in (3, half // 3, half // 2, half - 4):
+        query[place] = "G" if query[place] != "G" else "T"
+    refs, queries = [source, "ACGT" * 3], ["".join(query), "ACGT" * 2]
+    for costs, fields in ((da.Costs.affine(4, 6, 2), (4, 6, 2)), (da.Costs(), None)):
+        for ties in ("left", "right"):
+            found = da.alignments(refs, queries, costs, ties=ties)
+            for a, r, q in zip(found, refs, queries):
+                expected = (oracle.edit_cigar(r, q, right=ties == "right") if fields is None else
+                            oracle.affine_cigar(r, q, *fields, right=ties == "right"))
+                assert (a.cost, a.cigar) == expected
+
+
+def test_fronts_in_shared_blocks(da, oracle):
+    """Pairs whose fronts pass a warp's own arena, more of them than run at once without the shared blocks, among
+    short ones."""
+    rng = np.random.default_rng(41)
+    refs, queries = [], []
+    for trial in range(150):
+        source = _text(rng, 1500 if trial % 3 == 0 else 60)
+        refs.append(source)
+        queries.append(_mutated(rng, source, 0.14, "ACGT"))
+    found = da.alignments(refs, queries, da.Costs.affine(4, 6, 2))
+    assert [(a.cost, a.cigar) for a in found] == [oracle.affine_cigar(r, q, 4, 6, 2) for r, q in zip(refs, queries)]
