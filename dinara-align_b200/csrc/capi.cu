@@ -1860,15 +1860,11 @@ int64_t dinara_gpu_predictor_gradients(dinara_gpu *gpu, int64_t batch, const flo
         if (!gpu || !gpu->predictor_ready) throw Failure(DINARA_INVALID_MODE, "no parameters on this context");
         if (batch < 1 || batch > 65536) throw Failure(DINARA_INVALID_LENGTH, "a batch of 1 to 65,536 samples");
         DINARA_CUDA(cudaSetDevice(gpu->device));
-        std::vector<float> matrix(size_t(batch) * kPredictorInputs);
-        for (int64_t s = 0; s < batch; ++s)
-            for (int f = 0; f < kPredictorInputs; ++f)
-                matrix[size_t(int64_t(f) * batch + s)] = features[s * kPredictorInputs + f];
-        float *x = gpu->features.ensure<float>(matrix.size());
+        float *x = gpu->sketches.ensure<float>(size_t(batch) * kPredictorInputs);
         float *t = gpu->targets.ensure<float>(size_t(batch));
         float *g = gpu->gradients.ensure<float>(kPredictorParameters);
         float *l = gpu->counters.ensure<float>(64) + 60;
-        DINARA_CUDA(cudaMemcpyAsync(x, matrix.data(), matrix.size() * sizeof(float), cudaMemcpyHostToDevice, gpu->stream));
+        to_device(gpu, x, features, size_t(batch) * kPredictorInputs * sizeof(float), gpu->pinned_in);
         DINARA_CUDA(cudaMemcpyAsync(t, targets, size_t(batch) * sizeof(float), cudaMemcpyHostToDevice, gpu->stream));
         predictor_gradients(gpu, int(batch), x, t, g, l);
         float summed = 0.f;

@@ -391,7 +391,9 @@ void launch_features(dinara_gpu *gpu, const uint8_t *letters, const int64_t *off
 
 // C[m x n] (+)= op(A)[m x k] * op(B)[k x n], all row-major with leading dimensions; op transposes when
 // asked. A 64 x 64 tile a block of 256 threads, 4 x 4 outputs a thread, k in steps of 16 through shared
-// memory. `accumulate` adds to C; `bias` (length m) and `relu` finish the tile when given.
+// memory; an operand whose rows run along k is read 16 values of a row at a time, so a warp's reads are
+// whole sectors. `accumulate` adds to C; `bias` (length m) and `relu` finish the tile when given. Slice
+// blockIdx.z of gridDim.z takes its share of k into a C of its own, m * ldc apart (summed_kernel adds them).
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(256) product_kernel(int m, int n, int k, const float *A, int lda, const float *B,
                                                       int ldb, float *C, int ldc, const float *bias, bool relu,
@@ -401,17 +403,22 @@ __global__ void __launch_bounds__(256) product_kernel(int m, int n, int k, const
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
     const int row0 = blockIdx.y * 64, col0 = blockIdx.x * 64;
     float acc[4][4] = {{0.f}};
-    for (int kk = 0; kk < k; kk += 16) {
+    const int share = ((k + int(gridDim.z) - 1) / int(gridDim.z) + 15) & ~15;
+    const int k_begin = min(k, int(blockIdx.z) * share), k_end = min(k, k_begin + share);
+    C += int64_t(blockIdx.z) * m * ldc;
+    for (int kk = k_begin; kk < k_end; kk += 16) {
         for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-            const int kq = e / 64, i = e % 64;
-            const int r = row0 + i, kc = kk + kq;
+            // Consecutive threads along the operand's rows.
+            const int a_k = TA ? e / 64 : e % 16, a_i = TA ? e % 64 : e / 16;
+            const int r = row0 + a_i, a_kc = kk + a_k;
             float a = 0.f;
-            if (r < m && kc < k) a = TA ? A[int64_t(kc) * lda + r] : A[int64_t(r) * lda + kc];
-            As[kq][i] = a;
-            const int c = col0 + i;
+            if (r < m && a_kc < k_end) a = TA ? A[int64_t(a_kc) * lda + r] : A[int64_t(r) * lda + a_kc];
+            As[a_k][a_i] = a;
+            const int b_k = TB ? e % 16 : e / 64, b_i = TB ? e / 16 : e % 64;
+            const int c = col0 + b_i, b_kc = kk + b_k;
             float bv = 0.f;
-            if (c < n && kc < k) bv = TB ? B[int64_t(c) * ldb + kc] : B[int64_t(kc) * ldb + c];
-            Bs[kq][i] = bv;
+            if (c < n && b_kc < k_end) bv = TB ? B[int64_t(c) * ldb + b_kc] : B[int64_t(b_kc) * ldb + c];
+            Bs[b_k][b_i] = bv;
         }
         __syncthreads();
 #pragma unroll
@@ -451,6 +458,46 @@ void product(cudaStream_t stream, int m, int n, int k, const float *A, int lda, 
     dim3 grid(unsigned((n + 63) / 64), unsigned((m + 63) / 64));
     product_kernel<TA, TB><<<grid, 256, 0, stream>>>(m, n, k, A, lda, B, ldb, C, ldc, bias, relu, accumulate);
     DINARA_CUDA(cudaGetLastError());
+}
+
+// The sum of `slices` partial products of `count` values each, in the slices' order.
+__global__ void summed_kernel(const float *__restrict__ partial, int count, int slices, float *__restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    float sum = 0.f;
+    for (int z = 0; z < slices; ++z) sum += partial[int64_t(z) * count + i];
+    out[i] = sum;
+}
+
+// A weight gradient, A [m x k] times B [n x k] transposed into C [m x n], k the batch: its few tiles of the
+// output leave the GPU idle (five blocks for the first layer's, 530 us for 4,096 samples), so the batch is cut into
+// slices of 128 samples, a block a tile and slice, their partial sums kept apart and then added.
+constexpr int kSliceSamples = 128, kMostSlices = 32;
+void weight_gradient(cudaStream_t stream, int m, int n, int k, const float *A, int lda, const float *B, int ldb,
+                     float *partial, float *C) {
+    const int slices = std::min(kMostSlices, (k + kSliceSamples - 1) / kSliceSamples);
+    dim3 grid(unsigned((n + 63) / 64), unsigned((m + 63) / 64), unsigned(slices));
+    product_kernel<false, true><<<grid, 256, 0, stream>>>(m, n, k, A, lda, B, ldb, slices > 1 ? partial : C, n, nullptr,
+                                                        false, false);
+    DINARA_CUDA(cudaGetLastError());
+    if (slices == 1) return;
+    summed_kernel<<<(m * n + 255) / 256, 256, 0, stream>>>(partial, m * n, slices, C);
+    DINARA_CUDA(cudaGetLastError());
+}
+
+// Features pair-major (batch x kIn) to feature-major, 32 x 32 a block.
+__global__ void feature_major_kernel(const float *__restrict__ in, int batch, float *__restrict__ out) {
+    __shared__ float tile[32][33];
+    const int s0 = blockIdx.x * 32, f0 = blockIdx.y * 32;
+    for (int j = threadIdx.y; j < 32; j += 8) {
+        const int s = s0 + j, f = f0 + threadIdx.x;
+        if (s < batch && f < kIn) tile[j][threadIdx.x] = in[int64_t(s) * kIn + f];
+    }
+    __syncthreads();
+    for (int j = threadIdx.y; j < 32; j += 8) {
+        const int f = f0 + j, s = s0 + threadIdx.x;
+        if (s < batch && f < kIn) out[int64_t(f) * batch + s] = tile[threadIdx.x][j];
+    }
 }
 
 // The output layer and the loss: y = w3 . h2 + b3 for each sample; dy = 2 (y - target) / batch, and
@@ -641,7 +688,7 @@ constexpr int kW1 = 0, kB1 = kW1 + kIn * kH, kW2 = kB1 + kH, kB2 = kW2 + kH * kH
 void forward_backward(cudaStream_t stream, const float *params, const float *X, int ldx, const float *targets,
                       int batch, float *work, float *grads, float *loss) {
     float *h1 = work, *h2 = h1 + int64_t(kH) * batch, *y = h2 + int64_t(kH) * batch, *dy = y + batch;
-    float *dh2 = dy + batch, *dh1 = dh2 + int64_t(kH) * batch;
+    float *dh2 = dy + batch, *dh1 = dh2 + int64_t(kH) * batch, *partial = dh1 + int64_t(kH) * batch;
     // h1 = relu(W1^T X + b1): [kH x batch]; W1 is [kIn x kH] row-major, so op(A) = W1^T.
     product<true, false>(stream, kH, batch, kIn, params + kW1, kH, X, ldx, h1, batch, params + kB1, true);
     product<true, false>(stream, kH, batch, kH, params + kW2, kH, h1, batch, h2, batch, params + kB2, true);
@@ -650,7 +697,7 @@ void forward_backward(cudaStream_t stream, const float *params, const float *X, 
     output_backward_kernel<<<kH, 256, 0, stream>>>(h2, dy, batch, params + kW3, dh2, grads + kW3, grads + kB3);
     DINARA_CUDA(cudaGetLastError());
     // dW2[i][j] = sum_s h1[i][s] dh2[j][s]: [kH x kH] = h1 [kH x batch] * dh2^T.
-    product<false, true>(stream, kH, kH, batch, h1, batch, dh2, batch, grads + kW2, kH);
+    weight_gradient(stream, kH, kH, batch, h1, batch, dh2, batch, partial, grads + kW2);
     // db2: the rows of dh2.
     relu_backward_kernel<<<kH, 256, 0, stream>>>(h2, dh2, batch, grads + kB2);
     DINARA_CUDA(cudaGetLastError());
@@ -659,10 +706,10 @@ void forward_backward(cudaStream_t stream, const float *params, const float *X, 
     relu_backward_kernel<<<kH, 256, 0, stream>>>(h1, dh1, batch, grads + kB1);
     DINARA_CUDA(cudaGetLastError());
     // dW1[i][j] = sum_s X[i][s] dh1[j][s]: [kIn x kH].
-    product<false, true>(stream, kIn, kH, batch, X, ldx, dh1, batch, grads + kW1, kH);
+    weight_gradient(stream, kIn, kH, batch, X, ldx, dh1, batch, partial, grads + kW1);
 }
 
-size_t work_floats(int batch) { return size_t(batch) * (4 * kH + 2) + 64; }
+size_t work_floats(int batch) { return size_t(batch) * (4 * kH + 2) + size_t(kMostSlices) * kIn * kH + 64; }
 
 }  // namespace
 
@@ -680,8 +727,12 @@ void predictor_gradients(dinara_gpu *gpu, int batch, const float *features, cons
                          float *loss) {
     float *params = gpu->weights.as<float>();
     float *work = gpu->activations.ensure<float>(work_floats(batch));
+    float *columns = gpu->features.ensure<float>(size_t(batch) * kIn);
+    feature_major_kernel<<<dim3(unsigned(batch + 31) / 32, (kIn + 31) / 32), dim3(32, 8), 0, gpu->stream>>>(features, batch,
+                                                                                                       columns);
+    DINARA_CUDA(cudaGetLastError());
     DINARA_CUDA(cudaMemsetAsync(loss, 0, sizeof(float), gpu->stream));
-    forward_backward(gpu->stream, params, features, batch, targets, batch, work, grads, loss);
+    forward_backward(gpu->stream, params, columns, batch, targets, batch, work, grads, loss);
 }
 
 const int64_t *predict_thresholds(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const int64_t *offsets) {

@@ -188,3 +188,24 @@ def test_fronts_in_shared_blocks(da, oracle):
         queries.append(_mutated(rng, source, 0.14, "ACGT"))
     found = da.alignments(refs, queries, da.Costs.affine(4, 6, 2))
     assert [(a.cost, a.cigar) for a in found] == [oracle.affine_cigar(r, q, 4, 6, 2) for r, q in zip(refs, queries)]
+
+
+# ---- the predictor's gradients: the batch's slices -----------------------------------------------------------------
+
+@pytest.mark.parametrize("batch", [1, 31, 128, 129, 4096, 4097])
+def test_gradients_at_slice_edges(da, batch):
+    """Against 64 bits: an fp32 sum of `batch` products in slices is off by at most about (128 + 32) * 2^-24 of the sum
+    of their sizes, 1e-5; the sums here lie within ten times of their terms' sizes, so 1e-4 of the largest."""
+    import mlp_oracle
+    from dinara_align import learned
+
+    rng = np.random.default_rng(batch)
+    flat = rng.normal(0, 0.1, size=learned.PARAMETERS).astype(np.float32)
+    x = rng.normal(0, 0.5, size=(batch, learned.INPUTS)).astype(np.float32)
+    t = rng.uniform(0, 0.2, size=batch).astype(np.float32)
+    predictor = learned.Predictor()
+    predictor.install(flat, 1.0, 0.0)
+    got, loss = predictor.gradients(x, t)
+    expected, expected_loss = mlp_oracle.gradients(*(v.astype(np.float64) for v in (flat, x, t)))
+    np.testing.assert_allclose(got, expected, rtol=0, atol=1e-4 * np.abs(expected).max())
+    assert abs(loss - expected_loss) <= 1e-5 * expected_loss
