@@ -489,33 +489,71 @@ KernelFn pick_kernel(int cls, bool local, bool record, int bits, bool smem) {
 #undef DINARA_SHAPE
 }
 
-// The 16-bit pair score sweep for a whole-matrix shape class.
-KernelFn pick_pairs_kernel(int cls, bool local) {
-    switch (cls) {
-        case 0: return local ? &affine_pairs_kernel<4, 16, true> : &affine_pairs_kernel<4, 16, false>;
-        case 1: return local ? &affine_pairs_kernel<8, 16, true> : &affine_pairs_kernel<8, 16, false>;
-        case 2: return local ? &affine_pairs_kernel<16, 16, true> : &affine_pairs_kernel<16, 16, false>;
-        case 3: return local ? &affine_pairs_kernel<16, 20, true> : &affine_pairs_kernel<16, 20, false>;
-        default: return local ? &affine_pairs_kernel<32, 16, true> : &affine_pairs_kernel<32, 16, false>;
-    }
+// A 16-bit pair sweep's launch for a whole-matrix shape class: its kernel, its lanes and columns a lane, and the
+// threads and shared memory of a block. A profile form (8-bit letters) keeps 64 bytes a letter and column of a lane
+// for each warp, so its blocks are of four warps: two of them an SM under a 20-letter alphabet.
+struct PairsLaunch {
+    KernelFn fn;
+    int lanes, columns, threads;
+    size_t shared;
+};
+
+PairsLaunch pairs_launch(KernelFn two_bits, KernelFn bytes, int bits, int lanes, int columns, int letters) {
+    if (bits == 8) return {bytes, lanes, columns, kBlock / 2, size_t(kBlock / 64) * 64 * letters * columns};
+    return {two_bits, lanes, columns, kBlock, 0};
 }
 
-// The same keeping each hit's rows (local).
-KernelFn pick_hits_kernel(int cls) {
+// Scores, or (`hits`, local) each hit's rows. The 20-column shape is the two-bit form's alone.
+PairsLaunch pick_pairs(int cls, bool local, bool hits, int bits, int letters) {
+#define DINARA_PAIRS(G, C, G8)                                                                                       \
+    return pairs_launch(hits    ? &affine_pairs_kernel<G, C, true, true>                                             \
+                        : local ? &affine_pairs_kernel<G, C, true>                                                   \
+                                : &affine_pairs_kernel<G, C, false>,                                                 \
+                        hits    ? &affine_pairs_kernel<G8, 16, true, true, 8>                                        \
+                        : local ? &affine_pairs_kernel<G8, 16, true, false, 8>                                       \
+                                : &affine_pairs_kernel<G8, 16, false, false, 8>,                                     \
+                        bits, bits == 8 ? G8 : G, bits == 8 ? 16 : C, letters);
     switch (cls) {
-        case 0: return &affine_pairs_kernel<4, 16, true, true>;
-        case 1: return &affine_pairs_kernel<8, 16, true, true>;
-        case 2: return &affine_pairs_kernel<16, 16, true, true>;
-        case 3: return &affine_pairs_kernel<16, 20, true, true>;
-        default: return &affine_pairs_kernel<32, 16, true, true>;
+        case 0: DINARA_PAIRS(4, 16, 4)
+        case 1: DINARA_PAIRS(8, 16, 8)
+        case 2: DINARA_PAIRS(16, 16, 16)
+        case 3: DINARA_PAIRS(16, 20, 32)
+        default: DINARA_PAIRS(32, 16, 32)
     }
+#undef DINARA_PAIRS
 }
 
-int persistent_blocks(dinara_gpu *gpu, KernelFn fn) {
+int persistent_blocks(dinara_gpu *gpu, KernelFn fn, int threads = kBlock, size_t shared = 0) {
     int per_sm = 0;
-    DINARA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kBlock, 0));
+    if (shared > (size_t(48) << 10))
+        DINARA_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shared)));
+    DINARA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, shared));
     if (per_sm < 1) per_sm = 1;
     return per_sm * gpu->multiprocessors;
+}
+
+// Launches a 16-bit pair sweep over items [begin, end) of `args.order`, its carry slots one a lane group, each as
+// long as the tallest pair, where pairs may be wider than a strip.
+void launch_pairs(dinara_gpu *gpu, const AffineBatch &batch, const PairsLaunch &sweep, KernelArgs args,
+                  const TableArgs &targs, const int32_t *table32, int64_t begin, int64_t end) {
+    if (end <= begin) return;
+    const int64_t groups = sweep.threads / sweep.lanes;
+    const int64_t needed = (end - begin + 2 * groups - 1) / (2 * groups);
+    const int64_t blocks =
+        std::max<int64_t>(1, std::min<int64_t>(persistent_blocks(gpu, sweep.fn, sweep.threads, sweep.shared), needed));
+    args.carry = nullptr;
+    args.carry_stride = 0;
+    if (batch.max_columns > uint32_t(sweep.lanes * sweep.columns)) {
+        args.carry_stride = int64_t(batch.max_rows) + 1;
+        args.carry = gpu->carry.ensure<int2>(size_t(blocks * groups * args.carry_stride));
+    }
+    args.begin = uint32_t(begin);
+    args.end = uint32_t(end);
+    ClockSpan clock(gpu, kClassWhole, gpu->stream);
+    sweep.fn<<<unsigned(blocks), sweep.threads, sweep.shared, gpu->stream>>>(args, targs, table32);
+    DINARA_CUDA(cudaGetLastError());
+    clock.stop();
+    gpu->launches += 1;
 }
 
 TableArgs table_args(const AffineTable &table, bool local) {
@@ -782,19 +820,23 @@ void affine_launch_all(dinara_gpu *gpu, const AffineBatch &batch, const AffineTa
             widening_band(gpu, batch, table, schedule.order + b.begin[bucket], b.end[bucket] - b.begin[bucket], args);
             continue;
         }
+        if (pairs16) {
+            launch_pairs(gpu, batch, pick_pairs(cls, batch.local, false, batch.bits, table.size), args, targs, table32,
+                         b.begin[bucket], b.end[bucket]);
+            continue;
+        }
         KernelFn fn = band_record ? &affine_kernel<32, 16, false, true, 2, false, false, true>
                       : wide      ? (batch.local ? &affine_wide_kernel<true, false> : &affine_wide_kernel<false, false>)
-                      : pairs16   ? pick_pairs_kernel(cls, batch.local)
                                   : pick_kernel(cls, batch.local, record, batch.bits, smem);
-        const int G = wide ? kBlock : (smem && !pairs16) || band_record ? 32 : affine_lanes(cls);
-        const int groups_per_block = (pairs16 ? 2 : 1) * kBlock / G;
+        const int G = wide ? kBlock : smem || band_record ? 32 : affine_lanes(cls);
+        const int groups_per_block = kBlock / G;
         int64_t blocks = persistent_blocks(gpu, fn);
         const int64_t needed = (b.end[bucket] - b.begin[bucket] + groups_per_block - 1) / groups_per_block;
         if (blocks > needed) blocks = needed;
         if (blocks < 1) blocks = 1;
         // Carry slots, one a group, each as long as the tallest pair: only a launch whose pairs may be
         // wider than one strip reads them.
-        const int width = wide ? 16 * kBlock : (smem && !pairs16) || band_record ? 512 : affine_lanes(cls) * affine_columns(cls);
+        const int width = wide ? 16 * kBlock : smem || band_record ? 512 : affine_lanes(cls) * affine_columns(cls);
         args.carry = nullptr;
         args.carry_stride = 0;
         if (batch.max_columns > uint32_t(width)) {
@@ -827,15 +869,15 @@ int32_t pair_limit_of(const AffineTable &table) {
 }
 
 // Which whole-matrix pairs the 16-bit pair score sweep takes (a table of up to four letters on the 2-bit
-// tape): locally, a cell held less row x extend reaches at most the best entry times the columns swept
+// tape, or a larger one through profiles): locally, a cell held less row x extend reaches at most the best entry times the columns swept
 // plus the rows times -extend and falls no lower than a gap's first letter, so that sum is held to half of
 // 30,000 less the gaps;
 // globally, a shifted cell moves at most the largest step a cell, so rows and swept columns are each held
 // to half of 30,000 over it, every value within 30,000 of zero. Entries must fit a byte (shifted, globally).
 PairLimits whole_limits_of(const AffineBatch &batch, const AffineTable &table) {
     PairLimits limits;
-    if (batch.bits != 2 || !table.packed16) return limits;
-    limits.wide = 1;
+    if (batch.bits == 2 && !table.packed16) return limits;
+    limits.wide = batch.bits == 2 ? 1 : 0;
     limits.long_strips = long_serves(batch, table) ? 1 : 0;
     const int32_t gaps = std::abs(table.open) + std::abs(table.extend);
     if (gaps > 8000) return limits;
@@ -1106,14 +1148,13 @@ __global__ void extension_finish_kernel(const PairShape *__restrict__ shapes, in
         for (int j = 0; j < 4; ++j) spans[4 * k + j] = span[j];
 }
 
-// Which pairs the 16-bit free-end sweep takes (a table of up to four letters on the 2-bit tape, its shifted
-// entries a byte): a shifted cell reaches at most the best entry times the columns swept plus the rows and
+// Which pairs the 16-bit free-end sweeps take (a table whose shifted entries fit a byte): a shifted cell reaches at most the best entry times the columns swept plus the rows and
 // columns swept times -extend, held to half of 30,000 less the gaps for the sum of a group's two pairs, and
 // falls at most a few gap openings below zero.
 PairLimits free_limits_of(const AffineBatch &batch, const AffineTable &table) {
     PairLimits limits;
     const int32_t gaps = std::abs(table.open) + std::abs(table.extend);
-    if (batch.bits != 2 || !table.packed16 || gaps > 2000) return limits;
+    if ((batch.bits == 2 && !table.packed16) || gaps > 2000) return limits;
     int32_t best = 1;
     for (int r = 0; r < table.size; ++r)
         for (int c = 0; c < table.size; ++c) {
@@ -1128,58 +1169,56 @@ PairLimits free_limits_of(const AffineBatch &batch, const AffineTable &table) {
     return limits;
 }
 
-// An extension's sweep takes eight places a lane, twice a class's lanes at most.
-KernelFn pick_extension_kernel(int cls) {
+// Their launches. An extension's sweep takes eight places a lane, so twice a class's lanes, 32 at most.
+PairsLaunch pick_free(int cls, int bits, int letters) {
+#define DINARA_FREE(G, C, G8) \
+    return pairs_launch(&free_pairs_kernel<G, C>, &free_pairs_kernel<G8, 16, 8>, bits, bits == 8 ? G8 : G, bits == 8 ? 16 : C, letters);
     switch (cls) {
-        case 0: return &extension_pairs_kernel<8, 8>;
-        case 1: return &extension_pairs_kernel<16, 8>;
-        default: return &extension_pairs_kernel<32, 8>;
+        case 0: DINARA_FREE(4, 16, 4)
+        case 1: DINARA_FREE(8, 16, 8)
+        case 2: DINARA_FREE(16, 16, 16)
+        case 3: DINARA_FREE(16, 20, 32)
+        default: DINARA_FREE(32, 16, 32)
     }
+#undef DINARA_FREE
 }
 
-KernelFn pick_free_kernel(int cls) {
+PairsLaunch pick_extension(int cls, int bits, int letters) {
+#define DINARA_EXTENSION_SWEEP(G) \
+    return pairs_launch(&extension_pairs_kernel<G, 8>, &extension_pairs_kernel<G, 8, 8>, bits, G, 8, letters);
     switch (cls) {
-        case 0: return &free_pairs_kernel<4, 16>;
-        case 1: return &free_pairs_kernel<8, 16>;
-        case 2: return &free_pairs_kernel<16, 16>;
-        case 3: return &free_pairs_kernel<16, 20>;
-        default: return &free_pairs_kernel<32, 16>;
+        case 0: DINARA_EXTENSION_SWEEP(8)
+        case 1: DINARA_EXTENSION_SWEEP(16)
+        default: DINARA_EXTENSION_SWEEP(32)
     }
+#undef DINARA_EXTENSION_SWEEP
 }
 
 // One free-end sweep of a scheduled batch: the 16-bit classes' pairs, then the rest in 32 bits.
-void launch_free(dinara_gpu *gpu, const AffineBatch &batch, const Schedule &order, KernelFn general, KernelArgs args,
-                 const TableArgs &targs, const int32_t *table32) {
+void launch_free(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, const Schedule &order,
+                 KernelFn general, KernelArgs args, const TableArgs &targs, const int32_t *table32) {
     const Buckets b = buckets_of(order);
-    auto launch = [&](KernelFn fn, int lanes, int width, int pairs_a_group, int64_t begin, int64_t end) {
-        if (end <= begin) return;
-        const int64_t per_block = int64_t(pairs_a_group) * kBlock / lanes;
-        const int64_t blocks =
-            std::max<int64_t>(1, std::min<int64_t>(persistent_blocks(gpu, fn), (end - begin + per_block - 1) / per_block));
-        args.carry = nullptr;
-        args.carry_stride = 0;
-        if (batch.max_columns > uint32_t(width)) {
-            args.carry_stride = int64_t(batch.max_rows) + 1;
-            args.carry = gpu->carry.ensure<int2>(size_t(blocks * (kBlock / lanes) * args.carry_stride));
-        }
-        args.begin = uint32_t(begin);
-        args.end = uint32_t(end);
-        ClockSpan clock(gpu, kClassWhole, gpu->stream);
-        fn<<<dim3(unsigned(blocks)), kBlock, 0, gpu->stream>>>(args, targs, table32);
-        DINARA_CUDA(cudaGetLastError());
-        clock.stop();
-        gpu->launches += 1;
-    };
-    for (int cls = kAffineShapes - 1; cls >= 0; --cls) {
-        const int64_t begin = b.begin[kWholePairsClass + cls], end = b.end[kWholePairsClass + cls];
-        if (batch.extension) {
-            const int lanes = std::min(2 * affine_lanes(cls), 32);
-            launch(pick_extension_kernel(cls), lanes, 8 * lanes, 2, begin, end);
-        } else {
-            launch(pick_free_kernel(cls), affine_lanes(cls), affine_lanes(cls) * affine_columns(cls), 2, begin, end);
-        }
+    for (int cls = kAffineShapes - 1; cls >= 0; --cls)
+        launch_pairs(gpu, batch,
+                     batch.extension ? pick_extension(cls, batch.bits, table.size) : pick_free(cls, batch.bits, table.size),
+                     args, targs, table32, b.begin[kWholePairsClass + cls], b.end[kWholePairsClass + cls]);
+    const int64_t begin = b.begin[kAffineShapes - 1], end = b.end[0];
+    if (end <= begin) return;
+    const int64_t blocks = std::max<int64_t>(
+        1, std::min<int64_t>(persistent_blocks(gpu, general), (end - begin + kBlock / 32 - 1) / (kBlock / 32)));
+    args.carry = nullptr;
+    args.carry_stride = 0;
+    if (batch.max_columns > 512u) {
+        args.carry_stride = int64_t(batch.max_rows) + 1;
+        args.carry = gpu->carry.ensure<int2>(size_t(blocks * (kBlock / 32) * args.carry_stride));
     }
-    launch(general, 32, 512, 1, b.begin[kAffineShapes - 1], b.end[0]);
+    args.begin = uint32_t(begin);
+    args.end = uint32_t(end);
+    ClockSpan clock(gpu, kClassWhole, gpu->stream);
+    general<<<dim3(unsigned(blocks)), kBlock, 0, gpu->stream>>>(args, targs, table32);
+    DINARA_CUDA(cudaGetLastError());
+    clock.stop();
+    gpu->launches += 1;
 }
 
 // Global scores with free ends: pairs whose values fit it in the 16-bit pair sweep (free_limits_of), the rest
@@ -1296,7 +1335,7 @@ void free_end_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTabl
         DINARA_CUDA(cudaGetLastError());
         gpu->launches += 1;
     } else {
-        launch_free(gpu, batch, order, fn, args, targs, table32);
+        launch_free(gpu, batch, table, order, fn, args, targs, table32);
     }
     if (batch.extension) {
         extension_finish_kernel<<<unsigned((count * 32 + 255) / 256), 256, 0, gpu->stream>>>(
@@ -1323,7 +1362,7 @@ void free_end_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTabl
             back.free_reference_end = batch.free_reference_start;
             back.free_query_start = 0;
             back.free_query_end = batch.free_query_start;
-            launch_free(gpu, batch, order, fn, back, targs, table32);
+            launch_free(gpu, batch, table, order, fn, back, targs, table32);
         }
         free_spans_kernel<<<pair_blocks, 256, 0, gpu->stream>>>(ends, origin_starts ? ends : ends + count, count, spans);
         DINARA_CUDA(cudaGetLastError());
@@ -1350,6 +1389,8 @@ const PairShape *hit_shapes(dinara_gpu *gpu, const AffineBatch &batch, const Aff
         DINARA_CUDA(cudaMemcpyAsync(hits + first, batch.shapes + first, size_t(count) * sizeof(PairShape),
                                     cudaMemcpyDeviceToDevice, gpu->stream));
     const TableArgs targs = table_args(table, true);
+    int32_t *table32 = nullptr;
+    if (batch.bits == 8) upload_table32(gpu, table, true, &table32);
     KernelArgs args;
     std::memset(&args, 0, sizeof args);
     args.tape = batch.tape;
@@ -1362,28 +1403,9 @@ const PairShape *hit_shapes(dinara_gpu *gpu, const AffineBatch &batch, const Aff
     args.best_entry = limits.best;
     const Buckets b = buckets_of(order);
     PhaseTimer timer(gpu, &gpu->record_ms);
-    for (int cls = kAffineShapes - 1; cls >= 0; --cls) {
-        const int bucket = kWholePairsClass + cls;
-        const int64_t pairs = b.end[bucket] - b.begin[bucket];
-        if (pairs <= 0) continue;
-        KernelFn fn = pick_hits_kernel(cls);
-        const int groups_per_block = kBlock / affine_lanes(cls);
-        const int64_t needed = (pairs + 2 * groups_per_block - 1) / (2 * groups_per_block);
-        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(persistent_blocks(gpu, fn), needed));
-        args.carry = nullptr;
-        args.carry_stride = 0;
-        if (batch.max_columns > uint32_t(affine_lanes(cls) * affine_columns(cls))) {
-            args.carry_stride = int64_t(batch.max_rows) + 1;
-            args.carry = gpu->carry.ensure<int2>(size_t(blocks * groups_per_block * args.carry_stride));
-        }
-        args.begin = uint32_t(b.begin[bucket]);
-        args.end = uint32_t(b.end[bucket]);
-        ClockSpan clock(gpu, kClassWhole, gpu->stream);
-        fn<<<unsigned(blocks), kBlock, 0, gpu->stream>>>(args, targs, nullptr);
-        DINARA_CUDA(cudaGetLastError());
-        clock.stop();
-        gpu->launches += 1;
-    }
+    for (int cls = kAffineShapes - 1; cls >= 0; --cls)
+        launch_pairs(gpu, batch, pick_pairs(cls, true, true, batch.bits, table.size), args, targs, table32,
+                     b.begin[kWholePairsClass + cls], b.end[kWholePairsClass + cls]);
     timer.stop();
     return hits;
 }

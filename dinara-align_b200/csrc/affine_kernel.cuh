@@ -590,25 +590,81 @@ __device__ __forceinline__ uint32_t pair_selector(uint32_t a, uint32_t b) { retu
 __device__ __forceinline__ uint32_t half_selector_a(uint32_t y) { return 17u * y + 128u; }
 __device__ __forceinline__ uint32_t half_selector_b(uint32_t y) { return 17u * y + 196u; }
 
+// Alphabets of more than four letters (a byte a letter): a pair's query profile in shared memory, each letter's
+// entries against a lane's C columns as C bytes, so that a row's substitutions are one read a pair and the permutes
+// that spread them over the halves are the two-bit form's, with fixed selectors. A lane reads only what it wrote.
+extern __shared__ uint4 sweep_profiles[];
+
+template <int C>
+struct __align__(C % 16 == 0 ? 16 : C % 8 == 0 ? 8 : 4) ProfileRow {
+    uint32_t words[C / 4];
+};
+
+// Writes a lane's part of a profile: for each of the alphabet's `letters`, its entries against the letters
+// `letter_of(k)` of the lane's first `owned` columns, zero past them. Letter a's part is profile[a * stride].
+template <int C, class L>
+__device__ __forceinline__ void fill_profile(ProfileRow<C> *profile, int stride, int letters, const int8_t *table8,
+                                             int owned, L &&letter_of) {
+    uint32_t columns[C / 4];
+#pragma unroll
+    for (int j = 0; j < C / 4; ++j) {
+        columns[j] = 0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            if (4 * j + b < owned) columns[j] |= letter_of(4 * j + b) << (8 * b);
+    }
+    for (int a = 0; a < letters; ++a) {
+        ProfileRow<C> row;
+#pragma unroll
+        for (int j = 0; j < C / 4; ++j) {
+            uint32_t word = 0;
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+                if (4 * j + b < owned)
+                    word |= uint32_t(uint8_t(table8[32 * a + ((columns[j] >> (8 * b)) & 31u)])) << (8 * b);
+            row.words[j] = word;
+        }
+        profile[a * stride] = row;
+    }
+}
+
+// Column k's substitutions of both pairs from a row's profile words: byte k % 4 of each, sign-extended.
+template <int C>
+__device__ __forceinline__ uint32_t profile_entry(const ProfileRow<C> &a, const ProfileRow<C> &b, int k) {
+    return uint32_t(prmt(a.words[k / 4], b.words[k / 4],
+                         pair_selector(half_selector_a(uint32_t(k % 4)), half_selector_b(uint32_t(k % 4)))));
+}
+
+// Copies a launch's table (32 rows of 33 entries, device) to the block's bytes, each less `less`.
+__device__ __forceinline__ void load_table8(int8_t *table8, const int32_t *__restrict__ table32, int32_t less) {
+    for (int i = threadIdx.x; i < 32 * 32; i += blockDim.x) table8[i] = int8_t(table32[i / 32 * 33 + i % 32] - less);
+}
+
 // With TRACK (local), each half's best keeps the first row that reaches it (a strict rise moves it, a rare branch:
 // a hit raises its lane's best about once a row), and the pair's shape cut to its hit's rows goes to p.hits. A
 // local alignment then records those rows alone: every optimal path to the hit's end starts within them, so
 // along the walked path each cell is the whole matrix's and every other cell at most its own, and each
 // decision comes out the same.
-template <int G, int C, bool LOCAL, bool TRACK = false>
-__global__ void __launch_bounds__(kBlock) affine_pairs_kernel(KernelArgs p, TableArgs t, const int32_t *__restrict__) {
+template <int G, int C, bool LOCAL, bool TRACK = false, int BITS = 2>
+__global__ void __launch_bounds__(kBlock, 2) affine_pairs_kernel(KernelArgs p, TableArgs t, const int32_t *__restrict__ table32) {
     static_assert(LOCAL || !TRACK, "hits are local");
     constexpr int W = G * C;
     constexpr int GPW = 32 / G;
+    constexpr bool PROFILE = BITS == 8;
     __shared__ uint32_t rows8[4];
+    __shared__ int8_t table8[PROFILE ? 32 * 32 : 1];
     if (threadIdx.x < 4) rows8[threadIdx.x] = t.rows8[threadIdx.x];
+    if (PROFILE) load_table8(table8, table32, LOCAL ? p.extend : 0);
     __syncthreads();
 
     const int lane = threadIdx.x & 31;
     const int member = lane % G;
     const int group = lane / G;
-    const int warp = int((int64_t(blockIdx.x) * kBlock + threadIdx.x) >> 5);
-    const int warps = int((int64_t(gridDim.x) * kBlock) >> 5);
+    const int warp = int((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
+    const int warps = int((int64_t(gridDim.x) * blockDim.x) >> 5);
+    // This lane's part of its group's two profiles, letter a's of half h at [(h * t.size + a) * G].
+    ProfileRow<C> *profile = reinterpret_cast<ProfileRow<C> *>(sweep_profiles) +
+                             int64_t((threadIdx.x >> 5) * GPW + group) * 2 * t.size * G + member;
     const int32_t open = p.open, extend = p.extend;
     const int32_t opening = open - extend;
     const int32_t first_gap = open + extend;
@@ -649,9 +705,17 @@ __global__ void __launch_bounds__(kBlock) affine_pairs_kernel(KernelArgs p, Tabl
 #pragma unroll
             for (int h = 0; h < 2; ++h) strip_live[h] = s < strips[h];
             const int first_col = s * W + member * C;
-            uint32_t sel[C];
+            uint32_t sel[PROFILE ? 1 : C];
+            if (PROFILE) {
 #pragma unroll
-            for (int k = 0; k < C; ++k) {
+                for (int h = 0; h < 2; ++h)
+                    fill_profile<C>(profile + h * t.size * G, G, t.size, table8,
+                                    strip_live[h] ? min(max(cols[h] - first_col, 0), C) : 0, [&](int k) {
+                                        return letter_at<8>(p.tape, sh[h].second_word, uint32_t(first_col + k));
+                                    });
+            }
+#pragma unroll
+            for (int k = 0; k < (PROFILE ? 0 : C); ++k) {
                 const int col = first_col + k;
                 const uint32_t a = strip_live[0] && col < cols[0]
                                        ? half_selector_a(letter_at<2>(p.tape, sh[0].second_word, uint32_t(col)))
@@ -698,15 +762,25 @@ __global__ void __launch_bounds__(kBlock) affine_pairs_kernel(KernelArgs p, Tabl
                 above_left = leftH;
                 if (row >= 1 && row <= group_rows) {
                     uint32_t tr[2];
+                    ProfileRow<C> entries[PROFILE ? 2 : 1];
 #pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        tr[h] = strip_live[h] && row <= rows[h]
-                                    ? rows8[letter_at<2>(p.tape, sh[h].first_word, uint32_t(row - 1))]
-                                    : 0u;
+                    for (int h = 0; h < 2; ++h) {
+                        const bool inside = strip_live[h] && row <= rows[h];
+                        const uint32_t letter =
+                            PROFILE ? (inside ? letter_at<BITS>(p.tape, sh[h].first_word, uint32_t(row - 1)) : 0u)
+                                    : (inside ? letter_at<BITS>(p.tape, sh[h].first_word, uint32_t(row - 1)) : 0u);
+                        if (PROFILE) {
+                            entries[h] = profile[int(h * t.size + letter) * G];
+                            if (!inside) entries[h] = ProfileRow<C>{};
+                        } else {
+                            tr[h] = inside ? rows8[letter] : 0u;
+                        }
+                    }
                     uint32_t I = 0, Xprev = 0;
 #pragma unroll
                     for (int k = 0; k < C; ++k) {
-                        const uint32_t sub = uint32_t(prmt(tr[0], tr[1], sel[k]));
+                        const uint32_t sub = PROFILE ? profile_entry(entries[0], entries[PROFILE ? 1 : 0], k)
+                                                     : uint32_t(prmt(tr[0], tr[1], sel[PROFILE ? 0 : k]));
                         const uint32_t Hup = H[k], Dup = D[k];
                         uint32_t Dn, X, Hn;
                         Dn = __viaddmax_s16x2(Hup, LOCAL ? open_less_extend2 : opening2, Dup);
@@ -797,7 +871,7 @@ __global__ void __launch_bounds__(kBlock) affine_pairs_kernel(KernelArgs p, Tabl
                     // No hit (a best of 0) leaves no row to record.
                     const int first = hit_first_row(hit_row[h], cols[h], hit[h], p.best_entry, open, extend);
                     PairShape cut = sh[h];
-                    cut.first_word += uint32_t(first / 16);
+                    cut.first_word += uint32_t(first / (32 / BITS));
                     cut.rows = hit[h] > 0 ? uint32_t(hit_row[h] - first) : 0u;
                     p.hits[pair[h]] = cut;
                 }

@@ -37,19 +37,25 @@ __device__ __forceinline__ uint32_t sixteen_rows(const uint32_t *__restrict__ ta
 //
 // 16 places a lane move 32 cells in 96 DPX, permute and logic instructions, where the 32-bit form takes 80 for
 // 16 cells and a shared-memory read a cell.
-template <int G, int C>
-__global__ void __launch_bounds__(kBlock, 2) free_pairs_kernel(KernelArgs p, TableArgs t, const int32_t *__restrict__) {
+template <int G, int C, int BITS = 2>
+__global__ void __launch_bounds__(kBlock, 2) free_pairs_kernel(KernelArgs p, TableArgs t, const int32_t *__restrict__ table32) {
     constexpr int W = G * C;
     constexpr int GPW = 32 / G;
+    constexpr bool PROFILE = BITS == 8;
     __shared__ uint32_t rows8[4];
+    __shared__ int8_t table8[PROFILE ? 32 * 32 : 1];
     if (threadIdx.x < 4) rows8[threadIdx.x] = t.rows8[threadIdx.x];
+    if (PROFILE) load_table8(table8, table32, 0);
     __syncthreads();
 
     const int lane = threadIdx.x & 31;
     const int member = lane % G;
     const int group = lane / G;
-    const int warp = int((int64_t(blockIdx.x) * kBlock + threadIdx.x) >> 5);
-    const int warps = int((int64_t(gridDim.x) * kBlock) >> 5);
+    const int warp = int((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
+    const int warps = int((int64_t(gridDim.x) * blockDim.x) >> 5);
+    // This lane's part of its group's two profiles, letter a's of half h at [(h * t.size + a) * G].
+    ProfileRow<C> *profile = reinterpret_cast<ProfileRow<C> *>(sweep_profiles) +
+                             int64_t((threadIdx.x >> 5) * GPW + group) * 2 * t.size * G + member;
     const int32_t open = p.open, extend = p.extend;
     const int32_t opening = open - extend;
     const int32_t first_gap = open + extend;
@@ -102,7 +108,17 @@ __global__ void __launch_bounds__(kBlock, 2) free_pairs_kernel(KernelArgs p, Tab
 
         for (int s = 0; s < warp_strips; ++s) {
             const int first = s * W + member * C;
-            uint32_t sel[C], last[C];
+            uint32_t sel[PROFILE ? 1 : C], last[C];
+            if (PROFILE) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    fill_profile<C>(profile + h * t.size * G, G, t.size, table8,
+                                    s < strips[h] ? min(max(cols[h] - first, 0), C) : 0, [&](int k) {
+                                        const int col = first + k;
+                                        return letter_at<8>(p.tape, sh[h].second_word,
+                                                            uint32_t(backwards ? cols[h] - 1 - col : col));
+                                    });
+            }
 #pragma unroll
             for (int k = 0; k < C; ++k) {
                 uint32_t half_sel[2] = {kPadHalf, kPadHalf}, half_last[2] = {0, 0};
@@ -110,13 +126,15 @@ __global__ void __launch_bounds__(kBlock, 2) free_pairs_kernel(KernelArgs p, Tab
                 for (int h = 0; h < 2; ++h) {
                     const int col = first + k;
                     if (s < strips[h] && col < cols[h]) {
-                        const uint32_t y =
-                            letter_at<2>(p.tape, sh[h].second_word, uint32_t(backwards ? cols[h] - 1 - col : col));
-                        half_sel[h] = h == 0 ? half_selector_a(y) : half_selector_b(y);
+                        if (!PROFILE) {
+                            const uint32_t y =
+                                letter_at<2>(p.tape, sh[h].second_word, uint32_t(backwards ? cols[h] - 1 - col : col));
+                            half_sel[h] = h == 0 ? half_selector_a(y) : half_selector_b(y);
+                        }
                         if (col == cols[h] - 1) half_last[h] = 0xFFFFu;
                     }
                 }
-                sel[k] = pair_selector(half_sel[0], half_sel[1]);
+                if (!PROFILE) sel[PROFILE ? 0 : k] = pair_selector(half_sel[0], half_sel[1]);
                 last[k] = half_last[0] | (half_last[1] << 16);
             }
             bool holds_last[2];
@@ -142,18 +160,33 @@ __global__ void __launch_bounds__(kBlock, 2) free_pairs_kernel(KernelArgs p, Tab
             const int warp_steps = warp_max(steps);
 
             for (int step0 = 1; step0 <= warp_steps; step0 += 16) {
-                uint32_t codes[2];
+                uint32_t codes[2] = {0, 0};
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
+                for (int h = 0; h < (PROFILE ? 0 : 2); ++h)
                     codes[h] = sixteen_rows(p.tape, sh[h].first_word, live[h] ? rows[h] : 0, step0 - member, backwards);
 #pragma unroll 2
                 for (int u = 0; u < 16; ++u) {
                     const int row = step0 + u - member;
                     uint32_t leftH = __shfl_up_sync(kFull, edgeH, 1, G);
                     uint32_t leftI = __shfl_up_sync(kFull, edgeI, 1, G);
-                    const uint32_t trA = rows8[codes[0] & 3u], trB = rows8[codes[1] & 3u];
-                    codes[0] >>= 2;
-                    codes[1] >>= 2;
+                    uint32_t trA = 0, trB = 0;
+                    ProfileRow<C> entries[PROFILE ? 2 : 1];
+                    if (PROFILE) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            // A row outside the pair reads its nearest letter: no cell that counts uses it.
+                            const int r = min(max(row, 1), max(rows[h], 1));
+                            const uint32_t letter =
+                                s < strips[h] ? letter_at<8>(p.tape, sh[h].first_word, uint32_t(backwards ? rows[h] - r : r - 1))
+                                              : 0u;
+                            entries[PROFILE ? h : 0] = profile[int(h * t.size + letter) * G];
+                        }
+                    } else {
+                        trA = rows8[codes[0] & 3u];
+                        trB = rows8[codes[1] & 3u];
+                        codes[0] >>= 2;
+                        codes[1] >>= 2;
+                    }
                     if (member == 0) {
                         if (s == 0) {
                             const int r = max(row, 0);
@@ -174,7 +207,8 @@ __global__ void __launch_bounds__(kBlock, 2) free_pairs_kernel(KernelArgs p, Tab
                         uint32_t I = leftI, left = leftH, last_column = 0;
 #pragma unroll
                         for (int k = 0; k < C; ++k) {
-                            const uint32_t sub = uint32_t(prmt(trA, trB, sel[k]));
+                            const uint32_t sub = PROFILE ? profile_entry(entries[0], entries[PROFILE ? 1 : 0], k)
+                                                         : uint32_t(prmt(trA, trB, sel[PROFILE ? 0 : k]));
                             const uint32_t Hup = H[k];
                             const uint32_t Dn = __viaddmax_s16x2(Hup, opening2, D[k]);
                             const uint32_t X = __viaddmax_s16x2(diag, sub, Dn);
@@ -258,8 +292,9 @@ __global__ void __launch_bounds__(kBlock, 2) free_pairs_kernel(KernelArgs p, Tab
 // A row's key is bits 16-31 the cell, shifted as held, bits 0-15 the row; on one anti-diagonal every cell's
 // shift is the same. Columns past a pair's end join with a weight below every real key. Eight places a lane
 // keep both pairs' keys and weights in registers.
-template <int G, int C>
-__global__ void __launch_bounds__(kBlock, 2) extension_pairs_kernel(KernelArgs p, TableArgs t, const int32_t *__restrict__) {
+template <int G, int C, int BITS = 2>
+__global__ void __launch_bounds__(kBlock, 2) extension_pairs_kernel(KernelArgs p, TableArgs t,
+                                                                   const int32_t *__restrict__ table32) {
     constexpr int W = G * C;
     constexpr int GPW = 32 / G;
     // A real cell, held shifted, lies within two openings (4,000) below zero and 15,000 above, so real keys are at
@@ -267,15 +302,21 @@ __global__ void __launch_bounds__(kBlock, 2) extension_pairs_kernel(KernelArgs p
     // that, and both together above INT32_MIN.
     constexpr int32_t kNoKey = INT32_MIN, kLeast = -4576 * 65536, kPast = -1400000000;
     constexpr uint32_t kBelow = 0xE0000000u;
+    constexpr bool PROFILE = BITS == 8;
     __shared__ uint32_t rows8[4];
+    __shared__ int8_t table8[PROFILE ? 32 * 32 : 1];
     if (threadIdx.x < 4) rows8[threadIdx.x] = t.rows8[threadIdx.x];
+    if (PROFILE) load_table8(table8, table32, 0);
     __syncthreads();
 
     const int lane = threadIdx.x & 31;
     const int member = lane % G;
     const int group = lane / G;
-    const int warp = int((int64_t(blockIdx.x) * kBlock + threadIdx.x) >> 5);
-    const int warps = int((int64_t(gridDim.x) * kBlock) >> 5);
+    const int warp = int((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
+    const int warps = int((int64_t(gridDim.x) * blockDim.x) >> 5);
+    // This lane's part of its group's two profiles, letter a's of half h at [(h * t.size + a) * G].
+    ProfileRow<C> *profile = reinterpret_cast<ProfileRow<C> *>(sweep_profiles) +
+                             int64_t((threadIdx.x >> 5) * GPW + group) * 2 * t.size * G + member;
     const int32_t open = p.open, extend = p.extend;
     const int32_t opening = open - extend;
     const int32_t first_gap = open + extend;
@@ -317,8 +358,18 @@ __global__ void __launch_bounds__(kBlock, 2) extension_pairs_kernel(KernelArgs p
 
         for (int s = 0; s < warp_strips; ++s) {
             const int first = s * W + member * C;
-            uint32_t sel[C];
+            uint32_t sel[PROFILE ? 1 : C];
             int32_t weight[2][C], key[2][C];
+            if (PROFILE) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    fill_profile<C>(profile + h * t.size * G, G, t.size, table8,
+                                    s < strips[h] ? min(max(cols[h] - first, 0), C) : 0, [&](int k) {
+                                        const int col = first + k;
+                                        return letter_at<8>(p.tape, sh[h].second_word,
+                                                            uint32_t(backwards ? cols[h] - 1 - col : col));
+                                    });
+            }
 #pragma unroll
             for (int k = 0; k < C; ++k) {
                 uint32_t half_sel[2] = {kPadHalf, kPadHalf};
@@ -326,7 +377,7 @@ __global__ void __launch_bounds__(kBlock, 2) extension_pairs_kernel(KernelArgs p
                 for (int h = 0; h < 2; ++h) {
                     const int col = first + k;
                     const bool inside = s < strips[h] && col < cols[h];
-                    if (inside) {
+                    if (inside && !PROFILE) {
                         const uint32_t y =
                             letter_at<2>(p.tape, sh[h].second_word, uint32_t(backwards ? cols[h] - 1 - col : col));
                         half_sel[h] = h == 0 ? half_selector_a(y) : half_selector_b(y);
@@ -334,7 +385,7 @@ __global__ void __launch_bounds__(kBlock, 2) extension_pairs_kernel(KernelArgs p
                     weight[h][k] = inside ? 0 : kPast;
                     key[h][k] = kNoKey;
                 }
-                sel[k] = pair_selector(half_sel[0], half_sel[1]);
+                if (!PROFILE) sel[PROFILE ? 0 : k] = pair_selector(half_sel[0], half_sel[1]);
             }
             uint32_t H[C], D[C];
 #pragma unroll
@@ -351,18 +402,33 @@ __global__ void __launch_bounds__(kBlock, 2) extension_pairs_kernel(KernelArgs p
             const int warp_steps = warp_max(steps);
 
             for (int step0 = 1; step0 <= warp_steps; step0 += 16) {
-                uint32_t codes[2];
+                uint32_t codes[2] = {0, 0};
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
+                for (int h = 0; h < (PROFILE ? 0 : 2); ++h)
                     codes[h] = sixteen_rows(p.tape, sh[h].first_word, live[h] ? rows[h] : 0, step0 - member, backwards);
 #pragma unroll 2
                 for (int u = 0; u < 16; ++u) {
                     const int row = step0 + u - member;
                     uint32_t leftH = __shfl_up_sync(kFull, edgeH, 1, G);
                     uint32_t leftI = __shfl_up_sync(kFull, edgeI, 1, G);
-                    const uint32_t trA = rows8[codes[0] & 3u], trB = rows8[codes[1] & 3u];
-                    codes[0] >>= 2;
-                    codes[1] >>= 2;
+                    uint32_t trA = 0, trB = 0;
+                    ProfileRow<C> entries[PROFILE ? 2 : 1];
+                    if (PROFILE) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            // A row outside the pair reads its nearest letter: no cell that counts uses it.
+                            const int r = min(max(row, 1), max(rows[h], 1));
+                            const uint32_t letter =
+                                s < strips[h] ? letter_at<8>(p.tape, sh[h].first_word, uint32_t(backwards ? rows[h] - r : r - 1))
+                                              : 0u;
+                            entries[PROFILE ? h : 0] = profile[int(h * t.size + letter) * G];
+                        }
+                    } else {
+                        trA = rows8[codes[0] & 3u];
+                        trB = rows8[codes[1] & 3u];
+                        codes[0] >>= 2;
+                        codes[1] >>= 2;
+                    }
                     if (member == 0) {
                         if (s == 0) {
                             leftH = opening2;
@@ -383,7 +449,8 @@ __global__ void __launch_bounds__(kBlock, 2) extension_pairs_kernel(KernelArgs p
                         uint32_t I = leftI, left = leftH;
 #pragma unroll
                         for (int k = 0; k < C; ++k) {
-                            const uint32_t sub = uint32_t(prmt(trA, trB, sel[k]));
+                            const uint32_t sub = PROFILE ? profile_entry(entries[0], entries[PROFILE ? 1 : 0], k)
+                                                         : uint32_t(prmt(trA, trB, sel[PROFILE ? 0 : k]));
                             const uint32_t Hup = H[k];
                             const uint32_t Dn = __viaddmax_s16x2(Hup, opening2, D[k]);
                             const uint32_t X = __viaddmax_s16x2(diag, sub, Dn);

@@ -155,6 +155,24 @@ def test_free_ends_and_extensions_at_the_widths(da, oracle, alphabet, entries):
             assert [(a.score, a.cigar, _span(a)) for a in found] == expected
 
 
+# ---- larger alphabets through profiles --------------------------------------------------------------------
+
+@pytest.mark.parametrize("alphabet", ["ACGTN", PROTEIN, THIRTY_TWO])
+def test_profiles_score_globally_and_locally(da, oracle, alphabet):
+    rng = np.random.default_rng(7 * len(alphabet))
+    refs, queries = _placed_pairs(rng, alphabet)
+    refs += ["", alphabet[:3]]
+    queries += [alphabet[:2], ""]
+    tape = da.Tape.of(refs, queries)
+    coded = np.concatenate([oracle.codes(text, alphabet) for pair in zip(refs, queries) for text in pair if text])
+    # The second table's entries do not fit a byte once shifted: the 32-bit form.
+    for scoring in (_tabulated(da, rng, alphabet), _tabulated(da, rng, alphabet, -70, -66)):
+        op, ex = oracle.kernel_gaps(scoring.opening, scoring.extension)
+        for mode, how in ((da.Mode.GLOBAL, oracle.GLOBAL), (da.Mode.local(), oracle.LOCAL)):
+            expected = oracle.batch_scores(coded, tape.offsets, _table(scoring), len(alphabet), op, ex, how, threads=8)
+            np.testing.assert_array_equal(da.scores_tape(tape, scoring, mode), expected)
+
+
 # ---- alignments under Costs: kept fronts in 16 bits, in 32 and in the shared blocks ---------------------------
 
 @pytest.mark.parametrize("letters", [31_998, 32_002])
