@@ -162,8 +162,10 @@ bool is_pinned(const void *pointer) {
 }
 
 // Copies `bytes` of host memory to the device on the context's stream, through page-locked staging
-// unless the caller's memory is page-locked already.
-void to_device(dinara_gpu *gpu, void *device, const void *host, size_t bytes, dinara::PinnedBuffer &staging) {
+// unless the caller's memory is page-locked already. A copy of one slice is not waited for with `settled` false:
+// the entry point then uses that staging for nothing else, and waits for its stream before it returns.
+void to_device(dinara_gpu *gpu, void *device, const void *host, size_t bytes, dinara::PinnedBuffer &staging,
+               bool settled = true) {
     if (bytes == 0) return;
     if (is_pinned(host)) {
         DINARA_CUDA(cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, gpu->stream));
@@ -172,6 +174,12 @@ void to_device(dinara_gpu *gpu, void *device, const void *host, size_t bytes, di
     // Staged a slice at a time, each copy overlapping the next slice's memcpy.
     const size_t slice = size_t(64) << 20;
     uint8_t *stage = staging.ensure<uint8_t>(std::min(bytes, 2 * slice));
+    if (bytes <= slice) {
+        std::memcpy(stage, host, bytes);
+        DINARA_CUDA(cudaMemcpyAsync(device, stage, bytes, cudaMemcpyHostToDevice, gpu->stream));
+        if (settled) DINARA_CUDA(cudaStreamSynchronize(gpu->stream));
+        return;
+    }
     const uint8_t *from = static_cast<const uint8_t *>(host);
     uint8_t *to = static_cast<uint8_t *>(device);
     cudaEvent_t done[2];
@@ -783,7 +791,8 @@ void start_batch(StreamedBatch &out, dinara_gpu *gpu, int64_t pairs, const char 
         });
         device_offsets_host = relative.data();
     }
-    to_device(gpu, offsets_device, device_offsets_host, size_t(2 * pairs + 1) * sizeof(int64_t), gpu->pinned_small);
+    to_device(gpu, offsets_device, device_offsets_host, size_t(2 * pairs + 1) * sizeof(int64_t), gpu->pinned_small,
+              false);
     DINARA_CUDA(cudaEventCreateWithFlags(&out.inputs_ready, cudaEventDisableTiming));
     DINARA_CUDA(cudaEventRecord(out.inputs_ready, gpu->stream));
     out.upload = std::make_unique<LetterUpload>(gpu, letters_device,
@@ -1021,7 +1030,8 @@ void streamed_distances(dinara_gpu *gpu, int64_t pairs, const char *letters, con
                         starts = given + first;
                     else if (policy == DINARA_BAND_LEARNED)
                         starts = timed_predictions(ctx, count, letters_device, unit_offsets, &predict_ms);
-                    band_doubling(ctx, count, letters_device, unit_offsets, starts, plan ? plan->default_start : 0,
+                    band_doubling(ctx, count, letters_device, unit_offsets,
+                                  offsets[2 * (first + count)] - offsets[2 * first], starts, plan ? plan->default_start : 0,
                                   results_device + first, report ? &unit_reports[k] : nullptr);
                     unit_reports[k].predict_ms = predict_ms;
                 }
@@ -1489,19 +1499,19 @@ int64_t dinara_gpu_distances_tape(dinara_gpu *gpu, int64_t pairs, const char *le
             streamed_distances(gpu, pairs, letters, offsets, relative, plan, units, results, report);
             return 0;
         }
-        to_device(gpu, letters_device, letters + first, size_t(total), gpu->pinned_in);
-        to_device(gpu, offsets_device, relative.data(), relative.size() * sizeof(int64_t), gpu->pinned_small);
+        to_device(gpu, letters_device, letters + first, size_t(total), gpu->pinned_in, false);
+        to_device(gpu, offsets_device, relative.data(), relative.size() * sizeof(int64_t), gpu->pinned_small, false);
         const int64_t *starts = nullptr;
         double predict_ms = 0.0;
         if (policy == DINARA_BAND_GIVEN) {
             int64_t *device_starts = gpu->predictions.ensure<int64_t>(size_t(pairs));
-            to_device(gpu, device_starts, plan->start_thresholds, size_t(pairs) * sizeof(int64_t), gpu->pinned_small);
+            to_device(gpu, device_starts, plan->start_thresholds, size_t(pairs) * sizeof(int64_t), gpu->pinned_out);
             starts = device_starts;
         } else if (policy == DINARA_BAND_LEARNED) {
             starts = timed_predictions(gpu, pairs, letters_device, offsets_device, &predict_ms);
         }
         int64_t *results_device = gpu->scores.ensure<int64_t>(size_t(pairs));
-        band_doubling(gpu, pairs, letters_device, offsets_device, starts, plan ? plan->default_start : 0, results_device,
+        band_doubling(gpu, pairs, letters_device, offsets_device, total, starts, plan ? plan->default_start : 0, results_device,
                       report);
         if (report) report->predict_ms = predict_ms;
         to_host_now(gpu, results, results_device, size_t(pairs) * sizeof(int64_t));
@@ -1660,7 +1670,7 @@ int64_t dinara_gpu_resident_distances(dinara_gpu *gpu, const dinara_band_plan *p
         if (policy == DINARA_BAND_LEARNED)
             starts = timed_predictions(gpu, r.pairs, r.letters_device, r.offsets_device, &predict_ms);
         int64_t *results_device = r.results.ensure<int64_t>(size_t(r.pairs));
-        band_doubling(gpu, r.pairs, r.letters_device, r.offsets_device, starts, plan ? plan->default_start : 0,
+        band_doubling(gpu, r.pairs, r.letters_device, r.offsets_device, r.offsets.back(), starts, plan ? plan->default_start : 0,
                       results_device, report);
         if (report) report->predict_ms = predict_ms;
         if (report) report->full_cells = r.cells;
@@ -1694,8 +1704,8 @@ void upload_tape(dinara_gpu *gpu, int64_t pairs, const char *letters, const int6
     for (int64_t k = 0; k <= 2 * pairs; ++k) relative[size_t(k)] = offsets[k] - first;
     uint8_t *letters_device = gpu->letters.ensure<uint8_t>(size_t(total) + 16);
     int64_t *offsets_device = gpu->offsets.ensure<int64_t>(size_t(2 * pairs + 1));
-    to_device(gpu, letters_device, letters + first, size_t(total), gpu->pinned_in);
-    to_device(gpu, offsets_device, relative.data(), relative.size() * sizeof(int64_t), gpu->pinned_small);
+    to_device(gpu, letters_device, letters + first, size_t(total), gpu->pinned_in, false);
+    to_device(gpu, offsets_device, relative.data(), relative.size() * sizeof(int64_t), gpu->pinned_small, false);
     *letters_out = letters_device;
     *offsets_out = offsets_device;
 }
@@ -1864,7 +1874,7 @@ int64_t dinara_gpu_predictor_gradients(dinara_gpu *gpu, int64_t batch, const flo
         float *t = gpu->targets.ensure<float>(size_t(batch));
         float *g = gpu->gradients.ensure<float>(kPredictorParameters);
         float *l = gpu->counters.ensure<float>(64) + 60;
-        to_device(gpu, x, features, size_t(batch) * kPredictorInputs * sizeof(float), gpu->pinned_in);
+        to_device(gpu, x, features, size_t(batch) * kPredictorInputs * sizeof(float), gpu->pinned_in, false);
         DINARA_CUDA(cudaMemcpyAsync(t, targets, size_t(batch) * sizeof(float), cudaMemcpyHostToDevice, gpu->stream));
         predictor_gradients(gpu, int(batch), x, t, g, l);
         float summed = 0.f;

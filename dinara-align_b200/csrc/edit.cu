@@ -224,76 +224,27 @@ __device__ __forceinline__ bool four_refused(uint32_t word) {
     return ((complement - 0x01010101u) & ~complement & 0x80808080u) != 0u;
 }
 
-// A warp a pair: the pattern (the shorter side; the query on a tie, api.mojo:1286-1293), whether both
-// sides are DNA, and a refusal for a 0xFE or 0xFF byte (c/dinara.h:15-17). Both sides lie together on the
-// tape, read as aligned 16-byte chunks a lane (device letter buffers keep 16 bytes of room past the
-// last letter); bytes of a chunk outside the pair count as an A.
-__global__ void prepare_kernel(const uint8_t *__restrict__ letters, const int64_t *__restrict__ offsets, int64_t pairs,
-                               EditPair *__restrict__ out, int64_t *__restrict__ plane_words,
-                               int64_t *__restrict__ results, uint8_t *__restrict__ status) {
-    const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= pairs) return;
-    const int64_t r0 = offsets[2 * warp], q0 = offsets[2 * warp + 1], q1 = offsets[2 * warp + 2];
-    const int64_t rlen = q0 - r0, qlen = q1 - q0;
-    bool dna = true, refused = false;
-    const int64_t first_chunk = r0 >> 4, end_chunk = (q1 + 15) >> 4;
-    for (int64_t chunk = first_chunk + lane; chunk < end_chunk; chunk += 32) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(letters) + chunk);
-        const uint32_t words[4] = {v.x, v.y, v.z, v.w};
-        const int64_t at = chunk << 4;
-        const bool inside = at >= r0 && at + 16 <= q1;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            uint32_t word = words[j];
-            if (!inside) {
-                uint32_t keep = 0;
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const int64_t place = at + 4 * j + b;
-                    if (place >= r0 && place < q1) keep |= 0xFFu << (8 * b);
-                }
-                word = (word & keep) | (0x41414141u & ~keep);
-            }
-            dna = dna && four_dna(word);
-            refused = refused || four_refused(word);
-        }
-    }
-    dna = __all_sync(kFull, dna);
-    refused = __any_sync(kFull, refused);
-    if (lane != 0) return;
-    const bool query_pattern = qlen <= rlen;
-    EditPair e;
-    e.pattern = query_pattern ? q0 : r0;
-    e.text = query_pattern ? r0 : q0;
-    e.n = int32_t(query_pattern ? qlen : rlen);
-    e.m = int32_t(query_pattern ? rlen : qlen);
-    e.dna = dna ? 1 : 0;
-    e.words = (e.n + 63) / 64;
-    out[warp] = e;
-    plane_words[warp] = dna ? 4 * int64_t(e.words) : 0;
-    status[warp] = refused ? 1 : 0;
-    if (refused)
-        results[warp] = DINARA_UNSUPPORTED_SYMBOLS;
-    else if (e.n == 0)
-        results[warp] = e.m;  // api.mojo:1287-1288: an empty side costs the other's letters
-    else
-        results[warp] = -1000;  // not yet known
+// Where a pair's planes start, in words, `letters_before` letters into the batch: its pattern, the shorter side,
+// takes at most one word a plane for every 128 letters of the pair, and one more.
+__host__ __device__ inline int64_t plane_start(int64_t letters_before, int64_t pair) {
+    return 4 * (letters_before / 128 + pair);
 }
 
-// A warp a DNA pair: its pattern's four match planes, a word per 64 letters, 256 letters (four words) a
+// The first round's thresholds and list (thresholds null: none is wanted).
+struct StartArgs {
+    const int64_t *given;  // first thresholds, or null for the length difference plus `default_start`
+    int64_t default_start;
+    int64_t *thresholds, *firsts, *rounds, *cheapest;
+    uint32_t *pending;
+    unsigned int *pending_count;
+};
+
+// A DNA pattern's four match planes, a word per 64 letters, 256 letters (four words) a
 // pass. Lane l takes letters 8l .. 8l + 7 of the pass as one 8-byte value (two aligned loads, shifted
 // into place; device letter buffers keep 16 bytes of room past the last letter), and forms a byte of each
 // plane from them; a word's byte i of plane x is then lane 8w + i's byte x, gathered by eight shuffles, and
 // lanes 0-15 store the pass's 16 words together. Letters past the pattern match no plane.
-__global__ void planes_kernel(const uint8_t *__restrict__ letters, const EditPair *__restrict__ pairs, int64_t count,
-                              const int64_t *__restrict__ plane_offsets, uint64_t *__restrict__ planes) {
-    const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= count) return;
-    const EditPair e = pairs[warp];
-    if (!e.dna || e.n == 0) return;
-    uint64_t *out = planes + plane_offsets[warp];
+__device__ void write_planes(const uint8_t *__restrict__ letters, const EditPair &e, int lane, uint64_t *__restrict__ out) {
     const uintptr_t origin = reinterpret_cast<uintptr_t>(letters + e.pattern);
     const uint32_t shift = uint32_t(origin & 7u) * 8u;
     const uint64_t *aligned = reinterpret_cast<const uint64_t *>(origin & ~uintptr_t(7));
@@ -324,28 +275,82 @@ __global__ void planes_kernel(const uint8_t *__restrict__ letters, const EditPai
     }
 }
 
-// The first round's pending list and thresholds.
-__global__ void start_kernel(const EditPair *__restrict__ pairs, int64_t count, const int64_t *__restrict__ given,
-                             int64_t default_start, const uint8_t *__restrict__ status, int64_t *__restrict__ thresholds,
-                             int64_t *__restrict__ firsts, uint32_t *__restrict__ pending,
-                             unsigned int *__restrict__ pending_count) {
-    const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    const EditPair e = pairs[k];
-    if (status[k] || e.n == 0) return;
+// A warp a pair: the pattern (the shorter side; the query on a tie, api.mojo:1286-1293), whether both
+// sides are DNA, and a refusal for a 0xFE or 0xFF byte (c/dinara.h:15-17). Both sides lie together on the
+// tape, read as aligned 16-byte chunks a lane (device letter buffers keep 16 bytes of room past the
+// last letter); bytes of a chunk outside the pair count as an A. A DNA pair's planes follow, and with `start`
+// the pair's first threshold and its place on the first round's list: one launch where a check, a scan of the
+// planes' sizes, the planes and the start took five and a wait for the sizes' sum.
+__global__ void prepare_kernel(const uint8_t *__restrict__ letters, const int64_t *__restrict__ offsets, int64_t pairs,
+                               EditPair *__restrict__ out, int64_t *__restrict__ plane_offsets,
+                               uint64_t *__restrict__ planes, int64_t *__restrict__ results,
+                               uint8_t *__restrict__ status, StartArgs start) {
+    const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (warp >= pairs) return;
+    const int64_t r0 = offsets[2 * warp], q0 = offsets[2 * warp + 1], q1 = offsets[2 * warp + 2];
+    const int64_t rlen = q0 - r0, qlen = q1 - q0;
+    bool dna = true, refused = false;
+    const int64_t first_chunk = r0 >> 4, end_chunk = (q1 + 15) >> 4;
+    for (int64_t chunk = first_chunk + lane; chunk < end_chunk; chunk += 32) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(letters) + chunk);
+        const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+        const int64_t at = chunk << 4;
+        const bool inside = at >= r0 && at + 16 <= q1;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            uint32_t word = words[j];
+            if (!inside) {
+                uint32_t keep = 0;
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const int64_t place = at + 4 * j + b;
+                    if (place >= r0 && place < q1) keep |= 0xFFu << (8 * b);
+                }
+                word = (word & keep) | (0x41414141u & ~keep);
+            }
+            dna = dna && four_dna(word);
+            refused = refused || four_refused(word);
+        }
+    }
+    dna = __all_sync(kFull, dna);
+    refused = __any_sync(kFull, refused);
+    const bool query_pattern = qlen <= rlen;
+    EditPair e;
+    e.pattern = query_pattern ? q0 : r0;
+    e.text = query_pattern ? r0 : q0;
+    e.n = int32_t(query_pattern ? qlen : rlen);
+    e.m = int32_t(query_pattern ? rlen : qlen);
+    e.dna = dna ? 1 : 0;
+    e.words = (e.n + 63) / 64;
+    const int64_t planes_at = plane_start(r0 - offsets[0], warp);
+    if (e.dna && e.n > 0) write_planes(letters, e, lane, planes + planes_at);
+    if (lane != 0) return;
+    out[warp] = e;
+    plane_offsets[warp] = planes_at;
+    status[warp] = refused ? 1 : 0;
+    if (refused)
+        results[warp] = DINARA_UNSUPPORTED_SYMBOLS;
+    else if (e.n == 0)
+        results[warp] = e.m;  // api.mojo:1287-1288: an empty side costs the other's letters
+    else
+        results[warp] = -1000;  // not yet known
+    if (!start.thresholds || refused || e.n == 0) return;
     const int64_t delta = int64_t(e.m) - e.n;
-    int64_t t = given ? given[k] : delta + default_start;
+    int64_t t = start.given ? start.given[warp] : delta + start.default_start;
     if (t < delta) t = delta;
     if (t < 1) t = 1;
-    thresholds[k] = t;
-    firsts[k] = t;
-    pending[atomicAdd(pending_count, 1u)] = uint32_t(k);
+    start.thresholds[warp] = t;
+    start.firsts[warp] = t;
+    start.rounds[warp] = 0;
+    start.cheapest[warp] = INT64_MAX / 2;  // above any cost
+    start.pending[atomicAdd(start.pending_count, 1u)] = uint32_t(warp);
 }
 
-// The counters a band doubling run keeps on the device. The first two fields and the shape counts and
+// The counters a band doubling run keeps on the device. The pairs' counts and the shape counts and
 // work come back to the host together, in one read of the context's readback words.
 struct BandCounters {
-    unsigned pending, next;
+    unsigned pending[2];  // this round's pairs and the next's, by the round's parity
     unsigned shape_counts[kBandShapes + 1];
     unsigned long long shape_work[kBandShapes + 1];  // words x text letters, per shape
     unsigned queues[kBandShapes + 1];                // each shape's launch's next item
@@ -359,9 +364,9 @@ static_assert(kCountsBytes <= kReadbackBytes, "a round's counts fit the readback
 // Keys for the pending pairs: band shape in the top bits, then the text length, longest first; each
 // shape's pairs and its work (the words its launch sweeps), summed in the block first.
 __global__ void band_keys_kernel(const EditPair *__restrict__ pairs, const uint32_t *__restrict__ pending,
-                                 const unsigned int *__restrict__ pending_count, const int64_t *__restrict__ thresholds,
-                                 bool latency, BandTuning tuning, uint32_t *__restrict__ keys,
-                                 BandCounters *__restrict__ counters) {
+                                 const unsigned int *__restrict__ pending_count, unsigned int *__restrict__ next_count,
+                                 int64_t room, const int64_t *__restrict__ thresholds, bool latency, BandTuning tuning,
+                                 uint32_t *__restrict__ keys, BandCounters *__restrict__ counters) {
     __shared__ unsigned block_counts[kBandShapes];
     __shared__ unsigned long long block_work[kBandShapes];
     for (int s = threadIdx.x; s < kBandShapes; s += blockDim.x) {
@@ -370,6 +375,9 @@ __global__ void band_keys_kernel(const EditPair *__restrict__ pairs, const uint3
     }
     __syncthreads();
     const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k == 0) *next_count = 0;
+    // Places past the list's end sort after it: the lowest key, and the sort keeps equal keys in order.
+    if (k >= *pending_count && k < room) keys[k] = 0;
     if (k < *pending_count) {
         const uint32_t pair = pending[k];
         const EditPair e = pairs[pair];
@@ -497,32 +505,29 @@ __global__ void tally_kernel(const EditPair *__restrict__ pairs, int64_t count, 
 
 }  // namespace
 
-PreparedPairs prepare_pairs(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const int64_t *offsets,
-                            int64_t *results) {
-    cudaStream_t stream = gpu->stream;
+namespace {
+
+PreparedPairs prepare(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const int64_t *offsets,
+                      int64_t letters_total, int64_t *results, const StartArgs &start) {
     PreparedPairs p;
     p.info = gpu->shapes.ensure<EditPair>(size_t(pairs));
-    int64_t *plane_words = gpu->plane_offsets.ensure<int64_t>(2 * size_t(pairs + 1) + 2);
-    p.plane_offsets = plane_words + (pairs + 1);
+    p.plane_offsets = gpu->plane_offsets.ensure<int64_t>(size_t(pairs));
     p.status = gpu->flags.ensure<uint8_t>(size_t(pairs));
+    p.planes = gpu->planes.ensure<uint64_t>(size_t(plane_start(letters_total, pairs)) + 8);
     const int threads = 256;
     const unsigned warp_blocks = unsigned((pairs * 32 + threads - 1) / threads);
-    prepare_kernel<<<warp_blocks, threads, 0, stream>>>(letters, offsets, pairs, p.info, plane_words, results,
-                                                        p.status);
-    gpu->launches += 1;
-    DINARA_CUDA(cudaGetLastError());
-    DINARA_CUDA(cudaMemsetAsync(plane_words + pairs, 0, sizeof(int64_t), stream));
-    size_t scratch = 0;
-    DINARA_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scratch, plane_words, p.plane_offsets, int(pairs + 1), stream));
-    void *space = gpu->sort_scratch.ensure<uint8_t>(scratch + 256);
-    DINARA_CUDA(cub::DeviceScan::ExclusiveSum(space, scratch, plane_words, p.plane_offsets, int(pairs + 1), stream));
-    int64_t plane_total = 0;
-    read_back(gpu, &plane_total, p.plane_offsets + pairs, sizeof(int64_t));
-    p.planes = gpu->planes.ensure<uint64_t>(size_t(plane_total) + 4);
-    planes_kernel<<<warp_blocks, threads, 0, stream>>>(letters, p.info, pairs, p.plane_offsets, p.planes);
+    prepare_kernel<<<warp_blocks, threads, 0, gpu->stream>>>(letters, offsets, pairs, p.info, p.plane_offsets, p.planes,
+                                                           results, p.status, start);
     gpu->launches += 1;
     DINARA_CUDA(cudaGetLastError());
     return p;
+}
+
+}  // namespace
+
+PreparedPairs prepare_pairs(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const int64_t *offsets,
+                            int64_t letters_total, int64_t *results) {
+    return prepare(gpu, pairs, letters, offsets, letters_total, results, StartArgs{});
 }
 
 double band_shape_rate(dinara_gpu *gpu, int shape, int64_t pairs, const uint8_t *letters, const PreparedPairs &p,
@@ -577,18 +582,11 @@ int band_shape_blocks(dinara_gpu *gpu, int shape) {
 }
 
 void band_doubling(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const int64_t *offsets,
-                   const int64_t *first_thresholds_device, int64_t default_start, int64_t *results,
+                   int64_t letters_total, const int64_t *first_thresholds_device, int64_t default_start, int64_t *results,
                    dinara_band_report *report) {
     cudaStream_t stream = gpu->stream;
     const int threads = 256;
     const unsigned thread_blocks = unsigned((pairs + threads - 1) / threads);
-    const PreparedPairs prepared = prepare_pairs(gpu, pairs, letters, offsets, results);
-    EditPair *info = prepared.info;
-    const int64_t *plane_offsets = prepared.plane_offsets;
-    const uint64_t *planes = prepared.planes;
-    const uint8_t *status = prepared.status;
-    void *space = nullptr;
-
     int64_t *thresholds = gpu->thresholds.ensure<int64_t>(4 * size_t(pairs));
     int64_t *firsts = thresholds + pairs;
     int64_t *rounds = thresholds + 2 * pairs;
@@ -600,13 +598,21 @@ void band_doubling(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const
         gpu->counters.ensure<unsigned int>((sizeof(BandCounters) + 3) / 4));
     unsigned long long *swept = &counters->swept;
     DINARA_CUDA(cudaMemsetAsync(counters, 0, sizeof(BandCounters), stream));
-    DINARA_CUDA(cudaMemsetAsync(rounds, 0, size_t(pairs) * sizeof(int64_t), stream));
-    DINARA_CUDA(cudaMemsetAsync(cheapest, 0x7f, size_t(pairs) * sizeof(int64_t), stream));  // above any cost
-    start_kernel<<<thread_blocks, threads, 0, stream>>>(info, pairs, first_thresholds_device,
-                                                        default_start > 0 ? default_start : 256, status, thresholds,
-                                                        firsts, pending, &counters->pending);
-    gpu->launches += 1;
-    DINARA_CUDA(cudaGetLastError());
+    StartArgs start;
+    start.given = first_thresholds_device;
+    start.default_start = default_start > 0 ? default_start : 256;
+    start.thresholds = thresholds;
+    start.firsts = firsts;
+    start.rounds = rounds;
+    start.cheapest = cheapest;
+    start.pending = pending;
+    start.pending_count = &counters->pending[0];
+    const PreparedPairs prepared = prepare(gpu, pairs, letters, offsets, letters_total, results, start);
+    EditPair *info = prepared.info;
+    const int64_t *plane_offsets = prepared.plane_offsets;
+    const uint64_t *planes = prepared.planes;
+    const uint8_t *status = prepared.status;
+    void *space = nullptr;
     uint32_t *keys = gpu->keys.ensure<uint32_t>(size_t(pairs));
     uint32_t *keys_sorted = gpu->keys_sorted.ensure<uint32_t>(size_t(pairs));
     uint32_t *order_sorted = gpu->order_sorted.ensure<uint32_t>(size_t(pairs));
@@ -614,8 +620,8 @@ void band_doubling(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const
     const BandTuning tuned = gpu->band_tuning;
     alignas(8) unsigned char host_bytes[kCountsBytes];
     const BandCounters *host = reinterpret_cast<const BandCounters *>(host_bytes);
-    read_back(gpu, host_bytes, counters, sizeof(unsigned int));
-    int64_t count = host->pending;
+    // The first round's list is at most every pair; how many it holds comes back with the round's counts.
+    int64_t count = pairs;
     int64_t launches = 0;
     float kernel_ms = 0.f;
     int64_t round = 0;
@@ -623,10 +629,11 @@ void band_doubling(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const
     double round_ms[16] = {0.0};
     while (count > 0) {
         const int64_t launches_before = launches;
-        const int64_t round_count = count;
+        unsigned int *pending_count = &counters->pending[round & 1], *next_count = &counters->pending[(round + 1) & 1];
         // Order the round's pairs: by band shape, longest text first.
-        DINARA_CUDA(cudaMemsetAsync(&counters->next, 0, offsetof(BandCounters, swept) - offsetof(BandCounters, next),
-                                    stream));
+        if (round > 0)
+            DINARA_CUDA(cudaMemsetAsync(counters->shape_counts, 0,
+                                        offsetof(BandCounters, swept) - offsetof(BandCounters, shape_counts), stream));
         const unsigned blocks = unsigned((count + threads - 1) / threads);
         // A round of few pairs takes the one-word-a-lane windows: lanes to spare, and the sweep's time is
         // its longest pair's chain of steps.
@@ -635,7 +642,7 @@ void band_doubling(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const
         BandTuning tuning = tuned;
         if (tuned.chain_share > 0.f && !latency) {
             DINARA_CUDA(cudaMemsetAsync(&counters->round_work, 0, sizeof(unsigned long long), stream));
-            round_work_kernel<<<blocks, threads, 0, stream>>>(info, pending, &counters->pending, thresholds,
+            round_work_kernel<<<blocks, threads, 0, stream>>>(info, pending, pending_count, thresholds,
                                                               &counters->round_work);
             gpu->launches += 1;
             DINARA_CUDA(cudaGetLastError());
@@ -644,8 +651,8 @@ void band_doubling(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const
             const double per_lane = double(work) / (double(gpu->multiprocessors) * 1024.0);
             tuning.chain_words = std::max<int64_t>(tuned.chain_words, int64_t(tuned.chain_share * per_lane));
         }
-        band_keys_kernel<<<blocks, threads, 0, stream>>>(info, pending, &counters->pending, thresholds, latency,
-                                                         tuning, keys, counters);
+        band_keys_kernel<<<blocks, threads, 0, stream>>>(info, pending, pending_count, next_count, count, thresholds,
+                                                         latency, tuning, keys, counters);
         gpu->launches += 1;
         DINARA_CUDA(cudaGetLastError());
         size_t sort_bytes = 0;
@@ -655,12 +662,18 @@ void band_doubling(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const
         DINARA_CUDA(cub::DeviceRadixSort::SortPairsDescending(space, sort_bytes, keys, keys_sorted, pending,
                                                               order_sorted, int(count), 0, 32, stream));
         read_back(gpu, host_bytes, counters, kCountsBytes);
-        DINARA_CUDA(cudaEventRecord(gpu->start, stream));
+        const int64_t round_count = host->pending[round & 1];
+        if (round_count == 0) break;
+        if (report) DINARA_CUDA(cudaEventRecord(gpu->start, stream));
         ClockSpan clock(gpu, kClassUnitBand, stream);
         // Each shape's launch on a side stream, all forked from and joined back to the context's stream,
         // so they run at once. Each takes a share of the GPU's lanes in proportion to its share of the
-        // round's work, so that they end together; the longest chains start first within each.
-        DINARA_CUDA(cudaEventRecord(gpu->fork, stream));
+        // round's work, so that they end together; the longest chains start first within each. A round of one
+        // shape stays on the context's stream.
+        int shapes_used = 0;
+        for (int shape = 0; shape < kBandShapes; ++shape) shapes_used += host->shape_counts[shape] > 0;
+        const bool fork = shapes_used > 1;
+        if (fork) DINARA_CUDA(cudaEventRecord(gpu->fork, stream));
         bool used[dinara_gpu::kSideStreams] = {false};
         // A shape's share of the round's time: its words at its measured cost a word.
         double total_work = 0.0;
@@ -695,9 +708,9 @@ void band_doubling(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const
             const int64_t needed = (n_shape + groups_per_block - 1) / groups_per_block;
             grid = std::max<int64_t>(1, std::min(grid, needed));
             const int side = shape % dinara_gpu::kSideStreams;
-            if (!used[side]) DINARA_CUDA(cudaStreamWaitEvent(gpu->side[side], gpu->fork, 0));
-            used[side] = true;
-            fn<<<unsigned(grid), kBlock, 0, gpu->side[side]>>>(args);
+            if (fork && !used[side]) DINARA_CUDA(cudaStreamWaitEvent(gpu->side[side], gpu->fork, 0));
+            used[side] = fork;
+            fn<<<unsigned(grid), kBlock, 0, fork ? gpu->side[side] : stream>>>(args);
             gpu->launches += 1;
             DINARA_CUDA(cudaGetLastError());
             at += n_shape;
@@ -708,26 +721,25 @@ void band_doubling(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const
             DINARA_CUDA(cudaEventRecord(gpu->joins[side], gpu->side[side]));
             DINARA_CUDA(cudaStreamWaitEvent(stream, gpu->joins[side], 0));
         }
-        DINARA_CUDA(cudaEventRecord(gpu->stop, stream));
+        if (report) DINARA_CUDA(cudaEventRecord(gpu->stop, stream));
         clock.stop();
-        DINARA_CUDA(cudaMemsetAsync(&counters->next, 0, sizeof(unsigned int), stream));
-        settle_kernel<<<blocks, threads, 0, stream>>>(info, order_sorted, &counters->pending, thresholds, cheapest,
-                                                      banded, results, rounds, latency, tuning, next, &counters->next);
+        settle_kernel<<<blocks, threads, 0, stream>>>(info, order_sorted, pending_count, thresholds, cheapest, banded,
+                                                      results, rounds, latency, tuning, next, next_count);
         gpu->launches += 1;
         DINARA_CUDA(cudaGetLastError());
-        DINARA_CUDA(cudaMemcpyAsync(&counters->pending, &counters->next, sizeof(unsigned int), cudaMemcpyDeviceToDevice,
-                                    stream));
-        read_back(gpu, host_bytes, counters, sizeof(unsigned int));
-        float ms = 0.f;
-        DINARA_CUDA(cudaEventElapsedTime(&ms, gpu->start, gpu->stop));
-        kernel_ms += ms;
-        if (round < 16) {
-            round_pairs[round] = round_count;
-            round_launches[round] = launches - launches_before;
-            round_ms[round] = ms;
+        read_back(gpu, host_bytes, counters, 2 * sizeof(unsigned int));
+        if (report) {
+            float ms = 0.f;
+            DINARA_CUDA(cudaEventElapsedTime(&ms, gpu->start, gpu->stop));
+            kernel_ms += ms;
+            if (round < 16) {
+                round_pairs[round] = round_count;
+                round_launches[round] = launches - launches_before;
+                round_ms[round] = ms;
+            }
         }
         ++round;
-        count = host->pending;
+        count = host->pending[round & 1];
         std::swap(pending, next);
     }
     if (report) {

@@ -142,7 +142,7 @@ struct PreparedPairs {
     uint8_t *status;
 };
 PreparedPairs prepare_pairs(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const int64_t *offsets,
-                            int64_t *results);
+                            int64_t letters_total, int64_t *results);
 
 // The autotuner's probe: one launch of window shape `shape` over every prepared pair, on the context's
 // stream; returns the words it swept per millisecond. `scratch` holds 2 x pairs int64 (device).
@@ -157,10 +157,11 @@ void band_autotune(dinara_gpu *gpu, const dinara_band_tune_options &options, din
 void band_tuning_access(dinara_gpu *gpu, bool set, dinara_band_tuning *values);
 
 // Runs band doubling over a batch whose ASCII letters and offsets are on the device already; writes
-// every pair's distance (or its code) to `results` (device) and fills `report`. `letters` starts on a
+// every pair's distance (or its code) to `results` (device) and fills `report`, when given. `letters_total` is the
+// pairs' letters (offsets' last less its first). `letters` starts on a
 // 16-byte boundary and keeps 16 bytes of room past its last letter (the kernels read whole chunks).
 void band_doubling(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const int64_t *offsets,
-                   const int64_t *first_thresholds_device, int64_t default_start, int64_t *results,
+                   int64_t letters_total, const int64_t *first_thresholds_device, int64_t default_start, int64_t *results,
                    dinara_band_report *report);
 
 // The learned band's first thresholds for a batch on the device (learned.cu): the predictor's cost

@@ -795,7 +795,7 @@ void predictor_train(dinara_gpu *gpu, const dinara_train_options &options, dinar
     uint8_t *letters = generated.letters;
     // Their exact distances: the method's own, plain band doubling.
     int64_t *distances = gpu->features.ensure<int64_t>(size_t(pairs));
-    band_doubling(gpu, pairs, letters, offsets, nullptr, 0, distances, nullptr);
+    band_doubling(gpu, pairs, letters, offsets, generated.letters_total, nullptr, 0, distances, nullptr);
     // Targets (distance over mean length) and features.
     std::vector<int64_t> host_distances(static_cast<size_t>(pairs)), host_offsets(size_t(2 * pairs + 1));
     DINARA_CUDA(cudaMemcpyAsync(host_distances.data(), distances, size_t(pairs) * sizeof(int64_t),

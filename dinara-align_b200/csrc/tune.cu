@@ -50,7 +50,7 @@ void measure_shapes(dinara_gpu *gpu, uint64_t seed, int64_t length, double rate,
         const int64_t pairs = 2 * most;
         const GeneratedPairs generated = generate_pairs(gpu, seed, pairs, double(probe), double(probe), rate, rate);
         int64_t *results = gpu->distances.ensure<int64_t>(size_t(pairs));
-        const PreparedPairs prepared = prepare_pairs(gpu, pairs, generated.letters, generated.offsets, results);
+        const PreparedPairs prepared = prepare_pairs(gpu, pairs, generated.letters, generated.offsets, generated.letters_total, results);
         int64_t *scratch = gpu->predictions.ensure<int64_t>(2 * size_t(pairs));
         for (int s = 0; s < kBandShapes; ++s) {
             if (rates[s] > 0 || std::max<int64_t>(length, 64 * (band_capacity(s) + 8)) > probe) continue;
@@ -106,7 +106,7 @@ void band_autotune(dinara_gpu *gpu, const dinara_band_tune_options &options, din
     int64_t *results = gpu->features.ensure<int64_t>(2 * size_t(o.pairs));
     int64_t *starts = results + o.pairs;
     gpu->band_tuning = tuning;
-    band_doubling(gpu, o.pairs, generated.letters, generated.offsets, nullptr, 0, results, nullptr);
+    band_doubling(gpu, o.pairs, generated.letters, generated.offsets, generated.letters_total, nullptr, 0, results, nullptr);
     near_starts_kernel<<<unsigned((o.pairs + 255) / 256), 256, 0, gpu->stream>>>(results, o.pairs, starts);
     DINARA_CUDA(cudaGetLastError());
     gpu->launches += 1;
@@ -124,7 +124,7 @@ void band_autotune(dinara_gpu *gpu, const dinara_band_tune_options &options, din
             for (int repeat = 0; repeat < 2; ++repeat) {
                 dinara_band_report band;
                 std::memset(&band, 0, sizeof band);
-                band_doubling(gpu, o.pairs, generated.letters, generated.offsets, start ? starts : nullptr, 0, results,
+                band_doubling(gpu, o.pairs, generated.letters, generated.offsets, generated.letters_total, start ? starts : nullptr, 0, results,
                               &band);
                 if (repeat == 0 || band.kernel_ms < fastest_run) fastest_run = band.kernel_ms;
             }

@@ -576,7 +576,8 @@ def distances_tape(tape: Tape, *, policy: int = native.BAND_PLAIN, start_thresho
     summary = native.CBandReport()
     code = native.lib().dinara_gpu_distances_tape(handle, pairs, tape.letters.ctypes.data,
                                                    native.pointer(tape.offsets, ctypes.c_int64), ctypes.byref(plan),
-                                                   native.pointer(out, ctypes.c_int64), ctypes.byref(summary))
+                                                   native.pointer(out, ctypes.c_int64),
+                                                   ctypes.byref(summary) if report else None)
     native.check(code, handle)
     if report:
         return out[:pairs], summary.as_dict()

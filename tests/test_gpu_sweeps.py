@@ -208,6 +208,35 @@ def test_fronts_in_shared_blocks(da, oracle):
     assert [(a.cost, a.cigar) for a in found] == [oracle.affine_cigar(r, q, 4, 6, 2) for r, q in zip(refs, queries)]
 
 
+# ---- unit-cost distances: the first round's list ---------------------------------------------------------------
+
+@pytest.mark.parametrize("pairs", [1, 2, 33, 400])
+def test_distances_beside_pairs_that_take_no_round(da, oracle, pairs):
+    """Refused pairs, empty sides and letters other than DNA among pairs of up to three rounds: patterns at words
+    and a letter either side."""
+    rng = np.random.default_rng(pairs)
+    refs, queries = [], []
+    for k in range(pairs):
+        length = int(rng.choice([1, 3, 63, 64, 65, 127, 128, 129, 700, 3000]))
+        ref = _text(rng, length, "ACGT" if k % 4 else "ACGTNRY")
+        refs.append(ref)
+        queries.append(_text(rng, length) if k % 5 == 3 else _mutated(rng, ref, 0.1, "ACGT"))
+    refs = [r.encode() for r in refs]
+    queries = [q.encode() for q in queries]
+    for k in range(0, pairs, 7):
+        queries[k] = b"" if k % 2 else queries[k] + b"\xfe"
+    tape = da.Tape.of(refs, queries)
+    found, report = da.distances_tape(tape, report=True)
+    np.testing.assert_array_equal(found, da.distances_tape(tape))
+    for k in range(pairs):
+        if queries[k].endswith(b"\xfe"):
+            assert found[k] == da._native.UNSUPPORTED_SYMBOLS
+        else:
+            assert found[k] == oracle.edit_distance_dp(refs[k], queries[k])
+    swept = sum(1 for r, q in zip(refs, queries) if r and q and not q.endswith(b"\xfe"))
+    assert (report["round_pairs"][0] if report["round_pairs"] else 0) == swept
+
+
 # ---- the predictor's gradients: the batch's slices -----------------------------------------------------------------
 
 @pytest.mark.parametrize("batch", [1, 31, 128, 129, 4096, 4097])
