@@ -892,7 +892,8 @@ PairLimits whole_limits_of(const AffineBatch &batch, const AffineTable &table) {
         limits.local = 1;
         // Half of it a pair: a lane group sweeps its two pairs to the larger one's rows and strips, so the
         // cells past a pair's end reach at most the sum of the two pairs' terms.
-        limits.whole = (30000 - gaps) / 2;
+        // A cell is held two openings higher too (the bias that keeps every half at zero or more).
+        limits.whole = (30000 - gaps - 2 * std::abs(table.open) - std::abs(table.open - table.extend)) / 2;
         limits.best = best;
         limits.row_step = -table.extend;
         return limits;

@@ -583,6 +583,16 @@ __device__ __forceinline__ uint32_t halves(int32_t low, int32_t high) {
 __device__ __forceinline__ int32_t low_of(uint32_t v) { return int32_t(int16_t(uint16_t(v & 0xFFFFu))); }
 __device__ __forceinline__ int32_t high_of(uint32_t v) { return int32_t(int16_t(uint16_t(v >> 16))); }
 
+// Sixteen 2-bit letters of a sequence (`length` letters from packed word `first_word`) from letter `start` on,
+// lowest bits first. Letters before the sequence or past its end read as any code: no cell that counts reads one.
+__device__ __forceinline__ uint32_t sixteen_letters(const uint32_t *__restrict__ tape, uint32_t first_word, int length,
+                                                    int start) {
+    const int word = start >> 4, last = max(length - 1, 0) >> 4;
+    const uint32_t a = __ldg(tape + first_word + min(max(word, 0), last));
+    const uint32_t b = __ldg(tape + first_word + min(max(word + 1, 0), last));
+    return __funnelshift_r(a, b, uint32_t(start & 15) * 2u);
+}
+
 // A column's selector for both pairs: bytes 0-1 pick pair A's entry (sign-extended) from its row's
 // register, bytes 2-3 pair B's from the other; kPadHalf reads 0 or -1 (a sign of a byte, replicated).
 constexpr uint32_t kPadHalf = 0x99u;
@@ -671,11 +681,15 @@ __global__ void __launch_bounds__(kBlock, 2) affine_pairs_kernel(KernelArgs p, T
     const int64_t slot = int64_t(warp) * GPW + group;
     const uint32_t open2 = halves(open, open), extend2 = halves(extend, extend), opening2 = halves(opening, opening);
     const uint32_t floor2 = halves(-32768, -32768);
-    const int32_t top = LOCAL ? 0 : opening;
+    // Local cells are held `bias` above their value, more than two gap openings, so that no half is ever below
+    // zero and an opening is added to both by one 32-bit add.
+    const int32_t bias = LOCAL ? -open - opening + 1 : 0;
+    const int32_t top = LOCAL ? bias : opening;
     const uint32_t top2 = halves(top, top), top_gap2 = halves(top + first_gap, top + first_gap);
     // Local cells are held less row x extend (the table less extend too): a deletion run then climbs by
     // a constant, the zero floor becomes row-dependent, and the best is shifted back a row at a time.
     const uint32_t open_less_extend2 = halves(open - extend, open - extend);
+    const uint32_t open_both = uint32_t(open) + (uint32_t(open) << 16);  // of two halves, each left at zero or more
 
     for (uint32_t base = p.begin + uint32_t(warp) * 2 * GPW; base < p.end; base += uint32_t(warps) * 2 * GPW) {
         const uint32_t item = base + 2 * group;
@@ -695,7 +709,7 @@ __global__ void __launch_bounds__(kBlock, 2) affine_pairs_kernel(KernelArgs p, T
             strips[h] = live[h] && rows[h] > 0 && cols[h] > 0 ? (cols[h] + W - 1) / W : 0;
         }
         const int warp_strips = warp_max(max(strips[0], strips[1]));
-        uint32_t best2 = 0;
+        uint32_t best2 = halves(bias, bias);
         int32_t reported[2] = {0, 0};
         // TRACK: each half's best over the strips so far and its first row.
         int32_t hit[2] = {0, 0}, hit_row[2] = {0, 0}, strip_row[2] = {0, 0};
@@ -732,7 +746,7 @@ __global__ void __launch_bounds__(kBlock, 2) affine_pairs_kernel(KernelArgs p, T
                 D[k] = top_gap2;
             }
             uint32_t edgeH = top2, edgeI = top_gap2;
-            const int32_t corner = LOCAL ? 0 : (first_col == 0 ? 0 : opening);
+            const int32_t corner = LOCAL ? bias : (first_col == 0 ? 0 : opening);
             uint32_t above_left = halves(corner, corner);
             int group_rows = 0;
 #pragma unroll
@@ -740,17 +754,24 @@ __global__ void __launch_bounds__(kBlock, 2) affine_pairs_kernel(KernelArgs p, T
             const int steps = group_rows > 0 ? group_rows + G : 0;
             const int warp_steps = warp_max(steps);
 
+            uint32_t codes[2] = {0, 0};
             for (int step = 1; step <= warp_steps; ++step) {
                 const int row = step - member;
+                // Sixteen rows' letters at a time, the sweep's own rows whatever the lane's.
+                if (!PROFILE && (step & 15) == 1) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        codes[h] = sixteen_letters(p.tape, sh[h].first_word, strip_live[h] ? rows[h] : 0, row - 1);
+                }
                 // Local: this row's lift (row x -extend, at least 0), the floor of its held cells.
                 const int32_t lift = LOCAL ? -max(row, 0) * extend : 0;
-                const uint32_t floor_h2 = halves(lift, lift), floor_i2 = halves(open + lift, open + lift);
+                const uint32_t floor_h2 = halves(lift + bias, lift + bias);
                 uint32_t leftH = __shfl_up_sync(kFull, edgeH, 1, G);
                 uint32_t leftI = __shfl_up_sync(kFull, edgeI, 1, G);
                 if (member == 0) {
                     if (s == 0) {
                         leftH = LOCAL ? floor_h2 : top2;
-                        leftI = LOCAL ? halves(lift + first_gap, lift + first_gap) : top_gap2;
+                        leftI = LOCAL ? halves(lift + bias + first_gap, lift + bias + first_gap) : top_gap2;
                     } else {
                         const int r = min(max(row, 0), group_rows);
                         const int2 c = p.carry[slot * p.carry_stride + r];
@@ -760,6 +781,9 @@ __global__ void __launch_bounds__(kBlock, 2) affine_pairs_kernel(KernelArgs p, T
                 }
                 uint32_t diag = above_left;
                 above_left = leftH;
+                const uint32_t here[2] = {codes[0] & 3u, codes[1] & 3u};
+                codes[0] >>= 2;
+                codes[1] >>= 2;
                 if (row >= 1 && row <= group_rows) {
                     uint32_t tr[2];
                     ProfileRow<C> entries[PROFILE ? 2 : 1];
@@ -768,7 +792,7 @@ __global__ void __launch_bounds__(kBlock, 2) affine_pairs_kernel(KernelArgs p, T
                         const bool inside = strip_live[h] && row <= rows[h];
                         const uint32_t letter =
                             PROFILE ? (inside ? letter_at<BITS>(p.tape, sh[h].first_word, uint32_t(row - 1)) : 0u)
-                                    : (inside ? letter_at<BITS>(p.tape, sh[h].first_word, uint32_t(row - 1)) : 0u);
+                                    : here[h];
                         if (PROFILE) {
                             entries[h] = profile[int(h * t.size + letter) * G];
                             if (!inside) entries[h] = ProfileRow<C>{};
@@ -793,8 +817,9 @@ __global__ void __launch_bounds__(kBlock, 2) affine_pairs_kernel(KernelArgs p, T
                         }
                         if (LOCAL) {
                             Hn = __vimax3_s16x2(X, I, floor_h2);
-                            // The next cell's insertion reads the floored X plus an opening.
-                            Xprev = __viaddmax_s16x2(X, open2, floor_i2);
+                            // The next cell's insertion, from X plus an opening (no half of it below zero). From a
+                            // cell under the floor it stays under every later one: no floor of its own.
+                            Xprev = X + open_both;
                         } else {
                             Hn = __vimax3_s16x2(X, I, X);
                             Xprev = X;
@@ -842,14 +867,14 @@ __global__ void __launch_bounds__(kBlock, 2) affine_pairs_kernel(KernelArgs p, T
                 // The strip's best joins the others': higher, or as high from an earlier row.
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const int32_t value = h == 0 ? low_of(best2) : high_of(best2);
+                    const int32_t value = (h == 0 ? low_of(best2) : high_of(best2)) - bias;
                     if (value > hit[h] || (value == hit[h] && strip_row[h] < hit_row[h])) {
                         hit[h] = value;
                         hit_row[h] = strip_row[h];
                     }
                     strip_row[h] = 0;
                 }
-                best2 = 0;
+                best2 = halves(bias, bias);
             }
             __syncwarp();
         }
@@ -880,8 +905,8 @@ __global__ void __launch_bounds__(kBlock, 2) affine_pairs_kernel(KernelArgs p, T
 #pragma unroll
             for (int span = 1; span < G; span <<= 1) best2 = __vimax_s16x2_relu(best2, __shfl_xor_sync(kFull, best2, span, G));
             if (member == 0) {
-                if (live[0]) p.scores[pair[0]] = low_of(best2);
-                if (live[1]) p.scores[pair[1]] = high_of(best2);
+                if (live[0]) p.scores[pair[0]] = low_of(best2) - bias;
+                if (live[1]) p.scores[pair[1]] = high_of(best2) - bias;
             }
         } else {
 #pragma unroll

@@ -6,16 +6,6 @@
 namespace dinara {
 namespace sweep {
 
-// Sixteen 2-bit letters of a sequence (`length` letters from packed word `first_word`) from letter `start` on,
-// lowest bits first. Letters before the sequence or past its end read as any code: no cell that counts reads one.
-__device__ __forceinline__ uint32_t sixteen_letters(const uint32_t *__restrict__ tape, uint32_t first_word, int length,
-                                                    int start) {
-    const int word = start >> 4, last = max(length - 1, 0) >> 4;
-    const uint32_t a = __ldg(tape + first_word + min(max(word, 0), last));
-    const uint32_t b = __ldg(tape + first_word + min(max(word + 1, 0), last));
-    return __funnelshift_r(a, b, uint32_t(start & 15) * 2u);
-}
-
 // A row window: the letters of rows row0 .. row0 + 15, the first in the low bits, for a sequence read forwards,
 // or (backwards) its last `length` letters' mirror, row r reading letter length - r.
 __device__ __forceinline__ uint32_t sixteen_rows(const uint32_t *__restrict__ tape, uint32_t first_word, int length,
