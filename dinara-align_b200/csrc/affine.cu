@@ -1669,4 +1669,39 @@ void last_places(dinara_gpu *gpu, const uint8_t *letters, const int64_t *offsets
     gpu->launches += 1;
 }
 
+namespace {
+
+// Spans that do not lie within their pair's letters are emptied and their pair flagged (before its span is packed);
+// with `inner`, pairs whose span aligned globally scores otherwise than the span's own score are flagged.
+__global__ void check_spans_kernel(const int64_t *__restrict__ offsets, int64_t first_pair, int64_t count,
+                                   int64_t *__restrict__ spans, const int32_t *__restrict__ scores,
+                                   const int32_t *__restrict__ inner, uint8_t *__restrict__ flags) {
+    const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k >= count) return;
+    const int64_t pair = first_pair + k;
+    bool failed = false;
+    if (inner) {
+        failed = inner[pair] != scores[pair];
+    } else {
+        int64_t *span = spans + 4 * k;
+        const int64_t rows = offsets[2 * pair + 1] - offsets[2 * pair];
+        const int64_t columns = offsets[2 * pair + 2] - offsets[2 * pair + 1];
+        failed = !(0 <= span[0] && span[0] <= span[1] && span[1] <= rows && 0 <= span[2] && span[2] <= span[3] &&
+                   span[3] <= columns);
+        if (failed) span[0] = span[1] = span[2] = span[3] = 0;
+    }
+    if (failed && flags[pair] == 0) flags[pair] = kWalkFailed;
+}
+
+}  // namespace
+
+void check_spans(dinara_gpu *gpu, const int64_t *offsets, int64_t first_pair, int64_t count, int64_t *spans,
+                 const int32_t *scores, const int32_t *inner, uint8_t *flags) {
+    if (count <= 0) return;
+    check_spans_kernel<<<unsigned((count + 255) / 256), 256, 0, gpu->stream>>>(offsets, first_pair, count, spans, scores,
+                                                                             inner, flags);
+    DINARA_CUDA(cudaGetLastError());
+    gpu->launches += 1;
+}
+
 }  // namespace dinara

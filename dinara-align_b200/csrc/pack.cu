@@ -15,8 +15,8 @@ namespace dinara {
 // its scheduling key (shape class, strips, rows; sorted descending so the longest go first).
 __global__ void pack_pairs_kernel(const uint8_t *__restrict__ letters, const int64_t *__restrict__ offsets,
                                   int64_t first_pair, int64_t count, const uint8_t *__restrict__ codes, int bits,
-                                  uint32_t *__restrict__ tape, PairShape *__restrict__ shapes,
-                                  uint8_t *__restrict__ unknown) {
+                                  const int64_t *__restrict__ spans, uint32_t *__restrict__ tape,
+                                  PairShape *__restrict__ shapes, uint8_t *__restrict__ unknown) {
     __shared__ uint8_t code_of[256];
     code_of[threadIdx.x & 255] = codes[threadIdx.x & 255];
     __syncthreads();
@@ -31,9 +31,14 @@ __global__ void pack_pairs_kernel(const uint8_t *__restrict__ letters, const int
     uint32_t starts[2], lengths[2];
     for (int side = 0; side < 2; ++side) {
         const int64_t k = 2 * warp + side;
-        const int64_t start = offsets[k];
-        const int64_t length = offsets[k + 1] - start;
+        int64_t start = offsets[k];
+        int64_t length = offsets[k + 1] - start;
         const uint64_t word0 = packed_word_start(start, k, bits);
+        if (spans) {
+            const int64_t *span = spans + 4 * nth + 2 * side;
+            length = span[1] - span[0];
+            start += span[0];
+        }
         starts[side] = uint32_t(word0);
         lengths[side] = uint32_t(length);
         // Lane i packs output words i, i + 32, ... (consecutive lanes, consecutive words: coalesced both
@@ -79,7 +84,7 @@ __global__ void pack_pairs_kernel(const uint8_t *__restrict__ letters, const int
     if (lane == 0) {
         PairShape shape{starts[0], lengths[0], starts[1], lengths[1]};
         shapes[warp] = shape;
-        unknown[warp] = bad ? 1 : 0;
+        if (unknown) unknown[warp] = bad ? 1 : 0;
     }
 }
 
@@ -144,12 +149,12 @@ __global__ void schedule_keys_kernel(const PairShape *__restrict__ shapes, const
 
 void pack_pairs(dinara_gpu *gpu, const uint8_t *letters_device, const int64_t *offsets_device, int64_t first_pair,
                 int64_t count, const uint8_t *codes_device, int bits, uint32_t *tape, PairShape *shapes,
-                uint8_t *unknown) {
+                uint8_t *unknown, const int64_t *spans) {
     if (count <= 0) return;
     const int threads = 256;
     const int64_t blocks = (count * 32 + threads - 1) / threads;
     pack_pairs_kernel<<<dim3(unsigned(blocks)), threads, 0, gpu->stream>>>(
-        letters_device, offsets_device, first_pair, count, codes_device, bits, tape, shapes, unknown);
+        letters_device, offsets_device, first_pair, count, codes_device, bits, spans, tape, shapes, unknown);
     gpu->launches += 1;
     DINARA_CUDA(cudaGetLastError());
 }

@@ -12,7 +12,7 @@ namespace dinara {
 // flags packing it whole gives.
 void pack_pairs(dinara_gpu *gpu, const uint8_t *letters_device, const int64_t *offsets_device, int64_t first_pair,
                 int64_t count, const uint8_t *codes_device, int bits, uint32_t *tape, PairShape *shapes,
-                uint8_t *unknown);
+                uint8_t *unknown, const int64_t *spans = nullptr);
 
 // A batch's sweep order: pairs by class, classes in descending order, then strips and rows descending.
 // Classes: the whole-matrix shape classes 0-4 (affine_shape_for with `record`); with `band` the proven
