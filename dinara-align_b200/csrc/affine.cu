@@ -650,7 +650,7 @@ struct PhaseTimer {
 // columns) - 2 score) / (best - 2 extend). The pair goes round again at that width (at least twice the
 // last, rounded up to 256 diagonals) unless this is the `last` round or that band's strips of
 // `strip_columns` would sweep three fifths of its rows or more: then to the whole-matrix list. With `swept`
-// null, every pair is routed to `first_width`. With `proven`, a pair whose band proves its score leaves the
+// null, every pair is routed to `first_width`, or a wider band foreseen for it (`foreseen`, by pair, when given). With `proven`, a pair whose band proves its score leaves the
 // width there (by pair - proven_first).
 __global__ void wide_route_kernel(const PairShape *__restrict__ shapes, const uint32_t *__restrict__ pending,
                                   const int32_t *__restrict__ swept, int64_t count, int32_t first_width, bool last,
@@ -658,7 +658,8 @@ __global__ void wide_route_kernel(const PairShape *__restrict__ shapes, const ui
                                   uint32_t *__restrict__ next, int32_t *__restrict__ next_width,
                                   unsigned int *__restrict__ next_count, uint32_t *__restrict__ whole,
                                   unsigned int *__restrict__ whole_count, int32_t *__restrict__ proven,
-                                  int64_t proven_first, int32_t strip_columns) {
+                                  int64_t proven_first, int32_t strip_columns,
+                                  const int32_t *__restrict__ foreseen) {
     const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const uint32_t pair = pending[k];
@@ -679,13 +680,18 @@ __global__ void wide_route_kernel(const PairShape *__restrict__ shapes, const ui
             whole[atomicAdd(whole_count, 1u)] = pair;
             return;
         }
-        const int64_t g = (4 * (int64_t(open) - extend) + int64_t(best) * (rows + columns) - 2 * score) / per_letter + 2;
-        const int64_t delta = columns > rows ? columns - rows : rows - columns;
-        width = max(2 * done, g + delta + 2);
+        width = max(2 * done, band_width_to_prove(score, rows, columns, best, open, extend));
         width = (width + 255) / 256 * 256;
     }
-    const bool banded = !last && width < (int64_t(1) << 30) && band_low_for_width(rows, columns, width) != INT32_MIN &&
-                        10 * (strip_columns + width) < 6 * rows;
+    auto worth = [&](int64_t w) {
+        return w < (int64_t(1) << 30) && band_low_for_width(rows, columns, w) != INT32_MIN &&
+               10 * (strip_columns + w) < 6 * rows;
+    };
+    if (!swept && foreseen && foreseen[pair] > 0) {
+        const int64_t wanted = (int64_t(foreseen[pair]) + 255) / 256 * 256;
+        if (wanted > width && worth(wanted)) width = wanted;
+    }
+    const bool banded = !last && worth(width);
     if (banded) {
         const unsigned at = atomicAdd(next_count, 1u);
         next[at] = pair;
@@ -717,11 +723,30 @@ void sweep_long(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &ta
     args.carry_stride = int64_t(batch.max_rows) + 1;
     ClockSpan clock(gpu, kClassWhole, gpu->stream);
     if (long_serves(batch, table)) {
-        // Four warps a block when the batch fills the GPU with them, eight for a batch too small to.
-        const int warps = count >= 4 * int64_t(gpu->multiprocessors) ? kLongWarps / 2 : kLongWarps;
-        int per_sm = 0;
-        DINARA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, affine_long_kernel, 32 * warps, 0));
-        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(int64_t(per_sm) * gpu->multiprocessors, count));
+        // A cluster a pair, or for a batch with pairs enough to fill the GPU, a block of four warps a pair.
+        const bool cluster = count < 4 * int64_t(gpu->multiprocessors);
+        const int threads = 32 * (cluster ? kLongClusterWarps : kLongWarps / 2);
+        cudaLaunchConfig_t config = {};
+        cudaLaunchAttribute shape = {};
+        shape.id = cudaLaunchAttributeClusterDimension;
+        shape.val.clusterDim = {unsigned(cluster ? kLongCluster : 1), 1, 1};
+        config.blockDim = dim3(unsigned(threads));
+        config.stream = gpu->stream;
+        config.attrs = &shape;
+        config.numAttrs = 1;
+        int64_t in_flight = 0;
+        if (cluster) {
+            config.gridDim = dim3(kLongCluster);
+            int clusters = 0;
+            DINARA_CUDA(cudaOccupancyMaxActiveClusters(&clusters, affine_long_kernel<true>, &config));
+            in_flight = std::max(clusters, 1);
+        } else {
+            int per_sm = 0;
+            DINARA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, affine_long_kernel<false>, threads, 0));
+            in_flight = int64_t(std::max(per_sm, 1)) * gpu->multiprocessors;
+        }
+        in_flight = std::min(in_flight, count);
+        config.gridDim = dim3(unsigned(in_flight * (cluster ? kLongCluster : 1)));
         LongArgs a;
         std::memset(&a, 0, sizeof a);
         a.tape = args.tape;
@@ -734,8 +759,13 @@ void sweep_long(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &ta
         for (int r = 0; r < 4; ++r) a.rows8[r] = targs.rows8[r];
         a.scores = args.scores;
         a.carry_stride = args.carry_stride;
-        a.carry = gpu->carry.ensure<int2>(size_t(blocks * args.carry_stride));
-        affine_long_kernel<<<unsigned(blocks), 32 * warps, 0, gpu->stream>>>(a);
+        // The carried columns, then (clusters) the progress words.
+        a.carry = gpu->carry.ensure<int2>(size_t(in_flight) * size_t(args.carry_stride + 2 * kLongMostWarps));
+        a.progress = a.carry + in_flight * args.carry_stride;
+        if (cluster)
+            DINARA_CUDA(cudaLaunchKernelEx(&config, affine_long_kernel<true>, a));
+        else
+            DINARA_CUDA(cudaLaunchKernelEx(&config, affine_long_kernel<false>, a));
     } else {
         KernelFn fn = widths ? &affine_wide_kernel<false, true> : &affine_wide_kernel<false, false>;
         const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(persistent_blocks(gpu, fn), count));
@@ -760,7 +790,8 @@ void sweep_long(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &ta
 // is then worth its rounds when the recording's strips (kRecordStrip columns) would sweep few of a pair's
 // rows, where the scores' own strips are a block's 4,096 columns.
 void widening_band(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, const uint32_t *order,
-                   int64_t count, KernelArgs args, int32_t *proven = nullptr, int64_t proven_first = 0) {
+                   int64_t count, KernelArgs args, int32_t *proven = nullptr, int64_t proven_first = 0,
+                   const int32_t *foreseen = nullptr) {
     if (count <= 0) return;
     int32_t best = -128;
     for (int r = 0; r < table.size; ++r)
@@ -783,7 +814,7 @@ void widening_band(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
         wide_route_kernel<<<unsigned((left + 255) / 256), 256, 0, gpu->stream>>>(
             batch.shapes, pending, swept, left, first_width, round == kBandRounds, args.scores, best, table.open,
             table.extend, next, next_widths, counts, whole, counts + 1, proven, proven_first,
-            strip_columns);
+            strip_columns, foreseen);
         DINARA_CUDA(cudaGetLastError());
         gpu->launches += 1;
         unsigned int routed = 0;
@@ -800,7 +831,7 @@ void widening_band(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
 }
 
 void affine_launch_all(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, const Schedule &schedule,
-                       bool record, KernelArgs args) {
+                       bool record, KernelArgs args, const int32_t *foreseen = nullptr) {
     const bool smem = !table.packed16 || batch.bits == 8;
     const TableArgs targs = table_args(table, batch.local);
     int32_t *table32 = nullptr;
@@ -808,7 +839,7 @@ void affine_launch_all(dinara_gpu *gpu, const AffineBatch &batch, const AffineTa
     const Buckets b = buckets_of(schedule);
     args.order = schedule.order;
     for (int bucket = kClasses - 1; bucket >= 0; --bucket) {
-        if (bucket == kBandClass || bucket == kBandPairsClass) continue;
+        if (bucket == kBandClass || bucket == kBandPairsClass || bucket == schedule.skip) continue;
         if (b.end[bucket] <= b.begin[bucket]) continue;
         const bool wide = bucket == kWideClass;
         // Recording, a long global pair whose widening band proved a width: its strips over that band.
@@ -817,7 +848,8 @@ void affine_launch_all(dinara_gpu *gpu, const AffineBatch &batch, const AffineTa
         const int cls = pairs16 ? bucket - kWholePairsClass : wide || band_record ? 4 : bucket;
         if (wide && !batch.local && !record && band_serves(batch, table)) {
             // Long global pairs take the widening band first.
-            widening_band(gpu, batch, table, schedule.order + b.begin[bucket], b.end[bucket] - b.begin[bucket], args);
+            widening_band(gpu, batch, table, schedule.order + b.begin[bucket], b.end[bucket] - b.begin[bucket], args, nullptr,
+                          0, foreseen);
             continue;
         }
         if (pairs16) {
@@ -985,7 +1017,7 @@ int64_t band_pairs(const Schedule &schedule) {
 void launch_bands(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, const Schedule &schedule,
                   int32_t *scores, uint32_t *leftovers, unsigned int *leftover_count, bool record, uint64_t *decisions,
                   const int64_t *decision_offsets, int64_t first_pair, uint8_t *layouts,
-                  unsigned long long *band_cells) {
+                  unsigned long long *band_cells, int32_t *foreseen = nullptr) {
     for (int pass = 0; pass < 2; ++pass) {
         const bool pairs_of_16 = pass == 0;
         BandedBatch b = banded_batch(batch, table, schedule, scores, nullptr, leftovers, leftover_count, pairs_of_16);
@@ -995,6 +1027,7 @@ void launch_bands(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &
         b.first_pair = first_pair;
         b.band_cells = band_cells;
         if (!pairs_of_16) {
+            b.widths = foreseen;
             banded_launch(gpu, b, record, false);
             continue;
         }
@@ -1473,20 +1506,41 @@ void affine_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
     unsigned int *counters = gpu->class_counts.ensure<unsigned int>(20);
     unsigned int *leftover_count = counters + 8;
     uint32_t *leftovers = nullptr;
+    int32_t *foreseen = nullptr;  // bands foreseen for the pairs that leave theirs early
     if (band_pairs(schedule_all) > 0) {
-        leftovers = gpu->leftovers.ensure<uint32_t>(size_t(band_pairs(schedule_all)));
+        leftovers = gpu->leftovers.ensure<uint32_t>(size_t(band_pairs(schedule_all)) +
+                                                    2 * size_t(schedule_all.counts[kWideClass]));
         DINARA_CUDA(cudaMemsetAsync(leftover_count, 0, sizeof(unsigned int), gpu->stream));
+        if (schedule_all.counts[kBandClass] > 0 && long_serves(batch, table)) {
+            foreseen = gpu->record_widths.ensure<int32_t>(size_t(batch.pairs));
+            DINARA_CUDA(cudaMemsetAsync(foreseen + first, 0, size_t(count) * sizeof(int32_t), gpu->stream));
+        }
         launch_bands(gpu, batch, table, schedule_all, scores, leftovers, leftover_count, false, nullptr, nullptr, 0,
-                     nullptr, band_counter(gpu));
+                     nullptr, band_counter(gpu), foreseen);
     }
-    affine_launch_all(gpu, batch, table, schedule_all, false, args);
+    // Long pairs wait for the band's leftovers, which may be long too: one sweep then takes them all at once (four
+    // pairs of 50,000 letters, two of them the band's: 117 ms together, 233 one sweep after the other).
+    const int64_t long_pairs = band_pairs(schedule_all) > 0 ? schedule_all.counts[kWideClass] : 0;
+    Schedule rest = schedule_all;
+    if (long_pairs > 0) {
+        const int64_t at = buckets_of(schedule_all).begin[kWideClass];
+        // Kept past every place the leftovers, with these after them, may take.
+        DINARA_CUDA(cudaMemcpyAsync(leftovers + band_pairs(schedule_all) + long_pairs, schedule_all.order + at,
+                                    size_t(long_pairs) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, gpu->stream));
+        rest.skip = kWideClass;
+    }
+    affine_launch_all(gpu, batch, table, rest, false, args);
     unsigned int left = 0;
     if (band_pairs(schedule_all) > 0) {
         read_back(gpu, &left, leftover_count, sizeof left);
-        if (left > 0) {
-            const Schedule again = dinara::schedule(gpu, batch.shapes, leftovers, 0, left, false, false,
+        if (left + long_pairs > 0) {
+            if (long_pairs > 0)
+                DINARA_CUDA(cudaMemcpyAsync(leftovers + left, leftovers + band_pairs(schedule_all) + long_pairs,
+                                            size_t(long_pairs) * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
+                                            gpu->stream));
+            const Schedule again = dinara::schedule(gpu, batch.shapes, leftovers, 0, left + long_pairs, false, false,
                                                     whole_limits_of(batch, table));
-            affine_launch_all(gpu, batch, table, again, false, args);
+            affine_launch_all(gpu, batch, table, again, false, args, foreseen);
         }
     }
     timer.stop();

@@ -101,6 +101,15 @@ __host__ __device__ inline int32_t band_low_for_width(int64_t rows, int64_t colu
     return int32_t((delta < 0 ? delta : 0) - slack);
 }
 
+// How wide a band (about a pair's main and end diagonals) proves a score (band_proves_width): g gap letters
+// outside it must cost more than the score lacks of the best, g > (4 (open - extend) + best (rows + columns) -
+// 2 score) / (best - 2 extend). `best - 2 extend` above zero.
+__host__ __device__ inline int64_t band_width_to_prove(int64_t score, int64_t rows, int64_t columns, int64_t best,
+                                                       int64_t open, int64_t extend) {
+    const int64_t g = (4 * (open - extend) + best * (rows + columns) - 2 * score) / (best - 2 * extend) + 2;
+    return g + (columns > rows ? columns - rows : rows - columns) + 2;
+}
+
 // A band-recorded pair (affine_kernel<..., BANDED>): 32 lanes of 16 columns, strips of kRecordStrip
 // columns, strip s sweeping only the rows its columns share with the pair's band [low, high] of
 // diagonals (column less row) and keeping decisions for those rows alone.

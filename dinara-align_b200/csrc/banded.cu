@@ -108,20 +108,30 @@ __global__ void __launch_bounds__(kBlock) banded_kernel(BandedBatch b) {
             // columns outside the pair read letter 0, which no real cell's value depends on.
             // Every 64 rows a pair whose band can no longer prove its score is left to the whole-matrix sweep: from
             // here its score gains at most the best shifted entry a row. At 5% errors a pair of 50,000 letters
-            // leaves after some 500 rows, where its band took 9 ms to its end; a pair that the band proves goes on
-            // as before.
+            // leaves after some 2,000 rows, where its band took 9 ms to its end; a pair that the band proves goes on
+            // as before. A pair stays for an eighth of its rows, 2,048 at most, so that what its score lost in them
+            // foretells what it will lose in all: with a fifth more, that says how wide a band would prove it
+            // (wide_route_kernel), and one wider sweep serves where a first one had to find the score.
             if (r0 > 1 && (r0 & 63) == 1) {
                 int32_t most = H[0];
 #pragma unroll
                 for (int k = 1; k < C; ++k) most = max(most, H[k]);
 #pragma unroll
                 for (int span = 1; span < G; span <<= 1) most = max(most, __shfl_xor_sync(kFull, most, span, G));
-                const int64_t reach = int64_t(most) + int64_t(max(b.best - 2 * extend, 0)) * (rows - r0 + 1) +
-                                      int64_t(rows + cols) * extend;
-                if (live && r0 <= rows && !band_proves(reach, rows, cols, low, b.best, open, extend)) {
+                const int64_t step = max(b.best - 2 * extend, 0);
+                const int64_t done = r0 - 1;
+                const int64_t ends = int64_t(rows + cols) * extend;
+                if (live && r0 <= rows && done >= min(rows / 8, 2048) &&
+                    !band_proves(most + step * (rows - done) + ends, rows, cols, low, b.best, open, extend)) {
                     if (member == 0) {
                         if (b.proven) b.proven[pair] = 0;
                         b.leftovers[atomicAdd(b.leftover_count, 1u)] = pair;
+                        if (b.widths && step > 0) {
+                            const int64_t lost = (step * done - most) * rows / done;
+                            const int64_t score = step * min(rows, cols) - lost - lost / 5 + ends;
+                            const int64_t width = band_width_to_prove(score, rows, cols, b.best, open, extend);
+                            b.widths[pair] = int32_t(min(width, int64_t(1) << 30));
+                        }
                     }
                     live = false;
                     rows = 0;

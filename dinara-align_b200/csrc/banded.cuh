@@ -104,6 +104,9 @@ struct BandedBatch {
     // proved the pair. Counting, when given: the band cells the launch swept (rows x band width a pair).
     uint8_t *layouts;
     unsigned long long *band_cells;
+    // The 32-bit sweep, when given: by pair, the band width that would prove a pair's score, as foreseen from the
+    // rows it swept, for each pair it leaves early.
+    int32_t *widths;
 };
 
 // Launches the banded sweep (scores, or with `record` scores and decisions) over `batch.count` pairs; with

@@ -9,8 +9,12 @@ namespace sweep {
 // A strip is 64 virtual lanes of 16 columns: a lane's low halves hold 16 columns and its high halves the
 // next 16, one row behind, so each DPX instruction on 16-bit pairs moves two cells of the one pair.
 constexpr int kLongStrip = 1024;
-constexpr int kLongWarps = 8;   // most warps a block; a launch may take fewer
-constexpr int kLongChunk = 32;  // steps between the block's barriers
+constexpr int kLongWarps = 8;     // most warps a block without clusters; a launch may take fewer
+constexpr int kLongChunk = 32;    // steps between barriers
+constexpr int kLongCluster = 8;   // blocks a cluster, and each one's warps
+constexpr int kLongClusterWarps = 2;
+constexpr int kLongMostWarps = 16;  // a pair's, either way
+static_assert(kLongCluster * kLongClusterWarps <= kLongMostWarps && kLongWarps <= kLongMostWarps, "progress slots");
 
 // A lane's halves hold its cells less its base, a true 32-bit value that follows them: at each chunk the
 // lane's own middle cell becomes the base. Within a lane's 32 columns two reached cells of a row differ
@@ -32,9 +36,16 @@ struct LongArgs {
     int32_t open, extend;
     uint32_t rows8[4];           // the shifted table, a byte an entry
     int32_t *scores;
-    int2 *carry;                 // a column of (score, insertion) a block
+    int2 *carry;                 // a column of (score, insertion) a pair in flight
     int64_t carry_stride;
+    int2 *progress;              // clusters: 2 * kLongMostWarps words a pair in flight
 };
+
+// Every thread of a cluster's blocks meets here; what each wrote before, the others read after.
+__device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 // A strip's rows: those its columns share with the band [low, high] of diagonals (column less row).
 __device__ __forceinline__ int long_first_row(int s, int high) { return max(1, s * kLongStrip + 1 - high); }
@@ -42,7 +53,7 @@ __device__ __forceinline__ int long_last_row(int s, int rows, int columns, int l
     return min(rows, min((s + 1) * kLongStrip, columns) - low);
 }
 
-// The whole or banded score of one pair a block (score_groups.mojo's recurrence, cells shifted by (row +
+// The whole or banded score of one pair a block, or with CLUSTER a cluster of eight blocks (score_groups.mojo's recurrence, cells shifted by (row +
 // column) * extend). Warp w of the block's sweeps strips w, w + warps, ...: a strip's virtual lane v runs one
 // row behind lane v - 1, whose last column reaches it from the lane's own low half or by one shuffle, and the
 // column left of a strip comes from the strip before through `carry`, a chunk of 32 rows at a time. Warps
@@ -55,24 +66,43 @@ __device__ __forceinline__ int long_last_row(int s, int rows, int columns, int l
 // 32-bit sweep, affine_wide_kernel) and its strips of 4,096 columns, which sweep 4,096 rows beyond a band's
 // width, are what this one does without.
 //
+// Eight warps on one SM share its four issue ports, and a pair of 50,000 letters keeps them all for each of its
+// rows; a batch too small to fill the GPU with pairs takes a cluster a pair instead, neighbouring strips on
+// different SMs, a warp or less a port. Its warps meet at a cluster barrier a chunk and keep their progress in
+// global memory, which the barrier's release and acquire order.
+//
 // A banded strip sweeps its rows alone, every cell above or left of them unreached; the score is then
 // the best over paths within the swept rows, the whole matrix's when the band proves it
 // (band_proves_width).
-__global__ void __launch_bounds__(32 * kLongWarps, 2) affine_long_kernel(LongArgs p) {
+template <bool CLUSTER>
+__global__ void __launch_bounds__(32 * (CLUSTER ? kLongClusterWarps : kLongWarps), CLUSTER ? 8 : 2)
+    affine_long_kernel(LongArgs p) {
     constexpr int C = 16;
     __shared__ uint32_t rows8[4];
-    __shared__ int2 progress[2][kLongWarps];  // by round parity: each warp's strip and the steps it has done
+    // By round parity: each warp's strip and the steps it has done.
+    __shared__ int2 block_progress[CLUSTER ? 1 : 2 * kLongMostWarps];
     if (threadIdx.x < 4) rows8[threadIdx.x] = p.rows8[threadIdx.x];
 
     const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const int warps = blockDim.x >> 5;
+    const uint32_t first_item = CLUSTER ? blockIdx.x / kLongCluster : blockIdx.x;
+    const uint32_t items_apart = CLUSTER ? gridDim.x / kLongCluster : gridDim.x;
+    const int rank = CLUSTER ? int(blockIdx.x % kLongCluster) : 0;  // clusters are consecutive blocks
+    const int warps = int(blockDim.x >> 5) * (CLUSTER ? kLongCluster : 1);
+    const int warp = CLUSTER ? int(threadIdx.x >> 5) * kLongCluster + rank : int(threadIdx.x >> 5);
+    volatile int *progress =
+        reinterpret_cast<volatile int *>(CLUSTER ? p.progress + int64_t(first_item) * 2 * kLongMostWarps : block_progress);
+    auto meet = [&] {
+        if (CLUSTER)
+            cluster_barrier();
+        else
+            __syncthreads();
+    };
     const int32_t opening = p.open - p.extend;
     const int32_t first_gap = p.open + p.extend;
     const uint32_t opening2 = halves(opening, opening), floor2 = halves(kLongFloor, kLongFloor);
-    int2 *carry = p.carry + int64_t(blockIdx.x) * p.carry_stride;
+    int2 *carry = p.carry + int64_t(first_item) * p.carry_stride;
 
-    for (uint32_t item = blockIdx.x; item < p.count; item += gridDim.x) {
+    for (uint32_t item = first_item; item < p.count; item += items_apart) {
         const uint32_t pair = p.order[item];
         const PairShape sh = p.shapes[pair];
         const int rows = int(sh.rows), cols = int(sh.columns);
@@ -87,9 +117,12 @@ __global__ void __launch_bounds__(32 * kLongWarps, 2) affine_long_kernel(LongArg
                 high = from + width - 1;
             }
         }
-        __syncthreads();  // the last pair's progress and carry are read
-        if (threadIdx.x < 2 * kLongWarps) progress[threadIdx.x / kLongWarps][threadIdx.x % kLongWarps] = make_int2(-1, 0);
-        __syncthreads();
+        meet();  // the last pair's progress and carry are read
+        if (rank == 0 && threadIdx.x < 2 * kLongMostWarps) {
+            progress[2 * threadIdx.x] = -1;
+            progress[2 * threadIdx.x + 1] = 0;
+        }
+        meet();
 
         // The strip under this warp: its rows, its state and the steps it has done.
         int strip = warp, done = 0;
@@ -98,8 +131,11 @@ __global__ void __launch_bounds__(32 * kLongWarps, 2) affine_long_kernel(LongArg
         uint32_t edgeH = 0, edgeI = 0, above_left = 0, send = 0, before = 0;
         int32_t base = 0;
         // Every round some strip's chunk is ready (the first unfinished strip's always is), so the rounds
-        // end within the sum of all strips' chunks.
+        // end within the sum of all strips' chunks: when the last strip's warp has moved past it, which every
+        // warp reads as of the same barrier.
         for (int round = 0;; ++round) {
+            const int before_round = ((round + 1) & 1) * kLongMostWarps;
+            if (progress[2 * (before_round + (strips - 1) % warps)] > strips - 1) break;
             bool ready = strip < strips;
             if (ready && done == 0) {
                 first_row = long_first_row(strip, high);
@@ -112,8 +148,9 @@ __global__ void __launch_bounds__(32 * kLongWarps, 2) affine_long_kernel(LongArg
                 // step r - its first row + 64) by the last barrier.
                 const int last_read = min(first_row - 1 + done + kLongChunk, previous_last);
                 const int needed = last_read - long_first_row(strip - 1, high) + 64;
-                const int2 theirs = progress[(round + 1) & 1][(strip - 1) % warps];
-                ready = theirs.x > strip - 1 || (theirs.x == strip - 1 && theirs.y >= needed);
+                const int at = 2 * (before_round + (strip - 1) % warps);
+                const int their_strip = progress[at], their_done = progress[at + 1];
+                ready = their_strip > strip - 1 || (their_strip == strip - 1 && their_done >= needed);
             }
             if (ready) {
                 const bool from_top = first_row == 1;
@@ -256,8 +293,11 @@ __global__ void __launch_bounds__(32 * kLongWarps, 2) affine_long_kernel(LongArg
                     done = 0;
                 }
             }
-            if (lane == 0) progress[round & 1][warp] = make_int2(strip, done);
-            if (!__syncthreads_or(strip < strips)) break;
+            if (lane == 0) {
+                progress[2 * ((round & 1) * kLongMostWarps + warp)] = strip;
+                progress[2 * ((round & 1) * kLongMostWarps + warp) + 1] = done;
+            }
+            meet();
         }
     }
 }

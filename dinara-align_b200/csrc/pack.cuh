@@ -35,6 +35,7 @@ constexpr uint32_t kLongSide = 1024 + 1;
 struct Schedule {
     const uint32_t *order;
     int64_t counts[kClasses];
+    int skip = -1;  // a class the whole-matrix launches leave out
 };
 
 // Which pairs the 16-bit pair sweeps take: band pairs whose rows and columns sum to at most `band`; and,
