@@ -17,6 +17,7 @@
 #include <utility>
 #include <vector>
 
+#include <emmintrin.h>
 #include <sys/mman.h>
 
 #include "affine.cuh"
@@ -224,6 +225,29 @@ void parallel_copy(uint8_t *to, const uint8_t *from, size_t bytes, int threads =
         helpers[t - 1] = std::thread([=] { std::memcpy(to + begin, from + begin, end - begin); });
     }
     std::memcpy(to, from, std::min(bytes, part));
+    for (int t = 1; t < threads; ++t) helpers[t - 1].join();
+}
+
+// A copy into page-locked memory that a device copy reads next, past the caches: with the lines left dirty in eight
+// cores' caches the bus read them at 5 to 14 GB/s, from memory at 48. `to` starts on a 16-byte boundary.
+void copy_past_caches(uint8_t *to, const uint8_t *from, size_t bytes) {
+    const size_t whole = bytes / 16;
+    for (size_t k = 0; k < whole; ++k)
+        _mm_stream_si128(reinterpret_cast<__m128i *>(to) + k, _mm_loadu_si128(reinterpret_cast<const __m128i *>(from) + k));
+    _mm_sfence();
+    std::memcpy(to + 16 * whole, from + 16 * whole, bytes - 16 * whole);
+}
+
+// copy_past_caches shared by eight threads, or fewer for a small copy (about half a megabyte each).
+void stage_copy(uint8_t *to, const uint8_t *from, size_t bytes) {
+    const int threads = int(std::min<size_t>(8, bytes / (size_t(1) << 19) + 1));
+    const size_t part = ((bytes + threads - 1) / threads + 63) & ~size_t(63);
+    std::thread helpers[7];
+    for (int t = 1; t < threads; ++t) {
+        const size_t begin = std::min(bytes, t * part), end = std::min(bytes, begin + part);
+        helpers[t - 1] = std::thread([=] { copy_past_caches(to + begin, from + begin, end - begin); });
+    }
+    copy_past_caches(to, from, std::min(bytes, part));
     for (int t = 1; t < threads; ++t) helpers[t - 1].join();
 }
 
@@ -490,7 +514,7 @@ class LetterUpload {
                 if (piece >= 2) DINARA_CUDA(cudaEventSynchronize(events_[piece - 2]));
                 const size_t at = piece * kUploadPiece;
                 // Eight threads: from pageable memory this copy, not the bus, sets the upload's pace.
-                parallel_copy(buffer, host_ + at, std::min(kUploadPiece, bytes_ - at), 8);
+                stage_copy(buffer, host_ + at, std::min(kUploadPiece, bytes_ - at));
                 queue(piece, buffer);
                 {
                     std::lock_guard<std::mutex> lock(mutex_);
