@@ -56,7 +56,6 @@ struct WaveArgs {
     int32_t x, od, ed, oi, ei;  // the costs over their common factor; d a deletion's, i an insertion's
     int64_t scale;
     int64_t ceiling;         // the largest cost (over the common factor) a pair may take
-    bool reversed;           // Ties.LEFT: both sequences read back to front
     bool eqx;
     bool trace;
     uint8_t *arena;
@@ -73,42 +72,68 @@ struct WaveArgs {
     unsigned int *retry_count;
 };
 
-// Eight bytes from `at` on, which need not be aligned (device letter buffers start on a 16-byte boundary and keep 16
-// bytes of room past the last letter): the two aligned words they lie in.
+// Four and eight bytes from `at` on, which need not be aligned: the aligned words they lie in (device letter buffers
+// keep 16 bytes of room on either side of their letters).
+__device__ __forceinline__ uint32_t four_bytes(const uint8_t *at) {
+    const uintptr_t address = reinterpret_cast<uintptr_t>(at);
+    const uint32_t *aligned = reinterpret_cast<const uint32_t *>(address & ~uintptr_t(3));
+    return __funnelshift_r(__ldg(aligned), __ldg(aligned + 1), uint32_t(address & 3u) * 8u);
+}
 __device__ __forceinline__ uint64_t eight_bytes(const uint8_t *at) {
     const uintptr_t address = reinterpret_cast<uintptr_t>(at);
-    const uint64_t *aligned = reinterpret_cast<const uint64_t *>(address & ~uintptr_t(7));
-    const uint32_t shift = uint32_t(address & 7u) * 8u;
-    const uint64_t low = __ldg(aligned), high = __ldg(aligned + 1);
-    return shift ? (low >> shift) | (high << (64u - shift)) : low;
+    const uint32_t *aligned = reinterpret_cast<const uint32_t *>(address & ~uintptr_t(3));
+    const uint32_t shift = uint32_t(address & 3u) * 8u;
+    const uint32_t a = __ldg(aligned), b = __ldg(aligned + 1), c = __ldg(aligned + 2);
+    return (uint64_t(__funnelshift_r(b, c, shift)) << 32) | __funnelshift_r(a, b, shift);
 }
 
-// Eight letters of a sequence from letter `i` on as it is read: forwards, the first in the low byte; reversed, the
-// first in the high byte (letter i is then s[length - 1 - i]). No byte before `letters`, the buffer's first, is
-// read; what lies past the sequence is for the caller to leave out.
-__device__ __forceinline__ uint64_t eight_letters(const uint8_t *letters, const uint8_t *s, int32_t length, int32_t i,
-                                                  bool reversed) {
-    if (!reversed) return eight_bytes(s + i);
-    const int64_t at = (s - letters) + length - 8 - i;
-    return at >= 0 ? eight_bytes(letters + at) : eight_bytes(letters) << (-8 * at);
-}
-
-// The furthest column a diagonal's matches take a front from `column` (row column - diagonal), eight letters a
-// step: a letter at a time, each pair of loads waited for the one before.
-__device__ __forceinline__ int32_t slide(const uint8_t *letters, const uint8_t *first, int32_t columns,
-                                         const uint8_t *second, int32_t rows, int32_t column, int32_t diagonal,
-                                         bool reversed) {
-    int32_t left = min(columns - column, rows - (column - diagonal));
-    while (left > 0) {
-        const uint64_t apart = eight_letters(letters, first, columns, column, reversed) ^
-                               eight_letters(letters, second, rows, column - diagonal, reversed);
-        const int32_t alike = apart ? (reversed ? __clzll(apart) : __ffsll(apart) - 1) >> 3 : 8;
+// The furthest column a diagonal's matches take a front from `column` (row column - diagonal): four letters, which
+// end most slides, then eight a step. (A letter at a time, each pair of loads waited for the one before.) Reversed,
+// letter i is s[length - 1 - i], so a group's first letter is its highest byte. What lies past a sequence is left
+// out by `left`, the letters to its end.
+template <bool REVERSED>
+__device__ __forceinline__ int32_t slide(const uint8_t *first, int32_t columns, const uint8_t *second, int32_t rows,
+                                         int32_t column, int32_t diagonal) {
+    const int32_t row = column - diagonal;
+    int32_t left = min(columns - column, rows - row);
+    if (left <= 0) return column;
+    const uint8_t *x = REVERSED ? first + (columns - column) : first + column;  // the next letter's place, or one past
+    const uint8_t *y = REVERSED ? second + (rows - row) : second + row;
+    const uint32_t apart = REVERSED ? four_bytes(x - 4) ^ four_bytes(y - 4) : four_bytes(x) ^ four_bytes(y);
+    if (apart) return column + min((REVERSED ? __clz(apart) : __ffs(apart) - 1) >> 3, left);
+    if (left <= 4) return column + left;
+    column += 4;
+    left -= 4;
+    x += REVERSED ? -4 : 4;
+    y += REVERSED ? -4 : 4;
+    for (;;) {
+        const uint64_t wide = REVERSED ? eight_bytes(x - 8) ^ eight_bytes(y - 8) : eight_bytes(x) ^ eight_bytes(y);
+        const int32_t alike = wide ? (REVERSED ? __clzll(wide) : __ffsll(wide) - 1) >> 3 : 8;
         column += min(alike, left);
-        if (alike < 8) break;
         left -= 8;
+        if (alike < 8 || left <= 0) return column;
+        x += REVERSED ? -8 : 8;
+        y += REVERSED ? -8 : 8;
     }
-    return column;
 }
+
+// A source front as a cost's lanes read it: a layer's diagonals lo .. lo + width - 1 (width 0: none), diagonal k's
+// value at[k].
+template <class V>
+struct SourceLayer {
+    const V *at;
+    int32_t lo;
+    uint32_t width;
+    __device__ __forceinline__ SourceLayer(const uint8_t *arena, const CostEntry &e, int32_t layer) {
+        const int32_t places = e.hi - e.lo + 1;
+        lo = e.lo;
+        width = places > 0 ? uint32_t(places) : 0u;
+        at = reinterpret_cast<const V *>(arena + e.offset) + (int64_t(layer) * places - e.lo);
+    }
+    __device__ __forceinline__ int32_t operator[](int32_t k) const {
+        return uint32_t(k - lo) < width ? int32_t(at[k]) : kUnreached<V>;
+    }
+};
 
 // A front's value on a diagonal: unreached outside its diagonals, before cost zero, or where empty.
 template <class V>
@@ -324,8 +349,8 @@ __device__ bool trace_affine(const WaveArgs &a, const uint8_t *arena, const Cost
     return false;
 }
 
-template <bool EDIT, class V>
-__global__ void __launch_bounds__(kWaveBlock) wavefront_kernel(WaveArgs a) {
+template <bool EDIT, class V, bool REVERSED>
+__global__ void __launch_bounds__(kWaveBlock, 8) wavefront_kernel(WaveArgs a) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = (int64_t(blockIdx.x) * kWaveBlock + threadIdx.x) >> 5;
     // The warp's own arena (its cost entries, then fronts), and where its fronts go on once that is full: every
@@ -359,7 +384,8 @@ __global__ void __launch_bounds__(kWaveBlock) wavefront_kernel(WaveArgs a) {
             }
             // The diagonals any source reaches, within the matrix.
             int32_t lo, hi;
-            CostEntry same_e, open_first_e, ext_first_e, open_second_e, ext_second_e;
+            CostEntry same_e = entry_of(table, -1), open_first_e = same_e, ext_first_e = same_e, open_second_e = same_e,
+                      ext_second_e = same_e;
             if (s == 0) {
                 lo = hi = 0;
             } else if (EDIT) {
@@ -385,7 +411,12 @@ __global__ void __launch_bounds__(kWaveBlock) wavefront_kernel(WaveArgs a) {
             }
             lo = max(lo, -rows);
             hi = min(hi, columns);
-            const int32_t width = hi >= lo ? hi - lo + 1 : 0;
+            // A cost that no source reaches has an empty front: its lanes' first diagonals must not wrap past lo.
+            if (hi < lo) {
+                lo = 1;
+                hi = 0;
+            }
+            const int32_t width = hi - lo + 1;
             constexpr int64_t kPlaceBytes = EDIT ? int64_t(sizeof(V)) : 3 * int64_t(sizeof(V)) + 1;
             const int64_t bytes = (kPlaceBytes * width + 15) & ~int64_t(15);
             if (used + bytes > room_end) {
@@ -428,11 +459,16 @@ __global__ void __launch_bounds__(kWaveBlock) wavefront_kernel(WaveArgs a) {
                 table[s] = e;
             }
             V *aligned = reinterpret_cast<V *>(arena + used);
+            const SourceLayer<V> same_at(arena, same_e, kAligned);
+            const SourceLayer<V> open_first_at(arena, EDIT ? same_e : open_first_e, kAligned);
+            const SourceLayer<V> ext_first_at(arena, EDIT ? same_e : ext_first_e, EDIT ? kAligned : kFirst);
+            const SourceLayer<V> open_second_at(arena, EDIT ? same_e : open_second_e, kAligned);
+            const SourceLayer<V> ext_second_at(arena, EDIT ? same_e : ext_second_e, EDIT ? kAligned : kSecond);
             bool hit = false;
             for (int32_t k = lo + lane; k <= hi; k += 32) {
                 int32_t value;
                 if (s == 0) {
-                    value = slide(a.letters, first, columns, second, rows, 0, 0, a.reversed);
+                    value = slide<REVERSED>(first, columns, second, rows, 0, 0);
                     if (!EDIT) {
                         aligned[width + (k - lo)] = V(kUnreached<V>);
                         aligned[2 * width + (k - lo)] = V(kUnreached<V>);
@@ -440,15 +476,13 @@ __global__ void __launch_bounds__(kWaveBlock) wavefront_kernel(WaveArgs a) {
                     }
                 } else if (EDIT) {
                     int move;
-                    const int32_t best = furthest_source(front_at<V>(arena, same_e, 0, k), front_at<V>(arena, same_e, 0, k - 1),
-                                                         front_at<V>(arena, same_e, 0, k + 1), k, columns, rows, move);
-                    value = best < 0 ? kUnreached<V> : slide(a.letters, first, columns, second, rows, best, k, a.reversed);
+                    const int32_t best =
+                        furthest_source(same_at[k], same_at[k - 1], same_at[k + 1], k, columns, rows, move);
+                    value = best < 0 ? kUnreached<V> : slide<REVERSED>(first, columns, second, rows, best, k);
                 } else {
-                    const int32_t same = front_at<V>(arena, same_e, kAligned, k);
-                    const int32_t opened_below = front_at<V>(arena, open_first_e, kAligned, k - 1);
-                    const int32_t extended_below = front_at<V>(arena, ext_first_e, kFirst, k - 1);
-                    const int32_t opened_above = front_at<V>(arena, open_second_e, kAligned, k + 1);
-                    const int32_t extended_above = front_at<V>(arena, ext_second_e, kSecond, k + 1);
+                    const int32_t same = same_at[k];
+                    const int32_t opened_below = open_first_at[k - 1], extended_below = ext_first_at[k - 1];
+                    const int32_t opened_above = open_second_at[k + 1], extended_above = ext_second_at[k + 1];
                     const int32_t below = max(opened_below, extended_below);
                     const int32_t above = max(opened_above, extended_above);
                     const int32_t first_gap = below >= 0 && below < columns ? below + 1 : kUnreached<V>;
@@ -464,7 +498,7 @@ __global__ void __launch_bounds__(kWaveBlock) wavefront_kernel(WaveArgs a) {
                     if (opened_above > extended_above) flag |= kOpenedSecond;
                     if (!(substituted >= gapped)) flag |= first_gap >= second_gap ? kFirst : kSecond;
                     const int32_t start = max(substituted, gapped);
-                    value = start >= 0 ? slide(a.letters, first, columns, second, rows, start, k, a.reversed) : kUnreached<V>;
+                    value = start >= 0 ? slide<REVERSED>(first, columns, second, rows, start, k) : kUnreached<V>;
                     aligned[width + (k - lo)] = V(first_gap);
                     aligned[2 * width + (k - lo)] = V(second_gap);
                     (reinterpret_cast<uint8_t *>(aligned + 3 * width))[k - lo] = flag;
@@ -495,7 +529,7 @@ __global__ void __launch_bounds__(kWaveBlock) wavefront_kernel(WaveArgs a) {
                     CigarOut out;
                     out.slot = a.slots + a.slot_offsets[pair];
                     out.capacity = 2 * (int64_t(columns) + rows) + 8;
-                    out.forward = a.reversed;
+                    out.forward = REVERSED;
                     const bool traced = EDIT ? trace_edit<V>(a, arena, table, s, columns, rows, out)
                                              : trace_affine<V>(a, arena, table, s, columns, rows, out);
                     out.flush();
@@ -556,6 +590,13 @@ __global__ void wave_gather_kernel(const char *__restrict__ slots, const int64_t
 }
 
 using WaveFn = void (*)(WaveArgs);
+
+template <bool EDIT>
+WaveFn pick_wave(bool short_columns, bool reversed) {
+    if (short_columns)
+        return reversed ? &wavefront_kernel<EDIT, int16_t, true> : &wavefront_kernel<EDIT, int16_t, false>;
+    return reversed ? &wavefront_kernel<EDIT, int32_t, true> : &wavefront_kernel<EDIT, int32_t, false>;
+}
 
 int64_t gcd(int64_t a, int64_t b) {
     while (b) {
@@ -634,8 +675,8 @@ int64_t cost_alignments(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, 
     uint32_t longest = 0;  // the longest pair's letters, and one
     read_back(gpu, &longest, keys_sorted, sizeof longest);
     const bool short_columns = int64_t(longest) <= kShortLetters;
-    WaveFn fn = plan.edit ? (short_columns ? &wavefront_kernel<true, int16_t> : &wavefront_kernel<true, int32_t>)
-                          : (short_columns ? &wavefront_kernel<false, int16_t> : &wavefront_kernel<false, int32_t>);
+    const bool reversed = !right_ties;
+    WaveFn fn = plan.edit ? pick_wave<true>(short_columns, reversed) : pick_wave<false>(short_columns, reversed);
     char *slots = trace ? gpu->walk_out.ensure<char>(size_t(slot_total) + 8) : nullptr;
     int64_t *lengths = gpu->cigar_lengths.ensure<int64_t>(size_t(pairs) + 1);
     DINARA_CUDA(cudaMemsetAsync(lengths, 0, (size_t(pairs) + 1) * sizeof(int64_t), stream));
@@ -685,7 +726,6 @@ int64_t cost_alignments(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, 
         args.ei = int32_t(plan.ei);
         args.scale = plan.scale;
         args.ceiling = plan.ceiling;
-        args.reversed = !right_ties;
         args.eqx = eqx;
         args.trace = trace;
         args.arena = arena;
