@@ -162,6 +162,34 @@ bool is_pinned(const void *pointer) {
     return attributes.type == cudaMemoryTypeHost;
 }
 
+// A copy into page-locked memory that a device copy reads next, past the caches: with the lines left dirty in eight
+// cores' caches the bus read them at 5 to 14 GB/s, from memory at 48. `to` starts on a 16-byte boundary. A small
+// copy stays in this core's cache, where it costs less.
+void copy_past_caches(uint8_t *to, const uint8_t *from, size_t bytes) {
+    if (bytes < (size_t(1) << 16)) {
+        std::memcpy(to, from, bytes);
+        return;
+    }
+    const size_t whole = bytes / 16;
+    for (size_t k = 0; k < whole; ++k)
+        _mm_stream_si128(reinterpret_cast<__m128i *>(to) + k, _mm_loadu_si128(reinterpret_cast<const __m128i *>(from) + k));
+    _mm_sfence();
+    std::memcpy(to + 16 * whole, from + 16 * whole, bytes - 16 * whole);
+}
+
+// copy_past_caches shared by eight threads, or fewer for a small copy (about half a megabyte each).
+void stage_copy(uint8_t *to, const uint8_t *from, size_t bytes) {
+    const int threads = int(std::min<size_t>(8, bytes / (size_t(1) << 19) + 1));
+    const size_t part = ((bytes + threads - 1) / threads + 63) & ~size_t(63);
+    std::thread helpers[7];
+    for (int t = 1; t < threads; ++t) {
+        const size_t begin = std::min(bytes, t * part), end = std::min(bytes, begin + part);
+        helpers[t - 1] = std::thread([=] { copy_past_caches(to + begin, from + begin, end - begin); });
+    }
+    copy_past_caches(to, from, std::min(bytes, part));
+    for (int t = 1; t < threads; ++t) helpers[t - 1].join();
+}
+
 // Copies `bytes` of host memory to the device on the context's stream, through page-locked staging
 // unless the caller's memory is page-locked already. A copy of one slice is not waited for with `settled` false:
 // the entry point then uses that staging for nothing else, and waits for its stream before it returns.
@@ -172,12 +200,18 @@ void to_device(dinara_gpu *gpu, void *device, const void *host, size_t bytes, di
         DINARA_CUDA(cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, gpu->stream));
         return;
     }
-    // Staged a slice at a time, each copy overlapping the next slice's memcpy.
+    // Staged a slice at a time, each copy overlapping the next slice's staging.
     const size_t slice = size_t(64) << 20;
     uint8_t *stage = staging.ensure<uint8_t>(std::min(bytes, 2 * slice));
     if (bytes <= slice) {
-        std::memcpy(stage, host, bytes);
-        DINARA_CUDA(cudaMemcpyAsync(device, stage, bytes, cudaMemcpyHostToDevice, gpu->stream));
+        // One slice goes in quarters, or pieces of 2 MB, each copy overlapping the next piece's staging.
+        const size_t piece = std::max(size_t(2) << 20, ((bytes + 3) / 4 + 63) & ~size_t(63));
+        for (size_t at = 0; at < bytes; at += piece) {
+            const size_t n = std::min(piece, bytes - at);
+            stage_copy(stage + at, static_cast<const uint8_t *>(host) + at, n);
+            DINARA_CUDA(cudaMemcpyAsync(static_cast<uint8_t *>(device) + at, stage + at, n, cudaMemcpyHostToDevice,
+                                        gpu->stream));
+        }
         if (settled) DINARA_CUDA(cudaStreamSynchronize(gpu->stream));
         return;
     }
@@ -193,7 +227,7 @@ void to_device(dinara_gpu *gpu, void *device, const void *host, size_t bytes, di
         const size_t n = std::min(slice, bytes - at);
         uint8_t *buffer = stage + (bytes > slice ? half * slice : 0);
         if (used[half]) DINARA_CUDA(cudaEventSynchronize(done[half]));
-        std::memcpy(buffer, from + at, n);
+        stage_copy(buffer, from + at, n);
         DINARA_CUDA(cudaMemcpyAsync(to + at, buffer, n, cudaMemcpyHostToDevice, gpu->stream));
         DINARA_CUDA(cudaEventRecord(done[half], gpu->stream));
         used[half] = true;
@@ -225,29 +259,6 @@ void parallel_copy(uint8_t *to, const uint8_t *from, size_t bytes, int threads =
         helpers[t - 1] = std::thread([=] { std::memcpy(to + begin, from + begin, end - begin); });
     }
     std::memcpy(to, from, std::min(bytes, part));
-    for (int t = 1; t < threads; ++t) helpers[t - 1].join();
-}
-
-// A copy into page-locked memory that a device copy reads next, past the caches: with the lines left dirty in eight
-// cores' caches the bus read them at 5 to 14 GB/s, from memory at 48. `to` starts on a 16-byte boundary.
-void copy_past_caches(uint8_t *to, const uint8_t *from, size_t bytes) {
-    const size_t whole = bytes / 16;
-    for (size_t k = 0; k < whole; ++k)
-        _mm_stream_si128(reinterpret_cast<__m128i *>(to) + k, _mm_loadu_si128(reinterpret_cast<const __m128i *>(from) + k));
-    _mm_sfence();
-    std::memcpy(to + 16 * whole, from + 16 * whole, bytes - 16 * whole);
-}
-
-// copy_past_caches shared by eight threads, or fewer for a small copy (about half a megabyte each).
-void stage_copy(uint8_t *to, const uint8_t *from, size_t bytes) {
-    const int threads = int(std::min<size_t>(8, bytes / (size_t(1) << 19) + 1));
-    const size_t part = ((bytes + threads - 1) / threads + 63) & ~size_t(63);
-    std::thread helpers[7];
-    for (int t = 1; t < threads; ++t) {
-        const size_t begin = std::min(bytes, t * part), end = std::min(bytes, begin + part);
-        helpers[t - 1] = std::thread([=] { copy_past_caches(to + begin, from + begin, end - begin); });
-    }
-    copy_past_caches(to, from, std::min(bytes, part));
     for (int t = 1; t < threads; ++t) helpers[t - 1].join();
 }
 
@@ -1693,7 +1704,8 @@ void upload_tape(dinara_gpu *gpu, int64_t pairs, const char *letters, const int6
     const int64_t total = offsets[2 * pairs] - first;
     std::vector<int64_t> relative(size_t(2 * pairs + 1));
     for (int64_t k = 0; k <= 2 * pairs; ++k) relative[size_t(k)] = offsets[k] - first;
-    uint8_t *letters_device = gpu->letters.ensure<uint8_t>(size_t(total) + 16);
+    // Room for 16 bytes before the letters too: a slide over reversed letters reads whole words (ties.cu).
+    uint8_t *letters_device = gpu->letters.ensure<uint8_t>(size_t(total) + 32) + 16;
     int64_t *offsets_device = gpu->offsets.ensure<int64_t>(size_t(2 * pairs + 1));
     to_device(gpu, letters_device, letters + first, size_t(total), gpu->pinned_in, false);
     to_device(gpu, offsets_device, relative.data(), relative.size() * sizeof(int64_t), gpu->pinned_small, false);
