@@ -784,9 +784,7 @@ void sweep_long(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &ta
         for (int r = 0; r < 4; ++r) a.rows8[r] = targs.rows8[r];
         a.scores = args.scores;
         a.carry_stride = args.carry_stride;
-        // The carried columns, then (clusters) the progress words.
-        a.carry = gpu->carry.ensure<int2>(size_t(in_flight) * size_t(args.carry_stride + 2 * kLongMostWarps));
-        a.progress = a.carry + in_flight * args.carry_stride;
+        a.carry = gpu->carry.ensure<int2>(size_t(in_flight * args.carry_stride));
         if (cluster)
             DINARA_CUDA(cudaLaunchKernelEx(&config, affine_long_kernel<true>, a));
         else

@@ -10,11 +10,10 @@ namespace sweep {
 // next 16, one row behind, so each DPX instruction on 16-bit pairs moves two cells of the one pair.
 constexpr int kLongStrip = 1024;
 constexpr int kLongWarps = 8;     // most warps a block without clusters; a launch may take fewer
-constexpr int kLongChunk = 32;    // steps between barriers
+constexpr int kLongChunk = 32;    // steps of a chunk: a strip's letters and left column are read, and its base moved, once
+constexpr int kLongChunks = 2;    // chunks between barriers
 constexpr int kLongCluster = 8;   // blocks a cluster, and each one's warps
 constexpr int kLongClusterWarps = 2;
-constexpr int kLongMostWarps = 16;  // a pair's, either way
-static_assert(kLongCluster * kLongClusterWarps <= kLongMostWarps && kLongWarps <= kLongMostWarps, "progress slots");
 
 // A lane's halves hold its cells less its base, a true 32-bit value that follows them: at each chunk the
 // lane's own middle cell becomes the base. Within a lane's 32 columns two reached cells of a row differ
@@ -38,7 +37,6 @@ struct LongArgs {
     int32_t *scores;
     int2 *carry;                 // a column of (score, insertion) a pair in flight
     int64_t carry_stride;
-    int2 *progress;              // clusters: 2 * kLongMostWarps words a pair in flight
 };
 
 // Every thread of a cluster's blocks meets here; what each wrote before, the others read after.
@@ -53,12 +51,26 @@ __device__ __forceinline__ int long_last_row(int s, int rows, int columns, int l
     return min(rows, min((s + 1) * kLongStrip, columns) - low);
 }
 
+// Stores `value` at `place` in this block's shared memory, or in block `rank` of its cluster's.
+template <bool CLUSTER>
+__device__ __forceinline__ void leave_word(int *place, int rank, int value) {
+    if (CLUSTER) {
+        uint32_t remote;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                     : "=r"(remote)
+                     : "r"(uint32_t(__cvta_generic_to_shared(place))), "r"(rank));
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(value) : "memory");
+    } else {
+        *reinterpret_cast<volatile int *>(place) = value;
+    }
+}
+
 // The whole or banded score of one pair a block, or with CLUSTER a cluster of eight blocks (score_groups.mojo's recurrence, cells shifted by (row +
 // column) * extend). Warp w of the block's sweeps strips w, w + warps, ...: a strip's virtual lane v runs one
 // row behind lane v - 1, whose last column reaches it from the lane's own low half or by one shuffle, and the
 // column left of a strip comes from the strip before through `carry`, a chunk of 32 rows at a time. Warps
-// meet at one barrier a chunk; a warp takes its next chunk when the strip before has, by the last barrier,
-// left every row the chunk reads, else sits the round out. Strips of a band start lower one after
+// meet at one barrier every two chunks and leave how far they are with the warp of the next strip; a warp takes
+// a chunk when the strip before had, by the last barrier, left every row it reads, else waits for the next. Strips of a band start lower one after
 // another, so about (width + 1,024) / 1,100 of them run at once.
 //
 // Each step is 16 x 5 instructions of the DPX and permute pipe for 32 x 32 cells a warp (16-bit pairs run at the
@@ -68,8 +80,8 @@ __device__ __forceinline__ int long_last_row(int s, int rows, int columns, int l
 //
 // Eight warps on one SM share its four issue ports, and a pair of 50,000 letters keeps them all for each of its
 // rows; a batch too small to fill the GPU with pairs takes a cluster a pair instead, neighbouring strips on
-// different SMs, a warp or less a port. Its warps meet at a cluster barrier a chunk and keep their progress in
-// global memory, which the barrier's release and acquire order.
+// different SMs, a warp or less a port. Its warps meet at a cluster barrier, whose release and acquire order the
+// column in global memory and the words left in one another's shared memory.
 //
 // A banded strip sweeps its rows alone, every cell above or left of them unreached; the score is then
 // the best over paths within the swept rows, the whole matrix's when the band proves it
@@ -79,8 +91,9 @@ __global__ void __launch_bounds__(32 * (CLUSTER ? kLongClusterWarps : kLongWarps
     affine_long_kernel(LongArgs p) {
     constexpr int C = 16;
     __shared__ uint32_t rows8[4];
-    // By round parity: each warp's strip and the steps it has done.
-    __shared__ int2 block_progress[CLUSTER ? 1 : 2 * kLongMostWarps];
+    // By round parity: for each of the block's warps, the strip and steps of the warp before it; and whether the
+    // last strip is done.
+    __shared__ int left_by[2][CLUSTER ? kLongClusterWarps : kLongWarps][2], finished[2];
     if (threadIdx.x < 4) rows8[threadIdx.x] = p.rows8[threadIdx.x];
 
     const int lane = threadIdx.x & 31;
@@ -89,8 +102,9 @@ __global__ void __launch_bounds__(32 * (CLUSTER ? kLongClusterWarps : kLongWarps
     const int rank = CLUSTER ? int(blockIdx.x % kLongCluster) : 0;  // clusters are consecutive blocks
     const int warps = int(blockDim.x >> 5) * (CLUSTER ? kLongCluster : 1);
     const int warp = CLUSTER ? int(threadIdx.x >> 5) * kLongCluster + rank : int(threadIdx.x >> 5);
-    volatile int *progress =
-        reinterpret_cast<volatile int *>(CLUSTER ? p.progress + int64_t(first_item) * 2 * kLongMostWarps : block_progress);
+    const int own = int(threadIdx.x >> 5);  // the warp's place in its block, and the next strip's warp's
+    const int next_warp = (warp + 1) % warps;
+    const int next_own = CLUSTER ? next_warp / kLongCluster : next_warp, next_rank = CLUSTER ? next_warp % kLongCluster : 0;
     auto meet = [&] {
         if (CLUSTER)
             cluster_barrier();
@@ -117,10 +131,11 @@ __global__ void __launch_bounds__(32 * (CLUSTER ? kLongClusterWarps : kLongWarps
                 high = from + width - 1;
             }
         }
-        meet();  // the last pair's progress and carry are read
-        if (rank == 0 && threadIdx.x < 2 * kLongMostWarps) {
-            progress[2 * threadIdx.x] = -1;
-            progress[2 * threadIdx.x + 1] = 0;
+        meet();  // the last pair's words and column are read
+        if (lane < 2) {
+            left_by[lane][own][0] = -1;
+            left_by[lane][own][1] = 0;
+            finished[lane] = 0;
         }
         meet();
 
@@ -131,28 +146,29 @@ __global__ void __launch_bounds__(32 * (CLUSTER ? kLongClusterWarps : kLongWarps
         uint32_t edgeH = 0, edgeI = 0, above_left = 0, send = 0, before = 0;
         int32_t base = 0;
         // Every round some strip's chunk is ready (the first unfinished strip's always is), so the rounds
-        // end within the sum of all strips' chunks: when the last strip's warp has moved past it, which every
-        // warp reads as of the same barrier.
+        // end within the sum of all strips' chunks: when the last strip is done, which every warp reads as of the
+        // same barrier.
         for (int round = 0;; ++round) {
-            const int before_round = ((round + 1) & 1) * kLongMostWarps;
-            if (progress[2 * (before_round + (strips - 1) % warps)] > strips - 1) break;
-            bool ready = strip < strips;
-            if (ready && done == 0) {
-                first_row = long_first_row(strip, high);
-                last_row = long_last_row(strip, rows, cols, low);
-                previous_last = strip > 0 ? long_last_row(strip - 1, rows, cols, low) : rows;
-                total = last_row - first_row + 1 + 63;
-            }
-            if (ready && strip > 0) {
-                // The strip before has left every row of this chunk (its virtual lane 63 leaves row r at its
-                // step r - its first row + 64) by the last barrier.
-                const int last_read = min(first_row - 1 + done + kLongChunk, previous_last);
-                const int needed = last_read - long_first_row(strip - 1, high) + 64;
-                const int at = 2 * (before_round + (strip - 1) % warps);
-                const int their_strip = progress[at], their_done = progress[at + 1];
-                ready = their_strip > strip - 1 || (their_strip == strip - 1 && their_done >= needed);
-            }
-            if (ready) {
+            const int before_round = (round + 1) & 1;
+            if (*const_cast<volatile int *>(&finished[before_round])) break;
+            const int their_strip = *const_cast<volatile int *>(&left_by[before_round][own][0]);
+            const int their_done = *const_cast<volatile int *>(&left_by[before_round][own][1]);
+            for (int chunk = 0; chunk < kLongChunks; ++chunk) {
+                bool ready = strip < strips;
+                if (ready && done == 0) {
+                    first_row = long_first_row(strip, high);
+                    last_row = long_last_row(strip, rows, cols, low);
+                    previous_last = strip > 0 ? long_last_row(strip - 1, rows, cols, low) : rows;
+                    total = last_row - first_row + 1 + 63;
+                }
+                if (ready && strip > 0) {
+                    // The strip before has left every row of this chunk (its virtual lane 63 leaves row r at its
+                    // step r - its first row + 64) by the last barrier.
+                    const int last_read = min(first_row - 1 + done + kLongChunk, previous_last);
+                    const int needed = last_read - long_first_row(strip - 1, high) + 64;
+                    ready = their_strip > strip - 1 || (their_strip == strip - 1 && their_done >= needed);
+                }
+                if (!ready) break;
                 const bool from_top = first_row == 1;
                 const int t0 = done + 1;
                 if (done == 0) {
@@ -288,15 +304,15 @@ __global__ void __launch_bounds__(32 * (CLUSTER ? kLongClusterWarps : kLongWarps
                     }
                 }
                 done += kLongChunk;
-                if (done >= total) {
-                    strip += warps;
-                    done = 0;
-                }
+                if (done < total) continue;
+                // The strip is done.
+                if (strip + 1 == strips && lane < (CLUSTER ? kLongCluster : 1))
+                    leave_word<CLUSTER>(&finished[round & 1], lane, 1);
+                strip += warps;
+                done = 0;
+                break;
             }
-            if (lane == 0) {
-                progress[2 * ((round & 1) * kLongMostWarps + warp)] = strip;
-                progress[2 * ((round & 1) * kLongMostWarps + warp) + 1] = done;
-            }
+            if (lane < 2) leave_word<CLUSTER>(&left_by[round & 1][next_own][lane], next_rank, lane == 0 ? strip : done);
             meet();
         }
     }
