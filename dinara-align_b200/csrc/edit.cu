@@ -35,22 +35,24 @@ constexpr unsigned kFull = 0xffffffffu;
 // A DNA letter's code, the same for planes and text: bits 1-2 of its ASCII byte (A 0, C 1, T 2, G 3).
 __device__ __forceinline__ uint32_t dna_code(uint32_t byte) { return (byte >> 1) & 3u; }
 
-// The Myers/Hyyro step of one word (device_edit.mojo:56-75): `carry` is the step into the word's top
-// (-1, 0, +1); returns the step out of its bottom bit.
-__device__ __forceinline__ int myers_word(uint64_t equal, uint64_t &positive, uint64_t &negative, int carry) {
+// The Myers/Hyyro step of one word (device_edit.mojo:56-75): `up` and `down` say whether the step into the word's top
+// is +1 or -1 (at most one is set), and become the step out of its bottom bit. Two bits a step, not its sign: the bits
+// come out of the word and go into the next one by a shift each, with no comparison.
+__device__ __forceinline__ void myers_word(uint64_t equal, uint64_t &positive, uint64_t &negative, uint32_t &up,
+                                           uint32_t &down) {
     const uint64_t vp = positive, vm = negative;
-    const uint64_t carry_negative = carry < 0 ? 1ull : 0ull, carry_positive = carry > 0 ? 1ull : 0ull;
     const uint64_t crossing = equal | vm;
-    equal |= carry_negative;
+    equal |= uint64_t(down);
     const uint64_t horizontal = (((equal & vp) + vp) ^ vp) | equal;
     uint64_t plus = vm | ~(horizontal | vp);
     uint64_t minus = vp & horizontal;
-    const int out = int((plus >> 63) & 1ull) - int((minus >> 63) & 1ull);
-    plus = (plus << 1) | carry_positive;
-    minus = (minus << 1) | carry_negative;
+    const uint32_t up_out = uint32_t(plus >> 63), down_out = uint32_t(minus >> 63);
+    plus = (plus << 1) | uint64_t(up);
+    minus = (minus << 1) | uint64_t(down);
     positive = minus | ~(crossing | plus);
     negative = plus & crossing;
-    return out;
+    up = up_out;
+    down = down_out;
 }
 
 __device__ __forceinline__ uint64_t shfl_down64(uint64_t v, int width) {
@@ -134,10 +136,23 @@ __global__ void __launch_bounds__(kBlock) band_kernel(BandArgs a) {
         int next_slide = last > 0 ? delta + e + 1 + 64 : INT_MAX;
         int next_col = 1;
         int next_time = 1 + member + (next_slide == 1 ? 1 : 0);
-        uint32_t letter = live && m > 0 ? __ldg(text) : 0u;
-        int hout = 0;
+        // A column's words of its letter's plane are read a column early, and its letter two, so that no step waits
+        // for either (windows of more words a lane keep their registers and read them in the step).
+        constexpr bool AHEAD = K <= 6;
+        uint32_t letter = live && m > 0 ? __ldg(text) : 0u, letter_after = live && m > 1 ? __ldg(text + 1) : 0u;
+        uint64_t equals[AHEAD ? K : 1];
+        auto read_ahead = [&](const uint64_t *words_at, int held_words, uint32_t code) {
+#pragma unroll
+            for (int i = 0; i < K; ++i)
+                if (AHEAD) equals[AHEAD ? i : 0] = i < held_words ? __ldg(words_at + 4 * i + code) : 0ull;
+        };
+        if (AHEAD && dna && live && m > 0) {
+            const bool slides_first = next_slide == 1;
+            read_ahead(mine + (slides_first ? 4 : 0), held - (slides_first ? 1 : 0), dna_code(letter));
+        }
+        uint32_t hout = 0;  // the step out of the lane's last word: bit 0 up, bit 1 down
         for (int step = 1; step <= warp_steps; ++step) {
-            const int from_above = G > 1 ? __shfl_up_sync(kFull, hout, 1, G) : 0;
+            const uint32_t from_above = G > 1 ? __shfl_up_sync(kFull, hout, 1, G) : 0u;
             const bool due = live && next_col <= m && step == next_time;
             const bool slides = due && next_col == next_slide;
             uint64_t belowP = 0, belowM = 0;
@@ -167,28 +182,32 @@ __global__ void __launch_bounds__(kBlock) band_kernel(BandArgs a) {
                     next_slide = base < last ? next_slide + 64 : INT_MAX;
                 }
                 const uint32_t here = letter;
-                if (c < m) letter = __ldg(text + c);  // the next column's letter, early
-                int carry = member == 0 ? 1 : from_above;
+                letter = letter_after;
+                if (c + 1 < m) letter_after = __ldg(text + c + 1);
+                const uint32_t carry = member == 0 ? 1u : from_above;
+                uint32_t up = carry & 1u, down = carry >> 1;
                 const uint32_t code = dna_code(here);
 #pragma unroll
                 for (int i = 0; i < K; ++i) {
                     if (i < held) {
                         uint64_t eq;
                         if (dna) {
-                            eq = __ldg(mine + 4 * i + code);
+                            eq = AHEAD ? equals[AHEAD ? i : 0] : __ldg(mine + 4 * i + code);
                         } else {
                             eq = 0;
                             const int first_row = (base + member * K + i) * 64;
                             const int rows = min(64, n - first_row);
                             for (int j = 0; j < rows; ++j) eq |= uint64_t(pattern[first_row + j] == here) << j;
                         }
-                        carry = myers_word(eq, P[i], M[i], carry);
+                        myers_word(eq, P[i], M[i], up, down);
                     }
                 }
-                hout = carry;
+                hout = up | (down << 1);
                 if (member == 0) above += 1;
                 next_col = c + 1;
-                next_time = step + 1 + (next_col == next_slide ? 1 : 0);
+                const int slides_next = next_col == next_slide ? 1 : 0;
+                next_time = step + 1 + slides_next;
+                if (AHEAD && dna && next_col <= m) read_ahead(mine + 4 * slides_next, held - slides_next, dna_code(letter));
             }
         }
         // The distance: the row above the window plus every vertical step down to the pattern's last row.
