@@ -26,6 +26,7 @@
 #include "free_kernel.cuh"
 #include "long_kernel.cuh"
 #include "pack.cuh"
+#include "record_kernel.cuh"
 
 namespace dinara {
 
@@ -44,7 +45,8 @@ struct WalkArgs {
     const uint64_t *decisions;
     const uint64_t *decisions_extra;  // the band's leftovers, swept whole afterwards
     // Per pair: 0 whole matrix, 1 band, 2 whole matrix in decisions_extra, 3 and 4 the 16-bit pair band's
-    // planes over 64 and 32 diagonals, 5 a band-recorded pair's strips over its proven width (widths[k]).
+    // planes over 64 and 32 diagonals, 5 a band-recorded pair's strips over its proven width (widths[k]), 6 and 7
+    // the 16-bit pair sweep's planes of the whole matrix, in decisions and in decisions_extra.
     const uint8_t *layouts;
     const int32_t *widths;
     const int64_t *decision_offsets;
@@ -112,13 +114,15 @@ __global__ void walk_kernel(WalkArgs a) {
     };
     if (rows > 0 && cols > 0) {
         const int layout = a.layouts[k];
-        const uint64_t *decisions = layout == 2 ? a.decisions_extra : a.decisions;
-        const int G = record_lanes(uint32_t(cols), a.uniform);
+        const uint64_t *decisions = layout == 2 || layout == 7 ? a.decisions_extra : a.decisions;
+        const bool pair_planes = layout >= 6;  // its lanes' rows start together, and a stop sets both moves' bits
+        const int G = record_lanes(uint32_t(cols), a.uniform && !pair_planes);
         const int lane_shift = __ffs(G * 16) - 1;  // a strip is G lanes of 16 columns
         const bool banded = layout == 1 || layout == 3 || layout == 4;
-        const bool planes = layout == 3 || layout == 4;
+        const bool planes = layout == 3 || layout == 4 || pair_planes;
         const int width = layout == 4 ? kBandWidth / 2 : kBandWidth;  // layout 4: the narrow band's 32
-        const int rows_pad = banded ? ((rows + 3) & ~3) : (((rows + 2) | 3) + 1);
+        const int rows_pad = banded || pair_planes ? ((rows + 3) & ~3) : (((rows + 2) | 3) + 1);
+        const int skew = pair_planes ? 0 : 3;  // a lane's rows lie this far into their sectors, by its number
         const int low = banded ? band_low_for_width(rows, cols, width) : 0;
         const int64_t base = a.decision_offsets[k];
         // Layout 5: the strip under the walk, its swept rows and its first word (past the earlier strips').
@@ -145,7 +149,7 @@ __global__ void walk_kernel(WalkArgs a) {
         constexpr uint32_t per_word = 32 / BITS;
         uint32_t row_word_at = ~0u, column_word_at = ~0u, row_word = 0, column_word = 0;
         while (row > 0 && column > 0) {
-            int64_t at;
+            int64_t at, ahead;  // this step's word, and the one sixteen steps on along the diagonal
             int slot_in;
             if (layout == 5) {
                 // Strips are left behind right to left: step back over each one the column has passed.
@@ -166,6 +170,7 @@ __global__ void walk_kernel(WalkArgs a) {
                 const int member = within / 16;
                 slot_in = within % 16;
                 at = base + strip_at + int64_t(member) * strip_pad + (row - strip_first + (member & 3));
+                ahead = within >= 16 ? at - strip_pad - 16 : at - 16;
             } else {
                 // The band's layout: place o = column - row - low, a lane of 16 places a block of rows. The
                 // proof keeps every optimal path inside the band; a place outside it would read another
@@ -180,9 +185,10 @@ __global__ void walk_kernel(WalkArgs a) {
                 const int off = column - 1;
                 const int member = (off & ((1 << lane_shift) - 1)) >> 4;
                 const int64_t whole_at =
-                    base + int64_t((off >> lane_shift) * G + member) * rows_pad + (row - 1 + (member & 3));
+                    base + int64_t((off >> lane_shift) * G + member) * rows_pad + (row - 1 + (member & skew));
                 const int64_t band_at = base + int64_t(place >> 4) * rows_pad + (row - 1);
                 at = banded ? band_at : whole_at;
+                ahead = banded || off < 16 ? at - 16 : at - rows_pad - 16;  // the lane before's, or near it across strips
                 slot_in = (banded ? place : off) & 15;
             }
             if ((at & ~int64_t(3)) != sector) {
@@ -193,6 +199,9 @@ __global__ void walk_kernel(WalkArgs a) {
                 held1 = uint64_t(low_words.z) | (uint64_t(low_words.w) << 32);
                 held2 = uint64_t(high_words.x) | (uint64_t(high_words.y) << 32);
                 held3 = uint64_t(high_words.z) | (uint64_t(high_words.w) << 32);
+                // Most steps keep to the diagonal: the sector sixteen steps on, on its way from memory meanwhile (the
+                // decisions of a batch are past L2, and each read of them waited for alone).
+                if (row > 16 && ahead >= base) asm volatile("prefetch.global.L2 [%0];" ::"l"(decisions + ahead));
             }
             const int within_sector = int(at & 3);
             const uint64_t word = within_sector == 0   ? held0
@@ -203,7 +212,8 @@ __global__ void walk_kernel(WalkArgs a) {
             // insertion extending, 16 bits each; inserting wins over deleting as decide() orders them.
             // Otherwise a nibble a place.
             const uint32_t deleting = uint32_t(word >> slot_in) & 1u, inserting = uint32_t(word >> (16 + slot_in)) & 1u;
-            const uint32_t from_planes = (inserting ? 2u : deleting) | ((uint32_t(word >> (32 + slot_in)) & 1u) << 2) |
+            const uint32_t source = pair_planes ? deleting | (inserting << 1) : inserting ? 2u : deleting;
+            const uint32_t from_planes = source | ((uint32_t(word >> (32 + slot_in)) & 1u) << 2) |
                                          ((uint32_t(word >> (48 + slot_in)) & 1u) << 3);
             const uint32_t nibble = planes ? from_planes : uint32_t(word >> (4 * slot_in)) & 15u;
             if (a.local && state == 0 && (nibble & 3u) == 3u) break;
@@ -355,9 +365,18 @@ __global__ void cigar_text_kernel(const char *__restrict__ slots, const int64_t 
     }
 }
 
+// The words a whole-matrix pair records: its strips' lanes' rows, to a whole sector, skewed by the lane for the 32-bit
+// sweep, not for the 16-bit one's planes.
+__device__ __forceinline__ int64_t whole_words(const PairShape &sh, bool uniform, bool planes) {
+    const int G = record_lanes(sh.columns, uniform && !planes);
+    const int W = G * 16;
+    const int64_t rows_pad = planes ? (int64_t(sh.rows) + 3) & ~int64_t(3) : ((int64_t(sh.rows) + 2) | 3) + 1;
+    return (int64_t(sh.columns) + W - 1) / W * G * rows_pad;
+}
+
 __global__ void slot_sizes_kernel(const PairShape *__restrict__ shapes, int64_t first_pair, int64_t count, bool uniform,
-                                  int32_t band_pair_limit, bool band, const int32_t *__restrict__ widths,
-                                  int64_t *__restrict__ decision_words, int64_t *__restrict__ slot_bytes,
+                                  int32_t band_pair_limit, bool band, PairLimits limits,
+                                  const int32_t *__restrict__ widths, int64_t *__restrict__ decision_words, int64_t *__restrict__ slot_bytes,
                                   uint8_t *__restrict__ layouts) {
     const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (k >= count) return;
@@ -373,11 +392,10 @@ __global__ void slot_sizes_kernel(const PairShape *__restrict__ shapes, int64_t 
         layout = int64_t(sh.rows) + sh.columns <= band_pair_limit ? 3 : 1;
         words = int64_t(kBandLanes) * ((int64_t(sh.rows) + 3) & ~int64_t(3));
     } else if (sh.rows > 0 && sh.columns > 0) {
-        const int G = record_lanes(sh.columns, uniform);
-        const int W = G * 16;
-        const int64_t strips = (sh.columns + W - 1) / W;
-        const int64_t rows_pad = ((int64_t(sh.rows) + 2) | 3) + 1;
-        words = strips * G * rows_pad;
+        // The 16-bit pair sweep's planes (layout 6), or a nibble a cell.
+        const bool planes = takes_pairs16(limits, sh.rows, sh.columns, affine_shape_for(sh.columns, true), true);
+        words = whole_words(sh, uniform, planes);
+        if (planes) layout = 6;
     }
     decision_words[k] = words;
     slot_bytes[k] = 4 * (int64_t(sh.rows) + sh.columns) + 8;
@@ -413,13 +431,12 @@ __global__ void swept_cells_kernel(const PairShape *__restrict__ shapes, int64_t
 
 // The whole-matrix words of each leftover pair of the band.
 __global__ void leftover_words_kernel(const PairShape *__restrict__ shapes, const uint32_t *__restrict__ leftovers,
-                                      int64_t count, bool uniform, int64_t *__restrict__ words) {
+                                      int64_t count, bool uniform, PairLimits limits, int64_t *__restrict__ words) {
     const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const PairShape sh = shapes[leftovers[k]];
-    const int G = record_lanes(sh.columns, uniform);
-    const int W = G * 16;
-    words[k] = (int64_t(sh.columns) + W - 1) / W * G * (((int64_t(sh.rows) + 2) | 3) + 1);
+    words[k] = whole_words(
+        sh, uniform, takes_pairs16(limits, sh.rows, sh.columns, affine_shape_for(sh.columns, true), true));
 }
 
 // The pairs of [first, first + count) a block sweeps when scoring (kWideRows x kWideColumns or more), listed.
@@ -432,14 +449,16 @@ __global__ void long_pairs_kernel(const PairShape *__restrict__ shapes, int64_t 
 }
 
 // Points each leftover's decisions at its place in the extra buffer and marks its layout.
-__global__ void leftover_places_kernel(const uint32_t *__restrict__ leftovers, int64_t count, int64_t first_pair,
+__global__ void leftover_places_kernel(const PairShape *__restrict__ shapes, const uint32_t *__restrict__ leftovers,
+                                       int64_t count, int64_t first_pair, PairLimits limits,
                                        const int64_t *__restrict__ offsets, int64_t *__restrict__ decision_offsets,
                                        uint8_t *__restrict__ layouts) {
     const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const int64_t pair = int64_t(leftovers[k]) - first_pair;
+    const PairShape sh = shapes[leftovers[k]];
     decision_offsets[pair] = offsets[k];
-    layouts[pair] = 2;
+    layouts[pair] = takes_pairs16(limits, sh.rows, sh.columns, affine_shape_for(sh.columns, true), true) ? 7 : 2;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -521,6 +540,20 @@ PairsLaunch pick_pairs(int cls, bool local, bool hits, int bits, int letters) {
         default: DINARA_PAIRS(32, 16, 32)
     }
 #undef DINARA_PAIRS
+}
+
+// Recording; its classes are the recording sweep's (16 columns a lane).
+PairsLaunch pick_record(int cls, bool local, int bits, int letters) {
+#define DINARA_RECORD(G)                                                                                             \
+    return pairs_launch(local ? &record_pairs_kernel<G, true, 2> : &record_pairs_kernel<G, false, 2>,                \
+                        local ? &record_pairs_kernel<G, true, 8> : &record_pairs_kernel<G, false, 8>, bits, G, 16, letters);
+    switch (cls) {
+        case 0: DINARA_RECORD(4)
+        case 1: DINARA_RECORD(8)
+        case 2: DINARA_RECORD(16)
+        default: DINARA_RECORD(32)
+    }
+#undef DINARA_RECORD
 }
 
 int persistent_blocks(dinara_gpu *gpu, KernelFn fn, int threads = kBlock, size_t shared = 0) {
@@ -877,8 +910,9 @@ void affine_launch_all(dinara_gpu *gpu, const AffineBatch &batch, const AffineTa
             continue;
         }
         if (pairs16) {
-            pair_sweeps.push_back({pick_pairs(cls, batch.local, false, batch.bits, table.size), b.begin[bucket],
-                                   b.end[bucket]});
+            pair_sweeps.push_back({record ? pick_record(cls, batch.local, batch.bits, table.size)
+                                          : pick_pairs(cls, batch.local, false, batch.bits, table.size),
+                                   b.begin[bucket], b.end[bucket]});
             continue;
         }
         KernelFn fn = band_record ? &affine_kernel<32, 16, false, true, 2, false, false, true>
@@ -963,6 +997,35 @@ PairLimits whole_limits_of(const AffineBatch &batch, const AffineTable &table) {
             step = std::max(step, std::abs(v));
         }
     limits.whole = 30000 / std::max(step, 1) - 4;
+    return limits;
+}
+
+// Which whole-matrix pairs the 16-bit recording sweep takes: every half at zero or more, record_bias above its
+// value, and below 32,768. Locally a pair of the 16-bit score sweeps, its rows its hit's; globally, a
+// shifted cell reaches at most the largest shifted entry a column swept.
+PairLimits record_limits_of(const AffineBatch &batch, const AffineTable &table) {
+    PairLimits limits;
+    if (std::abs(table.open) + std::abs(table.extend) > 2000) return limits;
+    const int32_t bias = record_bias(table.open, table.extend);
+    if (batch.local) {
+        limits = whole_limits_of(batch, table);
+        limits.whole = std::max(limits.whole - bias, 0);
+    } else {
+        if (batch.bits == 2 && !table.packed16) return limits;
+        int32_t best = 1;
+        for (int r = 0; r < table.size; ++r)
+            for (int c = 0; c < table.size; ++c) {
+                const int32_t v = table.entries[r * 32 + c] - 2 * table.extend;
+                if (v < -128 || v > 127) return limits;
+                best = std::max(best, v);
+            }
+        limits.local = 1;  // the local form of the limit
+        limits.best = best;
+        limits.whole = 32000 - 2 * bias;
+    }
+    limits.wide = 0;
+    limits.long_strips = 0;
+    limits.record = 1;
     return limits;
 }
 
@@ -1603,8 +1666,16 @@ int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &whole_batch, const
     const int32_t *widths = band && !batch.local && batch.max_rows >= kWideRows && batch.max_columns >= kWideColumns
                                 ? proven_band_widths(gpu, batch, table, scores, first_pair, count)
                                 : nullptr;
+    PairLimits limits = record_limits_of(batch, table);
+    // A local pair without its hit found has no known end: only hits' rows take the 16-bit sweep.
+    if (batch.local && batch.shapes == whole_batch.shapes) limits.whole = 0;
+    // Two pairs a group pay where pairs fill the GPU: a global row takes the 16-bit sweep about twice as long, and
+    // a few hundred leftovers of a band 370 us against 195. Locally it is the shorter either way.
+    const int64_t full = 32 * int64_t(gpu->multiprocessors);
+    PairLimits left_limits = limits;
+    if (!batch.local && (band || count < full)) limits.whole = 0;
     slot_sizes_kernel<<<blocks, threads, 0, gpu->stream>>>(batch.shapes, first_pair, count, uniform, band_pair_limit,
-                                                           band, widths, words, slot_bytes, layouts);
+                                                           band, limits, widths, words, slot_bytes, layouts);
     gpu->launches += 1;
     DINARA_CUDA(cudaGetLastError());
     size_t scratch = 0;
@@ -1626,7 +1697,6 @@ int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &whole_batch, const
     int64_t *ends = gpu->spans.ensure<int64_t>(size_t(count) + 1);
     int64_t *lengths = gpu->cigar_lengths.ensure<int64_t>(2 * (size_t(count) + 1));
     int64_t *run_counts = lengths + (count + 1);
-    PairLimits limits;
     limits.band = band ? pair_limit_of(table) : 0;
     limits.band_widths = widths;
     limits.band_first = first_pair;
@@ -1665,11 +1735,12 @@ int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &whole_batch, const
         read_back(gpu, &left, leftover_count, sizeof left);
         if (left > 0) {
             // The band's leftovers, swept whole: their decisions in the extra buffer.
+            if (left < full) left_limits.whole = 0;
             int64_t *left_words = gpu->thresholds.ensure<int64_t>(2 * (size_t(left) + 1) + 2);
             int64_t *left_offsets = left_words + (left + 1);
             const unsigned left_blocks = unsigned((left + threads - 1) / threads);
             leftover_words_kernel<<<left_blocks, threads, 0, gpu->stream>>>(batch.shapes, leftovers, left, uniform,
-                                                                            left_words);
+                                                                            left_limits, left_words);
             gpu->launches += 1;
             DINARA_CUDA(cudaGetLastError());
             DINARA_CUDA(cudaMemsetAsync(left_words + left, 0, sizeof(int64_t), gpu->stream));
@@ -1680,11 +1751,11 @@ int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &whole_batch, const
             int64_t extra_total = 0;
             read_back(gpu, &extra_total, left_offsets + left, sizeof(int64_t));
             extra = gpu->decisions_extra.ensure<uint64_t>(size_t(extra_total) + 8);
-            leftover_places_kernel<<<left_blocks, threads, 0, gpu->stream>>>(leftovers, left, first_pair, left_offsets,
-                                                                             word_offsets, layouts);
+            leftover_places_kernel<<<left_blocks, threads, 0, gpu->stream>>>(batch.shapes, leftovers, left, first_pair,
+                                                                             left_limits, left_offsets, word_offsets, layouts);
             gpu->launches += 1;
             DINARA_CUDA(cudaGetLastError());
-            const Schedule again = dinara::schedule(gpu, batch.shapes, leftovers, 0, left, true, false);
+            const Schedule again = dinara::schedule(gpu, batch.shapes, leftovers, 0, left, true, false, left_limits);
             KernelArgs extra_args = args;
             extra_args.decisions = extra;
             affine_launch_all(gpu, batch, table, again, true, extra_args);

@@ -908,6 +908,7 @@ __global__ void __launch_bounds__(kBlock, 2) affine_pairs_kernel(KernelArgs p, T
                     cut.first_word += uint32_t(first / (32 / BITS));
                     cut.rows = hit[h] > 0 ? uint32_t(hit_row[h] - first) : 0u;
                     p.hits[pair[h]] = cut;
+                    p.scores[pair[h]] = hit[h];
                 }
             }
         } else if (LOCAL) {

@@ -20,6 +20,7 @@
 // Pairs the band does not prove go on a leftover list for the whole-matrix sweep.
 #include "affine_kernel.cuh"
 #include "banded.cuh"
+#include "record_kernel.cuh"
 
 namespace dinara {
 namespace {
@@ -278,28 +279,6 @@ __device__ __forceinline__ uint32_t pack2(int32_t low, int32_t high) {
 __device__ __forceinline__ int32_t low_half(uint32_t v) { return int32_t(int16_t(uint16_t(v & 0xFFFFu))); }
 __device__ __forceinline__ int32_t high_half(uint32_t v) { return int32_t(int16_t(uint16_t(v >> 16))); }
 
-// The halves' maximum: the DPX maximum floored at zero, which every value here already is at or above.
-__device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) { return __vimax_s16x2_relu(a, b); }
-
-// Adds to a plane `acc` (pair A's 16 places in the low half, pair B's in the high) place k's flags: set
-// where a half of `v` has bit 15 clear. `v` = b - a + 0x8000 in each half (halves in [0, 0x8000), so
-// nothing crosses between them) has bit 15 set exactly where b >= a, so a clear bit records a > b. The
-// flags move from bits 15 and 31 down to k and 16 + k by the high word of a product, added in the same
-// instruction (the FMA pipe's, leaving the ALU to the cells).
-__device__ __forceinline__ uint32_t gather_flag(uint32_t acc, uint32_t v, int k) {
-    const uint32_t flags = ~v & 0x80008000u;
-    return k == 15 ? acc + flags : __umulhi(flags, 1u << (17 + k)) + acc;
-}
-
-// b - a + c (the halves' sums in [0, 0x10000), so none crosses into the other) by two multiply-adds,
-// which the multiply-add pipe takes, leaving the ALU pipe, the recording sweep's bound, to the cells.
-__device__ __forceinline__ uint32_t difference_mad(uint32_t b, uint32_t a, uint32_t c) {
-    uint32_t biased, out;
-    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(biased) : "r"(b), "r"(1u), "r"(c));
-    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(out) : "r"(a), "r"(0xFFFFFFFFu), "r"(biased));
-    return out;
-}
-
 // LANES lanes of 16 places a lane group: a band of 32 diagonals (2 lanes, the narrow first pass) or 64
 // (4 lanes). In the narrow pass a pair whose band cannot hold both its ends goes straight to the leftover
 // list, which the wide pass takes; a pair the narrow band proves is marked as its layout 4.
@@ -426,7 +405,7 @@ __global__ void __launch_bounds__(kBlock, 2) banded_pairs_kernel(BandedBatch b) 
                         const uint32_t dn = __viaddmax_s16x2(Hup, opening2, Dup);
                         if (RECORD) {
                             const uint32_t xd = __viaddmax_s16x2(H[k], sub, 0u);  // H + sub: never below 0
-                            X[k] = max2(xd, dn);
+                            X[k] = max_halves(xd, dn);
                             // gotoh.mojo:173-186 decide: the source leaves the diagonal only where the
                             // deletion beats it; a deletion run extends only where extending beats opening.
                             deleting = gather_flag(deleting, difference_mad(xd, dn, at_least), k);               // dn > xd
@@ -445,9 +424,9 @@ __global__ void __launch_bounds__(kBlock, 2) banded_pairs_kernel(BandedBatch b) 
                     if (member == 0) reach = unreached2;
                     if (G > 2) {
                         const uint32_t further = __shfl_up_sync(kFull, reach, 1, G);
-                        if (member >= 1) reach = max2(reach, further);
+                        if (member >= 1) reach = max_halves(reach, further);
                         const uint32_t further2 = __shfl_up_sync(kFull, reach, 2, G);
-                        if (member >= 2) reach = max2(reach, further2);
+                        if (member >= 2) reach = max_halves(reach, further2);
                     }
                     if (RECORD) {
                         // Pass 2: the insertion layer (the best earlier X plus an opening), the scores, and the
@@ -460,7 +439,7 @@ __global__ void __launch_bounds__(kBlock, 2) banded_pairs_kernel(BandedBatch b) 
                         for (int k = 0; k < C; ++k) {
                             const uint32_t I = S2;
                             S2 = __viaddmax_s16x2(X[k], opening2, S2);
-                            H[k] = max2(X[k], I);
+                            H[k] = max_halves(X[k], I);
                             inserting = gather_flag(inserting, difference_mad(X[k], I, at_least), k);  // I > X
                             // The left cell's insertion beats its score plus an opening: the run extends.
                             if (k > 0) insertion_runs = gather_flag(insertion_runs, difference_mad(prevH, prevI, at_least_open), k);

@@ -108,10 +108,7 @@ __device__ void classify_pair(const PairShape *__restrict__ shapes, const uint32
         if (!record && limits.wide && shape.rows >= kWideRows && shape.columns >= kWideColumns) cls = kWideClass;
         const uint32_t width = cls == kWideClass ? 4096u : uint32_t(affine_lanes(cls) * affine_columns(cls));
         strips = empty ? 0 : (shape.columns + width - 1) / width;
-        const int64_t swept = int64_t(strips) * width;
-        const bool pairs16 = cls != kWideClass && !record && !empty && limits.whole > 0 &&
-                             (limits.local ? swept * limits.best + int64_t(shape.rows) * limits.row_step <= limits.whole
-                                           : 2 * swept <= limits.whole && 2 * int64_t(shape.rows) <= limits.whole);
+        const bool pairs16 = takes_pairs16(limits, shape.rows, shape.columns, cls, record != 0);
         if (pairs16) {
             cls += kWholePairsClass;
         } else if (!record && limits.long_strips && shape.rows >= kLongSide && shape.columns >= kLongSide) {

@@ -1,7 +1,7 @@
 // Packing the caller's letters on the device, and the longest-first schedule of a batch.
 #pragma once
 
-#include "internal.cuh"
+#include "affine.cuh"
 
 namespace dinara {
 
@@ -46,6 +46,7 @@ struct PairLimits {
     int32_t band = 0;
     int32_t whole = 0;
     int32_t local = 0;
+    int32_t record = 0;  // `whole` holds the recording sweep's pairs (else the score sweeps')
     int32_t wide = 0;
     // Scoring without a CIGAR, globally: the 16-bit strips of a long pair serve the batch's table. Then pairs of
     // at least kLongSide x kLongSide that no 16-bit pair sweep takes go to kWideClass too.
@@ -58,6 +59,17 @@ struct PairLimits {
     const int32_t *band_widths = nullptr;
     int64_t band_first = 0;
 };
+
+// Whether a non-empty pair of whole-matrix shape class `cls` takes a 16-bit pair sweep (`record`: recording).
+__host__ __device__ inline bool takes_pairs16(const PairLimits &limits, uint32_t rows, uint32_t columns, int cls,
+                                              bool record) {
+    if (limits.whole <= 0 || record != (limits.record != 0) || cls >= kWholePairsClass || rows == 0 || columns == 0)
+        return false;
+    const uint32_t width = uint32_t(affine_lanes(cls) * affine_columns(cls));
+    const int64_t swept = int64_t((columns + width - 1) / width) * width;
+    return limits.local ? swept * limits.best + int64_t(rows) * limits.row_step <= limits.whole
+                        : 2 * swept <= limits.whole && 2 * int64_t(rows) <= limits.whole;
+}
 
 // The order of pairs [first, first + count), or of the `count` pairs listed in `list` (device) when given.
 Schedule schedule(dinara_gpu *gpu, const PairShape *shapes, const uint32_t *list, int64_t first, int64_t count,
