@@ -510,7 +510,9 @@ KernelFn pick_kernel(int cls, bool local, bool record, int bits, bool smem) {
 
 // A 16-bit pair sweep's launch for a whole-matrix shape class: its kernel, its lanes and columns a lane, and the
 // threads and shared memory of a block. A profile form (8-bit letters) keeps 64 bytes a letter and column of a lane
-// for each warp, so its blocks are of four warps: two of them an SM under a 20-letter alphabet.
+// for each warp. Blocks are of two warps, so that a batch's longest pairs, which come first, go to an SM
+// each: eight warps a block gave one SM the sixteen longest (5,000 reads' hits: 4.7 ms).
+constexpr int kPairsThreads = 64;
 struct PairsLaunch {
     KernelFn fn;
     int lanes, columns, threads;
@@ -518,8 +520,8 @@ struct PairsLaunch {
 };
 
 PairsLaunch pairs_launch(KernelFn two_bits, KernelFn bytes, int bits, int lanes, int columns, int letters) {
-    if (bits == 8) return {bytes, lanes, columns, kBlock / 2, size_t(kBlock / 64) * 64 * letters * columns};
-    return {two_bits, lanes, columns, kBlock, 0};
+    return {bits == 8 ? bytes : two_bits, lanes, columns, kPairsThreads,
+            bits == 8 ? size_t(kPairsThreads / 32) * 64 * letters * columns : 0};
 }
 
 // Scores, or (`hits`, local) each hit's rows. The 20-column shape is the two-bit form's alone.
