@@ -1012,6 +1012,7 @@ PairLimits record_limits_of(const AffineBatch &batch, const AffineTable &table) 
     if (batch.local) {
         limits = whole_limits_of(batch, table);
         limits.whole = std::max(limits.whole - bias, 0);
+        limits.hits = 1;
     } else {
         if (batch.bits == 2 && !table.packed16) return limits;
         int32_t best = 1;
@@ -1025,7 +1026,6 @@ PairLimits record_limits_of(const AffineBatch &batch, const AffineTable &table) 
         limits.best = best;
         limits.whole = 32000 - 2 * bias;
     }
-    limits.wide = 0;
     limits.long_strips = 0;
     limits.record = 1;
     return limits;

@@ -47,6 +47,7 @@ struct PairLimits {
     int32_t whole = 0;
     int32_t local = 0;
     int32_t record = 0;  // `whole` holds the recording sweep's pairs (else the score sweeps')
+    int32_t hits = 0;    // recording: of hits' rows, so only pairs whose hits a score sweep has found
     int32_t wide = 0;
     // Scoring without a CIGAR, globally: the 16-bit strips of a long pair serve the batch's table. Then pairs of
     // at least kLongSide x kLongSide that no 16-bit pair sweep takes go to kWideClass too.
@@ -65,6 +66,8 @@ __host__ __device__ inline bool takes_pairs16(const PairLimits &limits, uint32_t
                                               bool record) {
     if (limits.whole <= 0 || record != (limits.record != 0) || cls >= kWholePairsClass || rows == 0 || columns == 0)
         return false;
+    // The score sweeps left a long pair (kWideClass) its whole shape and no hit.
+    if (limits.hits && limits.wide && rows >= kWideRows && columns >= kWideColumns) return false;
     const uint32_t width = uint32_t(affine_lanes(cls) * affine_columns(cls));
     const int64_t swept = int64_t((columns + width - 1) / width) * width;
     return limits.local ? swept * limits.best + int64_t(rows) * limits.row_step <= limits.whole

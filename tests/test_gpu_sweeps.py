@@ -108,6 +108,50 @@ def test_hits_in_long_targets(da, oracle, alphabet):
             assert a.query_start == (query.rfind(columns) if columns else 0)
 
 
+@pytest.mark.parametrize("entries", [(1, -1, 0, -1), (1, -3, -5, -2)])
+def test_long_pairs_beside_hits(da, oracle, entries):
+    """Pairs at and past 4,096 x 2,048 letters, whose hits no 16-bit sweep finds, in a batch of pairs whose hits it
+    does: their whole matrices are recorded."""
+    rng = np.random.default_rng(abs(sum(entries)) + 41)
+    scoring = da.Scoring.uniform(*entries)
+    refs, queries = [], []
+    for rows, columns in ((4095, 2048), (4096, 2047), (4096, 2048), (4200, 4150), (300, 200), (900, 600)):
+        source = _text(rng, columns)
+        refs.append((_text(rng, 100) + _mutated(rng, source, 0.05, "ACGT") + _text(rng, rows))[:rows])
+        queries.append(source)
+    tape = da.Tape.of(refs, queries)
+    coded = np.concatenate([oracle.codes(text) for pair in zip(refs, queries) for text in pair])
+    op, ex = oracle.kernel_gaps(scoring.opening, scoring.extension)
+    expected, cigars = oracle.batch_alignments(coded, tape.offsets, _table(scoring), 4, op, ex, oracle.LOCAL, threads=8)
+    found = da.alignments(refs, queries, scoring, da.Mode.local())
+    assert [a.score for a in found] == list(expected)
+    assert [a.cigar for a in found] == cigars
+
+
+@pytest.mark.parametrize("alphabet", ["ACGT", PROTEIN])
+@pytest.mark.parametrize("local", [False, True])
+def test_recorded_pairs_that_fill_the_gpu(da, oracle, alphabet, local):
+    """5,000 pairs: enough for the 16-bit recording globally, for a band's leftovers, and for its strips of 256
+    columns; widths a column either side of its lane groups', one strip and more, an odd pair out."""
+    rng = np.random.default_rng(len(alphabet) + local)
+    scoring = da.Scoring.uniform(2, -4, -4, -2, alphabet)
+    widths = (1, 15, 16, 17, 31, 32, 33, 64, 65, 128, 129)
+    refs, queries = [], []
+    for k in range(5001):
+        width = widths[k % len(widths)] if k >= 40 else (255, 256, 257, 512, 513, 600, 768, 769)[k % 8]
+        source = _text(rng, width, alphabet)
+        refs.append(_text(rng, 3 + k % 30, alphabet) + (source[:40 + width // 2] if k % 3 else ""))
+        queries.append(_mutated(rng, source, 0.1, alphabet) or alphabet[0])
+    tape = da.Tape.of(refs, queries)
+    coded = np.concatenate([oracle.codes(text, alphabet) for pair in zip(refs, queries) for text in pair])
+    op, ex = oracle.kernel_gaps(scoring.opening, scoring.extension)
+    expected, cigars = oracle.batch_alignments(coded, tape.offsets, _table(scoring), len(alphabet), op, ex,
+                                               oracle.LOCAL if local else oracle.GLOBAL, threads=8)
+    found = da.alignments(refs, queries, scoring, da.Mode.local() if local else da.Mode.GLOBAL)
+    assert [a.score for a in found] == list(expected)
+    assert [a.cigar for a in found] == cigars
+
+
 # ---- free ends and extensions in 16-bit halves ----------------------------------------------------------
 
 WIDTHS = (1, 8, 9, 15, 16, 17, 63, 64, 65, 127, 128, 129, 255, 256, 257, 320, 321, 512, 513, 700)
