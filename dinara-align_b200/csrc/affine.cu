@@ -1192,7 +1192,7 @@ __global__ void diagonal_counts_kernel(const PairShape *__restrict__ shapes, int
 __global__ void extension_finish_kernel(const PairShape *__restrict__ shapes, int64_t first, int64_t count,
                                         bool from_end, const int64_t *__restrict__ stops,
                                         const unsigned long long *__restrict__ diagonals,
-                                        const int64_t *__restrict__ diagonal_offsets, int64_t zdrop, int64_t slack,
+                                        const int64_t *__restrict__ diagonal_offsets, int64_t zdrop, int32_t extend,
                                         int64_t end_bonus, const int32_t *__restrict__ reach_scores,
                                         const int64_t *__restrict__ reach_spans, int32_t *__restrict__ scores,
                                         int64_t *__restrict__ spans) {
@@ -1203,6 +1203,7 @@ __global__ void extension_finish_kernel(const PairShape *__restrict__ shapes, in
     const PairShape sh = shapes[pair];
     const int64_t rows = sh.rows, columns = sh.columns;
     int64_t best = scores[pair], row = stops[k] >> 32, column = stops[k] & 0xffffffff;
+    const int64_t slack = -int64_t(extend);
     bool dropped = false;
     if (diagonals && rows > 0 && columns > 0) {
         const unsigned long long *kept = diagonals + diagonal_offsets[k];
@@ -1212,8 +1213,13 @@ __global__ void extension_finish_kernel(const PairShape *__restrict__ shapes, in
             const int64_t d = d0 + lane;
             const bool inside = d <= rows + columns;
             const unsigned long long word = inside ? kept[d] : 0ull;
-            const int32_t most = inside ? int32_t(uint32_t(word >> 32) ^ 0x80000000u) : 0;
-            const int64_t furthest = int64_t(word & 0xffffffffu);
+            // A 16-bit sweep's key (its high word zero: the cell, shifted, over its row), or a value over its row.
+            const bool key16 = word >> 32 == 0;
+            const int32_t key = int32_t(uint32_t(word) ^ 0x80000000u);
+            const int32_t most = !inside ? 0
+                                 : key16 ? (key >> 16) + int32_t(d) * extend
+                                         : int32_t(uint32_t(word >> 32) ^ 0x80000000u);
+            const int64_t furthest = key16 ? int64_t(key & 0xffff) : int64_t(word & 0xffffffffu);
             // The best up to and with this lane's: a value above zero, and the latest lane that has it (-1: the
             // best before these).
             int32_t through = inside && most > 0 && most >= best_so_far ? most : best_so_far;
@@ -1469,7 +1475,7 @@ void free_end_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTabl
     if (batch.extension) {
         extension_finish_kernel<<<unsigned((count * 32 + 255) / 256), 256, 0, gpu->stream>>>(
             batch.shapes, first, count, batch.from_end, ends, args.diagonals, args.diagonal_offsets, batch.zdrop,
-            -int64_t(table.extend), batch.end_bonus, reach_scores, reach_spans, scores, spans);
+            table.extend, batch.end_bonus, reach_scores, reach_spans, scores, spans);
         DINARA_CUDA(cudaGetLastError());
         gpu->launches += 1;
     } else if (spans) {

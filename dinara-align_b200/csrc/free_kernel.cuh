@@ -273,11 +273,12 @@ __global__ void __launch_bounds__(kBlock, 2) free_pairs_kernel(KernelArgs p, Tab
 // An extension's stop (scored.mojo:69-100 and 272-300, FROM_ORIGIN: the best cell anywhere above zero, of equal ones
 // the furthest along both sequences together, then along the reference) of two pairs a group of G lanes, in 16-bit
 // halves, no letter free. Each place's cells of a row join a key a pair, its value over its row, that moves one
-// place left a row with its anti-diagonal (row + column): place 0's key is then the lane's whole part of one
-// anti-diagonal, where later rows win ties, and only it is taken further, one a row instead of one a cell. With
-// p.diagonals it goes to that anti-diagonal's word by an atomic maximum (a Z-drop reads them in order); without,
-// to the lane's best, later anti-diagonals winning ties. Rows run on past a pair's last until its last keys
-// have moved out. (A compare and an atomic a cell in 32 bits held 10,000 pairs of 450 letters for 17.8 ms.)
+// place left a row with its anti-diagonal (row + column), from a lane's place 0 on to the place before: the lane
+// that starts the group then holds the strip's whole part of one anti-diagonal a row, where later rows win ties,
+// and it alone takes it further. With p.diagonals it goes to that anti-diagonal's word by an atomic maximum (a
+// Z-drop reads them in order); without, to the lane's best, later anti-diagonals winning ties. After the last row
+// each lane takes the keys it holds further itself. (A compare and an atomic a cell in 32 bits held 10,000 pairs
+// of 450 letters for 17.8 ms; an atomic a lane a row made their call 9.9 ms against 9.3.)
 //
 // A row's key is bits 16-31 the cell, shifted as held, bits 0-15 the row; on one anti-diagonal every cell's
 // shift is the same. Columns past a pair's end join with a weight below every real key. Eight places a lane
@@ -388,8 +389,16 @@ __global__ void __launch_bounds__(kBlock, 2) extension_pairs_kernel(KernelArgs p
             int group_rows = 0;
 #pragma unroll
             for (int h = 0; h < 2; ++h) group_rows = max(group_rows, s < strips[h] ? rows[h] : 0);
-            const int steps = group_rows > 0 ? group_rows + C - 1 + G : 0;
+            const int steps = group_rows > 0 ? group_rows - 1 + G : 0;
             const int warp_steps = warp_max(steps);
+            // A key of pair h's anti-diagonal `along`, taken further.
+            auto send = [&](int h, int32_t whole, int along) {
+                if (whole < kLeast) return;
+                if (p.diagonals)
+                    atomicMax(reinterpret_cast<uint32_t *>(p.diagonals + words[h] + along), uint32_t(whole) ^ 0x80000000u);
+                else
+                    offer(h, (whole >> 16) + along * extend, along, whole & 0xFFFF);
+            };
 
             for (int step0 = 1; step0 <= warp_steps; step0 += 16) {
                 uint32_t codes[2] = {0, 0};
@@ -399,6 +408,9 @@ __global__ void __launch_bounds__(kBlock, 2) extension_pairs_kernel(KernelArgs p
 #pragma unroll 2
                 for (int u = 0; u < 16; ++u) {
                     const int row = step0 + u - member;
+                    // The next lane's place 0 one row up, on the anti-diagonal of this lane's last place there.
+                    const int32_t further_a = __shfl_down_sync(kFull, key[0][0], 1, G);
+                    const int32_t further_b = __shfl_down_sync(kFull, key[1][0], 1, G);
                     uint32_t leftH = __shfl_up_sync(kFull, edgeH, 1, G);
                     uint32_t leftI = __shfl_up_sync(kFull, edgeI, 1, G);
                     uint32_t trA = 0, trB = 0;
@@ -432,7 +444,12 @@ __global__ void __launch_bounds__(kBlock, 2) extension_pairs_kernel(KernelArgs p
                     }
                     uint32_t diag = above_left;
                     above_left = leftH;
-                    if (row >= 1 && row < group_rows + C) {
+                    // Every lane of the group goes on until its last has swept the last row: its keys move with them.
+                    if (row >= 1 && row + member <= steps) {
+                        if (member < G - 1) {
+                            key[0][C - 1] = max(key[0][C - 1], further_a);
+                            key[1][C - 1] = max(key[1][C - 1], further_b);
+                        }
                         const uint32_t stamp = uint32_t(row) | kBelow;
                         const uint32_t key_a = row <= rows[0] ? 0x1054u : 0x7654u;
                         const uint32_t key_b = row <= rows[1] ? 0x3254u : 0x7654u;
@@ -458,21 +475,18 @@ __global__ void __launch_bounds__(kBlock, 2) extension_pairs_kernel(KernelArgs p
                         edgeI = I;
                         if (member == G - 1 && s + 1 < warp_strips && row <= group_rows)
                             p.carry[slot * p.carry_stride + row] = make_int2(int32_t(edgeH), int32_t(edgeI));
-                        const int along = row + first + 1;
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const int32_t whole = key[h][0];
-                            if (whole < kLeast) continue;
-                            const int32_t value = (whole >> 16) + along * extend;
-                            const int their_row = whole & 0xFFFF;
-                            if (p.diagonals)
-                                atomicMax(p.diagonals + words[h] + along,
-                                          (static_cast<unsigned long long>(uint32_t(value) ^ 0x80000000u) << 32) |
-                                              uint32_t(their_row));
-                            else
-                                offer(h, value, along, their_row);
+                        if (member == 0) {
+                            send(0, key[0][0], row + first + 1);
+                            send(1, key[1][0], row + first + 1);
                         }
                     }
+                }
+            }
+            if (steps > 0) {
+#pragma unroll
+                for (int k = 0; k < C; ++k) {
+                    send(0, key[0][k], steps - member + first + k + 1);
+                    send(1, key[1][k], steps - member + first + k + 1);
                 }
             }
             __syncwarp();
