@@ -380,33 +380,90 @@ struct BandCounters {
 constexpr size_t kCountsBytes = offsetof(BandCounters, queues);
 static_assert(kCountsBytes <= kReadbackBytes, "a round's counts fit the readback words");
 
-// Keys for the pending pairs: band shape in the top bits, then the text length, longest first; each
-// shape's pairs and its work (the words its launch sweeps), summed in the block first.
+// band_shape_for by a warp: a lane a shape (two for the first lanes), its order of choice in a 64-bit rank whose least
+// is the choice. `cost` holds the tuning's word costs.
+__device__ int band_shape_by_warp(const EditPair &e, int64_t t, bool latency, const BandTuning &tuning,
+                                  const float *cost) {
+    static_assert(kBandShapes <= 64, "two shapes a lane");
+    const int lane = int(threadIdx.x & 31);
+    const int64_t needed = band_words_needed(e.n, e.m, t);
+    int capacity[2], words[2];
+    int64_t smallest = INT32_MAX;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int s = min(lane + 32 * i, kBandShapes - 1);
+        capacity[i] = lane + 32 * i < kBandShapes ? int(band_capacity(s)) : -1;
+        words[i] = int(band_words_per_lane(s));
+        if (capacity[i] >= needed) smallest = min(smallest, int64_t(capacity[i]));
+    }
+#pragma unroll
+    for (int span = 16; span > 0; span >>= 1) smallest = min(smallest, __shfl_xor_sync(0xffffffffu, smallest, span));
+    if (smallest == INT32_MAX) return kWidestShape;
+    // The least rank of the shapes within `reach` quarters of the smallest window (`bounded`: whose chain fits).
+    auto least = [&](int64_t reach, bool bounded) {
+        unsigned long long best = ~0ull;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const unsigned s = unsigned(lane + 32 * i);
+            if (capacity[i] < needed || capacity[i] < 0 || 4 * int64_t(capacity[i]) > reach * smallest) continue;
+            if (bounded && int64_t(e.m) * words[i] > tuning.chain_words) continue;
+            // Costs are positive, so their bits order as they do.
+            const unsigned long long price = __float_as_uint(float(capacity[i]) * cost[s]);
+            const unsigned long long chain = e.m > 0 ? unsigned(words[i]) : 0u;
+            const unsigned long long rank = latency   ? (unsigned long long)(words[i]) << 32 | unsigned(capacity[i])
+                                            : bounded ? price
+                                                      : chain << 32 | price;
+            best = min(best, rank << 8 | s);
+        }
+#pragma unroll
+        for (int span = 16; span > 0; span >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, span));
+        return best;
+    };
+    unsigned long long best = ~0ull;
+    if (latency) {
+        best = least(8, false);
+    } else {
+        for (int reach = 5; reach <= tuning.reach && best == ~0ull; reach = reach < tuning.reach ? tuning.reach : reach + 1)
+            best = least(reach, true);
+        if (best == ~0ull) best = least(max(tuning.reach, 5), false);
+    }
+    return int(best & 0xff);
+}
+
+// Keys for the pending pairs, a warp a pair: band shape in the top six bits, then the text length, longest first, as
+// the five bits of its exponent and the first five below (pairs within 3% of one another keep their order:
+// two passes of the sort instead of four); each shape's pairs and its work (the words its launch sweeps), summed in
+// the block first. (A thread a pair looked at the 39 shapes one after another: 20 us for 10,000 pairs.)
+constexpr int kKeyShapeBit = 10;
 __global__ void band_keys_kernel(const EditPair *__restrict__ pairs, const uint32_t *__restrict__ pending,
                                  const unsigned int *__restrict__ pending_count, unsigned int *__restrict__ next_count,
                                  int64_t room, const int64_t *__restrict__ thresholds, bool latency, BandTuning tuning,
-                                 uint32_t *__restrict__ keys, BandCounters *__restrict__ counters) {
+                                 uint16_t *__restrict__ keys, BandCounters *__restrict__ counters) {
     __shared__ unsigned block_counts[kBandShapes];
     __shared__ unsigned long long block_work[kBandShapes];
+    __shared__ float cost[kBandShapes];
     for (int s = threadIdx.x; s < kBandShapes; s += blockDim.x) {
         block_counts[s] = 0;
         block_work[s] = 0;
+        cost[s] = tuning.word_cost[s];
     }
     __syncthreads();
-    const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k == 0) *next_count = 0;
+    const int64_t k = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int lane = int(threadIdx.x & 31);
+    if (k == 0 && lane == 0) *next_count = 0;
     // Places past the list's end sort after it: the lowest key, and the sort keeps equal keys in order.
-    if (k >= *pending_count && k < room) keys[k] = 0;
+    if (k >= *pending_count && k < room && lane == 0) keys[k] = 0;
     if (k < *pending_count) {
         const uint32_t pair = pending[k];
         const EditPair e = pairs[pair];
-        const int shape = band_shape_for(e.n, e.m, thresholds[pair], latency, tuning);
-        uint32_t length = uint32_t(e.m) >> 2;
-        if (length > 0xFFFFFFu) length = 0xFFFFFFu;
-        keys[k] = (uint32_t(shape) << 24) | length;
-        atomicAdd(&block_counts[shape], 1u);
-        const int64_t window = band_capacity(shape);
-        atomicAdd(&block_work[shape], (unsigned long long)(int64_t(e.m) * (window < e.words ? window : e.words)));
+        const int shape = band_shape_by_warp(e, thresholds[pair], latency, tuning, cost);
+        if (lane == 0) {
+            const uint32_t length = e.m > 0 ? (__float_as_uint(float(e.m)) >> 18) - (127u << 5) : 0u;
+            keys[k] = uint16_t((uint32_t(shape) << kKeyShapeBit) | min(length, (1u << kKeyShapeBit) - 1u));
+            atomicAdd(&block_counts[shape], 1u);
+            const int64_t window = band_capacity(shape);
+            atomicAdd(&block_work[shape], (unsigned long long)(int64_t(e.m) * (window < e.words ? window : e.words)));
+        }
     }
     __syncthreads();
     for (int s = threadIdx.x; s < kBandShapes; s += blockDim.x) {
@@ -448,8 +505,9 @@ __global__ void round_work_kernel(const EditPair *__restrict__ pairs, const uint
 __global__ void settle_kernel(const EditPair *__restrict__ pairs, const uint32_t *__restrict__ pending,
                               const unsigned int *__restrict__ pending_count, int64_t *__restrict__ thresholds,
                               int64_t *__restrict__ cheapest, const int64_t *__restrict__ banded,
-                              int64_t *__restrict__ results, int64_t *__restrict__ rounds, bool latency,
-                              BandTuning tuning, uint32_t *__restrict__ next, unsigned int *__restrict__ next_count) {
+                              int64_t *__restrict__ results, int64_t *__restrict__ rounds,
+                              const uint16_t *__restrict__ keys, uint32_t *__restrict__ next,
+                              unsigned int *__restrict__ next_count) {
     const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (k >= *pending_count) return;
     const uint32_t pair = pending[k];
@@ -457,8 +515,7 @@ __global__ void settle_kernel(const EditPair *__restrict__ pairs, const uint32_t
     const int64_t t = thresholds[pair];
     const int64_t found = banded[pair];
     rounds[pair] += 1;
-    const int shape = band_shape_for(e.n, e.m, t, latency, tuning);
-    const int64_t window = band_capacity(shape);
+    const int64_t window = band_capacity(keys[k] >> kKeyShapeBit);  // the round's sorted keys
     const bool whole = window >= e.words;  // the window holds every word: the whole matrix
     // The proof needs the window to cover the band; the widest window (512 words) falls short only for
     // patterns past 32,768 letters with bands wider than it, refused here (device memory, as the
@@ -632,8 +689,8 @@ void band_doubling(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const
     const uint64_t *planes = prepared.planes;
     const uint8_t *status = prepared.status;
     void *space = nullptr;
-    uint32_t *keys = gpu->keys.ensure<uint32_t>(size_t(pairs));
-    uint32_t *keys_sorted = gpu->keys_sorted.ensure<uint32_t>(size_t(pairs));
+    uint16_t *keys = gpu->keys.ensure<uint16_t>(size_t(pairs));
+    uint16_t *keys_sorted = gpu->keys_sorted.ensure<uint16_t>(size_t(pairs));
     uint32_t *order_sorted = gpu->order_sorted.ensure<uint32_t>(size_t(pairs));
     if (gpu->band_tuning.chain_words == 0) gpu->band_tuning = default_band_tuning();
     const BandTuning tuned = gpu->band_tuning;
@@ -670,16 +727,16 @@ void band_doubling(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const
             const double per_lane = double(work) / (double(gpu->multiprocessors) * 1024.0);
             tuning.chain_words = std::max<int64_t>(tuned.chain_words, int64_t(tuned.chain_share * per_lane));
         }
-        band_keys_kernel<<<blocks, threads, 0, stream>>>(info, pending, pending_count, next_count, count, thresholds,
-                                                         latency, tuning, keys, counters);
+        band_keys_kernel<<<unsigned((count * 32 + threads - 1) / threads), threads, 0, stream>>>(
+            info, pending, pending_count, next_count, count, thresholds, latency, tuning, keys, counters);
         gpu->launches += 1;
         DINARA_CUDA(cudaGetLastError());
         size_t sort_bytes = 0;
         DINARA_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, sort_bytes, keys, keys_sorted, pending,
-                                                              order_sorted, int(count), 0, 32, stream));
+                                                              order_sorted, int(count), 0, 16, stream));
         space = gpu->sort_scratch.ensure<uint8_t>(sort_bytes + 256);
         DINARA_CUDA(cub::DeviceRadixSort::SortPairsDescending(space, sort_bytes, keys, keys_sorted, pending,
-                                                              order_sorted, int(count), 0, 32, stream));
+                                                              order_sorted, int(count), 0, 16, stream));
         read_back(gpu, host_bytes, counters, kCountsBytes);
         const int64_t round_count = host->pending[round & 1];
         if (round_count == 0) break;
@@ -743,7 +800,7 @@ void band_doubling(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, const
         if (report) DINARA_CUDA(cudaEventRecord(gpu->stop, stream));
         clock.stop();
         settle_kernel<<<blocks, threads, 0, stream>>>(info, order_sorted, pending_count, thresholds, cheapest, banded,
-                                                      results, rounds, latency, tuning, next, next_count);
+                                                      results, rounds, keys_sorted, next, next_count);
         gpu->launches += 1;
         DINARA_CUDA(cudaGetLastError());
         read_back(gpu, host_bytes, counters, 2 * sizeof(unsigned int));
