@@ -710,8 +710,8 @@ struct PhaseTimer {
 // columns) - 2 score) / (best - 2 extend). The pair goes round again at that width (at least twice the
 // last, rounded up to 256 diagonals) unless this is the `last` round or that band's strips of
 // `strip_columns` would sweep three fifths of its rows or more: then to the whole-matrix list. With `swept`
-// null, every pair is routed to `first_width`, or a wider band foreseen for it (`foreseen`, by pair, when given). With `proven`, a pair whose band proves its score leaves the
-// width there (by pair - proven_first).
+// null, every pair is routed to `first_width`, or a wider band foreseen for it (`foreseen`, by pair, when
+// given). With `proven`, a pair whose band proves its score leaves the width there (by pair - proven_first).
 __global__ void wide_route_kernel(const PairShape *__restrict__ shapes, const uint32_t *__restrict__ pending,
                                   const int32_t *__restrict__ swept, int64_t count, int32_t first_width, bool last,
                                   const int32_t *__restrict__ scores, int32_t best, int32_t open, int32_t extend,
@@ -783,9 +783,17 @@ void sweep_long(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &ta
     args.carry_stride = int64_t(batch.max_rows) + 1;
     ClockSpan clock(gpu, kClassWhole, gpu->stream);
     if (long_serves(batch, table)) {
-        // A cluster a pair, or for a batch with pairs enough to fill the GPU, a block of four warps a pair.
+        // A cluster a pair, or for a batch with pairs enough to fill the GPU, a block of four warps a pair. Where
+        // clusters of 32 warps leave each port of the GPU four warps or fewer, a pair lasts as long as its rows'
+        // chain, and half the columns a lane shorten it: one pair of 50,000 letters at 5% 14.9 -> 13.1 ms, four at
+        // 30% 62.2 -> 50.9, 64 of 20,000 at 5% 12.9 -> 11.5. With more pairs the ports are the bound, which a row's
+        // fixed instructions share: 128 of 8,000 at 5% 6.5 -> 6.6, 300 of 6,000 7.7 -> 9.6.
         const bool cluster = count < 4 * int64_t(gpu->multiprocessors);
-        const int threads = 32 * (cluster ? kLongClusterWarps : kLongWarps / 2);
+        const bool narrow = 2 * count <= gpu->multiprocessors;
+        void (*fn)(LongArgs) = !cluster ? &affine_long_kernel<false, 16>
+                               : narrow ? &affine_long_kernel<true, 8>
+                                        : &affine_long_kernel<true, 16>;
+        const int threads = 32 * (cluster ? long_cluster_warps(narrow ? 8 : 16) : kLongWarps / 2);
         cudaLaunchConfig_t config = {};
         cudaLaunchAttribute shape = {};
         shape.id = cudaLaunchAttributeClusterDimension;
@@ -798,11 +806,11 @@ void sweep_long(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &ta
         if (cluster) {
             config.gridDim = dim3(kLongCluster);
             int clusters = 0;
-            DINARA_CUDA(cudaOccupancyMaxActiveClusters(&clusters, affine_long_kernel<true>, &config));
+            DINARA_CUDA(cudaOccupancyMaxActiveClusters(&clusters, fn, &config));
             in_flight = std::max(clusters, 1);
         } else {
             int per_sm = 0;
-            DINARA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, affine_long_kernel<false>, threads, 0));
+            DINARA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0));
             in_flight = int64_t(std::max(per_sm, 1)) * gpu->multiprocessors;
         }
         in_flight = std::min(in_flight, count);
@@ -820,10 +828,7 @@ void sweep_long(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &ta
         a.scores = args.scores;
         a.carry_stride = args.carry_stride;
         a.carry = gpu->carry.ensure<int2>(size_t(in_flight * args.carry_stride));
-        if (cluster)
-            DINARA_CUDA(cudaLaunchKernelEx(&config, affine_long_kernel<true>, a));
-        else
-            DINARA_CUDA(cudaLaunchKernelEx(&config, affine_long_kernel<false>, a));
+        DINARA_CUDA(cudaLaunchKernelEx(&config, fn, a));
     } else {
         KernelFn fn = widths ? &affine_wide_kernel<false, true> : &affine_wide_kernel<false, false>;
         const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(persistent_blocks(gpu, fn), count));

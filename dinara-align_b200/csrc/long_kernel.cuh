@@ -6,14 +6,15 @@
 namespace dinara {
 namespace sweep {
 
-// A strip is 64 virtual lanes of 16 columns: a lane's low halves hold 16 columns and its high halves the
-// next 16, one row behind, so each DPX instruction on 16-bit pairs moves two cells of the one pair.
+// A strip is 64 virtual lanes of C columns (16, or 8 for a batch of few pairs): a lane's low halves hold C columns and
+// its high halves the next C, one row behind, so each DPX instruction on 16-bit pairs moves two cells of the one
+// pair.
 constexpr int kLongStrip = 1024;
 constexpr int kLongWarps = 8;     // most warps a block without clusters; a launch may take fewer
 constexpr int kLongChunk = 32;    // steps of a chunk: a strip's letters and left column are read, and its base moved, once
 constexpr int kLongChunks = 2;    // chunks between barriers
-constexpr int kLongCluster = 8;   // blocks a cluster, and each one's warps
-constexpr int kLongClusterWarps = 2;
+constexpr int kLongCluster = 8;   // blocks a cluster
+__host__ __device__ constexpr int long_cluster_warps(int C) { return C == 8 ? 4 : 2; }  // and each one's warps
 
 // A lane's halves hold its cells less its base, a true 32-bit value that follows them: at each chunk the
 // lane's own middle cell becomes the base. Within a lane's 32 columns two reached cells of a row differ
@@ -46,9 +47,13 @@ __device__ __forceinline__ void cluster_barrier() {
 }
 
 // A strip's rows: those its columns share with the band [low, high] of diagonals (column less row).
-__device__ __forceinline__ int long_first_row(int s, int high) { return max(1, s * kLongStrip + 1 - high); }
+template <int STRIP>
+__device__ __forceinline__ int long_first_row(int s, int high) {
+    return max(1, s * STRIP + 1 - high);
+}
+template <int STRIP>
 __device__ __forceinline__ int long_last_row(int s, int rows, int columns, int low) {
-    return min(rows, min((s + 1) * kLongStrip, columns) - low);
+    return min(rows, min((s + 1) * STRIP, columns) - low);
 }
 
 // Stores `value` at `place` in this block's shared memory, or in block `rank` of its cluster's.
@@ -65,35 +70,35 @@ __device__ __forceinline__ void leave_word(int *place, int rank, int value) {
     }
 }
 
-// The whole or banded score of one pair a block, or with CLUSTER a cluster of eight blocks (score_groups.mojo's recurrence, cells shifted by (row +
-// column) * extend). Warp w of the block's sweeps strips w, w + warps, ...: a strip's virtual lane v runs one
-// row behind lane v - 1, whose last column reaches it from the lane's own low half or by one shuffle, and the
-// column left of a strip comes from the strip before through `carry`, a chunk of 32 rows at a time. Warps
-// meet at one barrier every two chunks and leave how far they are with the warp of the next strip; a warp takes
-// a chunk when the strip before had, by the last barrier, left every row it reads, else waits for the next. Strips of a band start lower one after
-// another, so about (width + 1,024) / 1,100 of them run at once.
+// The whole or banded score of one pair a block, or with CLUSTER a cluster of eight blocks (score_groups.mojo's
+// recurrence, cells shifted by (row + column) * extend). Warp w of them sweeps strips w, w + warps, ...: a strip's
+// virtual lane v runs one row behind lane v - 1, whose last column reaches it from the lane's own low half or by one
+// shuffle, and the column left of a strip comes from the strip before through `carry`, a chunk of 32 rows at a time.
+// Warps meet at one barrier every two chunks and leave how far they are with the warp of the next strip; a warp
+// takes a chunk when the strip before had, by the last barrier, left every row it reads, else waits for the next.
+// Strips of a band start lower one after another, so about (width + 64 C) / (64 C + 100) of them run at once.
 //
-// Each step is 16 x 5 instructions of the DPX and permute pipe for 32 x 32 cells a warp (16-bit pairs run at the
+// Each step is C x 5 instructions of the DPX and permute pipe for 32 x 2 C cells a warp (16-bit pairs run at the
 // 32-bit rate), so an SM's bound is 25.6 cells a cycle against 12.8 in 32 bits; a barrier a row (the block-wide
-// 32-bit sweep, affine_wide_kernel) and its strips of 4,096 columns, which sweep 4,096 rows beyond a band's
-// width, are what this one does without.
+// 32-bit sweep, affine_wide_kernel) and its strips of 4,096 columns, which sweep 4,096 rows beyond a band's width,
+// are what this one does without.
 //
 // Eight warps on one SM share its four issue ports, and a pair of 50,000 letters keeps them all for each of its
 // rows; a batch too small to fill the GPU with pairs takes a cluster a pair instead, neighbouring strips on
 // different SMs, a warp or less a port. Its warps meet at a cluster barrier, whose release and acquire order the
-// column in global memory and the words left in one another's shared memory.
+// column in global memory and the words left in one another's shared memory. A batch smaller still, whose ports wait
+// for a row's chain of insertions through a lane's C columns, takes C = 8 and twice the warps (sweep_long).
 //
-// A banded strip sweeps its rows alone, every cell above or left of them unreached; the score is then
-// the best over paths within the swept rows, the whole matrix's when the band proves it
-// (band_proves_width).
-template <bool CLUSTER>
-__global__ void __launch_bounds__(32 * (CLUSTER ? kLongClusterWarps : kLongWarps), CLUSTER ? 8 : 2)
-    affine_long_kernel(LongArgs p) {
-    constexpr int C = 16;
+// A banded strip sweeps its rows alone, every cell above or left of them unreached; the score is then the best over
+// paths within the swept rows, the whole matrix's when the band proves it (band_proves_width).
+template <bool CLUSTER, int C>
+__global__ void __launch_bounds__(32 * (CLUSTER ? long_cluster_warps(C) : kLongWarps),
+                                  CLUSTER ? 16 / long_cluster_warps(C) : 2) affine_long_kernel(LongArgs p) {
+    constexpr int STRIP = 64 * C;
     __shared__ uint32_t rows8[4];
     // By round parity: for each of the block's warps, the strip and steps of the warp before it; and whether the
     // last strip is done.
-    __shared__ int left_by[2][CLUSTER ? kLongClusterWarps : kLongWarps][2], finished[2];
+    __shared__ int left_by[2][CLUSTER ? long_cluster_warps(C) : kLongWarps][2], finished[2];
     if (threadIdx.x < 4) rows8[threadIdx.x] = p.rows8[threadIdx.x];
 
     const int lane = threadIdx.x & 31;
@@ -120,7 +125,7 @@ __global__ void __launch_bounds__(32 * (CLUSTER ? kLongClusterWarps : kLongWarps
         const uint32_t pair = p.order[item];
         const PairShape sh = p.shapes[pair];
         const int rows = int(sh.rows), cols = int(sh.columns);
-        const int strips = (cols + kLongStrip - 1) / kLongStrip;
+        const int strips = (cols + STRIP - 1) / STRIP;
         // The band's diagonals; a pair whose band cannot hold both ends is swept whole.
         int low = -rows, high = cols;
         if (p.band_widths) {
@@ -156,16 +161,16 @@ __global__ void __launch_bounds__(32 * (CLUSTER ? kLongClusterWarps : kLongWarps
             for (int chunk = 0; chunk < kLongChunks; ++chunk) {
                 bool ready = strip < strips;
                 if (ready && done == 0) {
-                    first_row = long_first_row(strip, high);
-                    last_row = long_last_row(strip, rows, cols, low);
-                    previous_last = strip > 0 ? long_last_row(strip - 1, rows, cols, low) : rows;
+                    first_row = long_first_row<STRIP>(strip, high);
+                    last_row = long_last_row<STRIP>(strip, rows, cols, low);
+                    previous_last = strip > 0 ? long_last_row<STRIP>(strip - 1, rows, cols, low) : rows;
                     total = last_row - first_row + 1 + 63;
                 }
                 if (ready && strip > 0) {
                     // The strip before has left every row of this chunk (its virtual lane 63 leaves row r at its
                     // step r - its first row + 64) by the last barrier.
                     const int last_read = min(first_row - 1 + done + kLongChunk, previous_last);
-                    const int needed = last_read - long_first_row(strip - 1, high) + 64;
+                    const int needed = last_read - long_first_row<STRIP>(strip - 1, high) + 64;
                     ready = their_strip > strip - 1 || (their_strip == strip - 1 && their_done >= needed);
                 }
                 if (!ready) break;
@@ -173,10 +178,11 @@ __global__ void __launch_bounds__(32 * (CLUSTER ? kLongClusterWarps : kLongWarps
                 const int t0 = done + 1;
                 if (done == 0) {
                     // A new strip: its columns' selectors, and every lane's base the value its cells start near.
-                    const int word = strip * (kLongStrip / 16) + 2 * lane;
+                    static_assert(C == 16 || C == 8, "a lane's letters are two words or one");
+                    const int word = strip * (STRIP / 16) + (C / 8) * lane;
                     const int last_word = (cols - 1) >> 4;
                     const uint32_t a = __ldg(p.tape + sh.second_word + min(word, last_word));
-                    const uint32_t b = __ldg(p.tape + sh.second_word + min(word + 1, last_word));
+                    const uint32_t b = C == 16 ? __ldg(p.tape + sh.second_word + min(word + 1, last_word)) : a >> 16;
 #pragma unroll
                     for (int k = 0; k < C; ++k)
                         sel[k] = pair_selector(half_selector_a((a >> (2 * k)) & 3u), half_selector_b((b >> (2 * k)) & 3u));
@@ -233,8 +239,8 @@ __global__ void __launch_bounds__(32 * (CLUSTER ? kLongClusterWarps : kLongWarps
                 const bool starting = t0 <= 64;
                 const bool leaves = strip + 1 < strips;
                 // The corner: its virtual lane reaches the last row at this step.
-                const int corner = cols - 1 - strip * kLongStrip;
-                const int corner_step = strip + 1 == strips ? rows - first_row + 1 + (corner >> 4) : -1;
+                const int corner = cols - 1 - strip * STRIP;
+                const int corner_step = strip + 1 == strips ? rows - first_row + 1 + corner / C : -1;
                 const int32_t top_h = held(opening), top_d = held(opening + first_gap);
 #pragma unroll 2
                 for (int u = 0; u < kLongChunk; ++u) {
@@ -296,11 +302,11 @@ __global__ void __launch_bounds__(32 * (CLUSTER ? kLongClusterWarps : kLongWarps
                         if (row >= first_row && row <= last_row)
                             carry[row] = make_int2(base + low_of(send), base + high_of(send));
                     }
-                    if (step == corner_step && lane == (corner >> 5)) {
+                    if (step == corner_step && lane == corner / (2 * C)) {
                         uint32_t value = 0;
 #pragma unroll
-                        for (int k = 0; k < C; ++k) value |= H[k] & (0u - uint32_t(k == (corner & 15)));
-                        p.scores[pair] = base + ((corner & 16) ? high_of(value) : low_of(value)) + (rows + cols) * p.extend;
+                        for (int k = 0; k < C; ++k) value |= H[k] & (0u - uint32_t(k == corner % C));
+                        p.scores[pair] = base + ((corner & C) ? high_of(value) : low_of(value)) + (rows + cols) * p.extend;
                     }
                 }
                 done += kLongChunk;

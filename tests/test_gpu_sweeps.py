@@ -66,6 +66,21 @@ def test_long_pairs_in_strips(da, oracle, entries):
     np.testing.assert_array_equal(da.scores_tape(tape, scoring), expected)
 
 
+@pytest.mark.parametrize("pairs", [75, 592])
+def test_many_long_pairs_in_strips(da, oracle, pairs):
+    """Enough long pairs for strips of 16 columns a lane: a cluster a pair, and a block a pair (10 pairs, above,
+    take eight columns a lane)."""
+    rng = np.random.default_rng(pairs)
+    scoring = da.Scoring.uniform(30, -40, -20, -3)
+    refs = [_text(rng, 1025 + int(rng.integers(0, 90))) for _ in range(pairs)]
+    queries = [_text(rng, 1025 + int(rng.integers(0, 90))) for _ in range(pairs)]
+    tape = da.Tape.of(refs, queries)
+    coded = np.concatenate([oracle.codes(text) for pair in zip(refs, queries) for text in pair])
+    op, ex = oracle.kernel_gaps(scoring.opening, scoring.extension)
+    expected = oracle.batch_scores(coded, tape.offsets, _table(scoring), 4, op, ex, oracle.GLOBAL, threads=8)
+    np.testing.assert_array_equal(da.scores_tape(tape, scoring), expected)
+
+
 # ---- local alignments recorded over their hits' rows ----------------------------------------------------
 
 @pytest.mark.parametrize("alphabet", ["ACGT", "ACGTN", PROTEIN])
