@@ -534,13 +534,22 @@ PairsLaunch pick_pairs(int cls, bool local, bool hits, int bits, int letters) {
                         : local ? &affine_pairs_kernel<G8, 16, true, false, 8>                                       \
                                 : &affine_pairs_kernel<G8, 16, false, false, 8>,                                     \
                         bits, bits == 8 ? G8 : G, bits == 8 ? 16 : C, letters);
+    // The finer strips are the two-bit scores' (PairLimits::fine).
+#define DINARA_FINE(C)                                                                                               \
+    return pairs_launch(local ? &affine_pairs_kernel<32, C, true> : &affine_pairs_kernel<32, C, false>, nullptr, 2,  \
+                        32, C, letters);
     switch (cls) {
         case 0: DINARA_PAIRS(4, 16, 4)
         case 1: DINARA_PAIRS(8, 16, 8)
         case 2: DINARA_PAIRS(16, 16, 16)
         case 3: DINARA_PAIRS(16, 20, 32)
-        default: DINARA_PAIRS(32, 16, 32)
+        case 4: DINARA_PAIRS(32, 16, 32)
+        case 5: DINARA_FINE(12)
+        case 6: DINARA_FINE(14)
+        case 7: DINARA_FINE(20)
+        default: DINARA_FINE(24)
     }
+#undef DINARA_FINE
 #undef DINARA_PAIRS
 }
 
@@ -570,15 +579,26 @@ int persistent_blocks(dinara_gpu *gpu, KernelFn fn, int threads = kBlock, size_t
 // A class's 16-bit pair sweep of a batch: items [begin, end) of the order.
 struct ClassSweep {
     PairsLaunch launch;
+    int cls;
     int64_t begin, end;
 };
+
+// The tallest pair a 16-bit pair sweep's limits let in, of a batch's.
+int64_t tallest_of(const AffineBatch &batch, const PairLimits &limits) {
+    int64_t rows = batch.max_rows;
+    if (limits.local && limits.row_step > 0) rows = std::min<int64_t>(rows, limits.whole / limits.row_step);
+    if (!limits.local) rows = std::min<int64_t>(rows, limits.whole / 2);
+    return rows;
+}
 
 // Launches a batch's classes' sweeps at once, each on a side stream forked from the context's and joined back to
 // it: one class's last pairs run beside the next one's, where one launch after the other ended each on its own
 // tail (5,000 reads' hits: 8.3 ms one by one). Each has carry slots of its own, one a lane group, each as long as
-// the tallest pair, where pairs may be wider than its strip. One class alone stays on the context's stream.
-void launch_together(dinara_gpu *gpu, const AffineBatch &batch, const std::vector<ClassSweep> &sweeps, KernelArgs args,
-                     const TableArgs &targs, const int32_t *table32) {
+// the tallest pair (`limits`), where a class's pairs may be wider than its strip. One class alone stays on the
+// context's stream.
+void launch_together(dinara_gpu *gpu, const AffineBatch &batch, const PairLimits &limits,
+                     const std::vector<ClassSweep> &sweeps, KernelArgs args, const TableArgs &targs,
+                     const int32_t *table32) {
     if (sweeps.empty()) return;
     std::vector<int64_t> blocks, slots;
     int64_t all_slots = 0;
@@ -588,10 +608,12 @@ void launch_together(dinara_gpu *gpu, const AffineBatch &batch, const std::vecto
         const int64_t needed = (sweep.end - sweep.begin + 2 * groups - 1) / (2 * groups);
         blocks.push_back(
             std::max<int64_t>(1, std::min<int64_t>(persistent_blocks(gpu, l.fn, l.threads, l.shared), needed)));
-        slots.push_back(batch.max_columns > uint32_t(l.lanes * l.columns) ? blocks.back() * groups : 0);
+        const int cls = sweep.cls;
+        const int64_t widest = cls < 4 ? affine_lanes(cls) * affine_columns(cls) : int64_t(batch.max_columns);
+        slots.push_back(widest > int64_t(l.lanes) * l.columns ? blocks.back() * groups : 0);
         all_slots += slots.back();
     }
-    const int64_t stride = int64_t(batch.max_rows) + 1;
+    const int64_t stride = tallest_of(batch, limits) + 1;
     int2 *carry = all_slots > 0 ? gpu->carry.ensure<int2>(size_t(all_slots * stride)) : nullptr;
     const bool fork = sweeps.size() > 1;
     if (fork) DINARA_CUDA(cudaEventRecord(gpu->fork, gpu->stream));
@@ -864,7 +886,7 @@ void widening_band(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
     uint32_t *lists = gpu->wide_pending.ensure<uint32_t>(5 * size_t(count));
     uint32_t *whole = lists + 2 * count;
     int32_t *widths = reinterpret_cast<int32_t *>(lists + 3 * count);
-    unsigned int *counts = gpu->class_counts.ensure<unsigned int>(20) + 9;  // [0] next, [1] whole
+    unsigned int *counts = gpu->class_counts.ensure<unsigned int>(kClassCounters) + 9;  // [0] next, [1] whole
     DINARA_CUDA(cudaMemsetAsync(counts + 1, 0, sizeof(unsigned int), gpu->stream));
     constexpr int kBandRounds = 2;
     const uint32_t *pending = order;
@@ -894,7 +916,7 @@ void widening_band(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
 }
 
 void affine_launch_all(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, const Schedule &schedule,
-                       bool record, KernelArgs args, const int32_t *foreseen = nullptr) {
+                       bool record, const PairLimits &limits, KernelArgs args, const int32_t *foreseen = nullptr) {
     const bool smem = !table.packed16 || batch.bits == 8;
     const TableArgs targs = table_args(table, batch.local);
     int32_t *table32 = nullptr;
@@ -908,7 +930,7 @@ void affine_launch_all(dinara_gpu *gpu, const AffineBatch &batch, const AffineTa
         const bool wide = bucket == kWideClass;
         // Recording, a long global pair whose widening band proved a width: its strips over that band.
         const bool band_record = bucket == kBandRecordClass;
-        const bool pairs16 = !wide && !band_record && bucket >= kWholePairsClass;
+        const bool pairs16 = bucket >= kWholePairsClass && bucket < kWholePairsClass + kPairShapes;
         const int cls = pairs16 ? bucket - kWholePairsClass : wide || band_record ? 4 : bucket;
         if (wide && !batch.local && !record && band_serves(batch, table)) {
             // Long global pairs take the widening band first.
@@ -919,7 +941,7 @@ void affine_launch_all(dinara_gpu *gpu, const AffineBatch &batch, const AffineTa
         if (pairs16) {
             pair_sweeps.push_back({record ? pick_record(cls, batch.local, batch.bits, table.size)
                                           : pick_pairs(cls, batch.local, false, batch.bits, table.size),
-                                   b.begin[bucket], b.end[bucket]});
+                                   cls, b.begin[bucket], b.end[bucket]});
             continue;
         }
         KernelFn fn = band_record ? &affine_kernel<32, 16, false, true, 2, false, false, true>
@@ -949,7 +971,7 @@ void affine_launch_all(dinara_gpu *gpu, const AffineBatch &batch, const AffineTa
         clock.stop();
         gpu->launches += 1;
     }
-    launch_together(gpu, batch, pair_sweeps, args, targs, table32);
+    launch_together(gpu, batch, limits, pair_sweeps, args, targs, table32);
 }
 
 // The largest rows + columns of a pair the 16-bit pair sweep takes under a table (band_pair_limit): the
@@ -966,10 +988,17 @@ int32_t pair_limit_of(const AffineTable &table) {
     return band_pair_limit(step, bytes_fit);
 }
 
+// Pairs an SM from which scores take the finer strips. They sweep fewer columns past a pair's last (pair_shape_for)
+// in more classes of fewer pairs, so they need pairs enough for each class to fill its share of the GPU. Local scores
+// of reads of 330 to 1,000 letters in targets of 1,000 to 5,000, strips of 512 against these: 2,500 of them 3.96
+// against 4.15 ms a call, 5,000 5.62 against 5.88, 7,500 7.55 against 7.02; 20,000 reads of 150 to 1,000 11.08
+// against 10.33. 5,000 local alignments, their hits swept so, 9.8 against 10.7.
+constexpr int64_t kFinerPairs = 48;
+
 // Which whole-matrix pairs the 16-bit pair score sweep takes (a table of up to four letters on the 2-bit
-// tape, or a larger one through profiles): locally, a cell held less row x extend reaches at most the best entry times the columns swept
-// plus the rows times -extend and falls no lower than a gap's first letter, so that sum is held to half of
-// 30,000 less the gaps;
+// tape, or a larger one through profiles): locally, a cell held less row x extend reaches at most the best
+// entry times the columns swept plus the rows times -extend and falls no lower than a gap's first letter, so
+// that sum is held to half of 30,000 less the gaps;
 // globally, a shifted cell moves at most the largest step a cell, so rows and swept columns are each held
 // to half of 30,000 over it, every value within 30,000 of zero. Entries must fit a byte (shifted, globally).
 PairLimits whole_limits_of(const AffineBatch &batch, const AffineTable &table) {
@@ -1005,6 +1034,11 @@ PairLimits whole_limits_of(const AffineBatch &batch, const AffineTable &table) {
         }
     limits.whole = 30000 / std::max(step, 1) - 4;
     return limits;
+}
+
+// Whether `count` pairs' scores take the finer strips past 320 columns.
+int finer_strips(dinara_gpu *gpu, const AffineBatch &batch, int64_t count) {
+    return batch.bits == 2 && count >= kFinerPairs * int64_t(gpu->multiprocessors) ? 1 : 0;
 }
 
 // Which whole-matrix pairs the 16-bit recording sweep takes: every half at zero or more, record_bias above its
@@ -1075,7 +1109,7 @@ BandedBatch banded_batch(const AffineBatch &batch, const AffineTable &table, con
 // by tally_swept.
 unsigned long long *band_counter(dinara_gpu *gpu) {
     if (!gpu->timing) return nullptr;
-    unsigned long long *counter = reinterpret_cast<unsigned long long *>(gpu->class_counts.ensure<unsigned int>(20) + 16);
+    unsigned long long *counter = reinterpret_cast<unsigned long long *>(gpu->class_counts.ensure<unsigned int>(kClassCounters) + 16);
     DINARA_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), gpu->stream));
     return counter;
 }
@@ -1086,14 +1120,14 @@ unsigned long long *band_counter(dinara_gpu *gpu) {
 void tally_swept(dinara_gpu *gpu, const PairShape *shapes, int64_t first, int64_t count, bool band,
                  const uint32_t *leftovers, int64_t left, const int32_t *widths = nullptr) {
     if (!gpu->timing) return;
-    unsigned long long *out = reinterpret_cast<unsigned long long *>(gpu->class_counts.ensure<unsigned int>(20) + 12);
+    unsigned long long *out = reinterpret_cast<unsigned long long *>(gpu->class_counts.ensure<unsigned int>(kClassCounters) + 12);
     DINARA_CUDA(cudaMemsetAsync(out, 0, 2 * sizeof(unsigned long long), gpu->stream));
     swept_cells_kernel<<<256, 256, 0, gpu->stream>>>(shapes, first, count, band, leftovers, left, widths, out);
     gpu->launches += 1;
     DINARA_CUDA(cudaGetLastError());
     unsigned long long host[2] = {0, 0};
     read_back(gpu, host, out, sizeof host);
-    if (band) read_back(gpu, &host[0], gpu->class_counts.ensure<unsigned int>(20) + 16, sizeof host[0]);
+    if (band) read_back(gpu, &host[0], gpu->class_counts.ensure<unsigned int>(kClassCounters) + 16, sizeof host[0]);
     gpu->swept_cells += int64_t(host[0] + host[1]);
     gpu->band_cells += int64_t(host[0]);
     gpu->whole_cells += int64_t(host[1]);
@@ -1129,7 +1163,7 @@ void launch_bands(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &
         // The 16-bit pair band in two passes: every pair over 32 diagonals first (most short pairs' scores
         // prove there, for half the cells), then the pairs it did not prove, or could not hold, over 64.
         uint32_t *narrow_left = gpu->narrow_leftovers.ensure<uint32_t>(size_t(b.count));
-        unsigned int *narrow_count = gpu->class_counts.ensure<unsigned int>(20) + 11;
+        unsigned int *narrow_count = gpu->class_counts.ensure<unsigned int>(kClassCounters) + 11;
         DINARA_CUDA(cudaMemsetAsync(narrow_count, 0, sizeof(unsigned int), gpu->stream));
         BandedBatch narrow = b;
         narrow.leftovers = narrow_left;
@@ -1283,9 +1317,9 @@ __global__ void extension_finish_kernel(const PairShape *__restrict__ shapes, in
         for (int j = 0; j < 4; ++j) spans[4 * k + j] = span[j];
 }
 
-// Which pairs the 16-bit free-end sweeps take (a table whose shifted entries fit a byte): a shifted cell reaches at most the best entry times the columns swept plus the rows and
-// columns swept times -extend, held to half of 30,000 less the gaps for the sum of a group's two pairs, and
-// falls at most a few gap openings below zero.
+// Which pairs the 16-bit free-end sweeps take (a table whose shifted entries fit a byte): a shifted cell reaches at
+// most the best entry times the columns swept plus the rows and columns swept times -extend, held to half of
+// 30,000 less the gaps for the sum of a group's two pairs, and falls at most a few gap openings below zero.
 PairLimits free_limits_of(const AffineBatch &batch, const AffineTable &table) {
     PairLimits limits;
     const int32_t gaps = std::abs(table.open) + std::abs(table.extend);
@@ -1339,9 +1373,9 @@ void launch_free(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &t
         if (last > first)
             sweeps.push_back({batch.extension ? pick_extension(cls, batch.bits, table.size)
                                               : pick_free(cls, batch.bits, table.size),
-                              first, last});
+                              cls, first, last});
     }
-    launch_together(gpu, batch, sweeps, args, targs, table32);
+    launch_together(gpu, batch, free_limits_of(batch, table), sweeps, args, targs, table32);
     const int64_t begin = b.begin[kAffineShapes - 1], end = b.end[0];
     if (end <= begin) return;
     const int64_t blocks = std::max<int64_t>(
@@ -1522,7 +1556,7 @@ const PairShape *hit_shapes(dinara_gpu *gpu, const AffineBatch &batch, const Aff
     if (limits.whole <= 0) return nullptr;
     const Schedule order = dinara::schedule(gpu, batch.shapes, nullptr, first, count, false, false, limits);
     int64_t taken = 0;
-    for (int cls = 0; cls < kAffineShapes; ++cls) taken += order.counts[kWholePairsClass + cls];
+    for (int cls = 0; cls < kPairShapes; ++cls) taken += order.counts[kWholePairsClass + cls];
     if (taken == 0) return nullptr;
     PairShape *hits = gpu->hits.ensure<PairShape>(size_t(batch.pairs));
     if (taken < count)
@@ -1544,11 +1578,11 @@ const PairShape *hit_shapes(dinara_gpu *gpu, const AffineBatch &batch, const Aff
     const Buckets b = buckets_of(order);
     PhaseTimer timer(gpu, &gpu->record_ms);
     std::vector<ClassSweep> sweeps;
-    for (int cls = kAffineShapes - 1; cls >= 0; --cls) {
+    for (int cls = kPairShapes - 1; cls >= 0; --cls) {
         const int64_t begin = b.begin[kWholePairsClass + cls], end = b.end[kWholePairsClass + cls];
-        if (end > begin) sweeps.push_back({pick_pairs(cls, true, true, batch.bits, table.size), begin, end});
+        if (end > begin) sweeps.push_back({pick_pairs(cls, true, true, batch.bits, table.size), cls, begin, end});
     }
-    launch_together(gpu, batch, sweeps, args, targs, table32);
+    launch_together(gpu, batch, limits, sweeps, args, targs, table32);
     timer.stop();
     return hits;
 }
@@ -1559,7 +1593,7 @@ const PairShape *hit_shapes(dinara_gpu *gpu, const AffineBatch &batch, const Aff
 int32_t *proven_band_widths(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, int32_t *scores,
                             int64_t first_pair, int64_t count) {
     uint32_t *list = gpu->long_pairs.ensure<uint32_t>(size_t(count));
-    unsigned int *listed = gpu->class_counts.ensure<unsigned int>(20) + 18;
+    unsigned int *listed = gpu->class_counts.ensure<unsigned int>(kClassCounters) + 18;
     DINARA_CUDA(cudaMemsetAsync(listed, 0, sizeof(unsigned int), gpu->stream));
     long_pairs_kernel<<<unsigned((count + 255) / 256), 256, 0, gpu->stream>>>(batch.shapes, first_pair, count, list,
                                                                              listed);
@@ -1603,6 +1637,7 @@ void affine_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
     const bool band = band_serves(batch, table);
     PairLimits limits = whole_limits_of(batch, table);
     limits.band = band ? pair_limit_of(table) : 0;
+    limits.fine = finer_strips(gpu, batch, count);
     const Schedule schedule_all = dinara::schedule(gpu, batch.shapes, nullptr, first, count, false, band, limits);
     PhaseTimer timer(gpu, &gpu->kernel_ms);
     KernelArgs args;
@@ -1612,7 +1647,7 @@ void affine_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
     args.open = table.open;
     args.extend = table.extend;
     args.scores = scores;
-    unsigned int *counters = gpu->class_counts.ensure<unsigned int>(20);
+    unsigned int *counters = gpu->class_counts.ensure<unsigned int>(kClassCounters);
     unsigned int *leftover_count = counters + 8;
     uint32_t *leftovers = nullptr;
     int32_t *foreseen = nullptr;  // bands foreseen for the pairs that leave theirs early
@@ -1638,7 +1673,7 @@ void affine_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
                                     size_t(long_pairs) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, gpu->stream));
         rest.skip = kWideClass;
     }
-    affine_launch_all(gpu, batch, table, rest, false, args);
+    affine_launch_all(gpu, batch, table, rest, false, limits, args);
     unsigned int left = 0;
     if (band_pairs(schedule_all) > 0) {
         read_back(gpu, &left, leftover_count, sizeof left);
@@ -1647,9 +1682,11 @@ void affine_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
                 DINARA_CUDA(cudaMemcpyAsync(leftovers + left, leftovers + band_pairs(schedule_all) + long_pairs,
                                             size_t(long_pairs) * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
                                             gpu->stream));
+            PairLimits left_limits = whole_limits_of(batch, table);
+            left_limits.fine = finer_strips(gpu, batch, left);
             const Schedule again = dinara::schedule(gpu, batch.shapes, leftovers, 0, left + long_pairs, false, false,
-                                                    whole_limits_of(batch, table));
-            affine_launch_all(gpu, batch, table, again, false, args, foreseen);
+                                                    left_limits);
+            affine_launch_all(gpu, batch, table, again, false, left_limits, args, foreseen);
         }
     }
     timer.stop();
@@ -1732,7 +1769,7 @@ int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &whole_batch, const
     args.ends = ends;
     args.first_pair = first_pair;
     args.band_widths = widths;
-    unsigned int *counters = gpu->class_counts.ensure<unsigned int>(20);
+    unsigned int *counters = gpu->class_counts.ensure<unsigned int>(kClassCounters);
     unsigned int *leftover_count = counters + 8;
     uint32_t *leftovers = nullptr;
     uint64_t *extra = nullptr;
@@ -1742,7 +1779,7 @@ int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &whole_batch, const
         launch_bands(gpu, batch, table, schedule_all, scores, leftovers, leftover_count, true, decisions, word_offsets,
                      first_pair, layouts, band_counter(gpu));
     }
-    affine_launch_all(gpu, batch, table, schedule_all, true, args);
+    affine_launch_all(gpu, batch, table, schedule_all, true, limits, args);
     unsigned int left = 0;
     if (band_pairs(schedule_all) > 0) {
         read_back(gpu, &left, leftover_count, sizeof left);
@@ -1771,7 +1808,7 @@ int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &whole_batch, const
             const Schedule again = dinara::schedule(gpu, batch.shapes, leftovers, 0, left, true, false, left_limits);
             KernelArgs extra_args = args;
             extra_args.decisions = extra;
-            affine_launch_all(gpu, batch, table, again, true, extra_args);
+            affine_launch_all(gpu, batch, table, again, true, left_limits, extra_args);
         }
     }
 

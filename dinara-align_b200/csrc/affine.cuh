@@ -13,13 +13,36 @@ constexpr int kAffineShapes = 5;
 __host__ __device__ inline int affine_lanes(int shape) {
     return shape == 0 ? 4 : shape == 1 ? 8 : shape == 2 ? 16 : shape == 3 ? 16 : 32;
 }
-__host__ __device__ inline int affine_columns(int shape) { return shape == 3 ? 20 : 16; }
+__host__ __device__ inline int affine_columns(int shape) {
+    return shape == 3 || shape == 7 ? 20 : shape == 5 ? 12 : shape == 6 ? 14 : shape == 8 ? 24 : 16;
+}
 __host__ __device__ inline int affine_shape_for(uint32_t columns, bool record) {
     if (columns <= 64) return 0;
     if (columns <= 128) return 1;
     if (columns <= 256) return 2;
     if (!record && columns <= 320) return 3;
     return 4;
+}
+
+// The shapes of the two-bit 16-bit pair score sweeps: those, and 32 lanes of 12, 14, 20 and 24 columns (5 to 8).
+constexpr int kPairShapes = 9;
+// The one that sweeps the fewest columns past a pair's last: past 320 columns, of strips of 384, 448, 512, 640 and
+// 768 the least sum that spans the pair, of equal ones the widest. (20,000 reads of 150 to 1,000 letters sweep 631
+// columns on average for their 575, 759 with strips of 512 alone.)
+__host__ __device__ inline int pair_shape_for(uint32_t columns) {
+    if (columns <= 320) return affine_shape_for(columns, false);
+    const int shapes[5] = {8, 7, 4, 6, 5};
+    int best = 4;
+    uint32_t least = ~0u;
+    for (int k = 0; k < 5; ++k) {
+        const uint32_t width = uint32_t(32 * affine_columns(shapes[k]));
+        const uint32_t swept = (columns + width - 1) / width * width;
+        if (swept < least) {
+            least = swept;
+            best = shapes[k];
+        }
+    }
+    return best;
 }
 
 // Lanes a pair's recording sweep takes: its shape class's, or 32 for the shared-memory table path,

@@ -100,26 +100,30 @@ __device__ void classify_pair(const PairShape *__restrict__ shapes, const uint32
     if (limits.band_widths && limits.band_widths[pair - limits.band_first] > 0) {
         cls = kBandRecordClass;
         strips = (shape.columns + 511) / 512;
-        if (strips > 255) strips = 255;
+        if (strips > 127) strips = 127;
     } else if (band && band_eligible(shape.rows, shape.columns)) {
         cls = int64_t(shape.rows) + shape.columns <= limits.band ? kBandPairsClass : kBandClass;
     } else {
         cls = empty ? 0 : affine_shape_for(shape.columns, record != 0);
         if (!record && limits.wide && shape.rows >= kWideRows && shape.columns >= kWideColumns) cls = kWideClass;
-        const uint32_t width = cls == kWideClass ? 4096u : uint32_t(affine_lanes(cls) * affine_columns(cls));
+        const int fitted = limits.fine && cls < kAffineShapes && !empty ? pair_shape_for(shape.columns) : cls;
+        const bool pairs16 =
+            cls != kWideClass && takes_pairs16(limits, shape.rows, shape.columns, fitted, record != 0);
+        const int swept_by = pairs16 ? fitted : cls;
+        const uint32_t width =
+            cls == kWideClass ? 4096u : uint32_t(affine_lanes(swept_by) * affine_columns(swept_by));
         strips = empty ? 0 : (shape.columns + width - 1) / width;
-        const bool pairs16 = takes_pairs16(limits, shape.rows, shape.columns, cls, record != 0);
         if (pairs16) {
-            cls += kWholePairsClass;
+            cls = kWholePairsClass + fitted;
         } else if (!record && limits.long_strips && shape.rows >= kLongSide && shape.columns >= kLongSide) {
             cls = kWideClass;
             strips = (shape.columns + 4095) / 4096;
         }
-        if (strips > 255) strips = 255;
+        if (strips > 127) strips = 127;
     }
     uint32_t rows = shape.rows >> 2;
     if (rows > 0xFFFFFu) rows = 0xFFFFFu;
-    keys[k] = (uint32_t(cls) << 28) | (strips << 20) | rows;
+    keys[k] = (uint32_t(cls) << 27) | (strips << 20) | rows;
     order[k] = pair;
     atomicAdd(&block_counts[cls], 1u);
 }
@@ -166,7 +170,7 @@ Schedule schedule(dinara_gpu *gpu, const PairShape *shapes, const uint32_t *list
     uint32_t *order = gpu->order.ensure<uint32_t>(count);
     uint32_t *keys_out = gpu->keys_sorted.ensure<uint32_t>(count);
     uint32_t *order_out = gpu->order_sorted.ensure<uint32_t>(count);
-    unsigned int *class_counts = gpu->class_counts.ensure<unsigned int>(kClasses);
+    unsigned int *class_counts = gpu->class_counts.ensure<unsigned int>(kClassCounters) + kScheduleCounts;
     DINARA_CUDA(cudaMemsetAsync(class_counts, 0, kClasses * sizeof(unsigned int), gpu->stream));
     const int threads = 256;
     schedule_keys_kernel<<<unsigned((count + threads - 1) / threads), threads, 0, gpu->stream>>>(

@@ -21,12 +21,16 @@ void pack_pairs(dinara_gpu *gpu, const uint8_t *letters_device, const int64_t *o
 // takes, kWholePairsClass plus the shape class; long pairs one block sweeps, kWideClass; and, recording,
 // pairs whose widening band proved a width (`limits.band_widths`), kBandRecordClass. `order` is valid on
 // the device until the next call.
-constexpr int kClasses = 14;
+constexpr int kClasses = 18;
 constexpr int kBandClass = 5;
 constexpr int kBandPairsClass = 6;
 constexpr int kWholePairsClass = 7;
-constexpr int kWideClass = 12;
-constexpr int kBandRecordClass = 13;
+constexpr int kWideClass = kWholePairsClass + kPairShapes;
+constexpr int kBandRecordClass = kWideClass + 1;
+static_assert(kBandRecordClass + 1 == kClasses && kClasses <= 32, "a class is five bits of a key");
+// A context's counters on the device (class_counts): the launches' own in the first words, a schedule's classes
+// from kScheduleCounts on.
+constexpr int kClassCounters = 64, kScheduleCounts = 32;
 // A pair a whole block sweeps (kWideClass), scoring without a CIGAR: at least this tall and this wide.
 constexpr uint32_t kWideRows = 4096, kWideColumns = 2048;
 // With the 16-bit strips: a pair of two strips or more, each way. (600 pairs of 3,000 letters: 8.6 ms in 32 bits,
@@ -46,6 +50,7 @@ struct PairLimits {
     int32_t band = 0;
     int32_t whole = 0;
     int32_t local = 0;
+    int32_t fine = 0;    // the score sweeps' own shapes past 320 columns too (pair_shape_for)
     int32_t record = 0;  // `whole` holds the recording sweep's pairs (else the score sweeps')
     int32_t hits = 0;    // recording: of hits' rows, so only pairs whose hits a score sweep has found
     int32_t wide = 0;
@@ -61,14 +66,13 @@ struct PairLimits {
     int64_t band_first = 0;
 };
 
-// Whether a non-empty pair of whole-matrix shape class `cls` takes a 16-bit pair sweep (`record`: recording).
-__host__ __device__ inline bool takes_pairs16(const PairLimits &limits, uint32_t rows, uint32_t columns, int cls,
+// Whether a pair takes the 16-bit pair sweep of shape `shape` (`record`: recording).
+__host__ __device__ inline bool takes_pairs16(const PairLimits &limits, uint32_t rows, uint32_t columns, int shape,
                                               bool record) {
-    if (limits.whole <= 0 || record != (limits.record != 0) || cls >= kWholePairsClass || rows == 0 || columns == 0)
-        return false;
+    if (limits.whole <= 0 || record != (limits.record != 0) || rows == 0 || columns == 0) return false;
     // The score sweeps left a long pair (kWideClass) its whole shape and no hit.
     if (limits.hits && limits.wide && rows >= kWideRows && columns >= kWideColumns) return false;
-    const uint32_t width = uint32_t(affine_lanes(cls) * affine_columns(cls));
+    const uint32_t width = uint32_t(affine_lanes(shape) * affine_columns(shape));
     const int64_t swept = int64_t((columns + width - 1) / width) * width;
     return limits.local ? swept * limits.best + int64_t(rows) * limits.row_step <= limits.whole
                         : 2 * swept <= limits.whole && 2 * int64_t(rows) <= limits.whole;

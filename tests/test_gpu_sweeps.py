@@ -143,6 +143,28 @@ def test_long_pairs_beside_hits(da, oracle, entries):
     assert [a.cigar for a in found] == cigars
 
 
+@pytest.mark.parametrize("entries", [(2, -4, -4, -2), (1, -3, -5, 0), (0, -4, -6, -2)])
+def test_scores_past_320_columns(da, oracle, entries):
+    """Enough two-bit pairs for the strips of 384 to 768 columns, at the widths where one gives way to the next, a
+    column either side, and past one strip of each; short and a few tall, no band proving them."""
+    rng = np.random.default_rng(abs(sum(entries)) + 11)
+    scoring = da.Scoring.uniform(*entries)
+    widths = [w + d for w in (320, 384, 448, 512, 640, 768, 896, 1024, 1152, 1280, 1536) for d in (-1, 0, 1)]
+    refs, queries = [], []
+    for k in range(9600):
+        source = _text(rng, widths[k % len(widths)])
+        refs.append(source[100:100 + 3 + k % 30] if k >= 66 else _text(rng, 60) + source[:700])
+        queries.append(source)
+    tape = da.Tape.of(refs, queries)
+    coded = np.concatenate([oracle.codes(text) for pair in zip(refs, queries) for text in pair])
+    op, ex = oracle.kernel_gaps(scoring.opening, scoring.extension)
+    for mode, kind in ((da.Mode.GLOBAL, oracle.GLOBAL), (da.Mode.local(), oracle.LOCAL)):
+        if kind == oracle.LOCAL and entries[0] <= 0:
+            continue
+        expected = oracle.batch_scores(coded, tape.offsets, _table(scoring), 4, op, ex, kind, threads=8)
+        np.testing.assert_array_equal(da.scores_tape(tape, scoring, mode), expected)
+
+
 @pytest.mark.parametrize("alphabet", ["ACGT", PROTEIN])
 @pytest.mark.parametrize("local", [False, True])
 def test_recorded_pairs_that_fill_the_gpu(da, oracle, alphabet, local):
