@@ -616,6 +616,7 @@ void launch_together(dinara_gpu *gpu, const AffineBatch &batch, const PairLimits
     const int64_t stride = tallest_of(batch, limits) + 1;
     int2 *carry = all_slots > 0 ? gpu->carry.ensure<int2>(size_t(all_slots * stride)) : nullptr;
     const bool fork = sweeps.size() > 1;
+    ClockSpan clock(gpu, kClassWhole, gpu->stream);  // one for all: they run at once
     if (fork) DINARA_CUDA(cudaEventRecord(gpu->fork, gpu->stream));
     for (size_t k = 0; k < sweeps.size(); ++k) {
         const PairsLaunch &l = sweeps[k].launch;
@@ -626,10 +627,8 @@ void launch_together(dinara_gpu *gpu, const AffineBatch &batch, const PairLimits
         if (slots[k] > 0) carry += slots[k] * stride;
         args.begin = uint32_t(sweeps[k].begin);
         args.end = uint32_t(sweeps[k].end);
-        ClockSpan clock(gpu, kClassWhole, stream);
         l.fn<<<unsigned(blocks[k]), l.threads, l.shared, stream>>>(args, targs, table32);
         DINARA_CUDA(cudaGetLastError());
-        clock.stop();
         gpu->launches += 1;
         if (fork) {
             DINARA_CUDA(cudaEventRecord(gpu->joins[k], stream));
