@@ -569,7 +569,8 @@ PairsLaunch pick_record(int cls, bool local, int bits, int letters) {
 
 int persistent_blocks(dinara_gpu *gpu, KernelFn fn, int threads = kBlock, size_t shared = 0) {
     int per_sm = 0;
-    if (shared > (size_t(48) << 10))
+    // A launch may take 48 KB, the kernel's own shared memory (a profile form's table) among them, without asking.
+    if (shared > 0)
         DINARA_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shared)));
     DINARA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, shared));
     if (per_sm < 1) per_sm = 1;

@@ -2,6 +2,10 @@
 16-bit forms at their limits and a step past them, hits cut to their rows, kept fronts at their sizes, the
 first round's list, and the gradients' slices. Every result is an exact integer or text, except the gradients."""
 
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -254,6 +258,42 @@ def test_profiles_score_globally_and_locally(da, oracle, alphabet):
             np.testing.assert_array_equal(da.scores_tape(tape, scoring, mode), expected)
 
 
+def _check_alphabet(da, oracle, size):
+    """Every profile sweep at `size` letters: scores, hits and recorded alignments, globally and locally, free ends
+    and an extension, in every lane group, globally in a batch large enough for the 16-bit recording."""
+    alphabet = THIRTY_TWO[:size]
+    rng = np.random.default_rng(size)
+    scoring = _tabulated(da, rng, alphabet)
+    op, ex = oracle.kernel_gaps(scoring.opening, scoring.extension)
+    refs, queries = [], []
+    for k in range(4800):
+        source = _text(rng, (60, 120, 250, 300, 500)[k] if k < 5 else 5 + k % 9, alphabet)
+        refs.append(_text(rng, k % 4, alphabet) + source)
+        queries.append(_mutated(rng, source, 0.1, alphabet) or alphabet[0])
+    tape = da.Tape.of(refs, queries)
+    coded = np.concatenate([oracle.codes(text, alphabet) for pair in zip(refs, queries) for text in pair])
+    for mode, how in ((da.Mode.local(), oracle.LOCAL), (da.Mode.GLOBAL, oracle.GLOBAL)):
+        expected, cigars = oracle.batch_alignments(coded, tape.offsets, _table(scoring), size, op, ex, how, threads=8)
+        np.testing.assert_array_equal(da.scores_tape(tape, scoring, mode), expected)
+        found = da.alignments(refs, queries, scoring, mode)
+        assert [(a.score, a.cigar) for a in found] == list(zip(expected, cigars))
+    coded = [(oracle.codes(r, alphabet), oracle.codes(q, alphabet)) for r, q in zip(refs[:40], queries[:40])]
+    found = da.alignments(refs[:40], queries[:40], scoring, da.Mode.INFIX)
+    assert [(a.score, a.cigar, _span(a)) for a in found] == [
+        oracle.free_ends_alignment(a, b, _table(scoring), size, op, ex, BIG, BIG, 0, 0) for a, b in coded]
+    found = da.alignments(refs[:40], queries[:40], scoring, da.Mode.extension(0, da.Anchor.START, zdrop=25))
+    assert [(a.score, a.cigar, _span(a)) for a in found] == [
+        oracle.extension_alignment(a, b, _table(scoring), size, op, ex, False, -1, zdrop=25) for a, b in coded]
+
+
+def test_alphabets_in_rising_order():
+    """A profile's bytes grow with the alphabet, past 48 KB from 24 letters on with the block's table. In a process of
+    its own: a larger alphabet's launch leaves its allowance with the kernel."""
+    run = subprocess.run([sys.executable, os.path.abspath(__file__), "23", "24", "25", "32"], capture_output=True,
+                         text=True, timeout=300)
+    assert run.returncode == 0, run.stdout[-2000:] + run.stderr[-2000:]
+
+
 # ---- alignments under Costs: kept fronts in 16 bits, in 32 and in the shared blocks ---------------------------
 
 @pytest.mark.parametrize("letters", [31_998, 32_002])
@@ -337,3 +377,13 @@ def test_gradients_at_slice_edges(da, batch):
     expected, expected_loss = mlp_oracle.gradients(*(v.astype(np.float64) for v in (flat, x, t)))
     np.testing.assert_allclose(got, expected, rtol=0, atol=1e-4 * np.abs(expected).max())
     assert abs(loss - expected_loss) <= 1e-5 * expected_loss
+
+
+if __name__ == "__main__":
+    # One process's alphabets in turn (test_alphabets_in_rising_order).
+    import conftest  # noqa: F401
+    import dinara_align
+    import oracle as cpu
+
+    for letters in sys.argv[1:]:
+        _check_alphabet(dinara_align, cpu, int(letters))
