@@ -516,12 +516,12 @@ constexpr int kPairsThreads = 64;
 struct PairsLaunch {
     KernelFn fn;
     int lanes, columns, threads;
-    size_t shared;
+    size_t shared, most_shared;  // this alphabet's, and the largest one's
 };
 
 PairsLaunch pairs_launch(KernelFn two_bits, KernelFn bytes, int bits, int lanes, int columns, int letters) {
-    return {bits == 8 ? bytes : two_bits, lanes, columns, kPairsThreads,
-            bits == 8 ? size_t(kPairsThreads / 32) * 64 * letters * columns : 0};
+    const size_t a_letter = bits == 8 ? size_t(kPairsThreads / 32) * 64 * columns : 0;
+    return {bits == 8 ? bytes : two_bits, lanes, columns, kPairsThreads, a_letter * letters, a_letter * 32};
 }
 
 // Scores, or (`hits`, local) each hit's rows. The 20-column shape is the two-bit form's alone.
@@ -567,11 +567,13 @@ PairsLaunch pick_record(int cls, bool local, int bits, int letters) {
 #undef DINARA_RECORD
 }
 
-int persistent_blocks(dinara_gpu *gpu, KernelFn fn, int threads = kBlock, size_t shared = 0) {
+int persistent_blocks(dinara_gpu *gpu, KernelFn fn, int threads = kBlock, size_t shared = 0, size_t most_shared = 0) {
     int per_sm = 0;
-    // A launch may take 48 KB, the kernel's own shared memory (a profile form's table) among them, without asking.
-    if (shared > 0)
-        DINARA_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shared)));
+    // A launch may take 48 KB, the kernel's own shared memory (a profile form's table) among them, without asking. The
+    // allowance is the kernel's for every context in the process, so each asks for the same, the largest any takes: one
+    // that asked for its own alphabet's would take it from another context between that one's asking and its launch.
+    if (most_shared > 0)
+        DINARA_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most_shared)));
     DINARA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, shared));
     if (per_sm < 1) per_sm = 1;
     return per_sm * gpu->multiprocessors;
@@ -608,7 +610,7 @@ void launch_together(dinara_gpu *gpu, const AffineBatch &batch, const PairLimits
         const int64_t groups = l.threads / l.lanes;
         const int64_t needed = (sweep.end - sweep.begin + 2 * groups - 1) / (2 * groups);
         blocks.push_back(
-            std::max<int64_t>(1, std::min<int64_t>(persistent_blocks(gpu, l.fn, l.threads, l.shared), needed)));
+            std::max<int64_t>(1, std::min<int64_t>(persistent_blocks(gpu, l.fn, l.threads, l.shared, l.most_shared), needed)));
         const int cls = sweep.cls;
         const int64_t widest = cls < 4 ? affine_lanes(cls) * affine_columns(cls) : int64_t(batch.max_columns);
         slots.push_back(widest > int64_t(l.lanes) * l.columns ? blocks.back() * groups : 0);

@@ -2,9 +2,11 @@
 16-bit forms at their limits and a step past them, hits cut to their rows, kept fronts at their sizes, the
 first round's list, and the gradients' slices. Every result is an exact integer or text, except the gradients."""
 
+import ctypes
 import os
 import subprocess
 import sys
+import threading
 
 import numpy as np
 import pytest
@@ -292,6 +294,38 @@ def test_alphabets_in_rising_order():
     run = subprocess.run([sys.executable, os.path.abspath(__file__), "23", "24", "25", "32"], capture_output=True,
                          text=True, timeout=300)
     assert run.returncode == 0, run.stdout[-2000:] + run.stderr[-2000:]
+
+
+def test_two_contexts_with_alphabets_apart(da):
+    """A kernel's shared-memory allowance is the process's: contexts on threads of their own, one at 25 letters and one
+    at 32, launch side by side. (One launch in some thousands was refused when each asked for its own size.)"""
+    lib, native = da._native.lib(), da._native
+    failures = []
+
+    def score(size):
+        context = lib.dinara_gpu_new(0)
+        rng = np.random.default_rng(size)
+        alphabet = THIRTY_TWO[:size]
+        tape = da.Tape.of([_text(rng, 200, alphabet)] * 8, [_text(rng, 200, alphabet)] * 8)
+        scoring, _table_kept, _alphabet_kept = da.Scoring.uniform(5, -2, -10, -1, alphabet)._struct()
+        mode = da.Mode.local()._struct()
+        scores, statuses = np.empty(8, np.int32), np.empty(8, np.int64)
+        for _ in range(15_000):
+            code = lib.dinara_gpu_scores_tape(context, 8, tape.letters.ctypes.data,
+                                              native.pointer(tape.offsets, ctypes.c_int64), ctypes.byref(scoring),
+                                              ctypes.byref(mode), native.pointer(scores, ctypes.c_int32),
+                                              native.pointer(statuses, ctypes.c_int64))
+            if code:
+                failures.append((size, code, lib.dinara_gpu_last_error(context)))
+                break
+        lib.dinara_gpu_free(context)
+
+    threads = [threading.Thread(target=score, args=(size,)) for size in (25, 32)]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    assert not failures, failures
 
 
 # ---- alignments under Costs: kept fronts in 16 bits, in 32 and in the shared blocks ---------------------------
