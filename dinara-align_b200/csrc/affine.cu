@@ -1881,35 +1881,68 @@ void last_places(dinara_gpu *gpu, const uint8_t *letters, const int64_t *offsets
 
 namespace {
 
-// Spans that do not lie within their pair's letters are emptied and their pair flagged (before its span is packed);
-// with `inner`, pairs whose span aligned globally scores otherwise than the span's own score are flagged.
+// Spans that do not lie within their pair's letters are emptied and their pair flagged (before its span is packed).
+// The spans' sizes are summed, and their sides' most found, a warp at a time.
 __global__ void check_spans_kernel(const int64_t *__restrict__ offsets, int64_t first_pair, int64_t count,
-                                   int64_t *__restrict__ spans, const int32_t *__restrict__ scores,
-                                   const int32_t *__restrict__ inner, uint8_t *__restrict__ flags) {
+                                   int64_t *__restrict__ spans, bool uniform, bool band, uint8_t *__restrict__ flags,
+                                   SpanSizes *__restrict__ sizes) {
     const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    const int64_t pair = first_pair + k;
-    bool failed = false;
-    if (inner) {
-        failed = inner[pair] != scores[pair];
-    } else {
+    unsigned long long words = 0;
+    uint32_t span_rows = 0, span_columns = 0;
+    if (k < count) {
+        const int64_t pair = first_pair + k;
         int64_t *span = spans + 4 * k;
         const int64_t rows = offsets[2 * pair + 1] - offsets[2 * pair];
         const int64_t columns = offsets[2 * pair + 2] - offsets[2 * pair + 1];
-        failed = !(0 <= span[0] && span[0] <= span[1] && span[1] <= rows && 0 <= span[2] && span[2] <= span[3] &&
-                   span[3] <= columns);
-        if (failed) span[0] = span[1] = span[2] = span[3] = 0;
+        if (0 <= span[0] && span[0] <= span[1] && span[1] <= rows && 0 <= span[2] && span[2] <= span[3] &&
+            span[3] <= columns) {
+            span_rows = uint32_t(span[1] - span[0]);
+            span_columns = uint32_t(span[3] - span[2]);
+            words = (unsigned long long)record_words(span_rows, span_columns, uniform, band);
+        } else {
+            span[0] = span[1] = span[2] = span[3] = 0;
+            if (flags[pair] == 0) flags[pair] = kWalkFailed;
+        }
     }
-    if (failed && flags[pair] == 0) flags[pair] = kWalkFailed;
+#pragma unroll
+    for (int apart = 16; apart > 0; apart >>= 1) words += __shfl_xor_sync(kFull, words, apart);
+    span_rows = __reduce_max_sync(kFull, span_rows);
+    span_columns = __reduce_max_sync(kFull, span_columns);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(reinterpret_cast<unsigned long long *>(&sizes->words), words);
+        atomicMax(&sizes->max_rows, span_rows);
+        atomicMax(&sizes->max_columns, span_columns);
+    }
+}
+
+// Pairs whose span aligned globally scores otherwise than the span's own score are flagged.
+__global__ void check_span_scores_kernel(int64_t first_pair, int64_t count, const int32_t *__restrict__ scores,
+                                         const int32_t *__restrict__ inner, uint8_t *__restrict__ flags) {
+    const int64_t pair = first_pair + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (pair < first_pair + count && inner[pair] != scores[pair] && flags[pair] == 0) flags[pair] = kWalkFailed;
 }
 
 }  // namespace
 
-void check_spans(dinara_gpu *gpu, const int64_t *offsets, int64_t first_pair, int64_t count, int64_t *spans,
-                 const int32_t *scores, const int32_t *inner, uint8_t *flags) {
+SpanSizes check_spans(dinara_gpu *gpu, const int64_t *offsets, int64_t first_pair, int64_t count, int64_t *spans,
+                      bool uniform, bool band, uint8_t *flags) {
+    SpanSizes sizes{0, 0, 0};
+    if (count <= 0) return sizes;
+    SpanSizes *out = reinterpret_cast<SpanSizes *>(gpu->class_counts.ensure<unsigned int>(kClassCounters) + 20);
+    DINARA_CUDA(cudaMemsetAsync(out, 0, sizeof(SpanSizes), gpu->stream));
+    check_spans_kernel<<<unsigned((count + 255) / 256), 256, 0, gpu->stream>>>(offsets, first_pair, count, spans,
+                                                                             uniform, band, flags, out);
+    DINARA_CUDA(cudaGetLastError());
+    gpu->launches += 1;
+    read_back(gpu, &sizes, out, sizeof sizes);
+    return sizes;
+}
+
+void check_span_scores(dinara_gpu *gpu, int64_t first_pair, int64_t count, const int32_t *scores, const int32_t *inner,
+                       uint8_t *flags) {
     if (count <= 0) return;
-    check_spans_kernel<<<unsigned((count + 255) / 256), 256, 0, gpu->stream>>>(offsets, first_pair, count, spans, scores,
-                                                                             inner, flags);
+    check_span_scores_kernel<<<unsigned((count + 255) / 256), 256, 0, gpu->stream>>>(first_pair, count, scores, inner,
+                                                                                   flags);
     DINARA_CUDA(cudaGetLastError());
     gpu->launches += 1;
 }

@@ -111,10 +111,21 @@ int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &batch, const Affin
 void last_places(dinara_gpu *gpu, const uint8_t *letters, const int64_t *offsets, int64_t first_pair, int64_t count,
                  int64_t *spans);
 
+// What a range's spans, as pairs of their own, hold: the words their recorded decisions take (record_words) and the
+// longest side of each kind.
+struct SpanSizes {
+    int64_t words;
+    uint32_t max_rows, max_columns;
+};
+
 // Flags (kWalkFailed, where a pair has no flag yet) the pairs of [first_pair, first_pair + count) whose span lies
-// outside its letters, emptying the span; or, with `inner`, those whose span's own score `scores` differs from its
-// global alignment's. Spans are 4 a pair of the range, the rest by pair (device).
-void check_spans(dinara_gpu *gpu, const int64_t *offsets, int64_t first_pair, int64_t count, int64_t *spans,
-                 const int32_t *scores, const int32_t *inner, uint8_t *flags);
+// outside its letters, emptying the span, and returns the spans' sizes. Spans are 4 a pair of the range, the flags by
+// pair (device).
+SpanSizes check_spans(dinara_gpu *gpu, const int64_t *offsets, int64_t first_pair, int64_t count, int64_t *spans,
+                      bool uniform, bool band, uint8_t *flags);
+
+// Flags likewise the pairs whose span's score `scores` differs from `inner`, its global alignment's (by pair, device).
+void check_span_scores(dinara_gpu *gpu, int64_t first_pair, int64_t count, const int32_t *scores, const int32_t *inner,
+                       uint8_t *flags);
 
 }  // namespace dinara

@@ -26,6 +26,14 @@ __host__ __device__ inline bool band_eligible(uint32_t rows, uint32_t columns) {
     return rows > 0 && columns > 0 && band_low_for(rows, columns) != INT32_MIN;
 }
 
+// The most 64-bit words a pair's recorded decisions take (affine.cu's recording kernels), its band's leftovers apart.
+__host__ __device__ inline int64_t record_words(int64_t rows, int64_t columns, bool uniform, bool band) {
+    if (rows <= 0 || columns <= 0) return 0;
+    if (band && band_eligible(uint32_t(rows), uint32_t(columns))) return int64_t(kBandLanes) * ((rows + 3) & ~int64_t(3));
+    const int64_t lanes = record_lanes(uint32_t(columns), uniform);
+    return (columns + lanes * 16 - 1) / (lanes * 16) * lanes * (((rows + 2) | 3) + 1);
+}
+
 // Whether a band score proves itself (the bound of band_groups.mojo:235-248, restated for a table's
 // best entry `best` and gaps in the kernels' terms): any path visiting a diagonal outside [low, high]
 // takes at least two gap runs and g gap letters, g from the nearest diagonal outside, so scores at most

@@ -384,12 +384,36 @@ Packed pack_batch(dinara_gpu *gpu, int64_t pairs, const char *letters, const int
 // Device memory a launch's recorded decisions may take before the batch is cut into chunks.
 constexpr int64_t kDecisionBudget = int64_t(8) << 30;
 
-// The 64-bit words a pair's recorded decisions take (the layout affine.cu's record kernels write).
-int64_t record_words(int64_t rows, int64_t columns, bool uniform, bool band) {
-    if (rows <= 0 || columns <= 0) return 0;
-    if (band && band_eligible(uint32_t(rows), uint32_t(columns))) return int64_t(kBandLanes) * ((rows + 3) & ~int64_t(3));
-    const int64_t lanes = record_lanes(uint32_t(columns), uniform);
-    return (columns + lanes * 16 - 1) / (lanes * 16) * lanes * (((rows + 2) | 3) + 1);
+// A placed unit's CIGARs, recorded in parts, on the host: their bytes, and their offsets (one a pair and one).
+struct RecordedParts {
+    std::vector<char> bytes;
+    std::vector<int64_t> offsets{0};
+};
+
+// Alignments of pairs [first, first + count) of a batch whose recorded decisions pass the budget, in parts that keep
+// it by the pairs' own sides (`spans`, on the device: 4 a pair of the range, the sides' first and last letters).
+void record_in_parts(dinara_gpu *gpu, const AffineBatch &batch, const dinara::AffineTable &table, bool eqx,
+                     bool uniform, bool band, const int64_t *spans, int64_t first, int64_t count, int32_t *scores,
+                     int64_t *walked, RecordedParts &out) {
+    std::vector<int64_t> sides(size_t(4 * count));
+    to_host_now(gpu, sides.data(), spans, sides.size() * sizeof(int64_t));
+    for (int64_t begin = 0; begin < count;) {
+        int64_t end = begin, words = 0;
+        for (; end < count; ++end) {
+            const int64_t *s = sides.data() + 4 * end;
+            const int64_t more = record_words(s[1] - s[0], s[3] - s[2], uniform, band);
+            if (end > begin && words + more > kDecisionBudget / 8) break;
+            words += more;
+        }
+        const int64_t total = affine_alignments(gpu, batch, table, eqx, scores, walked, first + begin, end - begin);
+        const size_t at = out.bytes.size();
+        out.bytes.resize(at + size_t(total));
+        to_host_now(gpu, out.bytes.data() + at, gpu->cigar_bytes.as<char>(), size_t(total));
+        std::vector<int64_t> ends(size_t(end - begin + 1));
+        to_host_now(gpu, ends.data(), gpu->cigar_offsets.as<int64_t>(), ends.size() * sizeof(int64_t));
+        for (size_t k = 1; k < ends.size(); ++k) out.offsets.push_back(int64_t(at) + ends[k]);
+        begin = end;
+    }
 }
 
 // Per-pair statuses of pairs [first, first + count): scores that could pass 2^28 (-3), then a walk that
@@ -1323,7 +1347,8 @@ int64_t dinara_gpu_alignments_tape(dinara_gpu *gpu, int64_t pairs, const char *l
             // The partners' units wait for these buffers too.
             DINARA_CUDA(cudaEventRecord(streamed.inputs_ready, gpu->stream));
         }
-        // Units whose recorded decisions stay within a budget of device memory.
+        // Units whose recorded decisions stay within a budget of device memory; a placed batch's, whose spans are
+        // not known yet, as its scores' (its recording keeps the budget once they are).
         const bool uniform = !checked.table.packed16 || checked.bits == 8;
         const bool band = band_serves(batch, checked.table);
         const auto units = plan_units(
@@ -1332,7 +1357,7 @@ int64_t dinara_gpu_alignments_tape(dinara_gpu *gpu, int64_t pairs, const char *l
                 return record_words(offsets[2 * p + 1] - offsets[2 * p], offsets[2 * p + 2] - offsets[2 * p + 1],
                                     uniform, band);
             },
-            true, kDecisionBudget / 8);
+            !placed, kDecisionBudget / 8);
         // Every unit's CIGAR bytes go straight into the caller's buffer.
         std::unique_ptr<char, void (*)(void *)> bytes(nullptr, std::free);
         size_t room = 0, size = 0;
@@ -1381,16 +1406,28 @@ int64_t dinara_gpu_alignments_tape(dinara_gpu *gpu, int64_t pairs, const char *l
             StagedUnit unit;
             unit.first = first;
             unit.count = count;
+            RecordedParts parts;
+            bool in_parts = false;
             if (placed) {
                 int64_t *placed_spans = ctx->placed.ensure<int64_t>(size_t(4 * count));
                 affine_scores(ctx, ends, checked.table, scores_device, first, count, placed_spans);
-                check_spans(ctx, streamed.offsets_device, first, count, placed_spans, nullptr, nullptr, packed.unknown);
+                const SpanSizes sizes = check_spans(ctx, streamed.offsets_device, first, count, placed_spans, uniform,
+                                                    band, packed.unknown);
                 pack_pairs(ctx, streamed.letters_device, streamed.offsets_device, first, count, streamed.codes_device,
                            checked.bits, inner_tape, inner_shapes, nullptr, placed_spans);
-                unit.total = affine_alignments(ctx, inner, checked.table, eqx != 0, inner_scores, spans_device, first,
-                                               count);
-                check_spans(ctx, streamed.offsets_device, first, count, nullptr, scores_device, inner_scores,
-                            packed.unknown);
+                AffineBatch spanned = inner;
+                spanned.max_rows = sizes.max_rows;
+                spanned.max_columns = sizes.max_columns;
+                in_parts = sizes.words > kDecisionBudget / 8;
+                if (in_parts) {
+                    record_in_parts(ctx, spanned, checked.table, eqx != 0, uniform, band, placed_spans, first, count,
+                                    inner_scores, spans_device, parts);
+                    unit.total = int64_t(parts.bytes.size());
+                } else {
+                    unit.total = affine_alignments(ctx, spanned, checked.table, eqx != 0, inner_scores, spans_device,
+                                                   first, count);
+                }
+                check_span_scores(ctx, first, count, scores_device, inner_scores, packed.unknown);
                 spans_device = placed_spans;
             } else {
                 unit.total = affine_alignments(ctx, batch, checked.table, eqx != 0, scores_device, spans_device, first,
@@ -1401,10 +1438,16 @@ int64_t dinara_gpu_alignments_tape(dinara_gpu *gpu, int64_t pairs, const char *l
             unit.layout = StageLayout(count, unit.total, local || placed);
             uint8_t *stage = finisher.stage_for(int64_t(k), unit.layout.bytes);
             unit.stage = stage;
-            DINARA_CUDA(cudaMemcpyAsync(stage + unit.layout.cigars, ctx->cigar_bytes.as<char>(), size_t(unit.total),
-                                        cudaMemcpyDeviceToHost, ctx->stream));
-            DINARA_CUDA(cudaMemcpyAsync(stage + unit.layout.cigar_offsets, ctx->cigar_offsets.as<int64_t>(),
-                                        size_t(count + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+            if (in_parts) {
+                std::memcpy(stage + unit.layout.cigars, parts.bytes.data(), parts.bytes.size());
+                std::memcpy(stage + unit.layout.cigar_offsets, parts.offsets.data(),
+                            parts.offsets.size() * sizeof(int64_t));
+            } else {
+                DINARA_CUDA(cudaMemcpyAsync(stage + unit.layout.cigars, ctx->cigar_bytes.as<char>(),
+                                            size_t(unit.total), cudaMemcpyDeviceToHost, ctx->stream));
+                DINARA_CUDA(cudaMemcpyAsync(stage + unit.layout.cigar_offsets, ctx->cigar_offsets.as<int64_t>(),
+                                            size_t(count + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+            }
             DINARA_CUDA(cudaMemcpyAsync(stage + unit.layout.scores, scores_device + first,
                                         size_t(count) * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
             DINARA_CUDA(cudaMemcpyAsync(stage + unit.layout.unknown, packed.unknown + first, size_t(count),

@@ -242,6 +242,78 @@ def test_free_ends_and_extensions_at_the_widths(da, oracle, alphabet, entries):
             assert [(a.score, a.cigar, _span(a)) for a in found] == expected
 
 
+def _tiled(da, refs, queries, times):
+    """The pairs over and over as one tape."""
+    once = da.Tape.of(refs, queries)
+    letters = int(once.offsets[-1])
+    starts = (np.arange(times)[:, None] * letters + once.offsets[None, :-1]).reshape(-1)
+    return da.Tape(np.tile(once.letters[:letters], times), np.append(starts, times * letters))
+
+
+def _assert_tiled(da, tape, scoring, mode, expected, times):
+    scores, spans, offsets, data, statuses = da.alignments_tape(tape, scoring, mode)
+    assert not statuses.any()
+    np.testing.assert_array_equal(scores, np.tile([score for score, _c, _s in expected], times))
+    np.testing.assert_array_equal(spans, np.tile([span for _s, _c, span in expected], (times, 1)))
+    np.testing.assert_array_equal(np.diff(offsets), np.tile([len(cigar) for _s, cigar, _p in expected], times))
+    assert data.tobytes() == "".join(cigar for _s, cigar, _p in expected).encode() * times
+
+
+def test_placed_alignments_in_several_units(da, oracle):
+    """140,000 pairs take four units on four lanes, which share the spans' tape, shapes and scores."""
+    rng = np.random.default_rng(140)
+    scoring = da.Scoring.uniform(2, -4, -4, -2)
+    op, ex = oracle.kernel_gaps(scoring.opening, scoring.extension)
+    refs, queries = [], []
+    for k in range(1400):
+        source = _text(rng, 1 + k % 40)
+        refs.append(_text(rng, k % 17) + source + _text(rng, k % 13))
+        queries.append(_mutated(rng, source, 0.1, "ACGT") if k % 50 else "")
+    coded = [(oracle.codes(r), oracle.codes(q)) for r, q in zip(refs, queries)]
+    tape = _tiled(da, refs, queries, 100)
+    expected = [oracle.free_ends_alignment(a, b, _table(scoring), 4, op, ex, BIG, BIG, 0, 0) for a, b in coded]
+    _assert_tiled(da, tape, scoring, da.Mode.INFIX, expected, 100)
+    for from_end in (False, True):
+        mode = da.Mode.extension(0, da.Anchor.END if from_end else da.Anchor.START, zdrop=12, end_bonus=4)
+        expected = [oracle.extension_alignment(a, b, _table(scoring), 4, op, ex, from_end, 4, zdrop=12)
+                    for a, b in coded]
+        _assert_tiled(da, tape, scoring, mode, expected, 100)
+
+
+def _check_spans_past_their_pairs_band(da, oracle):
+    """2,400 overlaps of 4,000 x 4,000 letters, which as global pairs would keep a band of 64 diagonals, and whose spans
+    of 3,800 x 3,900 do not: their recorded decisions take 18.7 GB, in parts of 8 GiB. Prints the device memory that
+    the call leaves taken."""
+    import torch
+
+    rng = np.random.default_rng(24)
+    scoring = da.Scoring.uniform(2, -4, -4, -2)
+    op, ex = oracle.kernel_gaps(scoring.opening, scoring.extension)
+    refs, queries = [], []
+    for _ in range(8):
+        core = _text(rng, 3800)
+        refs.append(_text(rng, 200) + core)
+        queries.append((_mutated(rng, core[:1900], 0.02, "ACGT") + _text(rng, 100) +
+                        _mutated(rng, core[1900:], 0.02, "ACGT") + _text(rng, 200))[:4000])
+    mode = da.Mode.ends_free(reference_start=BIG, query_end=BIG)
+    da.alignments(refs[:1], queries[:1], scoring, mode)
+    before = torch.cuda.mem_get_info()[0]
+    expected = [oracle.free_ends_alignment(oracle.codes(r), oracle.codes(q), _table(scoring), 4, op, ex, BIG, 0, 0, BIG)
+                for r, q in zip(refs, queries)]
+    assert all(abs((s[1] - s[0]) - (s[3] - s[2])) >= 64 for _s, _c, s in expected)
+    _assert_tiled(da, _tiled(da, refs, queries, 300), scoring, mode, expected, 300)
+    print("bytes", before - torch.cuda.mem_get_info()[0])
+
+
+def test_spans_past_their_pairs_band(da):
+    """In a process of its own, whose memory no earlier call has taken: 8 GiB of decisions and a quarter (what a buffer
+    grows by), and 2 GB for the rest of the call."""
+    run = subprocess.run([sys.executable, os.path.abspath(__file__), "spans"], capture_output=True, text=True,
+                         timeout=300)
+    assert run.returncode == 0, run.stdout[-2000:] + run.stderr[-2000:]
+    assert int(run.stdout.split("bytes")[1]) < 1.25 * 2 ** 33 + 2e9, run.stdout
+
+
 # ---- larger alphabets through profiles --------------------------------------------------------------------
 
 @pytest.mark.parametrize("alphabet", ["ACGTN", PROTEIN, THIRTY_TWO])
@@ -414,10 +486,13 @@ def test_gradients_at_slice_edges(da, batch):
 
 
 if __name__ == "__main__":
-    # One process's alphabets in turn (test_alphabets_in_rising_order).
+    # What needs a process of its own: the spans past their pairs' band, or alphabets in turn.
     import conftest  # noqa: F401
     import dinara_align
     import oracle as cpu
 
-    for letters in sys.argv[1:]:
-        _check_alphabet(dinara_align, cpu, int(letters))
+    if sys.argv[1] == "spans":
+        _check_spans_past_their_pairs_band(dinara_align, cpu)
+    else:
+        for letters in sys.argv[1:]:
+            _check_alphabet(dinara_align, cpu, int(letters))
