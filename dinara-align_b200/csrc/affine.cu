@@ -727,6 +727,9 @@ struct PhaseTimer {
     }
 };
 
+// The first band of pairs that the 16-bit strips do not sweep, and the second chance of those they record.
+constexpr int kWideBand = 2048;
+
 // A widening band round's routing. A pair swept over its band of `swept[k]` diagonals keeps its score
 // when the band proves it (band_proves_width), or when the band could not hold both ends (the sweep was
 // then whole). Otherwise the band's score, a real alignment's, says how wide a band would prove a score
@@ -735,7 +738,12 @@ struct PhaseTimer {
 // last, rounded up to 256 diagonals) unless this is the `last` round or that band's strips of
 // `strip_columns` would sweep three fifths of its rows or more: then to the whole-matrix list. With `swept`
 // null, every pair is routed to `first_width`, or a wider band foreseen for it (`foreseen`, by pair, when
-// given). With `proven`, a pair whose band proves its score leaves the width there (by pair - proven_first).
+// given).
+// With `proven`, a pair whose band proves its score leaves there (by pair - proven_first) the least width that proves
+// that score, for its recording: a path far off the diagonals first scores low in a narrow band, so that the
+// band that finds it is several times as wide as its score needs. And a pair whose band would be too wide for its
+// worth goes round at kWideBand, which may hold its path, unless its score is an unrelated pair's (which asks
+// for nine tenths of its rows and more under most tables).
 __global__ void wide_route_kernel(const PairShape *__restrict__ shapes, const uint32_t *__restrict__ pending,
                                   const int32_t *__restrict__ swept, int64_t count, int32_t first_width, bool last,
                                   const int32_t *__restrict__ scores, int32_t best, int32_t open, int32_t extend,
@@ -749,17 +757,26 @@ __global__ void wide_route_kernel(const PairShape *__restrict__ shapes, const ui
     const uint32_t pair = pending[k];
     const PairShape sh = shapes[pair];
     const int64_t rows = sh.rows, columns = sh.columns;
-    int64_t width = first_width;
+    int64_t width = first_width, done = 0;
     if (swept) {
-        const int64_t done = swept[k];
+        done = swept[k];
+        const int64_t per_letter = int64_t(best) - 2 * int64_t(extend);
         const int32_t low = band_low_for_width(rows, columns, done);
         if (low == INT32_MIN) return;
         const int64_t score = scores[pair];
         if (band_proves_width(score, rows, columns, low, done, best, open, extend)) {
-            if (proven) proven[pair - proven_first] = int32_t(done);
+            if (proven) {
+                int64_t least = done;
+                if (per_letter > 0) least = (band_width_to_prove(score, rows, columns, best, open, extend) + 15) & ~int64_t(15);
+                auto proves = [&](int64_t w) {
+                    const int32_t from = band_low_for_width(rows, columns, w);
+                    return from != INT32_MIN && band_proves_width(score, rows, columns, from, w, best, open, extend);
+                };
+                while (least < done && !proves(least)) least += 16;
+                proven[pair - proven_first] = int32_t(min(least, done));
+            }
             return;
         }
-        const int64_t per_letter = int64_t(best) - 2 * int64_t(extend);
         if (per_letter <= 0) {  // no band proves anything narrower than the matrix
             whole[atomicAdd(whole_count, 1u)] = pair;
             return;
@@ -775,6 +792,8 @@ __global__ void wide_route_kernel(const PairShape *__restrict__ shapes, const ui
         const int64_t wanted = (int64_t(foreseen[pair]) + 255) / 256 * 256;
         if (wanted > width && worth(wanted)) width = wanted;
     }
+    if (swept && proven && done < kWideBand && !worth(width) && 5 * width < 4 * rows && worth(kWideBand))
+        width = kWideBand;
     const bool banded = !last && worth(width);
     if (banded) {
         const unsigned at = atomicAdd(next_count, 1u);
@@ -868,14 +887,18 @@ void sweep_long(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &ta
     gpu->launches += 1;
 }
 
-// Scores of long global pairs (the block-a-pair class) by a widening band: a first round sweeps each pair
-// over 2,048 diagonals; a pair its band does not prove goes round once more at the width its band score
+// Scores of long global pairs (kWideClass) by a widening band: a first round sweeps each pair over 256
+// diagonals, or over a wider band foreseen for it (over 2,048 where the 16-bit strips do not hold the table's
+// cells); a pair its band does not prove goes round once more at the width its band score
 // says would prove it, or is swept whole when that band would cover most of its matrix (or its second
 // band proves nothing either). Every score is the whole matrix's. With `proven`, each pair whose band
-// proved its score leaves that band's width there (by pair - proven_first; the rest are left as they were),
+// proved its score leaves there the width to record (by pair - proven_first; the rest are left as they were),
+// a third round serves pairs whose second was at 2,048,
 // and the pairs left to the whole matrix are not swept here: their recording gives their scores; a band
 // is then worth its rounds when the recording's strips (kRecordStrip columns) would sweep few of a pair's
-// rows, where the scores' own strips are a block's 4,096 columns.
+// rows, where the scores' own strips are of 1,024 columns (a block's 4,096 in 32 bits).
+// (64 pairs of 20,000 letters with 300 put in at a third and taken out at two thirds: recorded over the bands that
+// proved them 182 ms a call, over what their scores need 68.)
 void widening_band(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, const uint32_t *order,
                    int64_t count, KernelArgs args, int32_t *proven = nullptr, int64_t proven_first = 0,
                    const int32_t *foreseen = nullptr) {
@@ -884,22 +907,22 @@ void widening_band(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
     for (int r = 0; r < table.size; ++r)
         for (int c = 0; c < table.size; ++c) best = std::max(best, table.entries[r * 32 + c]);
     const int32_t strip_columns = proven ? kRecordStrip : long_serves(batch, table) ? kLongStrip : 16 * kBlock;
-    const int32_t first_width = long_serves(batch, table) ? 256 : 2048;
+    const int32_t first_width = long_serves(batch, table) ? 256 : kWideBand;
     uint32_t *lists = gpu->wide_pending.ensure<uint32_t>(5 * size_t(count));
     uint32_t *whole = lists + 2 * count;
     int32_t *widths = reinterpret_cast<int32_t *>(lists + 3 * count);
     unsigned int *counts = gpu->class_counts.ensure<unsigned int>(kClassCounters) + 9;  // [0] next, [1] whole
     DINARA_CUDA(cudaMemsetAsync(counts + 1, 0, sizeof(unsigned int), gpu->stream));
-    constexpr int kBandRounds = 2;
+    const int rounds = proven ? 3 : 2;
     const uint32_t *pending = order;
     const int32_t *swept = nullptr;
     int64_t left = count;
-    for (int round = 0; round <= kBandRounds && left > 0; ++round) {
+    for (int round = 0; round <= rounds && left > 0; ++round) {
         uint32_t *next = lists + (round & 1) * count;
         int32_t *next_widths = widths + (round & 1) * count;
         DINARA_CUDA(cudaMemsetAsync(counts, 0, sizeof(unsigned int), gpu->stream));
         wide_route_kernel<<<unsigned((left + 255) / 256), 256, 0, gpu->stream>>>(
-            batch.shapes, pending, swept, left, first_width, round == kBandRounds, args.scores, best, table.open,
+            batch.shapes, pending, swept, left, first_width, round == rounds, args.scores, best, table.open,
             table.extend, next, next_widths, counts, whole, counts + 1, proven, proven_first,
             strip_columns, foreseen);
         DINARA_CUDA(cudaGetLastError());

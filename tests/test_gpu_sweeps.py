@@ -87,6 +87,58 @@ def test_many_long_pairs_in_strips(da, oracle, pairs):
     np.testing.assert_array_equal(da.scores_tape(tape, scoring), expected)
 
 
+def _shifted(rng, length, size, first, second, rate=0.01):
+    """A sequence, and its copy with `size` letters put in at the share `first` of it and as many taken out at
+    `second`: between the two the alignment lies `size` diagonals off."""
+    source = _text(rng, length)
+    copy = _mutated(rng, source, rate, "ACGT")
+    a, b = int(first * len(copy)), int(second * len(copy))
+    return source, copy[:a] + _text(rng, size) + copy[a:b] + copy[b + size:]
+
+
+# The last table's steps (180) are past the 16-bit strips: a first band of 2,048.
+@pytest.mark.parametrize("entries", [(2, -4, -4, -2), (0, -4, -6, -2), (60, -60, -100, -10)])
+def test_long_alignments_off_the_diagonals(da, oracle, entries):
+    """Alignments whose paths leave the main diagonals: bands proven at once, at the width a low score asked for, at
+    2,048 where that is too wide for its worth, and not at all; recorded over what their own scores need."""
+    rng = np.random.default_rng(abs(sum(entries)) + 97)
+    scoring = da.Scoring.uniform(*entries)
+    shapes = [(4200, 40, 0.3, 0.6), (4300, 300, 0.1, 0.9), (5000, 300, 0.2, 0.8), (5200, 700, 0.3, 0.7),
+              (7000, 120, 0.1, 0.95), (9000, 300, 0.3, 0.6), (9000, 900, 0.05, 0.9), (6000, 1500, 0.4, 0.5)]
+    pairs = [_shifted(rng, *shape) for shape in shapes]
+    pairs += [(b, a) for a, b in pairs[:4]]
+    pairs += [(_text(rng, 4500), _text(rng, 4400)), (_shifted(rng, 6000, 300, 0.2, 0.8)[0],
+                                                     _shifted(rng, 6000, 300, 0.2, 0.8)[1][:5200])]
+    refs, queries = [a for a, _b in pairs], [b for _a, b in pairs]
+    tape = da.Tape.of(refs, queries)
+    coded = np.concatenate([oracle.codes(text) for pair in pairs for text in pair])
+    op, ex = oracle.kernel_gaps(scoring.opening, scoring.extension)
+    expected, cigars = oracle.batch_alignments(coded, tape.offsets, _table(scoring), 4, op, ex, oracle.GLOBAL, threads=8)
+    found = da.alignments(refs, queries, scoring)
+    assert [a.score for a in found] == list(expected)
+    assert [a.cigar for a in found] == cigars
+
+
+def test_long_alignments_record_what_their_scores_need(da):
+    """20,000 letters with 300 put in and taken out: the score lies 3,600 below the best, so 600 gap letters or so
+    outside a band cost more, and with a strip of 512 columns no more than 2,048 places a row are recorded. (The
+    band that finds the score, from the low one that 256 diagonals give, takes some 6,000.)"""
+    import bench
+
+    rng = np.random.default_rng(20)
+    source, copy = _shifted(rng, 20_000, 300, 1 / 3, 2 / 3)
+    tape = da.Tape.of([source], [copy])
+    native, lib = da._native, da._native.lib()
+    handle = lib.dinara_gpu_new(0)
+    scoring, _table_kept, _alphabet_kept = da.Scoring.uniform(2, -4, -4, -2)._struct()
+    mode, timing = da.Mode.GLOBAL._struct(), bench.Timing()
+    native.check(lib.dinara_gpu_resident_load(handle, 1, tape.letters.ctypes.data,
+                                              native.pointer(tape.offsets, ctypes.c_int64), ctypes.byref(scoring)), handle)
+    native.check(lib.dinara_gpu_resident_align(handle, ctypes.byref(mode), 1, 1, ctypes.byref(timing)), handle)
+    lib.dinara_gpu_free(handle)
+    assert 0 < timing.whole_cells < 20_000 * 2_048
+
+
 # ---- local alignments recorded over their hits' rows ----------------------------------------------------
 
 @pytest.mark.parametrize("alphabet", ["ACGT", "ACGTN", PROTEIN])
