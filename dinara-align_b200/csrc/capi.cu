@@ -17,7 +17,6 @@
 #include <utility>
 #include <vector>
 
-#include <emmintrin.h>
 #include <sys/mman.h>
 
 #include "affine.cuh"
@@ -26,6 +25,7 @@
 #include "internal.cuh"
 #include "learned.cuh"
 #include "pack.cuh"
+#include "staging.cuh"
 #include "ties.cuh"
 
 using namespace dinara;
@@ -160,34 +160,6 @@ bool is_pinned(const void *pointer) {
         return false;
     }
     return attributes.type == cudaMemoryTypeHost;
-}
-
-// A copy into page-locked memory that a device copy reads next, past the caches: with the lines left dirty in eight
-// cores' caches the bus read them at 5 to 14 GB/s, from memory at 48. `to` starts on a 16-byte boundary. A small
-// copy stays in this core's cache, where it costs less.
-void copy_past_caches(uint8_t *to, const uint8_t *from, size_t bytes) {
-    if (bytes < (size_t(1) << 16)) {
-        std::memcpy(to, from, bytes);
-        return;
-    }
-    const size_t whole = bytes / 16;
-    for (size_t k = 0; k < whole; ++k)
-        _mm_stream_si128(reinterpret_cast<__m128i *>(to) + k, _mm_loadu_si128(reinterpret_cast<const __m128i *>(from) + k));
-    _mm_sfence();
-    std::memcpy(to + 16 * whole, from + 16 * whole, bytes - 16 * whole);
-}
-
-// copy_past_caches shared by eight threads, or fewer for a small copy (about half a megabyte each).
-void stage_copy(uint8_t *to, const uint8_t *from, size_t bytes) {
-    const int threads = int(std::min<size_t>(8, bytes / (size_t(1) << 19) + 1));
-    const size_t part = ((bytes + threads - 1) / threads + 63) & ~size_t(63);
-    std::thread helpers[7];
-    for (int t = 1; t < threads; ++t) {
-        const size_t begin = std::min(bytes, t * part), end = std::min(bytes, begin + part);
-        helpers[t - 1] = std::thread([=] { copy_past_caches(to + begin, from + begin, end - begin); });
-    }
-    copy_past_caches(to, from, std::min(bytes, part));
-    for (int t = 1; t < threads; ++t) helpers[t - 1].join();
 }
 
 // Copies `bytes` of host memory to the device on the context's stream, through page-locked staging

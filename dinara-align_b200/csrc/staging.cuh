@@ -1,0 +1,45 @@
+// Host copies into page-locked memory that the device's copies read next.
+#pragma once
+
+#include <algorithm>
+#include <cstddef>
+#include <cstdint>
+#include <cstring>
+#include <thread>
+
+#if defined(__SSE2__)
+#include <emmintrin.h>
+#endif
+
+namespace dinara {
+
+// A copy into page-locked memory that a device copy reads next, past the caches: with the lines left dirty in eight
+// cores' caches the bus read them at 5 to 14 GB/s, from memory at 48. `to` starts on a 16-byte boundary. A small
+// copy stays in this core's cache, where it costs less; so does any on a host without these stores.
+inline void copy_past_caches(uint8_t *to, const uint8_t *from, size_t bytes) {
+    size_t done = 0;
+#if defined(__SSE2__)
+    if (bytes >= (size_t(1) << 16)) {
+        for (; done + 16 <= bytes; done += 16)
+            _mm_stream_si128(reinterpret_cast<__m128i *>(to + done),
+                             _mm_loadu_si128(reinterpret_cast<const __m128i *>(from + done)));
+        _mm_sfence();
+    }
+#endif
+    std::memcpy(to + done, from + done, bytes - done);
+}
+
+// copy_past_caches shared by eight threads, or fewer for a small copy (about half a megabyte each).
+inline void stage_copy(uint8_t *to, const uint8_t *from, size_t bytes) {
+    const int threads = int(std::min<size_t>(8, bytes / (size_t(1) << 19) + 1));
+    const size_t part = ((bytes + threads - 1) / threads + 63) & ~size_t(63);
+    std::thread helpers[7];
+    for (int t = 1; t < threads; ++t) {
+        const size_t begin = std::min(bytes, t * part), end = std::min(bytes, begin + part);
+        helpers[t - 1] = std::thread([=] { copy_past_caches(to + begin, from + begin, end - begin); });
+    }
+    copy_past_caches(to, from, std::min(bytes, part));
+    for (int t = 1; t < threads; ++t) helpers[t - 1].join();
+}
+
+}  // namespace dinara
