@@ -5,6 +5,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <cstring>
+#include <system_error>
 #include <thread>
 
 #if defined(__SSE2__)
@@ -29,17 +30,24 @@ inline void copy_past_caches(uint8_t *to, const uint8_t *from, size_t bytes) {
     std::memcpy(to + done, from + done, bytes - done);
 }
 
-// copy_past_caches shared by eight threads, or fewer for a small copy (about half a megabyte each).
+// copy_past_caches shared by eight threads, or fewer for a small copy (about half a megabyte each). The shares of
+// threads that cannot be started are copied here: an exception would leave this call with others still running.
 inline void stage_copy(uint8_t *to, const uint8_t *from, size_t bytes) {
     const int threads = int(std::min<size_t>(8, bytes / (size_t(1) << 19) + 1));
     const size_t part = ((bytes + threads - 1) / threads + 63) & ~size_t(63);
-    std::thread helpers[7];
-    for (int t = 1; t < threads; ++t) {
+    const auto share = [=](int t) {
         const size_t begin = std::min(bytes, t * part), end = std::min(bytes, begin + part);
-        helpers[t - 1] = std::thread([=] { copy_past_caches(to + begin, from + begin, end - begin); });
+        copy_past_caches(to + begin, from + begin, end - begin);
+    };
+    std::thread helpers[7];
+    int started = 1;
+    try {
+        for (; started < threads; ++started) helpers[started - 1] = std::thread(share, started);
+    } catch (const std::system_error &) {
     }
-    copy_past_caches(to, from, std::min(bytes, part));
-    for (int t = 1; t < threads; ++t) helpers[t - 1].join();
+    share(0);
+    for (int t = started; t < threads; ++t) share(t);
+    for (int t = 1; t < started; ++t) helpers[t - 1].join();
 }
 
 }  // namespace dinara

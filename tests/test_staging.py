@@ -50,3 +50,24 @@ def test_copies(tmp_path, host):
         (tmp_path / "emmintrin.h").write_text("#error a header of other hosts\n")
         flags = ["-U__SSE2__", "-I", str(tmp_path)]
     _run(tmp_path, COPIES, *flags)
+
+
+# A thread cannot be started from the `ALLOWED`th on.
+FAILING = r"""
+#include <cerrno>
+#include <dlfcn.h>
+#include <pthread.h>
+extern "C" int pthread_create(pthread_t *thread, const pthread_attr_t *attributes, void *(*body)(void *), void *argument) {
+    static int calls = 0;
+    if (calls++ % 8 >= ALLOWED) return EAGAIN;
+    using Create = int (*)(pthread_t *, const pthread_attr_t *, void *(*)(void *), void *);
+    static Create create = reinterpret_cast<Create>(dlsym(RTLD_NEXT, "pthread_create"));
+    return create(thread, attributes, body, argument);
+}
+"""
+
+
+@pytest.mark.parametrize("allowed", [0, 1, 3])
+def test_copies_where_threads_cannot_start(tmp_path, allowed):
+    """They end with every byte copied, not with the process."""
+    _run(tmp_path, FAILING + COPIES, f"-DALLOWED={allowed}", "-rdynamic", "-ldl")
