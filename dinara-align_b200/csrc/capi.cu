@@ -1355,6 +1355,7 @@ int64_t dinara_gpu_alignments_tape(dinara_gpu *gpu, int64_t pairs, const char *l
                 for (int64_t k = begin; k < end; ++k) {
                     const int64_t p = unit.first + k;
                     if (cigar_offsets) cigar_offsets[p + 1] = at + ends[k + 1];
+                    if (!spans) continue;
                     const int64_t rows = offsets[2 * p + 1] - offsets[2 * p];
                     const int64_t columns = offsets[2 * p + 2] - offsets[2 * p + 1];
                     int64_t *span = spans + 4 * p;

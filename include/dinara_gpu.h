@@ -130,8 +130,8 @@ int64_t dinara_gpu_alignments(dinara_gpu *gpu, int64_t pairs, const char *const 
 /*
  * Alignments over one tape with every CIGAR in one buffer: pair i's CIGAR is
  * cigar_bytes[cigar_offsets[i] .. cigar_offsets[i+1]) (no NULs), its score scores[i], its spans
- * spans[4i .. 4i+4) = reference_start, reference_end, query_start, query_end. `*cigar_bytes` is
- * allocated here (dinara_free). Same walk and placement as dinara_gpu_alignments.
+ * spans[4i .. 4i+4) = reference_start, reference_end, query_start, query_end (`spans` may be null).
+ * `*cigar_bytes` is allocated here (dinara_free). Same walk and placement as dinara_gpu_alignments.
  */
 int64_t dinara_gpu_alignments_tape(dinara_gpu *gpu, int64_t pairs, const char *letters, const int64_t *offsets,
                                    const dinara_scoring *scoring, const dinara_mode *mode, int64_t eqx,

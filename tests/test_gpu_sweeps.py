@@ -332,6 +332,31 @@ def test_placed_alignments_in_several_units(da, oracle):
         _assert_tiled(da, tape, scoring, mode, expected, 100)
 
 
+@pytest.mark.parametrize("mode_name", ["INFIX", "GLOBAL"])
+def test_alignments_without_spans(da, mode_name):
+    """A caller that wants no spans gives none: the scores and CIGARs are those with them."""
+    rng = np.random.default_rng(8)
+    refs = [_text(rng, 60) for _ in range(20)]
+    queries = [_mutated(rng, ref[10:50], 0.1, "ACGT") for ref in refs]
+    mode = getattr(da.Mode, mode_name)
+    tape = da.Tape.of(refs, queries)
+    native, lib = da._native, da._native.lib()
+    scoring, _table_kept, _alphabet_kept = da.Scoring.dna()._struct()
+    mode_struct = mode._struct()
+    scores, offsets, statuses = np.empty(20, np.int32), np.empty(21, np.int64), np.empty(20, np.int64)
+    buffer = ctypes.c_void_p()
+    handle = native.context(0)
+    native.check(lib.dinara_gpu_alignments_tape(
+        handle, 20, tape.letters.ctypes.data, native.pointer(tape.offsets, ctypes.c_int64), ctypes.byref(scoring),
+        ctypes.byref(mode_struct), 1, native.pointer(scores, ctypes.c_int32), None,
+        native.pointer(offsets, ctypes.c_int64), ctypes.byref(buffer), native.pointer(statuses, ctypes.c_int64)), handle)
+    data = ctypes.string_at(buffer.value, int(offsets[20]))
+    lib.dinara_free(buffer.value)
+    expected = da.alignments(refs, queries, da.Scoring.dna(), mode)
+    assert list(scores) == [a.score for a in expected]
+    assert [data[offsets[p]:offsets[p + 1]].decode() for p in range(20)] == [a.cigar for a in expected]
+
+
 def _check_spans_past_their_pairs_band(da, oracle):
     """2,400 overlaps of 4,000 x 4,000 letters, which as global pairs would keep a band of 64 diagonals, and whose spans
     of 3,800 x 3,900 do not: their recorded decisions take 18.7 GB, in parts of 8 GiB. Prints the device memory that
