@@ -137,7 +137,11 @@ __global__ void __launch_bounds__(kBlock) band_kernel(BandArgs a) {
         int next_col = 1;
         int next_time = 1 + member + (next_slide == 1 ? 1 : 0);
         // A column's words of its letter's plane are read a column early, and its letter two, so that no step waits
-        // for either (windows of more words a lane keep their registers and read them in the step).
+        // for either. It takes registers: 8 resident blocks become 7 at K = 2, 8 and 7 become 7 to 6 at 3 and 4, 7
+        // and 6 become 5 at 5 and 6. All the same the rounds' time with it up to K = 6, at K = 1 alone and without
+        // it: 200,000 uneven pairs 114.4, 122.3 and 123.0 ms, 30,000 of 2 to 4 kb at 10% errors 5.3, 7.7 and 7.8,
+        // 8,000 of 10 to 20 kb at 10% from near starts, where warps count most, 12.8, 12.3 and 12.6. Windows of 8
+        // words a lane and more keep their registers and read them in the step.
         constexpr bool AHEAD = K <= 6;
         uint32_t letter = live && m > 0 ? __ldg(text) : 0u, letter_after = live && m > 1 ? __ldg(text + 1) : 0u;
         uint64_t equals[AHEAD ? K : 1];
@@ -380,8 +384,7 @@ struct BandCounters {
 constexpr size_t kCountsBytes = offsetof(BandCounters, queues);
 static_assert(kCountsBytes <= kReadbackBytes, "a round's counts fit the readback words");
 
-// band_shape_for by a warp: a lane a shape (two for the first lanes), its order of choice in a 64-bit rank whose least
-// is the choice. `cost` holds the tuning's word costs.
+// band_shape_for by a warp, a lane a shape (two for the first lanes). `cost` holds the tuning's word costs.
 __device__ int band_shape_by_warp(const EditPair &e, int64_t t, bool latency, const BandTuning &tuning,
                                   const float *cost) {
     static_assert(kBandShapes <= 64, "two shapes a lane");
@@ -393,41 +396,24 @@ __device__ int band_shape_by_warp(const EditPair &e, int64_t t, bool latency, co
     for (int i = 0; i < 2; ++i) {
         const int s = min(lane + 32 * i, kBandShapes - 1);
         capacity[i] = lane + 32 * i < kBandShapes ? int(band_capacity(s)) : -1;
-        words[i] = int(band_words_per_lane(s));
+        words[i] = band_words_per_lane(s);
         if (capacity[i] >= needed) smallest = min(smallest, int64_t(capacity[i]));
     }
 #pragma unroll
-    for (int span = 16; span > 0; span >>= 1) smallest = min(smallest, __shfl_xor_sync(0xffffffffu, smallest, span));
+    for (int span = 16; span > 0; span >>= 1) smallest = min(smallest, __shfl_xor_sync(kFull, smallest, span));
     if (smallest == INT32_MAX) return kWidestShape;
-    // The least rank of the shapes within `reach` quarters of the smallest window (`bounded`: whose chain fits).
-    auto least = [&](int64_t reach, bool bounded) {
+    return band_shape_choice(latency, tuning.reach, [&](int64_t reach, bool bounded) {
         unsigned long long best = ~0ull;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const unsigned s = unsigned(lane + 32 * i);
-            if (capacity[i] < needed || capacity[i] < 0 || 4 * int64_t(capacity[i]) > reach * smallest) continue;
-            if (bounded && int64_t(e.m) * words[i] > tuning.chain_words) continue;
-            // Costs are positive, so their bits order as they do.
-            const unsigned long long price = __float_as_uint(float(capacity[i]) * cost[s]);
-            const unsigned long long chain = e.m > 0 ? unsigned(words[i]) : 0u;
-            const unsigned long long rank = latency   ? (unsigned long long)(words[i]) << 32 | unsigned(capacity[i])
-                                            : bounded ? price
-                                                      : chain << 32 | price;
-            best = min(best, rank << 8 | s);
-        }
+        for (int i = 0; i < 2; ++i)
+            if (capacity[i] >= 0)
+                best = min(best, (unsigned long long)band_shape_rank(lane + 32 * i, capacity[i], words[i],
+                                                                     cost[lane + 32 * i], e.m, needed, smallest, reach,
+                                                                     bounded, latency, tuning.chain_words));
 #pragma unroll
-        for (int span = 16; span > 0; span >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, span));
-        return best;
-    };
-    unsigned long long best = ~0ull;
-    if (latency) {
-        best = least(8, false);
-    } else {
-        for (int reach = 5; reach <= tuning.reach && best == ~0ull; reach = reach < tuning.reach ? tuning.reach : reach + 1)
-            best = least(reach, true);
-        if (best == ~0ull) best = least(max(tuning.reach, 5), false);
-    }
-    return int(best & 0xff);
+        for (int span = 16; span > 0; span >>= 1) best = min(best, __shfl_xor_sync(kFull, best, span));
+        return uint64_t(best);
+    });
 }
 
 // Keys for the pending pairs, a warp a pair: band shape in the top six bits, then the text length, longest first, as

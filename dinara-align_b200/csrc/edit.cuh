@@ -61,6 +61,44 @@ __host__ __device__ inline int64_t band_reach(int64_t n, int64_t m, int64_t wind
 // for a long chain); failing that, the shortest chain. For a round of few pairs (`latency`: the GPU has lanes to spare and the round
 // lasts as long as its longest chain), the fewest words a lane within twice the smallest window. A band
 // past the widest shape takes the widest. The tuning's figures are BandTuning's (internal.cuh).
+//
+// A shape's place in that order, the least first (its number in the low byte, which breaks ties), or ~0 where its
+// `capacity` does not hold the band's `needed` words, lies past `reach` quarters of the smallest window that does or
+// (`bounded`) its chain past the tuning's; `words` a lane, and `word_cost` the tuning's. One thread (band_shape_for)
+// and a warp (a round's keys, edit.cu) look for the least by it.
+__host__ __device__ inline uint64_t band_shape_rank(int shape, int capacity, int words, float word_cost, int64_t m,
+                                                    int64_t needed, int64_t smallest, int64_t reach, bool bounded,
+                                                    bool latency, int64_t chain_words) {
+    if (capacity < needed || 4 * int64_t(capacity) > reach * smallest) return ~uint64_t(0);
+    if (bounded && m * words > chain_words) return ~uint64_t(0);
+    uint64_t rank;
+    if (latency) {
+        rank = uint64_t(words) << 32 | uint32_t(capacity);
+    } else {
+        // Costs are positive, so their bits order as they do.
+        const float price = float(capacity) * word_cost;
+        uint32_t bits;
+        memcpy(&bits, &price, sizeof bits);
+        rank = bounded || m <= 0 ? bits : uint64_t(words) << 32 | bits;
+    }
+    return rank << 8 | uint64_t(shape);
+}
+
+// The least rank, by least(reach, bounded): band_shape_rank's over every shape.
+template <class L>
+__host__ __device__ inline int band_shape_choice(bool latency, int tuning_reach, L &&least) {
+    uint64_t best = ~uint64_t(0);
+    if (latency) {
+        best = least(8, false);
+    } else {
+        for (int reach = 5; reach <= tuning_reach && best == ~uint64_t(0);
+             reach = reach < tuning_reach ? tuning_reach : reach + 1)
+            best = least(reach, true);
+        if (best == ~uint64_t(0)) best = least(tuning_reach > 5 ? tuning_reach : 5, false);
+    }
+    return int(best & 0xff);
+}
+
 __host__ __device__ inline int band_shape_for(int64_t n, int64_t m, int64_t t, bool latency,
                                               const BandTuning &tuning) {
     const int64_t needed = band_words_needed(n, m, t);
@@ -70,53 +108,15 @@ __host__ __device__ inline int band_shape_for(int64_t n, int64_t m, int64_t t, b
         if (c >= needed && c < smallest) smallest = c;
     }
     if (smallest == INT64_MAX) return kWidestShape;
-    if (latency) {
-        int best = -1;
-        int64_t best_k = INT64_MAX, best_capacity = INT64_MAX;
+    return band_shape_choice(latency, tuning.reach, [&](int64_t reach, bool bounded) {
+        uint64_t best = ~uint64_t(0);
         for (int s = 0; s < kBandShapes; ++s) {
-            const int64_t c = band_capacity(s), k = band_words_per_lane(s);
-            if (c < needed || c > 2 * smallest) continue;
-            if (best < 0 || k < best_k || (k == best_k && c < best_capacity)) {
-                best = s;
-                best_k = k;
-                best_capacity = c;
-            }
+            const uint64_t rank = band_shape_rank(s, int(band_capacity(s)), band_words_per_lane(s), tuning.word_cost[s], m,
+                                                  needed, smallest, reach, bounded, latency, tuning.chain_words);
+            if (rank < best) best = rank;
         }
         return best;
-    }
-    // The cheapest shape whose chain fits, among those within a quarter of the smallest, then within the
-    // tuning's reach.
-    for (int reach = 5; reach <= tuning.reach; reach = reach < tuning.reach ? tuning.reach : reach + 1) {
-        int best = -1;
-        float best_cost = 0.f;
-        for (int s = 0; s < kBandShapes; ++s) {
-            const int64_t c = band_capacity(s);
-            if (c < needed || 4 * c > reach * smallest) continue;
-            if (m * band_words_per_lane(s) > tuning.chain_words) continue;
-            const float cost = float(c) * tuning.word_cost[s];
-            if (best < 0 || cost < best_cost) {
-                best = s;
-                best_cost = cost;
-            }
-        }
-        if (best >= 0) return best;
-    }
-    // No chain fits: the shortest, then the cheapest, within the reach.
-    int best = -1;
-    int64_t best_chain = INT64_MAX;
-    float best_cost = 0.f;
-    for (int s = 0; s < kBandShapes; ++s) {
-        const int64_t c = band_capacity(s);
-        if (c < needed || 4 * c > (tuning.reach > 5 ? tuning.reach : 5) * smallest) continue;
-        const int64_t chain = m * band_words_per_lane(s);
-        const float cost = float(c) * tuning.word_cost[s];
-        if (best < 0 || chain < best_chain || (chain == best_chain && cost < best_cost)) {
-            best = s;
-            best_chain = chain;
-            best_cost = cost;
-        }
-    }
-    return best;
+    });
 }
 
 // The tuning a context starts with: a word step costs its 40 operations plus a lane's work a column besides
