@@ -545,8 +545,9 @@ def test_distances_beside_pairs_that_take_no_round(da, oracle, pairs):
 
 @pytest.mark.parametrize("batch", [1, 31, 128, 129, 4096, 4097])
 def test_gradients_at_slice_edges(da, batch):
-    """Against 64 bits: an fp32 sum of `batch` products in slices is off by at most about (128 + 32) * 2^-24 of the sum
-    of their sizes, 1e-5; the sums here lie within ten times of their terms' sizes, so 1e-4 of the largest."""
+    """Against 64 bits: an fp32 sum of `batch` products in slices of 128 and then 32 is off by some sqrt(160) * 2^-24 of
+    its terms' root of squares, 8e-7, where roundings are as likely up as down. Six seeds a batch: at most 3e-7 of the
+    largest gradient from 31 samples on, 8e-7 at one, whose residual cancels."""
     import mlp_oracle
     from dinara_align import learned
 
@@ -554,11 +555,18 @@ def test_gradients_at_slice_edges(da, batch):
     flat = rng.normal(0, 0.1, size=learned.PARAMETERS).astype(np.float32)
     x = rng.normal(0, 0.5, size=(batch, learned.INPUTS)).astype(np.float32)
     t = rng.uniform(0, 0.2, size=batch).astype(np.float32)
+    # A sample with a unit within fp32's rounding of its bend may pass on either side of it: drawn anew.
+    while True:
+        _y, (_x, first, _h1, second, _h2) = mlp_oracle.forward(mlp_oracle.unpack(flat), x.astype(np.float64))
+        bent = np.minimum(np.abs(first).min(axis=1), np.abs(second).min(axis=1)) < 5e-6
+        if not bent.any():
+            break
+        x[bent] = rng.normal(0, 0.5, size=(int(bent.sum()), learned.INPUTS))
     predictor = learned.Predictor()
     predictor.install(flat, 1.0, 0.0)
     got, loss = predictor.gradients(x, t)
     expected, expected_loss = mlp_oracle.gradients(*(v.astype(np.float64) for v in (flat, x, t)))
-    np.testing.assert_allclose(got, expected, rtol=0, atol=1e-4 * np.abs(expected).max())
+    np.testing.assert_allclose(got, expected, rtol=0, atol=(1e-6 if batch >= 31 else 4e-6) * np.abs(expected).max())
     assert abs(loss - expected_loss) <= 1e-5 * expected_loss
 
 
