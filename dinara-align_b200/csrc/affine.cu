@@ -1571,10 +1571,11 @@ void free_end_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTabl
 }
 
 // Each local pair's shape cut to the rows its best alignment can span (by pair), from a score sweep of the pairs
-// the 16-bit pair sweeps take; the rest keep their whole shape. Recording a cell costs about seven times
-// scoring it in 16-bit pairs (its flags, their packing and the decisions' store, in 32 bits), so the cut
-// pays for its sweep once it leaves out a seventh of a pair's rows: a read of 575 letters in a target of
-// 3,000 leaves out three quarters. Null when no pair takes a 16-bit sweep.
+// the 16-bit pair sweeps take; the rest keep their whole shape. A read of 575 letters in a target of 3,000 leaves
+// out three quarters of its rows, and a hit found lets record_pairs_kernel take its rows in 16 bits, so the sweep
+// pays even where a hit spans its target: 5,000 reads of 600 letters in targets as long 8.8 ms a call recorded
+// whole in 32 bits, 5.5 so. (Recording a cell in 32 bits costs about seven times scoring it here.) Null when no
+// pair takes a 16-bit sweep.
 const PairShape *hit_shapes(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, int32_t *scores,
                             int64_t first, int64_t count) {
     const PairLimits limits = whole_limits_of(batch, table);
@@ -1744,8 +1745,11 @@ int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &whole_batch, const
     PairLimits limits = record_limits_of(batch, table);
     // A local pair without its hit found has no known end: only hits' rows take the 16-bit sweep.
     if (batch.local && batch.shapes == whole_batch.shapes) limits.whole = 0;
-    // Two pairs a group pay where pairs fill the GPU: a global row takes the 16-bit sweep about twice as long, and
-    // a few hundred leftovers of a band 370 us against 195. Locally it is the shorter either way.
+    // Two pairs a group pay where pairs fill the GPU: a global row takes the 16-bit sweep about twice as long. A call's
+    // global alignments, in 32 bits and in 16: proteins of 300 to 600 letters 1.59 and 1.70 ms for 150 pairs, 2.07 and
+    // 2.13 for 2,000, 4.5 and 4.4 for 7,000; DNA pairs of 600 to 1,200 that no band proves 6.4 and 6.8 for 1,000,
+    // 10.2 and 10.2 for 4,800, 29.0 and 29.3 for 20,000. Shorter pairs gain below the line too (proteins of 100 to
+    // 300, 1,000 pairs 1.06 and 0.81), so it is the longest's. Locally it is the shorter either way.
     const int64_t full = 32 * int64_t(gpu->multiprocessors);
     PairLimits left_limits = limits;
     if (!batch.local && (band || count < full)) limits.whole = 0;

@@ -68,11 +68,12 @@ struct KernelArgs {
     int32_t free_highest;
     // An extension's Z-drop (affine_kernel<..., ORIGIN>): each anti-diagonal's best cell, its true score
     // (offset by 2^31) in the high 32 bits and its row in the low, kept by atomic maximum at
-    // diagonals[diagonal_offsets[pair - first_pair] + row + column].
+    // diagonals[diagonal_offsets[pair - first_pair] + row + column]. (extension_pairs_kernel's keys are a cell as
+    // held over its row, offset by 2^31, in the low 32 bits alone.)
     unsigned long long *diagonals;
     const int64_t *diagonal_offsets;
     // Local hits' rows (affine_pairs_kernel<..., TRACK>): each pair's shape cut to the rows its best alignment
-    // can span (hit_rows), by pair, for a recording sweep of those rows alone; `best_entry` the table's.
+    // can span (from hit_first_row on), by pair, for a recording sweep of those rows alone; `best_entry` the table's.
     PairShape *hits;
     int32_t best_entry;
     const int32_t *known;  // free_pairs_kernel, sweeping back: each pair's score, by pair

@@ -105,8 +105,6 @@ __global__ void __launch_bounds__(kBlock) banded_kernel(BandedBatch b) {
         uint64_t buffered[4] = {0, 0, 0, 0};
 
         for (int r0 = 1; r0 <= warp_rows; r0 += 16) {
-            // Selectors of the 32 letters from column r0 + low + first_place on (letter index one less);
-            // columns outside the pair read letter 0, which no real cell's value depends on.
             // Every 64 rows a pair whose band can no longer prove its score is left to the whole-matrix sweep: from
             // here its score gains at most the best shifted entry a row. At 5% errors a pair of 50,000 letters
             // leaves after some 2,000 rows, where its band took 9 ms to its end; a pair that the band proves goes on
@@ -140,6 +138,8 @@ __global__ void __launch_bounds__(kBlock) banded_kernel(BandedBatch b) {
                 warp_rows = warp_max(live ? rows : 0);
                 if (warp_rows < r0) break;
             }
+            // Selectors of the 32 letters from column r0 + low + first_place on (letter index one less);
+            // columns outside the pair read letter 0, which no real cell's value depends on.
             uint32_t codes[2];
             run_of_letters(b.tape, sh.second_word, live ? cols : 0, r0 + low + first_place - 1, codes);
             uint32_t window[32];

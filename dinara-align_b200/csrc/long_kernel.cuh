@@ -1,4 +1,5 @@
-// Scores of one long pair a block, by warps that each sweep a strip of columns in 16-bit halves.
+// Scores of one long pair a block, or a cluster of blocks, by warps that each sweep a strip of columns in 16-bit
+// halves.
 #pragma once
 
 #include "affine_kernel.cuh"

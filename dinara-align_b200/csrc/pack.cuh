@@ -33,8 +33,9 @@ static_assert(kBandRecordClass + 1 == kClasses && kClasses <= 32, "a class is fi
 constexpr int kClassCounters = 64, kScheduleCounts = 32;
 // A pair a whole block sweeps (kWideClass), scoring without a CIGAR: at least this tall and this wide.
 constexpr uint32_t kWideRows = 4096, kWideColumns = 2048;
-// With the 16-bit strips: a pair of two strips or more, each way. (600 pairs of 3,000 letters: 8.6 ms in 32 bits,
-// a warp a pair, 5.2 in strips; 4,000 of them 25.3 and 16.7.)
+// With the 16-bit strips: a pair of two strips or more, each way. (In 32 bits, a warp a pair, and in strips: 50 pairs of
+// 1,100 letters 2.98 and 0.58 ms, 500 3.53 and 2.81, 5,000 7.45 and 4.61; of 2,500 letters 12.0 and 1.6, 12.6 and 9.3,
+// 25.1 and 19.1.)
 constexpr uint32_t kLongSide = 1024 + 1;
 struct Schedule {
     const uint32_t *order;
