@@ -1909,7 +1909,7 @@ void last_places(dinara_gpu *gpu, const uint8_t *letters, const int64_t *offsets
 namespace {
 
 // Spans that do not lie within their pair's letters are emptied and their pair flagged (before its span is packed).
-// The spans' sizes are summed, and their sides' most found, a warp at a time.
+// With `sizes`, the spans' sizes are summed, and their sides' most found, a warp at a time.
 __global__ void check_spans_kernel(const int64_t *__restrict__ offsets, int64_t first_pair, int64_t count,
                                    int64_t *__restrict__ spans, bool uniform, bool band, uint8_t *__restrict__ flags,
                                    SpanSizes *__restrict__ sizes) {
@@ -1931,6 +1931,7 @@ __global__ void check_spans_kernel(const int64_t *__restrict__ offsets, int64_t 
             if (flags[pair] == 0) flags[pair] = kWalkFailed;
         }
     }
+    if (!sizes) return;
 #pragma unroll
     for (int apart = 16; apart > 0; apart >>= 1) words += __shfl_xor_sync(kFull, words, apart);
     span_rows = __reduce_max_sync(kFull, span_rows);
@@ -1951,18 +1952,20 @@ __global__ void check_span_scores_kernel(int64_t first_pair, int64_t count, cons
 
 }  // namespace
 
-SpanSizes check_spans(dinara_gpu *gpu, const int64_t *offsets, int64_t first_pair, int64_t count, int64_t *spans,
-                      bool uniform, bool band, uint8_t *flags) {
-    SpanSizes sizes{0, 0, 0};
-    if (count <= 0) return sizes;
-    SpanSizes *out = reinterpret_cast<SpanSizes *>(gpu->class_counts.ensure<unsigned int>(kClassCounters) + 20);
-    DINARA_CUDA(cudaMemsetAsync(out, 0, sizeof(SpanSizes), gpu->stream));
+void check_spans(dinara_gpu *gpu, const int64_t *offsets, int64_t first_pair, int64_t count, int64_t *spans,
+                 bool uniform, bool band, uint8_t *flags, SpanSizes *sizes) {
+    if (sizes) *sizes = {0, 0, 0};
+    if (count <= 0) return;
+    SpanSizes *out = nullptr;
+    if (sizes) {
+        out = reinterpret_cast<SpanSizes *>(gpu->class_counts.ensure<unsigned int>(kClassCounters) + 20);
+        DINARA_CUDA(cudaMemsetAsync(out, 0, sizeof(SpanSizes), gpu->stream));
+    }
     check_spans_kernel<<<unsigned((count + 255) / 256), 256, 0, gpu->stream>>>(offsets, first_pair, count, spans,
                                                                              uniform, band, flags, out);
     DINARA_CUDA(cudaGetLastError());
     gpu->launches += 1;
-    read_back(gpu, &sizes, out, sizeof sizes);
-    return sizes;
+    if (sizes) read_back(gpu, sizes, out, sizeof *sizes);
 }
 
 void check_span_scores(dinara_gpu *gpu, int64_t first_pair, int64_t count, const int32_t *scores, const int32_t *inner,

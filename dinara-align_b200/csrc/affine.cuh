@@ -119,10 +119,10 @@ struct SpanSizes {
 };
 
 // Flags (kWalkFailed, where a pair has no flag yet) the pairs of [first_pair, first_pair + count) whose span lies
-// outside its letters, emptying the span, and returns the spans' sizes. Spans are 4 a pair of the range, the flags by
-// pair (device).
-SpanSizes check_spans(dinara_gpu *gpu, const int64_t *offsets, int64_t first_pair, int64_t count, int64_t *spans,
-                      bool uniform, bool band, uint8_t *flags);
+// outside its letters, emptying the span; with `sizes`, waits for the spans' sizes. Spans are 4 a pair of the range,
+// the flags by pair (device).
+void check_spans(dinara_gpu *gpu, const int64_t *offsets, int64_t first_pair, int64_t count, int64_t *spans,
+                 bool uniform, bool band, uint8_t *flags, SpanSizes *sizes);
 
 // Flags likewise the pairs whose span's score `scores` differs from `inner`, its global alignment's (by pair, device).
 void check_span_scores(dinara_gpu *gpu, int64_t first_pair, int64_t count, const int32_t *scores, const int32_t *inner,

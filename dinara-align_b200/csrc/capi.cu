@@ -356,6 +356,9 @@ Packed pack_batch(dinara_gpu *gpu, int64_t pairs, const char *letters, const int
 // Device memory a launch's recorded decisions may take before the batch is cut into chunks.
 constexpr int64_t kDecisionBudget = int64_t(8) << 30;
 
+// What a placed unit's carried columns may take before its spans' own longest side is looked for.
+constexpr int64_t kCarryRoom = int64_t(256) << 20;
+
 // A placed unit's CIGARs, recorded in parts, on the host: their bytes, and their offsets (one a pair and one).
 struct RecordedParts {
     std::vector<char> bytes;
@@ -1384,8 +1387,14 @@ int64_t dinara_gpu_alignments_tape(dinara_gpu *gpu, int64_t pairs, const char *l
             if (placed) {
                 int64_t *placed_spans = ctx->placed.ensure<int64_t>(size_t(4 * count));
                 affine_scores(ctx, ends, checked.table, scores_device, first, count, placed_spans);
-                const SpanSizes sizes = check_spans(ctx, streamed.offsets_device, first, count, placed_spans, uniform,
-                                                    band, packed.unknown);
+                // The spans' own sizes are waited for where pairs as large as the batch's largest sides could pass
+                // the decisions' budget, or their carried columns kCarryRoom.
+                SpanSizes sizes{0, packed.max_rows, packed.max_columns};
+                const bool bounded = count * record_words(packed.max_rows, packed.max_columns, uniform, false) <=
+                                         kDecisionBudget / 8 &&
+                                     count * (int64_t(packed.max_rows) + 1) * int64_t(sizeof(int2)) <= kCarryRoom;
+                check_spans(ctx, streamed.offsets_device, first, count, placed_spans, uniform, band, packed.unknown,
+                            bounded ? nullptr : &sizes);
                 pack_pairs(ctx, streamed.letters_device, streamed.offsets_device, first, count, streamed.codes_device,
                            checked.bits, inner_tape, inner_shapes, nullptr, placed_spans);
                 AffineBatch spanned = inner;
