@@ -617,6 +617,18 @@ void launch_together(dinara_gpu *gpu, const AffineBatch &batch, const PairLimits
         all_slots += slots.back();
     }
     const int64_t stride = tallest_of(batch, limits) + 1;
+    // Past the context's limit each class that carries keeps its share of it, on fewer blocks.
+    const int64_t room = std::max<int64_t>(gpu->carry_limit / (stride * int64_t(sizeof(int2))), 1);
+    if (all_slots > room) {
+        const double share = double(room) / double(all_slots);
+        all_slots = 0;
+        for (size_t k = 0; k < sweeps.size(); ++k) {
+            if (slots[k] == 0) continue;
+            blocks[k] = std::max<int64_t>(1, int64_t(double(blocks[k]) * share));
+            slots[k] = blocks[k] * (sweeps[k].launch.threads / sweeps[k].launch.lanes);
+            all_slots += slots[k];
+        }
+    }
     int2 *carry = all_slots > 0 ? gpu->carry.ensure<int2>(size_t(all_slots * stride)) : nullptr;
     const bool fork = sweeps.size() > 1;
     ClockSpan clock(gpu, kClassWhole, gpu->stream);  // one for all: they run at once

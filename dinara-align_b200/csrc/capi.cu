@@ -840,6 +840,7 @@ dinara_gpu *partner_of(dinara_gpu *gpu) {
         gpu->partner = dinara_gpu_new(gpu->device);
         if (!gpu->partner) throw Failure(DINARA_DEVICE_FAILURE, "a second stream for a batch's units: " + new_error);
     }
+    gpu->partner->carry_limit = gpu->carry_limit;
     return gpu->partner;
 }
 

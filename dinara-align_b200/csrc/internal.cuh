@@ -183,6 +183,9 @@ struct dinara_gpu {
     dinara::DeviceBuffer features, weights, gradients, optimizer, predictions, targets, activations, sketches;
     // Alignments under Costs: each warp's arena of kept fronts (ties.cu).
     dinara::DeviceBuffer wavefront;
+    // Bytes that the columns carried by sweeps that run at once may take together (a server's slot: what its request
+    // was admitted with).
+    int64_t carry_limit = INT64_MAX;
     dinara::BandTuning band_tuning{};
     bool predictor_ready = false;
     double predictor_margin = 1.25;    // the largest of the classes' margins (reported)

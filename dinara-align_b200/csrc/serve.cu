@@ -43,6 +43,7 @@ struct Request {
     std::vector<int64_t> statuses;
     int64_t code = 0;
     int64_t estimate = 0;  // device bytes the request's run may hold
+    int64_t max_rows = 0;  // its tallest pair's
     double submitted = 0, admitted = 0, finished = 0;
     bool done = false;
 };
@@ -67,18 +68,23 @@ void release_buffers(dinara_gpu *g) {
     if (g->partner) release_buffers(g->partner);
 }
 
+// The carried columns of pairs wider than one strip: a group's slot as long as the tallest pair, for every group a
+// launch that fills the GPU runs.
+int64_t carried_bytes(int64_t max_rows, int multiprocessors) {
+    return int64_t(multiprocessors) * 2 * 8 * (max_rows + 1) * 8;
+}
+
 // What a request's scores may hold on the device: its letters and their packed copy, per-pair shapes,
-// keys, orders and results, and the carried columns of pairs wider than one strip (a group's slot as long
-// as the tallest pair, for every group the widest launch runs).
-int64_t estimate_bytes(const Request &r, int multiprocessors) {
+// keys, orders and results, and its carried columns.
+int64_t estimate_bytes(Request &r, int multiprocessors) {
     int64_t letters = r.offsets.empty() ? 0 : r.offsets.back() - r.offsets.front();
-    int64_t max_rows = 0, max_columns = 0;
+    int64_t max_columns = 0;
     for (int64_t p = 0; p < r.pairs; ++p) {
-        max_rows = std::max(max_rows, r.offsets[size_t(2 * p + 1)] - r.offsets[size_t(2 * p)]);
+        r.max_rows = std::max(r.max_rows, r.offsets[size_t(2 * p + 1)] - r.offsets[size_t(2 * p)]);
         max_columns = std::max(max_columns, r.offsets[size_t(2 * p + 2)] - r.offsets[size_t(2 * p + 1)]);
     }
     int64_t bytes = 2 * letters + 160 * r.pairs + (int64_t(64) << 20);
-    if (max_columns > 256) bytes += int64_t(multiprocessors) * 2 * 8 * (max_rows + 1) * 8;
+    if (max_columns > 256) bytes += carried_bytes(r.max_rows, multiprocessors);
     return bytes;
 }
 
@@ -128,10 +134,14 @@ struct dinara_server {
         Request &first = *batch.front();
         dinara_scoring scoring{first.alphabet.data(), int64_t(first.alphabet.size()), first.table.data(),
                                first.opening, first.extension};
+        int64_t max_rows = 0;
         for (Request *q : batch) {
+            max_rows = std::max(max_rows, q->max_rows);
             q->scores.assign(size_t(std::max<int64_t>(q->pairs, 1)), 0);
             q->statuses.assign(size_t(std::max<int64_t>(q->pairs, 1)), 0);
         }
+        // Classes of pairs that sweep at once carry their columns at once, each in slots of its own.
+        slot->carry_limit = carried_bytes(max_rows, slot->multiprocessors);
         if (batch.size() == 1)
             return dinara_gpu_scores_tape(slot, first.pairs, first.letters.data(), first.offsets.data(), &scoring,
                                           &first.mode, first.scores.data(), first.statuses.data());

@@ -67,3 +67,27 @@ def test_wait_runs_out_then_completes(da):
         assert code == 0
         np.testing.assert_array_equal(scores, expected)
         assert (statuses == 0).all()
+
+
+def test_sweeps_at_once_keep_the_budget(da):
+    """8,000 local pairs of five strip widths in targets of 12,000 letters: each width's sweep carries columns of its own
+    at the same time as the others', within the 227 MB that the request's estimate (498 MB) holds for them."""
+    from dinara_align import serving
+
+    rng = np.random.default_rng(26)
+    letters = np.frombuffer(b"ACGT", np.uint8)
+    target = letters[rng.integers(0, 4, 12_000)]
+    pieces, lengths = [], []
+    for k in range(8_000):
+        query = letters[rng.integers(0, 4, 400 + (k * 75) % 1_100)]
+        pieces += [target, query]
+        lengths += [len(target), len(query)]
+    offsets = np.concatenate([[0], np.cumsum(lengths)])
+    tape = da.Tape(np.concatenate(pieces), offsets)
+    scoring = da.Scoring.uniform(2, -4, -4, -1)
+    with serving.Server(slots=1, device_bytes=520_000_000) as server:
+        code, scores, statuses, _ = server.wait(server.submit(tape, scoring, da.Mode.local()), timeout=600)
+        assert code == 0 and (statuses == 0).all()
+        stats = server.stats()
+        assert stats["resident_bytes"] <= stats["budget_bytes"], stats
+    np.testing.assert_array_equal(scores, da.scores_tape(tape, scoring, da.Mode.local()))
