@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include <cstring>
+#include <initializer_list>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -281,6 +282,30 @@ inline void read_back(dinara_gpu *gpu, void *host, const void *device, size_t by
     DINARA_CUDA(cudaMemcpyAsync(gpu->readback, device, bytes, cudaMemcpyDeviceToHost, gpu->stream));
     DINARA_CUDA(cudaStreamSynchronize(gpu->stream));
     std::memcpy(host, gpu->readback, bytes);
+}
+
+// Several such copies, each in 64 bytes of the readback words, with one wait.
+struct ReadBack {
+    void *host;
+    const void *device;
+    size_t bytes;
+};
+inline void read_back(dinara_gpu *gpu, std::initializer_list<ReadBack> reads) {
+    constexpr size_t kEach = 64;
+    uint8_t *words = reinterpret_cast<uint8_t *>(gpu->readback);
+    size_t at = 0;
+    for (const ReadBack &r : reads) {
+        if (r.bytes > kEach || at + kEach > kReadbackBytes)
+            throw Failure(DINARA_DEVICE_FAILURE, "a read back past the readback words");
+        DINARA_CUDA(cudaMemcpyAsync(words + at, r.device, r.bytes, cudaMemcpyDeviceToHost, gpu->stream));
+        at += kEach;
+    }
+    DINARA_CUDA(cudaStreamSynchronize(gpu->stream));
+    at = 0;
+    for (const ReadBack &r : reads) {
+        std::memcpy(r.host, words + at, r.bytes);
+        at += kEach;
+    }
 }
 
 }  // namespace dinara

@@ -670,28 +670,28 @@ int64_t cost_alignments(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, 
     DINARA_CUDA(cub::DeviceScan::ExclusiveSum(space, scan_bytes, slot_bytes, slot_offsets, int(pairs + 1), stream));
     DINARA_CUDA(cub::DeviceRadixSort::SortPairsDescending(space, sort_bytes, keys, keys_sorted, identity, order,
                                                           int(pairs), 0, 32, stream));
+    // Pairs with a refused letter sort last (key zero) and are left out of the launches, by their count.
+    unsigned int *counters = gpu->counters.ensure<unsigned int>(64);
+    DINARA_CUDA(cudaMemsetAsync(counters, 0, 64 * sizeof(unsigned int), stream));
+    size_t count_bytes = 0;
+    DINARA_CUDA(cub::DeviceReduce::Sum(nullptr, count_bytes, refused, counters + 8, int(pairs), stream));
+    space = gpu->sort_scratch.ensure<uint8_t>(std::max({scan_bytes, sort_bytes, count_bytes}) + 256);
+    DINARA_CUDA(cub::DeviceReduce::Sum(space, count_bytes, refused, counters + 8, int(pairs), stream));
+    // The slots' bytes, the longest pair's letters and one, and that count, with one wait.
     int64_t slot_total = 0;
-    read_back(gpu, &slot_total, slot_offsets + pairs, sizeof(int64_t));
-    uint32_t longest = 0;  // the longest pair's letters, and one
-    read_back(gpu, &longest, keys_sorted, sizeof longest);
+    uint32_t longest = 0;
+    unsigned int refused_count = 0;
+    read_back(gpu, {{&slot_total, slot_offsets + pairs, sizeof slot_total},
+                    {&longest, keys_sorted, sizeof longest},
+                    {&refused_count, counters + 8, sizeof refused_count}});
     const bool short_columns = int64_t(longest) <= kShortLetters;
     const bool reversed = !right_ties;
     WaveFn fn = plan.edit ? pick_wave<true>(short_columns, reversed) : pick_wave<false>(short_columns, reversed);
     char *slots = trace ? gpu->walk_out.ensure<char>(size_t(slot_total) + 8) : nullptr;
     int64_t *lengths = gpu->cigar_lengths.ensure<int64_t>(size_t(pairs) + 1);
     DINARA_CUDA(cudaMemsetAsync(lengths, 0, (size_t(pairs) + 1) * sizeof(int64_t), stream));
-    // Pairs with a refused letter sort last (key zero) and are left out of the launches.
-    unsigned int *counters = gpu->counters.ensure<unsigned int>(64);
     uint32_t *retry = gpu->pending.ensure<uint32_t>(size_t(pairs));
     uint32_t *retry_next = gpu->pending_next.ensure<uint32_t>(size_t(pairs));
-    // The refused pairs' count, to leave them out.
-    DINARA_CUDA(cudaMemsetAsync(counters, 0, 64 * sizeof(unsigned int), stream));
-    size_t count_bytes = 0;
-    DINARA_CUDA(cub::DeviceReduce::Sum(nullptr, count_bytes, refused, counters + 8, int(pairs), stream));
-    space = gpu->sort_scratch.ensure<uint8_t>(std::max({scan_bytes, sort_bytes, count_bytes}) + 256);
-    DINARA_CUDA(cub::DeviceReduce::Sum(space, count_bytes, refused, counters + 8, int(pairs), stream));
-    unsigned int refused_count = 0;
-    read_back(gpu, &refused_count, counters + 8, sizeof(unsigned int));
     int64_t live = pairs - int64_t(refused_count);
     const uint32_t *launch_order = order;
     // Arenas: 256 KB a warp at first, for every resident warp; a pair that outgrows its arena runs again
