@@ -1032,6 +1032,18 @@ int32_t pair_limit_of(const AffineTable &table) {
 // against 10.33. 5,000 local alignments, their hits swept so, 9.8 against 10.7.
 constexpr int64_t kFinerPairs = 48;
 
+// Larger alphabets' scores take 16 bits from so many pairs on: a row through profiles takes longer than in 32 bits, and
+// one pair leaves half of every register idle. Local scores under 20 letters, 32 bits and 16: one pair of 400 to 500
+// letters 0.29 and 0.31 ms, four 0.30 and 0.34, eight 0.35 and 0.34; of 600 to 900 0.54 and 0.65, 0.70 and 0.84, 0.79 and
+// 0.78. Globally the two are even below it up to about 16 letters.
+constexpr int64_t kProfilePairs = 8;
+
+// Whether every pair of a batch falls in one shape class. Where they fall in several, the 16-bit classes' sweeps run at
+// once and the 32-bit ones' one after another, which outweighs a small batch's other costs.
+bool one_class(const AffineBatch &batch, bool record) {
+    return affine_shape_for(batch.min_columns, record) == affine_shape_for(batch.max_columns, record);
+}
+
 // Which whole-matrix pairs the 16-bit pair score sweep takes (a table of up to four letters on the 2-bit
 // tape, or a larger one through profiles): locally, a cell held less row x extend reaches at most the best
 // entry times the columns swept plus the rows times -extend and falls no lower than a gap's first letter, so
@@ -1354,13 +1366,29 @@ __global__ void extension_finish_kernel(const PairShape *__restrict__ shapes, in
         for (int j = 0; j < 4; ++j) spans[4 * k + j] = span[j];
 }
 
+// Larger alphabets' free ends in 16 bits (free_pairs_kernel through profiles): a row of it takes longer than in 32 bits
+// (two pairs' letters and profile rows to read, one after the other), which pays once pairs fill the GPU, and a profile's
+// shared memory leaves it fewer warps from some letters on. Infix scores a call, in 32 bits and in 16, 20 letters: 300
+// pairs of 260 to 320 0.39 and 0.43 ms, 1,000 0.44 and 0.48, 1,500 0.52 and 0.53, 1,776 0.70 and 0.55; 20,000 of 400 to 500 5.6 and 5.0, of
+// 600 to 900 12.8 and 13.6; 32 letters: of 260 to 320 4.2 and 4.4, of 600 to 900 13.1 and 16.6; 10 letters: 13.0 and
+// 11.3. Extensions keep 16 bits at every size (their other form is twice as long).
+constexpr int64_t kFreeProfilePairs = 10;      // an SM, at least
+constexpr int32_t kProfileLetters = 16;        // up to so many letters pairs of any columns,
+constexpr int32_t kFreeProfileCells = 10240;   // past them of so many columns x letters at most (256 columns from 27
+                                               // letters on, where a profile leaves three blocks an SM)
+
 // Which pairs the 16-bit free-end sweeps take (a table whose shifted entries fit a byte): a shifted cell reaches at
 // most the best entry times the columns swept plus the rows and columns swept times -extend, held to half of
 // 30,000 less the gaps for the sum of a group's two pairs, and falls at most a few gap openings below zero.
-PairLimits free_limits_of(const AffineBatch &batch, const AffineTable &table) {
+PairLimits free_limits_of(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, int64_t count) {
     PairLimits limits;
     const int32_t gaps = std::abs(table.open) + std::abs(table.extend);
     if ((batch.bits == 2 && !table.packed16) || gaps > 2000) return limits;
+    if (batch.bits == 8 && !batch.extension) {
+        if (count < kFreeProfilePairs * gpu->multiprocessors) return limits;
+        if (table.size > kProfileLetters)
+            limits.columns = table.size <= 26 ? kFreeProfileCells / table.size : 256;
+    }
     int32_t best = 1;
     for (int r = 0; r < table.size; ++r)
         for (int c = 0; c < table.size; ++c) {
@@ -1401,8 +1429,8 @@ PairsLaunch pick_extension(int cls, int bits, int letters) {
 }
 
 // One free-end sweep of a scheduled batch: the 16-bit classes' pairs, then the rest in 32 bits.
-void launch_free(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, const Schedule &order,
-                 KernelFn general, KernelArgs args, const TableArgs &targs, const int32_t *table32) {
+void launch_free(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &table, const PairLimits &limits,
+                 const Schedule &order, KernelFn general, KernelArgs args, const TableArgs &targs, const int32_t *table32) {
     const Buckets b = buckets_of(order);
     std::vector<ClassSweep> sweeps;
     for (int cls = kAffineShapes - 1; cls >= 0; --cls) {
@@ -1412,7 +1440,7 @@ void launch_free(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable &t
                                               : pick_free(cls, batch.bits, table.size),
                               cls, first, last});
     }
-    launch_together(gpu, batch, free_limits_of(batch, table), sweeps, args, targs, table32);
+    launch_together(gpu, batch, limits, sweeps, args, targs, table32);
     const int64_t begin = b.begin[kAffineShapes - 1], end = b.end[0];
     if (end <= begin) return;
     const int64_t blocks = std::max<int64_t>(
@@ -1484,7 +1512,7 @@ void free_end_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTabl
         reach_spans = gpu->reach_spans.ensure<int64_t>(4 * size_t(count));
         free_end_scores(gpu, reaching, table, reach_scores, first, count, reach_spans);
     }
-    const PairLimits limits = free_limits_of(batch, table);
+    const PairLimits limits = free_limits_of(gpu, batch, table, count);
     const Schedule order = dinara::schedule(gpu, batch.shapes, nullptr, first, count, false, false, limits);
     int32_t *table32 = nullptr;
     upload_table32(gpu, table, false, &table32);
@@ -1546,7 +1574,7 @@ void free_end_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTabl
         DINARA_CUDA(cudaGetLastError());
         gpu->launches += 1;
     } else {
-        launch_free(gpu, batch, table, order, fn, args, targs, table32);
+        launch_free(gpu, batch, table, limits, order, fn, args, targs, table32);
     }
     if (batch.extension) {
         extension_finish_kernel<<<unsigned((count * 32 + 255) / 256), 256, 0, gpu->stream>>>(
@@ -1573,7 +1601,7 @@ void free_end_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTabl
             back.free_reference_end = batch.free_reference_start;
             back.free_query_start = 0;
             back.free_query_end = batch.free_query_start;
-            launch_free(gpu, batch, table, order, fn, back, targs, table32);
+            launch_free(gpu, batch, table, limits, order, fn, back, targs, table32);
         }
         free_spans_kernel<<<pair_blocks, 256, 0, gpu->stream>>>(ends, origin_starts ? ends : ends + count, count, spans);
         DINARA_CUDA(cudaGetLastError());
@@ -1674,6 +1702,9 @@ void affine_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
     }
     const bool band = band_serves(batch, table);
     PairLimits limits = whole_limits_of(batch, table);
+    if (batch.bits == 8 && count < kProfilePairs && (batch.local || table.size > kProfileLetters) &&
+        one_class(batch, false))
+        limits.whole = 0;
     limits.band = band ? pair_limit_of(table) : 0;
     limits.fine = finer_strips(gpu, batch, count);
     const Schedule schedule_all = dinara::schedule(gpu, batch.shapes, nullptr, first, count, false, band, limits);

@@ -70,6 +70,8 @@ struct AffineBatch {
     // Per-pair flags (the packing's unknown-letter flags): a walk that finds its path leaving the proven
     // band sets its pair's to kWalkFailed, which the host reports as DINARA_DEVICE_FAILURE. May be null.
     uint8_t *flags = nullptr;
+    // The shortest query's letters (0 where it is not known).
+    uint32_t min_columns = 0;
     // Global scores with free ends (scored.mojo:69-240): letters at the reference's start and end and the
     // query's start and end that may go unaligned for nothing (at most INT32_MAX; a pair reads at most
     // its own length). `free_ends` is set when any is nonzero.

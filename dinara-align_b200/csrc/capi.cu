@@ -274,7 +274,7 @@ struct Packed {
     uint32_t *tape = nullptr;
     PairShape *shapes = nullptr;
     uint8_t *unknown = nullptr;
-    uint32_t max_rows = 0, max_columns = 0;
+    uint32_t max_rows = 0, max_columns = 0, min_columns = 0;
 };
 
 // Runs work(begin, end) over [0, count) on eight threads when the count is large, else on this one; each
@@ -306,22 +306,27 @@ void check_offsets(int64_t pairs, const int64_t *offsets) {
     if (pairs > 0 && offsets[0] < 0) throw Failure(DINARA_INVALID_LENGTH, "an offset below zero");
 }
 
-// The batch's longest reference and longest query.
-void shape_maxima(int64_t pairs, const int64_t *offsets, uint32_t *max_rows, uint32_t *max_columns) {
-    std::atomic<uint32_t> rows{0}, columns{0};
+// The batch's longest reference, and its longest and shortest query.
+void shape_maxima(int64_t pairs, const int64_t *offsets, Packed &out) {
+    std::atomic<uint32_t> rows{0}, columns{0}, least{UINT32_MAX};
     split_work(pairs, [&](int64_t begin, int64_t end) {
-        uint32_t r = 0, c = 0;
+        uint32_t r = 0, c = 0, l = UINT32_MAX;
         for (int64_t p = begin; p < end; ++p) {
+            const uint32_t query = uint32_t(offsets[2 * p + 2] - offsets[2 * p + 1]);
             r = std::max<uint32_t>(r, uint32_t(offsets[2 * p + 1] - offsets[2 * p]));
-            c = std::max<uint32_t>(c, uint32_t(offsets[2 * p + 2] - offsets[2 * p + 1]));
+            c = std::max(c, query);
+            l = std::min(l, query);
+        }
+        for (uint32_t seen = least.load(); seen > l && !least.compare_exchange_weak(seen, l);) {
         }
         for (uint32_t seen = rows.load(); seen < r && !rows.compare_exchange_weak(seen, r);) {
         }
         for (uint32_t seen = columns.load(); seen < c && !columns.compare_exchange_weak(seen, c);) {
         }
     });
-    *max_rows = rows.load();
-    *max_columns = columns.load();
+    out.max_rows = rows.load();
+    out.max_columns = columns.load();
+    out.min_columns = least.load();
 }
 
 Packed pack_batch(dinara_gpu *gpu, int64_t pairs, const char *letters, const int64_t *offsets, const uint8_t codes[256],
@@ -338,7 +343,7 @@ Packed pack_batch(dinara_gpu *gpu, int64_t pairs, const char *letters, const int
         for (int64_t k = 0; k <= 2 * pairs; ++k) relative[size_t(k)] = offsets[k] - first;
         device_offsets_host = relative.data();
     }
-    shape_maxima(pairs, offsets, &out.max_rows, &out.max_columns);
+    shape_maxima(pairs, offsets, out);
     uint8_t *letters_device = gpu->letters.ensure<uint8_t>(size_t(total) + 16);
     int64_t *offsets_device = gpu->offsets.ensure<int64_t>(size_t(2 * pairs + 1));
     uint8_t *codes_device = gpu->code_table.ensure<uint8_t>(256);
@@ -831,7 +836,7 @@ void start_batch(StreamedBatch &out, dinara_gpu *gpu, int64_t pairs, const char 
     DINARA_CUDA(cudaEventRecord(out.inputs_ready, gpu->stream));
     out.upload = std::make_unique<LetterUpload>(gpu, letters_device,
                                                 reinterpret_cast<const uint8_t *>(letters) + out.base, size_t(total));
-    shape_maxima(pairs, offsets, &out.packed.max_rows, &out.packed.max_columns);
+    shape_maxima(pairs, offsets, out.packed);
 }
 
 // The context's partner, set up at its first use and freed with the context.
@@ -1200,6 +1205,7 @@ void run_scores(dinara_gpu *gpu, int64_t pairs, const char *letters, const int64
     start_batch(streamed, gpu, pairs, letters, offsets, checked.codes, checked.bits);
     const Packed &packed = streamed.packed;
     AffineBatch batch{pairs, checked.bits, local, packed.tape, packed.shapes, packed.max_rows, packed.max_columns};
+    batch.min_columns = packed.min_columns;
     batch.free_ends = ends.free_ends;
     batch.free_reference_start = ends.free_reference_start;
     batch.free_reference_end = ends.free_reference_end;
@@ -1299,6 +1305,7 @@ int64_t dinara_gpu_alignments_tape(dinara_gpu *gpu, int64_t pairs, const char *l
         const Packed &packed = streamed.packed;
         AffineBatch batch{pairs, checked.bits, local, packed.tape, packed.shapes, packed.max_rows, packed.max_columns,
                           packed.unknown};
+        batch.min_columns = packed.min_columns;
         int32_t *scores_device = streamed.scores;
         // A placed batch's spans, as pairs of their own.
         AffineBatch inner = batch;
@@ -1637,6 +1644,7 @@ int64_t dinara_gpu_resident_align(dinara_gpu *gpu, const dinara_mode *mode, int6
         Timer timer(gpu);
         AffineBatch batch{r.pairs, r.checked.bits, local, r.packed.tape, r.packed.shapes, r.packed.max_rows,
                           r.packed.max_columns, r.packed.unknown};
+        batch.min_columns = r.packed.min_columns;
         batch.free_ends = ends.free_ends;
         batch.free_reference_start = ends.free_reference_start;
         batch.free_reference_end = ends.free_reference_end;

@@ -54,6 +54,7 @@ struct PairLimits {
     int32_t fine = 0;    // the score sweeps' own shapes past 320 columns too (pair_shape_for)
     int32_t record = 0;  // `whole` holds the recording sweep's pairs (else the score sweeps')
     int32_t hits = 0;    // recording: of hits' rows, so only pairs whose hits a score sweep has found
+    int32_t columns = 0; // above 0: only pairs of at most so many columns
     int32_t wide = 0;
     // Scoring without a CIGAR, globally: the 16-bit strips of a long pair serve the batch's table. Then pairs of
     // at least kLongSide x kLongSide that no 16-bit pair sweep takes go to kWideClass too.
@@ -71,6 +72,7 @@ struct PairLimits {
 __host__ __device__ inline bool takes_pairs16(const PairLimits &limits, uint32_t rows, uint32_t columns, int shape,
                                               bool record) {
     if (limits.whole <= 0 || record != (limits.record != 0) || rows == 0 || columns == 0) return false;
+    if (limits.columns > 0 && columns > uint32_t(limits.columns)) return false;
     // The score sweeps left a long pair (kWideClass) its whole shape and no hit.
     if (limits.hits && limits.wide && rows >= kWideRows && columns >= kWideColumns) return false;
     const uint32_t width = uint32_t(affine_lanes(shape) * affine_columns(shape));

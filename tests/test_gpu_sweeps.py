@@ -332,6 +332,29 @@ def test_placed_alignments_in_several_units(da, oracle):
         _assert_tiled(da, tape, scoring, mode, expected, 100)
 
 
+# 5 letters and 20; 26 and 27, either side of the fewer columns; pairs of each up to those columns, at and past them.
+@pytest.mark.parametrize("size", [5, 20, 26, 27])
+def test_free_ends_through_profiles(da, oracle, size):
+    """Larger alphabets' free ends in batches that fill the GPU, in 16 bits up to the columns that their profiles pay for,
+    the same pairs in a batch that does not, in 32 bits."""
+    alphabet = THIRTY_TWO[:size]
+    rng = np.random.default_rng(size)
+    scoring = _tabulated(da, rng, alphabet)
+    op, ex = oracle.kernel_gaps(scoring.opening, scoring.extension)
+    refs, queries = _placed_pairs(rng, alphabet)
+    for width in (255, 256, 257, 393, 394, 512, 513):
+        source = _text(rng, width, alphabet)
+        refs.append(_text(rng, 30, alphabet) + source + _text(rng, 20, alphabet))
+        queries.append(source)
+    coded = [(oracle.codes(r, alphabet), oracle.codes(q, alphabet)) for r, q in zip(refs, queries)]
+    tape = _tiled(da, refs, queries, 20)
+    for counts in ((BIG, BIG, 0, 0), (0, 0, BIG, BIG), (9, 20, 0, 4)):
+        mode = da.Mode.ends_free(*counts)
+        expected = [oracle.free_ends_alignment(a, b, _table(scoring), size, op, ex, *counts) for a, b in coded]
+        _assert_tiled(da, tape, scoring, mode, expected, 20)
+        _assert_tiled(da, _tiled(da, refs, queries, 1), scoring, mode, expected, 1)
+
+
 @pytest.mark.parametrize("mode_name", ["INFIX", "GLOBAL"])
 def test_alignments_without_spans(da, mode_name):
     """A caller that wants no spans gives none: the scores and CIGARs are those with them."""
@@ -428,13 +451,13 @@ def _check_alphabet(da, oracle, size):
         np.testing.assert_array_equal(da.scores_tape(tape, scoring, mode), expected)
         found = da.alignments(refs, queries, scoring, mode)
         assert [(a.score, a.cigar) for a in found] == list(zip(expected, cigars))
-    coded = [(oracle.codes(r, alphabet), oracle.codes(q, alphabet)) for r, q in zip(refs[:40], queries[:40])]
-    found = da.alignments(refs[:40], queries[:40], scoring, da.Mode.INFIX)
+    coded = [(oracle.codes(r, alphabet), oracle.codes(q, alphabet)) for r, q in zip(refs, queries)]
+    found = da.alignments(refs, queries, scoring, da.Mode.INFIX)
     assert [(a.score, a.cigar, _span(a)) for a in found] == [
         oracle.free_ends_alignment(a, b, _table(scoring), size, op, ex, BIG, BIG, 0, 0) for a, b in coded]
     found = da.alignments(refs[:40], queries[:40], scoring, da.Mode.extension(0, da.Anchor.START, zdrop=25))
     assert [(a.score, a.cigar, _span(a)) for a in found] == [
-        oracle.extension_alignment(a, b, _table(scoring), size, op, ex, False, -1, zdrop=25) for a, b in coded]
+        oracle.extension_alignment(a, b, _table(scoring), size, op, ex, False, -1, zdrop=25) for a, b in coded[:40]]
 
 
 def test_alphabets_in_rising_order():
