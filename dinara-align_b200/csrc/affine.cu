@@ -1762,11 +1762,29 @@ void affine_scores(dinara_gpu *gpu, const AffineBatch &batch, const AffineTable 
     tally_swept(gpu, batch.shapes, first, count, band, leftovers, left);
 }
 
+namespace {
+
+// Whether a small local batch's hits are worth their sweep, its schedule and its wait (some 40 us), by its largest sides:
+// each row cut off spares its recording, and each row recorded gains by two pairs a lane group, but not in
+// batches of two to seven DNA pairs, where a group of two waits longer than two groups. (Recorded whole in 32 bits and with
+// hits: one DNA pair of 100 letters in a target as long 0.38 and 0.41 ms, in one of 200 0.51 and 0.44; 32 pairs of
+// 40 in 40 0.31 and 0.35, of 150 in 150 0.60 and 0.58; four proteins of 40 in 50 0.36 and 0.38, of 100 in 100 even;
+// 700 proteins of 60 to 70 letters, in two classes, 0.61 and 0.46.) Units are a twentieth of a microsecond.
+bool hits_pay(dinara_gpu *gpu, const AffineBatch &batch, int64_t count) {
+    if (count >= 8 * int64_t(gpu->multiprocessors) || !one_class(batch, true)) return true;
+    const int64_t rows = batch.max_rows, cut = std::max<int64_t>(rows - int64_t(batch.max_columns), 0);
+    if (batch.bits == 8) return 17 * cut + 6 * rows >= (count >= 16 ? 450 : 600);
+    if (count == 1) return 17 * cut + 2 * rows >= 800;
+    return count >= 8 ? 17 * cut + 6 * rows >= 900 : 17 * cut - 3 * rows >= 400;
+}
+
+}  // namespace
+
 int64_t affine_alignments(dinara_gpu *gpu, const AffineBatch &whole_batch, const AffineTable &table, bool eqx,
                           int32_t *scores, int64_t *spans, int64_t first_pair, int64_t count) {
     // A local batch records each pair's hit's rows alone: its pairs, from here on, are those rows.
     AffineBatch batch = whole_batch;
-    if (batch.local) {
+    if (batch.local && hits_pay(gpu, batch, count)) {
         const PairShape *hits = hit_shapes(gpu, batch, table, scores, first_pair, count);
         if (hits) batch.shapes = hits;
     }
