@@ -695,9 +695,19 @@ int64_t cost_alignments(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, 
     int64_t live = pairs - int64_t(refused_count);
     const uint32_t *launch_order = order;
     // Arenas: 256 KB a warp at first, for every resident warp; a pair that outgrows its arena runs again
-    // with sixteen times the room on as many warps as the budget holds.
+    // with more room on as many warps as the budget holds. A few pairs have at once what the longest could need, up to
+    // 64 MB each and 1 GB in all: a first run that ends for want of room lasts longer with the pool's blocks. (One pair of
+    // 3,000 letters at 15% errors took 28 ms by arenas of 256 KB, 4 and 64 MB, 44 with blocks between, and 26 so.)
+    constexpr int64_t kFewPairs = 32, kMostRoom = int64_t(64) << 20;
     int64_t arena_bytes = int64_t(256) << 10;
     const int64_t budget = int64_t(2) << 30;
+    if (live > 0 && live <= kFewPairs) {
+        const double letters = double(longest), place = (short_columns ? 2.0 : 4.0) * (plan.edit ? 1.0 : 3.5);
+        const double costs = double(plan.od + plan.oi) + letters * double(std::max(plan.ed, plan.ei)) + 2.0;
+        const double need = costs * (1.1 * letters * place + 512.0);
+        const int64_t each = std::min(kMostRoom, (int64_t(1) << 30) / ((live + 3) / 4 * 4));
+        arena_bytes = std::max(arena_bytes, int64_t(std::min(need, double(each))) & ~int64_t(255));
+    }
     int per_sm = 0;
     DINARA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kWaveBlock, 0));
     const int64_t resident_warps = int64_t(gpu->multiprocessors) * std::max(per_sm, 1) * (kWaveBlock / 32);
@@ -709,7 +719,9 @@ int64_t cost_alignments(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, 
         const int64_t blocks = (warps + warps_per_block - 1) / warps_per_block;
         // The first launch's pool: room for every pair's blocks, up to 1 GB in all.
         const int64_t own_bytes = blocks * warps_per_block * arena_bytes;
-        const int64_t pool = rounds == 0 ? std::min<int64_t>(kMostBlocks, (kBlocksAPair * live + 31) / 32 * 32) : 0;
+        const int64_t pool = rounds == 0 && live > kFewPairs
+                                 ? std::min<int64_t>(kMostBlocks, (kBlocksAPair * live + 31) / 32 * 32)
+                                 : 0;
         uint8_t *arena = gpu->wavefront.ensure<uint8_t>(size_t(own_bytes + pool * kBlockBytes));
         DINARA_CUDA(cudaMemsetAsync(counters, 0, 64 * sizeof(unsigned int), stream));
         WaveArgs args;
@@ -749,7 +761,20 @@ int64_t cost_alignments(dinara_gpu *gpu, int64_t pairs, const uint8_t *letters, 
         read_back(gpu, &again, counters + 1, sizeof(unsigned int));
         live = again;
         if (live == 0) break;
-        arena_bytes *= 16;
+        // Sixteen times the room, 64 MB and then 1 GB; a few pairs have 64 MB at once. The pool's blocks added 4 MB to the
+        // first run, so pairs of about 1,000 letters each way, which seldom need 8, have up to that where the budget
+        // holds it for each (500 of them at 30% errors 39.1 and 21.4 ms); longer ones mostly need more, and a longer
+        // run that ends for want of it (64 of 3,000 at 15% 73 and 81).
+        constexpr int64_t kFirstRoom = int64_t(4) << 20;
+        constexpr uint32_t kMidLetters = 3000;
+        if (arena_bytes >= kMostRoom)
+            arena_bytes *= 16;
+        else if (live <= kFewPairs || arena_bytes >= kFirstRoom)
+            arena_bytes = kMostRoom;
+        else
+            arena_bytes = longest > kMidLetters
+                              ? kFirstRoom
+                              : std::max(kFirstRoom, std::min(2 * kFirstRoom, (budget / live) & ~int64_t(255)));
         ++rounds;
         if (arena_bytes > budget || rounds > 3) {
             // Fronts past the whole budget: those pairs are refused for device memory.

@@ -535,6 +535,19 @@ def test_fronts_in_shared_blocks(da, oracle):
     assert [(a.cost, a.cigar) for a in found] == [oracle.affine_cigar(r, q, 4, 6, 2) for r, q in zip(refs, queries)]
 
 
+@pytest.mark.parametrize("pairs", [1, 32, 40])
+def test_fronts_past_their_first_room(da, oracle, pairs):
+    """A few dear pairs, which have the room that the longest could need at once, and more than a few, which run again in
+    rooms of up to 8 MB and of 64 MB: unrelated pairs of 1,400 letters, some of 1,000 at 40% errors, a short one."""
+    rng = np.random.default_rng(pairs)
+    refs, queries = [], []
+    for k in range(pairs):
+        refs.append(_text(rng, 1400 if k % 4 == 0 else 1000 if k % 4 < 3 else 50))
+        queries.append(_text(rng, 1380) if k % 4 == 0 else _mutated(rng, refs[-1], 0.4, "ACGT"))
+    found = da.alignments(refs, queries, da.Costs.affine(4, 6, 2))
+    assert [(a.cost, a.cigar) for a in found] == [oracle.affine_cigar(r, q, 4, 6, 2) for r, q in zip(refs, queries)]
+
+
 # ---- unit-cost distances: the first round's list ---------------------------------------------------------------
 
 @pytest.mark.parametrize("pairs", [1, 2, 33, 400])
